@@ -21,7 +21,7 @@ LIB = os.path.join(LIBDIR, "libhcore_gb300.so")
 SOURCES = ["hc_kernels.cu", "hc_plan.cu", "hc_dropin.cu", "hc_dense.cu", "hc_noalloc.cu",
            "hc_mlp.cu", "hc_tlr.cu", "hc_compress.cu", "hc_probe.cu",
            "hc_panel.cu", "hc_zkernels.cu", "hc_rebuild_tc.cu", "hc_qr_tc.cu",
-           "hc_stack_tc.cu"]
+           "hc_stack_tc.cu", "hc_svd.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 
 
@@ -38,7 +38,7 @@ def _flags() -> list[str]:
 
 
 def _headers() -> list[str]:
-    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith(".h")]
+    hs = [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f.endswith((".h", ".cuh"))]
     hs += [os.path.join(ROOT, "include", f) for f in os.listdir(os.path.join(ROOT, "include"))]
     return hs
 

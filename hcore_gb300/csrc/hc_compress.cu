@@ -352,6 +352,7 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             LaunchShape shape;
             shape.maxM = pM;
             shape.maxK = maxK;
+            shape.updates = nd;
             fill_buckets(descs, shape);
             e = cudaMemcpyAsync(d_desc, descs.data(), nd * sizeof(Desc), cudaMemcpyHostToDevice, s);
             if (e == cudaSuccess)

@@ -93,8 +93,10 @@ struct LaunchShape {
     // min(k, storage_rank): the rebuild's grid (0: maxK)
     int maxR = 0;
     // tuning: lanes per column pair of shared-memory SVD buckets with <= 24,
-    // <= 64 and more pairs; rank-bucket edge spacing
-    int svd_lanes[3] = {2, 2, 2};
+    // <= 64 and more pairs (-1: by `updates`, the number of updates that
+    // share the GPU); rank-bucket edge spacing
+    int svd_lanes[3] = {-1, -1, -1};
+    int updates = 1;
     int bucket_width = 8;
     int qr_warps = 4;   // warps per QR CTA (2, 4 or 8)
     bool mixed = false;  // FP32 factor products and rebuild (HCORE_GPU_MIXED_FACTORS)
@@ -127,6 +129,15 @@ template <typename T>
 cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status,
                               int *d_info, const LaunchShape &shape, cudaStream_t s,
                               unsigned phases);
+// SVD of updates whose two Jacobi matrices fit shared memory (hc_svd.cu):
+// configure sets the kernel's shared-memory attribute (not capturable) and
+// returns the largest such k; launch runs n updates of k <= K with G lanes
+// per column pair
+template <typename T>
+cudaError_t configure_svd_smem(int optin, int *kmax);
+template <typename T>
+void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
+                     int G, cudaStream_t s);
 // rebuild phase only, for listed updates whose status is STORAGE (set to
 // OK; d_cap, if not null, caps their rank)
 template <typename T>

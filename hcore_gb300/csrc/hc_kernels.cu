@@ -29,6 +29,7 @@
 #include <mutex>
 
 #include "hc_internal.h"
+#include "hc_scalar.cuh"
 
 namespace hc {
 
@@ -42,40 +43,6 @@ template <>
 struct Lim<float> {
     static constexpr float eps = FLT_EPSILON;
 };
-
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-template <typename T>
-__device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
-// binary exponent (floor(log2|x|), subnormals included), per precision
-__device__ __forceinline__ int binary_exponent(double x) { return ilogb(x); }
-__device__ __forceinline__ int binary_exponent(float x) { return ilogbf(x); }
-// 2^n built from its bits, n within the normal exponent range
-template <typename T>
-__device__ __forceinline__ T exp2i(int n);
-template <>
-__device__ __forceinline__ double exp2i<double>(int n) {
-    return __longlong_as_double((long long)(n + 1023) << 52);
-}
-template <>
-__device__ __forceinline__ float exp2i<float>(int n) {
-    return __int_as_float((n + 127) << 23);
-}
-// x * 2^n for |n| up to twice the normal exponent range: two exact multiplies
-template <typename T>
-__device__ __forceinline__ T mul_exp2(T x, int n) {
-    return (x * exp2i<T>(n / 2)) * exp2i<T>(n - n / 2);
-}
 
 // -x by its sign bit (integer pipe; exact, NaN payloads kept)
 __device__ __forceinline__ double flip_sign(double x) {
@@ -388,67 +355,47 @@ struct JacobiLim<float> {
     static constexpr float tiny_scale = 1e-12f;
 };
 
-// Lanes per column pair in the Jacobi sweeps of a bucket whose largest k is
-// K.  A group of G lanes shares a pair's rows, which divides the per-round
-// latency of one update by about G but repeats the rotation parameters in
-// every lane of the group.  Shared-memory buckets take the plan's tuning
-// (lanes for buckets of up to 24, up to 64 and more pairs; default two
-// throughout, the autotuner's usual pick on a TLR panel).  Workspace buckets (k beyond the
-// shared-memory limit): four lanes per pair, up to 1024 threads, to keep
-// enough loads in flight on the L2-resident matrices.
+// Lanes per column pair of the workspace SVD (below): four, up to 1024
+// threads, to keep enough loads in flight on the L2-resident matrices.
 constexpr int kSvdMaxThreads = 1024;
-// A tuning value of 0 fills the warps: one lane per pair needs ceil(np/32)
-// warps, and the pairs take as many lanes each (a power of two) as still fit
-// in them.  On this GPU one FP64 warp instruction holds a sub-partition's
-// pipe for about 64 cycles whatever its active lanes, so lanes left idle in a
-// warp are free to share a pair's rows, while an extra warp would repeat the
-// rotation-parameter arithmetic.
-__host__ __device__ inline int svd_group(int K, bool smem, const int *lanes) {
+static int svd_group(int K) {
     const int np = (K + 1) / 2;
-    if (smem) {
-        int g = np <= 24 ? lanes[0] : (np <= 64 ? lanes[1] : lanes[2]);
-        if (g == 0) {
-            const int w = (np + 31) / 32;
-            g = 1;
-            while (g < 32 && 2 * g * np <= 32 * w) g *= 2;
-        }
-        return g;
-    }
     return np <= kSvdMaxThreads / 4 ? 4 : (np <= kSvdMaxThreads / 2 ? 2 : 1);
 }
-// Threads per CTA of the SVD kernel: G lanes for each of the K/2 pairs.
-__host__ __device__ inline int svd_threads(int K, bool smem, const int *lanes) {
-    const int np = (K + 1) / 2;
-    const int cap = smem ? kThreads : kSvdMaxThreads;
-    const int t = ((np * svd_group(K, smem, lanes) + 31) / 32) * 32;
-    return t < 32 ? 32 : (t > cap ? cap : t);
+static int svd_threads(int K) {
+    const int t = (((K + 1) / 2 * svd_group(K) + 31) / 32) * 32;
+    return t < 32 ? 32 : (t > kSvdMaxThreads ? kSvdMaxThreads : t);
 }
-__host__ __device__ inline int svd_ld(int k) { return k | 1; }
+// Lanes per column pair of the shared-memory SVD (hc_svd.cu), by the plan's
+// tuning for buckets of up to 24, up to 64 and more pairs.  A tuning value of
+// 0 takes as many lanes (a power of two) as fit in the warps that one lane
+// per pair needs.  Without a tuning (-1): eight lanes while every update has
+// an SM of its own and they fit in eight warps (two a sub-partition), else
+// four.  More lanes shorten a round's rows, but each warp repeats the
+// rotation parameters, which counts once the FP64 pipes are shared.  SVD
+// phase with 2, 4 and 8 lanes (us): 16 updates of k 8-24 410, 287, 250; one
+// of k = 64 2839, 1753, 1453; 24 of k 80-116 8262, 5794, 6099; 384 of k
+// 12-68 4120, 3220, 3205 (whole plan 10787, 9669, 10455); 1900 of the same
+// 6216, 5747, 6881.
+static int svd_smem_lanes(int K, const int *lanes, int updates) {
+    const int np = (K + 1) / 2;
+    int g = np <= 24 ? lanes[0] : (np <= 64 ? lanes[1] : lanes[2]);
+    if (g < 0) g = updates <= 152 && 8 * np <= 256 ? 8 : 4;
+    if (g == 0) {
+        const int w = (np + 31) / 32;
+        g = 1;
+        while (g < 32 && 2 * g * np <= 32 * w) g *= 2;
+    }
+    return g;
+}
 
-// Dynamic shared memory of the SVD kernel: `mats` K x ld matrices (2, 1 or 0:
+// Dynamic shared memory of the workspace SVD: `mats` K x ld matrices (1 or 0:
 // the launch mode), then the column scales, squared norms, singular values,
 // Householder scalars, and two index arrays.
 template <typename T>
-__host__ __device__ inline size_t svd_smem_bytes(int K, int mats) {
+static size_t svd_smem_bytes(int K, int mats) {
     return (size_t)mats * K * svd_ld(K) * sizeof(T) + (size_t)4 * (K + 1) * sizeof(T) +
            (size_t)2 * (K + 1) * sizeof(int) + 64;
-}
-
-// Squared deflation bound of the SVD kernel's QR (described there): delta^2
-// for an FP64 update ranked by accuracy, -1 (no deflation) otherwise.  f2 is
-// ||T||_F^2 of T scaled by 2^-sexp.  One thread computes it once per update
-// (a warp-wide sum there cost the Jacobi loops registers).
-template <typename T>
-__device__ __forceinline__ T deflation_bound2(T f2, int k, int rk, int rule, double acc, int sexp) {
-    if constexpr (sizeof(T) != sizeof(double)) {
-        return T(-1);
-    } else {
-        if (rk != 0 || !(acc > 0.0)) return T(-1);
-        const T fro = sqrt(f2);
-        const T thr = (rule & kRuleRelative) ? (T)acc * fro * rsqrt(T(k)) : mul_exp2((T)acc, -sexp);
-        const T dl = min(T(1e-13) * thr, T(1e-16) * fro);
-        return isfinite(dl) ? dl * dl : T(-1);
-    }
 }
 
 // SVD of T = R_A R_B^T (k x k) by QR-preconditioned one-sided Jacobi
@@ -499,24 +446,22 @@ __global__ void __launch_bounds__(kSvdMaxThreads) gesvd_kernel(const Desc *__res
     // the k x k working matrices: column-major in shared memory (odd ld: a
     // lane walking its own column is free of bank conflicts), row-major in
     // the workspace (the lanes of a warp own consecutive columns in the
-    // tournament and in every lane-per-column loop: coalesced).  MODE 1: both
-    // in shared memory; 2: B (R^T) in shared memory, A (V_J) in the
-    // workspace; 0: both in the workspace.
-    constexpr bool A_SM = MODE == 1, B_SM = MODE >= 1;
-    const int ldA = A_SM ? svd_ld(k) : k, ldB = B_SM ? svd_ld(k) : k;
+    // tournament and in every lane-per-column loop: coalesced).  MODE 2: B
+    // (R^T) in shared memory, A (V_J) in the workspace; 0: both in the
+    // workspace.  (Both in shared memory: svd_smem_kernel, hc_svd.cu.)
+    constexpr bool B_SM = MODE == 2;
+    const int ldA = k, ldB = B_SM ? svd_ld(k) : k;
     // distance of rows i and i + 1 in a column
-    const size_t rsA = A_SM ? 1 : (size_t)ldA, rsB = B_SM ? 1 : (size_t)ldB;
+    const size_t rsA = (size_t)ldA, rsB = B_SM ? 1 : (size_t)ldB;
     auto ixA = [ldA](int i, int j) -> size_t {
-        return A_SM ? (size_t)j * ldA + i : (size_t)i * ldA + j;
+        return (size_t)i * ldA + j;
     };
     auto ixB = [ldB](int i, int j) -> size_t {
         return B_SM ? (size_t)j * ldB + i : (size_t)i * ldB + j;
     };
-    T *A = A_SM ? reinterpret_cast<T *>(smem_raw) : base + L.W;   // T, then QR, then V_J
-    T *B = B_SM ? reinterpret_cast<T *>(smem_raw) + (A_SM ? (size_t)maxK * svd_ld(maxK) : 0)
-                : base + L.V;                                       // R^T, rotated
-    const int nsm = (A_SM ? 1 : 0) + (B_SM ? 1 : 0);
-    T *aux = reinterpret_cast<T *>(smem_raw + (size_t)nsm * maxK * svd_ld(maxK) * sizeof(T));
+    T *A = base + L.W;                                                   // T, then QR, then V_J
+    T *B = B_SM ? reinterpret_cast<T *>(smem_raw) : base + L.V;         // R^T, rotated
+    T *aux = reinterpret_cast<T *>(smem_raw) + (B_SM ? (size_t)maxK * svd_ld(maxK) : 0);
     T *s_d = aux, *s_nrm = aux + (maxK + 1), *s_sig = aux + 2 * (maxK + 1);
     T *s_tau = aux + 3 * (maxK + 1);
     int *s_perm = reinterpret_cast<int *>(aux + 4 * (maxK + 1));   // Jacobi sort
@@ -527,7 +472,7 @@ __global__ void __launch_bounds__(kSvdMaxThreads) gesvd_kernel(const Desc *__res
     T amax = 0;
     for (int o = 0; o < k; ++o)
         for (int t = tid; t < k; t += nthr) {   // the lanes walk the contiguous index
-            const int i = A_SM ? t : o, j = A_SM ? o : t;
+            const int i = o, j = t;
             T s = 0;
             for (int l = max(i, j); l < k; ++l) s += UA[(size_t)l * M + i] * VB[(size_t)l * M + j];
             A[ixA(i, j)] = s;
@@ -1179,14 +1124,15 @@ static cudaError_t configure_recompress_once(int dev, int *svd_smem_kmax, int *s
     int optin = 0;
     cudaError_t e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     if (e != cudaSuccess) return e;
-    // dynamic shared memory the SVD kernel may take next to its static arrays
+    int kmax = 0;
+    e = configure_svd_smem<T>(optin, &kmax);
+    if (e != cudaSuccess) return e;
+    *svd_smem_kmax = kmax;
+    // dynamic shared memory the workspace SVD may take next to its static arrays
     cudaFuncAttributes fa;
-    e = cudaFuncGetAttributes(&fa, gesvd_kernel<T, 1>);
+    e = cudaFuncGetAttributes(&fa, gesvd_kernel<T, 2>);
     if (e != cudaSuccess) return e;
     const int dyn_max = optin - (int)fa.sharedSizeBytes;
-    int kmax = 0;
-    while (kmax < kMaxK && svd_smem_bytes<T>(kmax + 1, 2) <= (size_t)dyn_max) ++kmax;
-    *svd_smem_kmax = kmax;
     int khalf = kmax;
     while (khalf < kMaxK && svd_smem_bytes<T>(khalf + 1, 1) <= (size_t)dyn_max) ++khalf;
     if (svd_half_kmax) *svd_half_kmax = khalf;
@@ -1198,12 +1144,8 @@ static cudaError_t configure_recompress_once(int dev, int *svd_smem_kmax, int *s
     if (e != cudaSuccess) return e;
     // the attribute is per kernel, not per plan: allow the largest size any
     // plan may launch with, so plans of different k coexist
-    e = cudaFuncSetAttribute(gesvd_kernel<T, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             dyn_max);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(gesvd_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 dyn_max);
-    return e;
+    return cudaFuncSetAttribute(gesvd_kernel<T, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                dyn_max);
 }
 
 int bucket_edge(int k, int width) {
@@ -1266,11 +1208,10 @@ cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int
             const int mode = K <= shape.svd_smem_kmax ? 1 : (K <= shape.svd_half_kmax ? 2 : 0);
             cudaStream_t sb = forked ? shape.side[b] : s;
             if (forked) cudaStreamWaitEvent(sb, shape.fork, 0);
-            const int G = svd_group(K, mode == 1, shape.svd_lanes);
-            const int nt = svd_threads(K, mode == 1, shape.svd_lanes);
+            const int G = svd_group(K), nt = svd_threads(K);
             if (mode == 1)
-                gesvd_kernel<T, 1><<<bk.count, nt, svd_smem_bytes<T>(K, 2), sb>>>(
-                    d_desc + bk.start, ws, d_rank, d_status, d_info, K, G);
+                launch_svd_smem<T>(d_desc + bk.start, bk.count, ws, d_rank, d_status, d_info, K,
+                                   svd_smem_lanes(K, shape.svd_lanes, shape.updates), sb);
             else if (mode == 2)
                 gesvd_kernel<T, 2><<<bk.count, nt, svd_smem_bytes<T>(K, 1), sb>>>(
                     d_desc + bk.start, ws, d_rank, d_status, d_info, K, G);

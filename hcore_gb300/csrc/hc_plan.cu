@@ -449,9 +449,9 @@ extern "C" int hcore_gpu_tuning_default(hcore_gpu_tuning *t) {
     t->stream_groups = 16;
     if (const char *env = getenv("HCORE_GPU_STREAMS")) t->stream_groups = atoi(env);
     t->stream_groups = std::max(1, std::min(t->stream_groups, 64));
-    t->svd_lanes[0] = 2;   // the autotuner's pick on a TLR panel of 1953 updates
-    t->svd_lanes[1] = 2;
-    t->svd_lanes[2] = 2;
+    t->svd_lanes[0] = 4;   // the fastest on a TLR panel's updates (svd_smem_lanes)
+    t->svd_lanes[1] = 4;
+    t->svd_lanes[2] = 4;
     t->bucket_width = 8;
     t->phase_sync = 0;
     t->qr_warps = 4;
@@ -514,7 +514,8 @@ extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, 
     int ngroups = std::max(1, std::min(tune.stream_groups, n > 0 ? n : 1));
     p->phase_sync = tune.phase_sync != 0;
     auto set_shape_tuning = [&](LaunchShape &sh) {
-        for (int q = 0; q < 3; ++q) sh.svd_lanes[q] = tune.svd_lanes[q];
+        for (int q = 0; q < 3 && tuning; ++q) sh.svd_lanes[q] = tune.svd_lanes[q];
+        sh.updates = n;
         sh.bucket_width = tune.bucket_width;
         sh.qr_warps = tune.qr_warps;
     };

@@ -1,0 +1,693 @@
+// hcore-gb300 — the core SVD of an update whose two k x k Jacobi matrices fit
+// one SM's shared memory (k <= 119 in FP64, 168 in FP32): T = R_A R_B^T, QR
+// with column pivoting, one-sided Jacobi, rank rule, U_r and V_r S_r
+// (reference step: src/compute/hcore_dgemm.c:296-503, __svd).
+//
+// The method is the one of the workspace kernel (gesvd_kernel in
+// hc_kernels.cu: Drmac-Veselic preconditioning, scaled rotations, deflation);
+// this kernel is written for latency, because a CTA's serial chain of Jacobi
+// rounds and QR steps is what the SVD phase waits for.  One FP64 warp
+// instruction holds a sub-partition's FP64 pipe for about 64 cycles and a
+// dependent one cannot start earlier, so what counts is the number of FP64
+// warp instructions in a round's chain, not the bytes or the lanes:
+//   * a rotation's tangent is computed in FP32 from the leading bits of the
+//     three FP64 inner products (integer instructions extract them).  The
+//     tangent only has to bring the pair's inner product down by 2^-20 or so
+//     (the sweeps converge quadratically, and the last sweep starts below
+//     sqrt(tol)); what has to hold in FP64 is c^2 + s^2 = 1 for the tangent
+//     used, and that is done in FP64;
+//   * square roots and reciprocals in FP64 take an FP32 seed and one
+//     third-order Householder iteration (A. S. Householder, "The Numerical
+//     Treatment of a Single Nonlinear Equation", 1970), 5 and 3 instructions;
+//   * the scales keep their reciprocals, so no rotation divides;
+//   * comparisons of non-negative values run on the integer pipe;
+//   * the pivoted QR moves no column (a permutation instead), every warp
+//     finds the pivot and builds the reflector itself, so a step has one
+//     barrier; G lanes share a column there and in U_r = Q V_J as in the
+//     Jacobi.
+// SVD phase, before (two and, alone, four lanes per pair) and now, one GB300,
+// us: one update of k = 64 2388 -> 1453; 16 of k 8-24 485 -> 250; 384 of k
+// 12-68 4524 -> 3220; 1900 of the same 7272 -> 5747; FP32, 256 of k 10-48
+// 1139 -> 1050.  What bounds it now is the FP64 pipe of the one SM: in a round
+// at k = 64 each of eight warps issues about 8 instructions of inner product,
+// 22 of rotation parameters and 32 of rows, two warps a sub-partition, at 64
+// cycles each (4.0 us of the 4.3 us measured).
+#include <cfloat>
+#include <climits>
+
+#include "hc_internal.h"
+#include "hc_scalar.cuh"
+
+namespace hc {
+namespace {
+
+// ---- numbers from their bits -------------------------------------------------
+// x = m 2^(e - 1023), m in [1, 2) as FP32 (truncated); e = 0 for zero and
+// subnormals (their m is meaningless and not used)
+__device__ __forceinline__ void split(double x, float &m, int &e) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    e = (int)((hi >> 20) & 0x7FFu);
+    m = __uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+}
+// q 2^d as FP64 for a positive normal FP32 q; 0 when the result is not normal
+__device__ __forceinline__ double widen(float q, int d) {
+    const unsigned b = __float_as_uint(q);
+    const int e = (int)(b >> 23) + (1023 - 127) + d;
+    if (e <= 0) return 0.0;
+    return __hiloint2double((int)(((unsigned)e << 20) | ((b & 0x7FFFFFu) >> 3)), (int)(b << 29));
+}
+__device__ __forceinline__ float fsqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float frsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1 / sqrt(x), x normal and positive: y (1 + e/2 + 3 e^2/8), e = 1 - x y^2
+__device__ __forceinline__ double inv_sqrt(double x) {
+    float m;
+    int e;
+    split(x, m, e);
+    const int ex = e - 1023, odd = ex & 1, half = (ex - odd) >> 1;
+    const double y = widen(frsqrt_fast(odd ? 2.f * m : m), -half);
+    const double r = fma(-x * y, y, 1.0);
+    return fma(y * r, fma(0.375, r, 0.5), y);
+}
+__device__ __forceinline__ float inv_sqrt(float x) { return 1.f / sqrtf(x); }
+// 1 / x, x normal and positive: y (1 + e + e^2), e = 1 - x y
+__device__ __forceinline__ double inv(double x) {
+    float m;
+    int e;
+    split(x, m, e);
+    const double y = widen(__fdividef(1.f, m), 1023 - e);
+    const double r = fma(-x, y, 1.0);
+    return fma(y, fma(r, r, r), y);
+}
+__device__ __forceinline__ float inv(float x) { return 1.f / x; }
+
+// integer keys that order non-negative values (a negative value's key is
+// negative), and the key of x / 2^n for a value far above the smallest normal
+__device__ __forceinline__ long long key(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ int key(float x) { return __float_as_int(x); }
+__device__ __forceinline__ bool below_pow2(double x, double y, int n) {  // x < y 2^-n, y >= 0
+    return __double2hiint(x) < __double2hiint(y) - (n << 20);
+}
+__device__ __forceinline__ bool below_pow2(float x, float y, int n) {
+    return __float_as_int(x) < __float_as_int(y) - (n << 23);
+}
+
+template <typename T>
+struct SvLim;
+template <>
+struct SvLim<double> {
+    static constexpr double safmin = DBL_MIN / DBL_EPSILON;
+    static constexpr double tiny_scale = 1e-60;   // fold a column scale below this
+};
+template <>
+struct SvLim<float> {
+    static constexpr float safmin = FLT_MIN / FLT_EPSILON;
+    static constexpr float tiny_scale = 1e-12f;
+};
+
+// Is the pair to be rotated, a_pq^2 > tol^2 a_pp a_qq (rot), and was it above
+// the stopping level, a_pq^2 > tol a_pp a_qq (big)?
+__device__ __forceinline__ bool pair_test(double app, double aqq, double apq, float tol, bool &big) {
+    float mp, mq, ma;
+    int ep, eq, ea;
+    split(app, mp, ep);
+    split(aqq, mq, eq);
+    split(apq, ma, ea);
+    // at most about 2^2 (Cauchy-Schwarz); below 2^-110 < tol^2 no rotation
+    const int ex = 2 * ea - ep - eq;
+    if (ea == 0 || ex < -110) return false;
+    const float x = ma * ma * __int_as_float((min(ex, 60) + 127) << 23), y = mp * mq;
+    big = x > tol * y;
+    return x > tol * tol * y;
+}
+__device__ __forceinline__ bool pair_test(float app, float aqq, float apq, float tol, bool &big) {
+    const float x = apq * apq, y = app * aqq;
+    big = x > tol * y;
+    return apq != 0.f && x > tol * tol * y;
+}
+
+// t = v / (|w| + sqrt(w^2 + v^2)) with the sign of w v (w = 0: of v), the
+// tangent of the rotation that makes the pair orthogonal, w = a_qq - a_pp,
+// v = 2 a_pq
+__device__ __forceinline__ double tangent(double app, double aqq, double apq) {
+    const double w = aqq - app;
+    float mw, mv;
+    int ew, ev;
+    split(w, mw, ew);
+    split(apq, mv, ev);
+    ev += 1;
+    if (ew == 0) {   // equal norms: 45 degrees
+        mw = 0.f;
+        ew = ev;
+    }
+    const int em = max(ew, ev), dv = ev - em;
+    const float fw = mw * __int_as_float((max(ew - em, -60) + 127) << 23);
+    const float fv = mv * __int_as_float((max(dv, -60) + 127) << 23);
+    const float q = __fdividef(mv, fw + fsqrt_fast(fmaf(fw, fw, fv * fv)));
+    const double t = widen(q, dv);
+    const int sgn = ((ew == ev && mw == 0.f ? 0 : __double2hiint(w)) ^ __double2hiint(apq)) & (int)0x80000000;
+    return __hiloint2double(__double2hiint(t) | sgn, __double2loint(t));
+}
+__device__ __forceinline__ float tangent(float app, float aqq, float apq) {
+    const float w = aqq - app, v = 2.f * apq;
+    const float h = sqrtf(fmaf(w, w, v * v));
+    const float t = fabsf(v) / (fabsf(w) + h);
+    return (w < 0.f) != (v < 0.f) ? -t : t;
+}
+
+// Sum of f(i) over start <= i < k by a group of G lanes (rows i = lig mod G
+// each): eight partial sums by i mod 8, added in one fixed tree, so the result
+// does not depend on G.
+template <int G, typename T, typename F>
+__device__ __forceinline__ T group_sum(bool act, int start, int k, int lig, F f) {
+    constexpr int NA = 8 / G;
+    T a[NA];
+#pragma unroll
+    for (int m = 0; m < NA; ++m) a[m] = 0;
+    if (act) {
+        int i = (start & ~7) + lig;
+#pragma unroll
+        for (int m = 0; m < NA; ++m)   // the first eight rows may begin before start
+            if (i + G * m >= start && i + G * m < k) a[m] += f(i + G * m);
+        for (i += 8; i + G * (NA - 1) < k; i += 8)
+#pragma unroll
+            for (int m = 0; m < NA; ++m) a[m] += f(i + G * m);
+#pragma unroll
+        for (int m = 0; m + 1 < NA; ++m)
+            if (i + G * m < k) a[m] += f(i + G * m);
+    }
+#pragma unroll
+    for (int h = NA / 2; h > 0; h /= 2)
+#pragma unroll
+        for (int m = 0; m < h; ++m) a[m] += a[m + h];
+    T v = a[0];
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+
+constexpr int kSvThreads = 512;
+constexpr int kSvRows = 6;   // 32-row pieces of the largest k (168)
+
+template <typename T, int G>
+__global__ void __launch_bounds__(kSvThreads, 1)
+    svd_smem_kernel(const Desc *__restrict__ descs, T *__restrict__ ws, int *__restrict__ rank,
+                    int *__restrict__ status, int *__restrict__ info, int maxK) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ T s_wmax[kSvThreads / 32];
+    __shared__ int s_rank;
+    const Desc d = descs[blockIdx.x];
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
+    const int nw = nthr >> 5;
+    if (d.status0) {
+        if (tid == 0) {
+            status[d.idx] = d.status0;
+            rank[d.idx] = 0;
+            if (info) info[d.idx] = 0;
+        }
+        return;
+    }
+    const int M = d.M, k = d.k;
+    const WsLayout L = ws_layout(d);
+    T *base = ws + d.ws;
+    const T *UA = base + L.UA, *VB = base + L.VB;
+    // column-major with an odd leading dimension: lanes that walk a column
+    // are free of bank conflicts
+    const int ld = svd_ld(k);
+    const size_t mat = (size_t)maxK * svd_ld(maxK);
+    T *A = reinterpret_cast<T *>(smem_raw);   // R_A, T, its QR, then V_J
+    T *B = A + mat;                           // R_B, then R^T, rotated; at the end Q's reflectors
+    T *X0 = B + mat, *X1 = X0 + (maxK + 1), *s_d = X1 + (maxK + 1);
+    T *s_rd = s_d + (maxK + 1);               // R's diagonal, then 1 / s_d
+    T *s_tau = s_rd + (maxK + 1);             // 1 / g of reflector j, H = I - v v^T / g
+    short *s_perm = reinterpret_cast<short *>(s_tau + (maxK + 1));
+    short *s_pcol = s_perm + (maxK + 1);
+    T *Yg = base + L.Uo;   // reflectors of Q (k x k, ld k) in the Uo slot until U_r is written
+    const int grp = tid / G, lig = tid & (G - 1), ngrp = nthr / G;
+
+    // ---- T = triu(R_A) triu(R_B)^T (hcore_dgemm.c:330-387): a warp per row,
+    // the row of T replaces the row of R_A that only it reads --------------------
+    for (int l = warp; l < k; l += nw)
+        for (int i = lane; i < k; i += 32) {
+            A[(size_t)l * ld + i] = i <= l ? UA[(size_t)l * M + i] : T(0);
+            B[(size_t)l * ld + i] = i <= l ? VB[(size_t)l * M + i] : T(0);
+        }
+    __syncthreads();
+    T amax = 0;
+    bool bad = false;
+    for (int i = warp; i < k; i += nw) {
+        T acc[kSvRows];
+#pragma unroll
+        for (int c = 0; c < kSvRows; ++c) {
+            acc[c] = 0;
+            if (32 * c < k) {
+                const T *b = B + min(lane + 32 * c, k - 1);
+                T s0 = 0, s1 = 0;
+                int l = max(i, 32 * c);
+                for (; l + 1 < k; l += 2) {
+                    s0 += A[(size_t)l * ld + i] * b[(size_t)l * ld];
+                    s1 += A[(size_t)(l + 1) * ld + i] * b[(size_t)(l + 1) * ld];
+                }
+                if (l < k) s0 += A[(size_t)l * ld + i] * b[(size_t)l * ld];
+                acc[c] = s0 + s1;
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < kSvRows; ++c) {
+            const int j = lane + 32 * c;
+            if (j < k) {
+                A[(size_t)j * ld + i] = acc[c];
+                amax = max(amax, abs(acc[c]));
+                bad = bad || !isfinite(acc[c]);
+            }
+        }
+    }
+    amax = warp_max(amax);
+    if (lane == 0) s_wmax[warp] = amax;
+    if (__syncthreads_or(bad)) {
+        // a NaN or infinity: no decomposition; the update is not written
+        for (int t = tid; t < k; t += nthr) base[L.sig + t] = T(NAN);
+        if (tid == 0) {
+            int r = d.rk != 0 && d.rk < k ? d.rk : k;
+            if ((d.rule & kRuleCapRank) && r > d.max_rank) r = d.max_rank;
+            rank[d.idx] = r;
+            status[d.idx] = HCORE_GPU_S_NOCONV;
+            if (info) info[d.idx] = 0;
+        }
+        return;
+    }
+    // scale T by 2^-sexp, sexp the exponent of its largest entry
+    amax = 0;
+    for (int w = 0; w < nw; ++w) amax = max(amax, s_wmax[w]);
+    const int sexp = amax > T(0) ? binary_exponent(amax) : 0;
+
+    // squared column norms (G lanes per column), scaled columns
+    for (int c0 = 0; c0 < k; c0 += ngrp) {
+        const int c = c0 + grp;
+        T *ac = A + (size_t)c * ld;
+        const T s = group_sum<G, T>(c < k, 0, k, lig, [&](int i) {
+            const T x = sexp != 0 ? mul_exp2(ac[i], -sexp) : ac[i];
+            ac[i] = x;
+            return x * x;
+        });
+        if (c < k && lig == 0) {
+            X0[c] = s;    // norms of rows j.. of column c, squared; -1: pivoted already
+            s_d[c] = s;   // the same at the last exact computation
+        }
+    }
+    __syncthreads();
+    // squared deflation bound (see gesvd_kernel), the same in every thread
+    T f2 = 0;
+    for (int c = lane; c < k; c += 32) f2 += X0[c];
+    const T defl2 = deflation_bound2(warp_sum(f2), k, d.rk, d.rule, d.acc, sexp);
+    const int kfloor = d.rank_start < k ? (d.rank_start > 0 ? d.rank_start : 0) : k;
+
+    // ---- QR with column pivoting, T P = Q R ------------------------------------
+    int kk = k;
+    for (int j = 0; j < k; ++j) {
+        const T *nr = (j & 1) ? X1 : X0;
+        T *nr2 = (j & 1) ? X0 : X1;
+        // pivot: the largest remaining norm, the lowest column on a tie
+        auto best = key(T(-1));
+        int pv = 0;
+        for (int c = lane; c < k; c += 32) {
+            const auto x = key(nr[c]);
+            if (x > best) {
+                best = x;
+                pv = c;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const auto ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, pv, o);
+            if (ob > best || (ob == best && oi < pv)) {
+                best = ob;
+                pv = oi;
+            }
+        }
+        if (j >= kfloor && defl2 >= T(0) && best <= key(defl2)) {
+            T tail = 0;
+            for (int c = lane; c < k; c += 32) tail += max(nr[c], T(0));
+            if (warp_sum(tail) <= defl2) {
+                kk = j;
+                break;
+            }
+        }
+        // the reflector of column pv, rows j.., unscaled: v = (alpha - beta, x),
+        // beta = -sign(alpha) ||(alpha, x)|| (dlarfg's), g = beta (beta - alpha)
+        const T *ap = A + (size_t)pv * ld;
+        const T alpha = ap[j];
+        T ss = 0;
+        for (int i = j + 1 + lane; i < k; i += 32) ss += ap[i] * ap[i];
+        ss = warp_sum(ss);
+        T beta = alpha, vj = 0, ginv = 0;
+        if (ss > SvLim<T>::safmin) {
+            const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
+            T nb = n2 * rs;
+            nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
+            beta = -copysign(nb, alpha);
+            vj = alpha - beta;
+            ginv = inv(fma(-alpha, beta, n2));
+        }
+        if (tid == 0) {
+            s_pcol[j] = (short)pv;
+            s_rd[j] = beta;
+            s_tau[j] = ginv;
+        }
+        // apply it to the other remaining columns and downdate their norms
+        // (dlaqp2's rule), G lanes per column
+        const int i0 = j + 1 + ((lig - (j + 1)) & (G - 1));
+        for (int c0 = 0; c0 < k; c0 += ngrp) {
+            const int c = c0 + grp;
+            const T nc = c < k ? nr[c] : T(-1);
+            const bool act = c < k && c != pv && key(nc) >= 0;
+            T *ac = A + (size_t)c * ld;
+            const bool upd = act && ginv != T(0);
+            const T acj = upd && lig == 0 ? ac[j] : T(0);
+            // (row j's term, in lane 0's hands, is added to the sum of the rows below)
+            T s = group_sum<G, T>(upd, j + 1, k, lig, [&](int i) { return ap[i] * ac[i]; });
+            s = ginv * fma(vj, __shfl_sync(0xffffffffu, acj, lane & ~(G - 1)), s);
+            T nn = 0;
+            bool redo = false;
+            if (act) {
+                if (upd)
+                    for (int i = i0; i < k; i += G) ac[i] -= s * ap[i];
+                if (lig == 0) {
+                    const T r = upd ? acj - s * vj : ac[j];
+                    ac[j] = r;
+                    nn = nc - r * r;
+                    redo = !(key(nn) > 0) || below_pow2(nn, s_d[c], 10);
+                }
+            }
+            if (__any_sync(0xffffffffu, redo)) {
+                redo = __shfl_sync(0xffffffffu, (int)redo, lane & ~(G - 1)) != 0;
+                const T q = group_sum<G, T>(redo, j + 1, k, lig, [&](int i) { return ac[i] * ac[i]; });
+                if (redo && lig == 0) {
+                    nn = q;
+                    s_d[c] = q;
+                }
+            }
+            if (c < k && lig == 0) nr2[c] = act ? nn : T(-1);
+        }
+        __syncthreads();
+    }
+    {
+        // columns that the deflation left: positions kk.. in column order
+        const T *nr = (kk & 1) ? X1 : X0;
+        if (kk < k)
+            for (int c = tid; c < k; c += nthr)
+                if (key(nr[c]) >= 0) {
+                    int pos = kk;
+                    for (int q = 0; q < c; ++q) pos += key(nr[q]) >= 0;
+                    s_pcol[pos] = (short)c;
+                }
+    }
+    __syncthreads();
+    // Q's reflectors to the workspace, B = R^T (its columns kk.. are zero)
+    for (int h = warp; h < k; h += nw) {
+        const T *ah = A + (size_t)s_pcol[h] * ld;
+        for (int i = lane; i < k; i += 32) {
+            const T x = ah[i];
+            if (h < kk) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rd[h] : T(0));
+            // R(i, h)
+            B[(size_t)i * ld + h] = i < kk ? (i < h ? x : (i == h ? s_rd[h] : T(0))) : T(0);
+        }
+    }
+    __syncthreads();
+    for (int c = warp; c < k; c += nw)
+        for (int i = lane; i < k; i += 32) A[(size_t)c * ld + i] = i == c ? T(1) : T(0);
+    T *s_nrm = X0, *s_sig = X1;
+    auto column_norms = [&](bool fold) {
+        for (int c0 = 0; c0 < k; c0 += ngrp) {
+            const int c = c0 + grp;
+            T dj = 1;
+            T *xj = B + (size_t)c * ld;
+            if (c < kk) {
+                if (fold) {
+                    dj = s_d[c];
+                    if (dj < SvLim<T>::tiny_scale) {   // fold a scale before it underflows
+                        T *vj = A + (size_t)c * ld;
+                        for (int i = lig; i < k; i += G) {
+                            xj[i] *= dj;
+                            vj[i] *= dj;
+                        }
+                        dj = 1;
+                    }
+                }
+            }
+            const T s = group_sum<G, T>(c < kk, 0, k, lig, [&](int i) { return xj[i] * xj[i]; });
+            if (c < k && lig == 0) {
+                s_nrm[c] = c < kk ? dj * dj * s : T(0);
+                s_d[c] = dj;
+                s_rd[c] = fold && c < kk ? inv(dj) : T(1);
+            }
+        }
+    };
+    column_norms(false);
+    __syncthreads();
+
+    // ---- one-sided Jacobi on B = R^T, rotations accumulated in A ----------------
+    // (stopping rule and scaled rotations as in gesvd_kernel; columns kk.. of B
+    // are zero and take no part, V_J's rows kk.. stay zero)
+    const int n = kk + (kk & 1), np = n / 2;
+    const float tol = (float)(k > 8 ? k : 8) * (sizeof(T) == 8 ? (float)DBL_EPSILON : FLT_EPSILON);
+    bool converged = kk <= 1;
+    int sweeps = 0;
+    for (; sweeps < kMaxSweeps && !converged; ++sweeps) {
+        bool big = false;   // this thread rotated a pair above sqrt(tol)
+        for (int round = 0; round < n - 1; ++round) {
+            for (int b0 = 0; b0 < np; b0 += ngrp) {
+                // circle-method tournament: pair 0 is (n - 1, round), pair i
+                // (round + i, round - i) mod n - 1
+                const int pi = b0 + grp;
+                int p = round + pi, q = round - pi;
+                if (p >= n - 1) p -= n - 1;
+                if (q < 0) q += n - 1;
+                if (pi == 0) p = n - 1;
+                const bool valid = pi < np && p < kk && q < kk;
+                T *xp = B + (size_t)p * ld, *xq = B + (size_t)q * ld;
+                T app = 0, aqq = 0, dp = 1, dq = 1;
+                if (valid) {
+                    app = s_nrm[p];
+                    aqq = s_nrm[q];
+                    dp = s_d[p];
+                    dq = s_d[q];
+                }
+                const T dot = group_sum<G, T>(valid, 0, k, lig, [&](int i) { return xp[i] * xq[i]; });
+                bool rot = false, redo_p = false, redo_q = false;
+                T np_ = 0, nq_ = 0, dp2 = 1, dq2 = 1, rdp2 = 1, rdq2 = 1;
+                if (valid) {
+                    const T apq = (dp * dq) * dot;
+                    bool bigp = false;
+                    rot = key(app) > key(SvLim<T>::safmin) && key(aqq) > key(SvLim<T>::safmin) &&
+                          pair_test(app, aqq, apq, tol, bigp);
+                    if (rot) {
+                        big |= bigp;
+                        // true columns p' = c (p - t q), q' = c (q + t p), in B and
+                        // V_J; with column scales d: f1 = t dq / dp, f2 = t dp / dq
+                        const T t = tangent(app, aqq, apq);
+                        // (FP32 divides: it is cheap there, and the tracked
+                        // reciprocals' drift of one rounding a rotation is not)
+                        const T rdp = sizeof(T) == 8 ? s_rd[p] : T(1) / dp;
+                        const T rdq = sizeof(T) == 8 ? s_rd[q] : T(1) / dq;
+                        const T u = fma(t, t, T(1)), cs = inv_sqrt(u);
+                        const T f1 = t * (dq * rdp), f2 = t * (dp * rdq);
+                        np_ = app - t * apq;
+                        nq_ = aqq + t * apq;
+                        dp2 = dp * cs;
+                        dq2 = dq * cs;
+                        redo_p = below_pow2(np_, app, 6);
+                        redo_q = below_pow2(nq_, aqq, 6);
+                        T *vp = A + (size_t)p * ld, *vq = A + (size_t)q * ld;
+                        int i = lig;
+                        for (; i < kk; i += G) {
+                            const T a = xp[i], b = xq[i], c = vp[i], e = vq[i];
+                            xp[i] = a - f1 * b;
+                            xq[i] = b + f2 * a;
+                            vp[i] = c - f1 * e;
+                            vq[i] = e + f2 * c;
+                        }
+                        for (; i < k; i += G) {
+                            const T a = xp[i], b = xq[i];
+                            xp[i] = a - f1 * b;
+                            xq[i] = b + f2 * a;
+                        }
+                        const T ics = u * cs;   // 1 / c
+                        rdp2 = rdp * ics;
+                        rdq2 = rdq * ics;
+                    }
+                }
+                // strong cancellation in a tracked norm: recompute
+                if (__any_sync(0xffffffffu, redo_p || redo_q)) {
+                    const T sp = group_sum<G, T>(redo_p, 0, k, lig, [&](int i) { return xp[i] * xp[i]; });
+                    const T sq = group_sum<G, T>(redo_q, 0, k, lig, [&](int i) { return xq[i] * xq[i]; });
+                    if (redo_p) np_ = dp2 * dp2 * sp;
+                    if (redo_q) nq_ = dq2 * dq2 * sq;
+                }
+                if (rot && lig == 0) {
+                    s_nrm[p] = np_;
+                    s_nrm[q] = nq_;
+                    s_d[p] = dp2;
+                    s_d[q] = dq2;
+                    s_rd[p] = rdp2;
+                    s_rd[q] = rdq2;
+                }
+            }
+            __syncthreads();
+        }
+        column_norms(true);   // exact norms once per sweep
+        converged = !__syncthreads_or(big);
+    }
+
+    // singular values = true column norms of B (of the scaled T), descending,
+    // ties by index, NaN last: a total order whatever the values
+    bool nonfinite = false;
+    for (int j = tid; j < k; j += nthr) {
+        const T s = sqrt(s_nrm[j]);
+        nonfinite = nonfinite || !isfinite(s);
+        s_sig[j] = s == s ? s : T(-1);
+    }
+    if (tid == 0) s_rank = k;
+    const bool finite = !__syncthreads_or(nonfinite);
+    for (int j = tid; j < k; j += nthr) {
+        const auto sj = key(s_sig[j]);
+        int pos = 0;
+        for (int i = 0; i < k; ++i) {
+            const auto si = key(s_sig[i]);
+            pos += (si > sj) || (si == sj && i < j);
+        }
+        s_perm[pos] = (short)j;
+    }
+    __syncthreads();
+    // rank rule (hcore_dgemm.c:444-464; the fast rules start at i = 2; the
+    // compressor's starts at 0, may compare with acc * sigma_max and caps the
+    // rank at max_rank)
+    const T thr = (d.rule & kRuleRelative) ? (T)d.acc * mul_exp2(s_sig[s_perm[0]], sexp) : (T)d.acc;
+    for (int t = tid; t < k; t += nthr) {
+        const T s = s_sig[s_perm[t]];
+        const T v = key(s) < 0 ? T(NAN) : mul_exp2(s, sexp);
+        base[L.sig + t] = v;
+        if (d.rk == 0 && t >= d.rank_start && v < thr) atomicMin(&s_rank, t);
+    }
+    __syncthreads();
+    int r = d.rk != 0 ? (d.rk < k ? d.rk : k) : s_rank;
+    if ((d.rule & kRuleCapRank) && r > d.max_rank) r = d.max_rank;
+    int st = HCORE_GPU_S_OK;
+    if (!converged || !finite) st = HCORE_GPU_S_NOCONV;
+    else if (r > d.max_rank) st = HCORE_GPU_S_RANK_MAX;
+    else if (r > d.storage_rank) st = HCORE_GPU_S_STORAGE;
+
+    // U_r and V_r S_r of an accepted update, and of one whose rank only
+    // exceeds its storage limit (rebuilt later into larger storage)
+    if (st == HCORE_GPU_S_OK || st == HCORE_GPU_S_STORAGE) {
+        // V_r S_r = P (B's true columns): row P(i) of the output is row i of B
+        // (the rows S V^T of hcore_dgemm.c:484-489, transposed)
+        T *Uo = base + L.Uo, *Vo = base + L.Vo;
+        for (int t = warp; t < r; t += nw) {
+            const int j = s_perm[t];
+            const T f = s_d[j];
+            for (int i = lane; i < k; i += 32)
+                Vo[(size_t)t * k + s_pcol[i]] = mul_exp2(f * B[(size_t)j * ld + i], sexp);
+        }
+        __syncthreads();
+        // U_r = Q (V_J's true columns), Q = H_0 ... H_{kk-1}: the reflectors
+        // come into B's place, each group applies them, last to first, to its
+        // columns of V_J
+        for (int h = warp; h < kk; h += nw)
+            for (int i = lane; i < k; i += 32) B[(size_t)h * ld + i] = Yg[(size_t)h * k + i];
+        __syncthreads();
+        for (int t0 = 0; t0 < r; t0 += ngrp) {
+            const int t = t0 + grp;
+            const bool act = t < r;
+            const int j = act ? s_perm[t] : 0;
+            T *x = A + (size_t)j * ld;   // each group owns the column of its own j
+            if (act) {
+                const T dj = s_d[j];
+                for (int i = lig; i < k; i += G) x[i] *= dj;
+            }
+            for (int h = kk - 1; h >= 0; --h) {
+                const T gi = s_tau[h];
+                if (gi == T(0)) continue;
+                const T *y = B + (size_t)h * ld;
+                const int i0 = h + ((lig - h) & (G - 1));
+                const T s = gi * group_sum<G, T>(act, h, k, lig, [&](int i) { return y[i] * x[i]; });
+                if (act)
+                    for (int i = i0; i < k; i += G) x[i] -= s * y[i];
+            }
+            if (act)
+                for (int i = lig; i < k; i += G) Uo[(size_t)t * k + i] = x[i];
+        }
+    }
+    if (tid == 0) {
+        rank[d.idx] = r;
+        status[d.idx] = st;
+        if (info) info[d.idx] = sweeps;
+    }
+}
+
+// matrices, five arrays of k + 1 values, two index arrays
+template <typename T>
+size_t smem_bytes(int K) {
+    return (size_t)2 * K * svd_ld(K) * sizeof(T) + (size_t)5 * (K + 1) * sizeof(T) +
+           (size_t)2 * (K + 1) * sizeof(short) + 16;
+}
+
+}  // namespace
+
+template <typename T>
+cudaError_t configure_svd_smem(int optin, int *kmax) {
+    using K = void (*)(const Desc *, T *, int *, int *, int *, int);
+    const K kernels[] = {svd_smem_kernel<T, 1>, svd_smem_kernel<T, 2>, svd_smem_kernel<T, 4>,
+                         svd_smem_kernel<T, 8>};
+    int dyn = optin;
+    for (K f : kernels) {
+        cudaFuncAttributes fa;
+        const cudaError_t e = cudaFuncGetAttributes(&fa, f);
+        if (e != cudaSuccess) return e;
+        dyn = dyn < optin - (int)fa.sharedSizeBytes ? dyn : optin - (int)fa.sharedSizeBytes;
+    }
+    int k = 0;
+    while (k < 32 * kSvRows && smem_bytes<T>(k + 1) <= (size_t)dyn) ++k;
+    *kmax = k;
+    for (K f : kernels) {
+        const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+template <typename T, int G>
+static void launch_svd_g(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info,
+                         int K, cudaStream_t s) {
+    const int np = (K + 1) / 2, t = (np * G + 31) / 32 * 32;
+    svd_smem_kernel<T, G><<<n, t < kSvThreads ? t : kSvThreads, smem_bytes<T>(K), s>>>(
+        d_desc, ws, d_rank, d_status, d_info, K);
+}
+
+template <typename T>
+void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
+                     int G, cudaStream_t s) {
+    if (G >= 8) launch_svd_g<T, 8>(d_desc, n, ws, d_rank, d_status, d_info, K, s);
+    else if (G >= 4) launch_svd_g<T, 4>(d_desc, n, ws, d_rank, d_status, d_info, K, s);
+    else if (G >= 2) launch_svd_g<T, 2>(d_desc, n, ws, d_rank, d_status, d_info, K, s);
+    else launch_svd_g<T, 1>(d_desc, n, ws, d_rank, d_status, d_info, K, s);
+}
+
+template cudaError_t configure_svd_smem<double>(int, int *);
+template cudaError_t configure_svd_smem<float>(int, int *);
+template void launch_svd_smem<double>(const Desc *, int, double *, int *, int *, int *, int, int,
+                                      cudaStream_t);
+template void launch_svd_smem<float>(const Desc *, int, float *, int *, int *, int *, int, int,
+                                     cudaStream_t);
+
+}  // namespace hc

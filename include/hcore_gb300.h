@@ -175,16 +175,18 @@ int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
  *                      finishes a phase before any group starts the next
  *   qr_warps           warps per Householder-QR CTA: 8 (shortest path per
  *                      update), 4 or 2 (two or four times the CTAs per SM)
- * hcore_gpu_tuning_default fills the built-in choice (16 groups, 2 lanes per
+ * hcore_gpu_tuning_default fills the built-in choice (16 groups, 4 lanes per
  * pair, width 8, no phase sync, 4 QR warps: the autotuner's pick on a TLR
- * panel of 1953 updates; HCORE_GPU_STREAMS overrides the groups).  hcore_gpu_autotune
+ * panel of 1953 updates; HCORE_GPU_STREAMS overrides the groups; a plan
+ * created without a tuning also gives a short list of small updates eight
+ * lanes).  hcore_gpu_autotune
  * times plans of the given tasks over a search of these parameters
  * (coordinate descent; each candidate's execute captured in a CUDA graph on
  * a private stream and replayed `reps` times) and returns the fastest; the
  * tasks' outputs must not alias their inputs (the batch runs many times)
  * and are overwritten.  `stream` is not used (reserved).  Results do not
- * depend on the tuning beyond rounding (the SVD's reduction order follows
- * the lanes). */
+ * depend on the tuning beyond rounding (the lanes do not change them at all:
+ * the SVD adds in one fixed order). */
 typedef struct hcore_gpu_tuning {
     int stream_groups;
     int svd_lanes[3];
