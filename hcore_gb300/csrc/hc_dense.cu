@@ -11,245 +11,125 @@
 //       C = alpha op(A) op(B) + beta C
 //
 // Every contribution is first reduced to a rank-K' product beta CD +
-// coef * P Q^T with P of size M x K' and Q of size N x K' (prep kernels: one
-// CTA per syrk/gemmcd task, a tiled GEMM for the gemmbdcd product
-// Q = BD^T AV; uncompress needs none), and all tasks that hit the same tile
-// are then applied in list order by one tile kernel that keeps a 64 x 64
-// block of CD in registers.  Zeroing the
-// strict upper triangle after each syrk task reproduces the reference's
-// sequential semantics exactly; the syrk's own upper-triangle products are
-// never computed since they are overwritten by zero.
+// coef * P Q^T with P of size M x K' and Q of size N x K' (syrk and gemmcd: the
+// kernels below; gemmbdcd's Q = BD^T AV is a product of the next kind itself;
+// uncompress needs none), and all tasks that hit the same tile are then
+// applied in list order on the tensor cores (hc_dense_tc.cu).  Zeroing
+// the strict upper triangle where a run of syrk tasks ends is the reference's
+// sequential semantics; the syrk's own products strictly above the diagonal
+// are not computed since they are overwritten by zero.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <climits>
 
 #include "hc_internal.h"
 
 namespace hc {
 
-template <typename T>
-__device__ __forceinline__ T wsum(T v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
-}
-
-// S = X^T Y (p x q, reduce over n rows), then the computed factor:
-//   syrk:                       P = AU S                 (M x K)
-//   gemmcd, a > b:              P = Au rr                (M x b)
-//   gemmcd, a <= b:             Q = Bu rr^T              (M x a)
-__global__ void __launch_bounds__(256) dense_prep_kernel(const hcore_dense_task *tasks,
-                                                         const DenseWork *work, double *ws) {
+// A task's inner product S = X^T Y (p x q over n rows): AV^T AV over lda rows
+// for syrk (hcore_dsyrk.c:57,103), Av^T Bv over M rows for gemmcd
+// (hcore_dgemmcd.c:66-70); then the factor that it makes:
+//   syrk:                       P = AU S                 (M x a)
+//   gemmcd, a > b:              P = Au S                 (M x b)
+//   gemmcd, a <= b:             Q = Bu S^T               (M x a)
+//
+// Both kernels are bound by FP64 issue (one warp instruction per 64 cycles and
+// sub-partition), so what was saved is instructions: a warp takes four entries
+// of S at a time, whose sums are reduced together (6 shuffled additions
+// instead of 20 beside 4 M / 32 FMAs), and syrk's S is formed on and above the
+// diagonal only.  Tasks are split over CTAs (entries of S, rows of the factor)
+// so that uneven ranks and short lists fill the GPU.  768 tasks of ranks 8-32,
+// M = 1024: 2097 us in one kernel of a CTA per task, 825 + 723 us in these two.
+__global__ void __launch_bounds__(256) dense_inner_kernel(const hcore_dense_task *tasks,
+                                                          const DenseWork *work, double *ws) {
     const hcore_dense_task t = tasks[blockIdx.x];
-    if (t.kind > 1) return;  // uncompress: no prep; gemmbdcd: bdcd_prep_kernel
-    const DenseWork w = work[blockIdx.x];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    double *S = ws + w.ws;
-    const double *X, *Y;
-    int p, q, n, ldx, ldy;
-    if (t.kind == 0) {  // AV^T AV over LDAU rows (hcore_dsyrk.c:57,103)
-        X = t.Av; Y = t.Av; p = t.a; q = t.a; n = t.lda; ldx = t.lda; ldy = t.lda;
-    } else {            // Av^T Bv over M rows (hcore_dgemmcd.c:66-70)
-        X = t.Av; Y = t.Bv; p = t.a; q = t.b; n = t.M; ldx = t.M; ldy = t.M;
-    }
-    for (int e = warp; e < p * q; e += 8) {
-        const int i = e % p, j = e / p;
-        double s = 0;
-        for (int l = lane; l < n; l += 32) s += X[(size_t)i * ldx + l] * Y[(size_t)j * ldy + l];
-        s = wsum(s);
-        if (lane == 0) S[(size_t)j * p + i] = s;
-    }
-    __syncthreads();
-    double *out = S + (size_t)p * q;
-    const int M = t.M;
-    if (t.kind == 0) {  // P = AU S (M x a)
-        for (long long e = tid; e < (long long)M * t.a; e += 256) {
-            const int i = (int)(e % M), j = (int)(e / M);
-            double s = 0;
-            for (int l = 0; l < t.a; ++l) s += t.Au[(size_t)l * t.lda + i] * S[(size_t)j * p + l];
-            out[(size_t)j * M + i] = s;
+    if (t.kind > 1) return;  // uncompress: no prep; gemmbdcd: its own product
+    double *S = ws + work[blockIdx.x].ws;
+    const bool syrk = t.kind == 0;
+    const double *X = t.Av, *Y = syrk ? t.Av : t.Bv;
+    const int p = t.a, q = syrk ? t.a : t.b, n = syrk ? t.lda : t.M;
+    const int lane = threadIdx.x & 31, warp = blockIdx.y * 8 + (threadIdx.x >> 5);
+    const int quads = (p + 3) / 4;
+    for (int e = warp; e < quads * q; e += gridDim.y * 8) {
+        const int i0 = e % quads * 4, j = e / quads;
+        if (syrk && i0 > j) continue;
+        const double *y = Y + (size_t)j * n;
+        const double *x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = X + (size_t)min(i0 + u, p - 1) * n;
+        double s[4] = {};
+#pragma unroll 2
+        for (int l = lane; l < n; l += 32) {
+            const double yv = y[l];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] += x[u][l] * yv;
         }
-    } else if (t.a > t.b) {  // P = Au rr (M x b)
-        for (long long e = tid; e < (long long)M * t.b; e += 256) {
-            const int i = (int)(e % M), j = (int)(e / M);
-            double s = 0;
-            for (int l = 0; l < t.a; ++l) s += t.Au[(size_t)l * M + i] * S[(size_t)j * p + l];
-            out[(size_t)j * M + i] = s;
-        }
-    } else {  // Q = Bu rr^T (M x a)
-        for (long long e = tid; e < (long long)M * t.a; e += 256) {
-            const int i = (int)(e % M), j = (int)(e / M);
-            double s = 0;
-            for (int l = 0; l < t.b; ++l) s += t.Bu[(size_t)l * M + i] * S[(size_t)l * p + j];
-            out[(size_t)j * M + i] = s;
+        // lanes 8 u .. 8 u + 7 end with sum u
+        const bool h16 = lane & 16, h8 = lane & 8;
+        double a = (h16 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h16 ? s[0] : s[2], 16);
+        double b = (h16 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h16 ? s[1] : s[3], 16);
+        double c = (h8 ? b : a) + __shfl_xor_sync(0xffffffffu, h8 ? a : b, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+        const int i = i0 + (lane >> 3);
+        if ((lane & 7) == 0 && i < p && (!syrk || i <= j)) {
+            S[(size_t)j * p + i] = c;
+            if (syrk) S[(size_t)i * p + j] = c;
         }
     }
 }
 
-// One CTA per (64 x 64 tile of CD, group).  Thread (tx, ty) owns a 4 x 4
-// register block; K' is staged in chunks of 16 through shared memory.
-constexpr int TB = 64, TK = 16;
-
-// gemmbdcd prep: Q = BD^T AV (N x a, ld N) into the task's workspace, i.e.
-// (AV^T BD)^T of hcore_dgemmbdcd.c:80-87/:99-106, summed over kdim rows.
-// One CTA per (64 rows of Q, 64 columns of Q, task); both operands are read
-// along their contiguous dimension (16 consecutive rows of a column).
-__global__ void __launch_bounds__(256) bdcd_prep_kernel(const hcore_dense_task *tasks,
-                                                        const DenseWork *work, const int *idx,
-                                                        int tilesN, int tilesA, double *ws) {
-    __shared__ double sB[TK][TB + 1];
-    __shared__ double sA[TK][TB + 1];
-    const int ti = blockIdx.x % tilesN;
-    const int tj = (blockIdx.x / tilesN) % tilesA;
-    const int q = blockIdx.x / (tilesN * tilesA);
-    const int task = idx[q];
-    const hcore_dense_task t = tasks[task];
-    const int N = t.N ? t.N : t.M, K = t.kdim ? t.kdim : t.M, a = t.a;
-    const int row0 = ti * TB, col0 = tj * TB;  // rows of Q (columns of BD), columns of Q
-    if (row0 >= N || col0 >= a) return;
-    double *Q = ws + work[task].ws;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += TK) {
-        for (int e = threadIdx.x; e < TK * TB; e += 256) {
-            const int kk = e % TK, r = e / TK;
-            const int kg = k0 + kk;
-            sB[kk][r] = (kg < K && row0 + r < N) ? t.Bd[(size_t)(row0 + r) * t.ldb + kg] : 0.0;
-            sA[kk][r] = (kg < K && col0 + r < a) ? t.Av[(size_t)(col0 + r) * t.lda + kg] : 0.0;
+// out(i, j) = sum_l F(i, l) S'(l, j), a thread per row, four columns at a time
+__global__ void __launch_bounds__(128) dense_factor_kernel(const hcore_dense_task *tasks,
+                                                           const DenseWork *work, double *ws) {
+    const hcore_dense_task t = tasks[blockIdx.x];
+    if (t.kind > 1) return;
+    const int i = blockIdx.y * 128 + threadIdx.x;
+    if (i >= t.M) return;
+    const bool syrk = t.kind == 0, left = syrk || t.a > t.b;
+    const int p = t.a, q = syrk ? t.a : t.b;
+    const double *S = ws + work[blockIdx.x].ws;
+    double *out = ws + work[blockIdx.x].ws + (size_t)p * q;
+    // S'(l, j) = S(l, j), or S(j, l) for Bu S^T
+    const double *F = (left ? t.Au : t.Bu) + i;
+    const size_t ldf = syrk ? t.lda : t.M;
+    const int inner = left ? p : q, cols = left ? q : p;
+    const size_t sl = left ? 1 : p, sj = left ? p : 1;
+    for (int j = 0; j < cols; j += 4) {
+        double s[4] = {};
+        const double *b[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) b[u] = S + (size_t)min(j + u, cols - 1) * sj;
+#pragma unroll 4
+        for (int l = 0; l < inner; ++l) {
+            const double f = F[(size_t)l * ldf];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] += f * b[u][(size_t)l * sl];
         }
-        __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            double bv[4], av[4];
-#pragma unroll
-            for (int u = 0; u < 4; ++u) bv[u] = sB[kk][tx + 16 * u];
-#pragma unroll
-            for (int v = 0; v < 4; ++v) av[v] = sA[kk][ty + 16 * v];
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] += bv[u] * av[v];
-        }
-        __syncthreads();
+        for (int u = 0; u < 4; ++u)
+            if (j + u < cols) out[(size_t)(j + u) * t.M + i] = s[u];
     }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int i = row0 + tx + 16 * u, j = col0 + ty + 16 * v;
-            if (i < N && j < a) Q[(size_t)j * N + i] = acc[u][v];
-        }
 }
 
-__global__ void __launch_bounds__(256) dense_tile_kernel(const hcore_dense_task *tasks,
-                                                         const DenseWork *work,
-                                                         const int *group_start,
-                                                         const int *group_tasks, int tiles_per_dim) {
-    __shared__ double sP[TK][TB + 1];
-    __shared__ double sQ[TK][TB + 1];
-    const int g = blockIdx.y;
-    const int tile = blockIdx.x;
-    const int bi = tile % tiles_per_dim, bj = tile / tiles_per_dim;
-    const int g0 = group_start[g], g1 = group_start[g + 1];
-    if (g0 == g1) return;
-    const hcore_dense_task t0 = tasks[group_tasks[g0]];
-    const int M = t0.M, N = t0.N ? t0.N : t0.M;
-    const int row0 = bi * TB, col0 = bj * TB;
-    if (row0 >= M || col0 >= N) return;
-    double *CD = t0.CD;
-    const int ldcd = t0.ldcd;
-    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-    double acc[4][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int i = row0 + tx + 16 * u, j = col0 + ty + 16 * v;
-            acc[u][v] = (i < M && j < N) ? CD[(size_t)j * ldcd + i] : 0.0;
-        }
-    const bool strictly_upper = row0 + TB <= col0;  // every (i, j) here has i < j
-    for (int gi = g0; gi < g1; ++gi) {
-        const DenseWork w = work[group_tasks[gi]];
-        if (w.beta != 1.0) {  // beta = 0 does not read CD (BLAS convention)
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v) acc[u][v] = w.beta == 0.0 ? 0.0 : w.beta * acc[u][v];
-        }
-        if (!(w.syrk && strictly_upper)) {
-            for (int k0 = 0; k0 < w.kk; k0 += TK) {
-                // the task's coefficient is folded into P as it is staged
-                // (once per element, not once per use)
-                for (int e = threadIdx.x; e < TK * TB; e += 256) {
-                    const int kk = e / TB, r = e % TB;
-                    const int kg = k0 + kk;
-                    sP[kk][r] = (kg < w.kk && row0 + r < M) ? w.coef * w.P[(size_t)kg * w.ldp + row0 + r] : 0.0;
-                    sQ[kk][r] = (kg < w.kk && col0 + r < N) ? w.Q[(size_t)kg * w.ldq + col0 + r] : 0.0;
-                }
-                __syncthreads();
-#pragma unroll
-                for (int kk = 0; kk < TK; ++kk) {
-                    double pv[4], qv[4];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) pv[u] = sP[kk][tx + 16 * u];
-#pragma unroll
-                    for (int v = 0; v < 4; ++v) qv[v] = sQ[kk][ty + 16 * v];
-#pragma unroll
-                    for (int u = 0; u < 4; ++u)
-#pragma unroll
-                        for (int v = 0; v < 4; ++v) acc[u][v] += pv[u] * qv[v];
-                }
-                __syncthreads();
-            }
-        }
-        if (w.syrk) {
-#pragma unroll
-            for (int u = 0; u < 4; ++u)
-#pragma unroll
-                for (int v = 0; v < 4; ++v)
-                    if (row0 + tx + 16 * u < col0 + ty + 16 * v) acc[u][v] = 0.0;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < 4; ++u)
-#pragma unroll
-        for (int v = 0; v < 4; ++v) {
-            const int i = row0 + tx + 16 * u, j = col0 + ty + 16 * v;
-            if (i < M && j < N) CD[(size_t)j * ldcd + i] = acc[u][v];
-        }
-}
 
 cudaError_t launch_dense_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work, int n,
-                              double *ws, cudaStream_t s) {
+                              int maxM, double *ws, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
-    dense_prep_kernel<<<n, 256, 0, s>>>(d_tasks, d_work, ws);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_bdcd_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work,
-                             const int *d_idx, int n_idx, int maxN, int maxA, double *ws,
-                             cudaStream_t s) {
-    if (n_idx <= 0 || maxN <= 0 || maxA <= 0) return cudaSuccess;
-    const int tn = (maxN + TB - 1) / TB, ta = (maxA + TB - 1) / TB;
-    const long long blocks = (long long)tn * ta * n_idx;
-    if (blocks > INT_MAX) return cudaErrorInvalidValue;
-    bdcd_prep_kernel<<<(unsigned)blocks, 256, 0, s>>>(d_tasks, d_work, d_idx, tn, ta, ws);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_dense_tiles(const hcore_dense_task *d_tasks, const DenseWork *d_work,
-                               const int *d_group_start, const int *d_group_tasks, int ngroups,
-                               int maxDim, cudaStream_t s) {
-    if (ngroups <= 0) return cudaSuccess;
-    const int tpd = (maxDim + TB - 1) / TB;
-    dense_tile_kernel<<<dim3(tpd * tpd, ngroups), 256, 0, s>>>(d_tasks, d_work, d_group_start,
-                                                               d_group_tasks, tpd);
+    // about four CTAs an SM and more: a task's entries over up to eight CTAs
+    const int split = std::max(1, std::min(8, 1216 / n));
+    dense_inner_kernel<<<dim3(n, split), 256, 0, s>>>(d_tasks, d_work, ws);
+    dense_factor_kernel<<<dim3(n, (maxM + 127) / 128), 128, 0, s>>>(d_tasks, d_work, ws);
     return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------
 // plain dense GEMM, C = alpha op(A) op(B) + beta C (HCORE_dgemm_dense)
 // ---------------------------------------------------------------------------
+// Tiles of 64 x 64: thread (tx, ty) owns a 4 x 4 register block; the inner
+// dimension is staged in chunks of 16 through shared memory.
+constexpr int TB = 64, TK = 16;
 template <typename T>
 __global__ void __launch_bounds__(256) gemm_dense_kernel(int ta, int tb, int M, int N, int K,
                                                          T alpha, const T *A, int lda, const T *B,

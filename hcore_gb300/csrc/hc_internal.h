@@ -199,17 +199,45 @@ struct DenseWork {
     double coef;      // CD = beta CD + coef P Q^T
     double beta;
     int syrk;         // 1: zero the strict upper triangle after this task
+    int tr;           // 1: P is stored transposed (K' x M), 2: Q, 3: both
     long long ws;     // workspace offset (doubles): S (p x q), then the computed factor
 };
+// S and the computed factor of the syrk and gemmcd tasks (of n tasks of all kinds)
 cudaError_t launch_dense_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work, int n,
-                              double *ws, cudaStream_t s);
-// Q = Bd^T Av (N x a) of the gemmbdcd tasks listed in d_idx
-cudaError_t launch_bdcd_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work,
-                             const int *d_idx, int n_idx, int maxN, int maxA, double *ws,
-                             cudaStream_t s);
-cudaError_t launch_dense_tiles(const hcore_dense_task *d_tasks, const DenseWork *d_work,
-                               const int *d_group_start, const int *d_group_tasks, int ngroups,
-                               int maxDim, cudaStream_t s);
+                              int maxM, double *ws, cudaStream_t s);
+// the products on the tensor cores (hc_dense_tc.cu): the tasks of a tile laid
+// out along K in chunks of up to 128 columns.  cols[c] = (task, its column l).
+struct DenseChunk {
+    long long p, q;   // byte offsets of P's and Q's digit slices
+    int ep, eq;       // row scales of P and Q (ints)
+    int col0, ncol;   // columns of the K axis
+    int M, N;
+    double beta;      // CD is scaled by it before this chunk
+    int zero_upper;   // the strict upper triangle is zero after this chunk
+    int scale;        // 0: beta = 1, 1: another value, 2: zero
+};
+struct DenseJob {     // one tile and chunks of its list
+    double *cd;
+    int ldcd, task;   // task: one of the tile's products
+    int M, N, chunk0, nchunks;
+    int tile0;        // its first tile in the batch
+};
+struct DenseBatch {   // jobs that share the slice buffer at one time
+    int job0, njobs, ntiles, chunk0, nchunks, maxM, maxN;
+};
+// shared-memory attribute of the tile kernel on the current device
+cudaError_t configure_dense_tc();
+// bytes of a chunk's slices, and where Q's start
+size_t dense_slice_bytes(int M, int N, int ncol);
+size_t dense_slice_q_offset(int M, int ncol);
+int dense_tiles(int M, int N);   // tiles of one job
+// the balance of ncols columns (transposed: of products with both operands
+// stored transposed)
+cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, const int2 *d_dims, int ncols,
+                                 bool transposed, int *d_shift, cudaStream_t s);
+cudaError_t launch_dense_tiles_tc(const DenseWork *d_work, const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
+                                  const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
+                                  int *d_exps, cudaStream_t s);
 template <typename T>
 cudaError_t launch_gemm_dense(int ta, int tb, int M, int N, int K, T alpha, const T *A, int lda,
                               const T *B, int ldb, T beta, T *C, int ldc, cudaStream_t s);
