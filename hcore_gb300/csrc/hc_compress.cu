@@ -6,16 +6,23 @@
 // optional relative rule (sigma_i >= acc * sigma_max) for TLR matrices whose
 // tiles span many orders of magnitude.
 //
-// Method.  The reference runs a full dgesvd of the tile.  Here a truncated
-// Householder QR with column pivoting first finds the tile's numerical range,
-//     D P = Q [R11 R12; 0 R22],   ||R22||_F <= delta,
-// with delta = 1e-3 of the truncation threshold (at least 64 eps ||D||_F):
-// D = Q1 [R11 R12] P^T + E, ||E||_2 <= delta, so every singular value of
-// the k-column product Q1 R~ P^T is within delta of D's.  That product is
-// exactly the low-rank form the recompression plan takes (UA = Q1,
-// VB = P R~^T), so the plan's QR, Jacobi SVD and rebuild phases finish the
+// Method.  The reference runs a full dgesvd of the tile.  Here the tile's
+// numerical range is found first,
+//     D = Q B^T + E,   ||E||_F <= delta,
+// with delta = 1e-3 of the truncation threshold (at least 64 eps ||D||_F), so
+// that every singular value of the k-column product Q B^T is within delta of
+// D's.  That product is exactly the low-rank form the recompression plan takes
+// (UA = Q, VB = B), so the plan's QR, Jacobi SVD and rebuild phases finish the
 // job with the compressor's rank rule.  Ranks agree with the reference's
 // except where a singular value lies within delta of the threshold.
+//
+// The range comes from blocks of random test vectors whose products run on the
+// tensor cores (find_ranges): the tile is read and written a few times per 32
+// columns.  A truncated Householder QR with column pivoting (qrcp_kernel) does
+// the same one column at a time; it applies 3 M^2 FP64 FMAs per column on one
+// SM (98 ms for 48 tiles of 1024 and ranks 8-40 at 1e-8, where the blocks take
+// 7 ms and the whole call went from 120.7 to 19.3 ms), so it is kept for what
+// the blocks leave: small tiles, wide ranges, non-finite tiles.
 //
 // qrcp_kernel: one CTA per tile; the tile is copied into a workspace and
 // factored there, one pivot column per step (argmax of the trailing column
@@ -31,6 +38,7 @@
 #include <vector>
 
 #include "hc_host.h"
+#include "hc_products.h"
 
 namespace hc {
 
@@ -50,8 +58,138 @@ struct FormWork {
     const int *perm;
     double *UA, *VB;  // the plan workspace's UA and VB regions (M x k, ld M)
     int M, k;
+    const double *Q, *B;  // a range found by products: M x k each (else null)
 };
 
+// ---- the range by products ---------------------------------------------------
+// A tile of the blocked range finder: its residual E, the basis Q and B = E^T Q
+// found so far (M x k, ld M).
+struct RangeTile {
+    const double *D;
+    int ldd, M;
+    double *E, *Q, *B;
+};
+constexpr int kSumParts = 32;   // partial sums of squares per tile
+
+// E = D (load) and the partial sums of E's squares
+__global__ void __launch_bounds__(256) range_norm_kernel(const RangeTile *tiles, const int *list, bool load,
+                                                         double *part) {
+    __shared__ double s_sum[8];
+    const int q = list[blockIdx.x];
+    const RangeTile t = tiles[q];
+    const long long n = (long long)t.M * t.M, step = (long long)kSumParts * 256;
+    double s = 0.0;
+    for (long long e = (long long)blockIdx.y * 256 + threadIdx.x; e < n; e += step) {
+        double x;
+        if (load) {
+            x = t.D[(size_t)(e / t.M) * t.ldd + e % t.M];
+            t.E[e] = x;
+        } else {
+            x = t.E[e];
+        }
+        s += x * x;
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < 8; ++w) s += s_sum[w];
+        part[(size_t)q * kSumParts + blockIdx.y] = s;
+    }
+}
+
+// test vectors of one block: n values in (-1, 1), a fixed sequence (the
+// SplitMix64 mixing function of Steele, Lea and Flood, 2014)
+__global__ void range_test_vectors_kernel(double *omega, int n, int base) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    unsigned long long z = (unsigned long long)(base + i + 1) * 0x9E3779B97F4A7C15ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    omega[i] = (double)(long long)z * 0x1p-63;
+}
+
+// Columns c0 .. c0 + nc of each listed tile's Q made orthonormal among
+// themselves (modified Gram-Schmidt; a warp keeps the column it updates in
+// registers, RPL rows per lane).  Twice: a block spans several decades of
+// singular values, and what one pass leaves (about 1e-9) would stay in E far
+// above delta and be found again as new directions (160 columns instead of 80
+// for 1024-tiles of rank 40 at 1e-8).  They need not be orthogonal to the
+// earlier ones to rounding: E = D - Q B holds whatever Q is, and the plan
+// factors Q.
+template <int RPL>
+__global__ void __launch_bounds__(256, 1) range_orth_kernel(const RangeTile *tiles, const int *list, int c0,
+                                                            int nc) {
+    __shared__ double s_q[2][32 * RPL];
+    const RangeTile t = tiles[list[blockIdx.x]];
+    double *Q = t.Q + (size_t)c0 * t.M;
+    const int M = t.M, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    double x[RPL];
+    auto load = [&](int col) {
+#pragma unroll
+        for (int r = 0; r < RPL; ++r) {
+            const int i = lane + 32 * r;
+            x[r] = i < M ? Q[(size_t)col * M + i] : 0.0;
+        }
+    };
+    auto store = [&](int col) {
+#pragma unroll
+        for (int r = 0; r < RPL; ++r) {
+            const int i = lane + 32 * r;
+            if (i < M) Q[(size_t)col * M + i] = x[r];
+        }
+    };
+    auto publish = [&](double *q) {   // x / ||x|| (a zero column stays zero)
+        double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+        for (int r = 0; r < RPL; r += 2) {
+            s0 += x[r] * x[r];
+            s1 += x[r + 1] * x[r + 1];
+        }
+        s0 += s1;
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
+        const double f = s0 > 0.0 ? rsqrt(s0) : 0.0;
+#pragma unroll
+        for (int r = 0; r < RPL; ++r) {
+            x[r] *= f;
+            q[lane + 32 * r] = x[r];
+        }
+    };
+    for (int pass = 0; pass < 2; ++pass) {
+        if (warp == 0) {
+            load(0);
+            publish(s_q[0]);
+            store(0);
+        }
+        __syncthreads();
+        for (int j = 0; j + 1 < nc; ++j) {
+            const double *q = s_q[j & 1];
+            for (int col = j + 1 + warp; col < nc; col += 8) {
+                load(col);
+                double d0 = 0.0, d1 = 0.0;
+#pragma unroll
+                for (int r = 0; r < RPL; r += 2) {
+                    d0 += q[lane + 32 * r] * x[r];
+                    d1 += q[lane + 32 * (r + 1)] * x[r + 1];
+                }
+                d0 += d1;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, o);
+                const volatile double *qv = q;   // re-read rather than held in registers
+#pragma unroll
+                for (int r = 0; r < RPL; ++r) x[r] -= d0 * qv[lane + 32 * r];
+                if (col == j + 1) publish(s_q[(j + 1) & 1]);
+                store(col);
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// ---- the range by a pivoted QR ---------------------------------------------------
 __device__ __forceinline__ double wsum_d(double v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -209,6 +347,13 @@ __global__ void __launch_bounds__(256) qrcp_kernel(const QrcpTask *tasks, int *k
 __global__ void __launch_bounds__(256) compress_form_kernel(const FormWork *work) {
     const FormWork f = work[blockIdx.x];
     const int M = f.M, k = f.k, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (f.Q) {
+        for (long long e = tid; e < (long long)M * k; e += 256) {
+            f.UA[e] = f.Q[e];
+            f.VB[e] = f.B[e];
+        }
+        return;
+    }
     for (long long e = tid; e < (long long)M * k; e += 256) {
         const int l = (int)(e % M), i = (int)(e / M);
         f.VB[(size_t)i * M + f.perm[l]] = i <= l ? f.W[(size_t)l * M + i] : 0.0;
@@ -230,7 +375,157 @@ __global__ void __launch_bounds__(256) compress_form_kernel(const FormWork *work
     }
 }
 
+
 static size_t al256c(size_t x) { return (x + 255) & ~(size_t)255; }
+
+// Which tiles take the range finder, and its widest range: smaller tiles (and
+// wider ranges) are cheap for (need) the pivoted QR.
+constexpr int kRangeMinM = 128, kRangeMaxK = 256;
+static int range_cap(int M) { return M < kRangeMinM ? 0 : std::min(kRangeMaxK, M / 2 / 32 * 32); }
+
+// The range of tiles [0, nt) by products: blocks of columns Y = E Omega (random
+// test vectors), orthonormalised to Q_i, B_i = E^T Q_i, E <- E - Q_i B_i^T until
+// ||E||_F <= kRangeShare * delta (the blocked scheme of Martinsson and Voronin,
+// "A randomized blocked algorithm for efficiently computing rank-revealing
+// factorizations of matrices", 2016; the residual is formed, so what is found
+// does not depend on chance, only how soon).  k[q] becomes the columns found;
+// -1 leaves the tile to the pivoted QR (not finite, out of the range of squares,
+// or wider than its cap).
+static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compress_task *const *tasks,
+                               const RangeTile *d_tiles, int maxM, std::vector<int> &k, cudaStream_t s) {
+    k.assign(nt, -1);
+    if (nt == 0) return cudaSuccess;
+    std::vector<int> active(nt);
+    for (int q = 0; q < nt; ++q) active[q] = q;
+    char *buf = nullptr;   // list, partial sums, test vectors
+    const size_t b_list = al256c(nt * sizeof(int)), b_part = al256c((size_t)nt * kSumParts * sizeof(double));
+    cudaError_t e = cudaMalloc(&buf, b_list + b_part + (size_t)maxM * 32 * sizeof(double));
+    if (e != cudaSuccess) return e;
+    int *d_list = (int *)buf;
+    double *d_part = (double *)(buf + b_list), *d_omega = (double *)(buf + b_list + b_part);
+    std::vector<double> part((size_t)nt * kSumParts), limit(nt);
+    auto norms = [&](bool load) -> cudaError_t {
+        cudaError_t r = cudaMemcpyAsync(d_list, active.data(), active.size() * sizeof(int),
+                                        cudaMemcpyHostToDevice, s);
+        if (r == cudaSuccess) {
+            range_norm_kernel<<<dim3((unsigned)active.size(), kSumParts), 256, 0, s>>>(d_tiles, d_list, load,
+                                                                                       d_part);
+            r = cudaGetLastError();
+        }
+        if (r == cudaSuccess)
+            r = cudaMemcpyAsync(part.data(), d_part, part.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
+        return r == cudaSuccess ? cudaStreamSynchronize(s) : r;
+    };
+    auto sum_of = [&](int q) {
+        double x = 0.0;
+        for (int y = 0; y < kSumParts; ++y) x += part[(size_t)q * kSumParts + y];
+        return x;
+    };
+    char *arena = nullptr;
+    size_t arena_bytes = 0;
+    std::vector<char> host;
+    // run a list of products: upload its layout and launch it
+    auto products = [&](DenseProducts &p) -> cudaError_t {
+        size_t up = 0;
+        p.place_host(up);
+        size_t all = up;
+        p.place_device(all);
+        if (all > arena_bytes) {
+            cudaError_t r = cudaStreamSynchronize(s);
+            cudaFree(arena);
+            arena = nullptr;
+            arena_bytes = 0;
+            if (r == cudaSuccess) r = cudaMalloc(&arena, all);
+            if (r != cudaSuccess) return r;
+            arena_bytes = all;
+        }
+        host.resize(up);
+        p.pack(host.data());
+        // (from pageable memory: the copy has left `host` when it returns)
+        const cudaError_t r = cudaMemcpyAsync(arena, host.data(), up, cudaMemcpyHostToDevice, s);
+        return r == cudaSuccess ? p.launch(arena, s) : r;
+    };
+    e = configure_dense_tc();
+    if (e == cudaSuccess) e = norms(true);
+    std::vector<int> found(nt, 0);
+    for (int c0 = 0; e == cudaSuccess;) {
+        // tiles that are done, refused or full leave the list
+        std::vector<int> next;
+        for (int q : active) {
+            const hcore_compress_task &t = *tasks[q];
+            const double x = sum_of(q);
+            if (c0 == 0) {
+                if (!(x == 0.0 || (x > 1e-280 && x < 1e280))) continue;
+                const double d = kRangeShare * range_delta(sqrt(x), t.M, t.relative != 0, t.acc);
+                limit[q] = d * d;
+            }
+            if (!(x <= limit[q])) {
+                if (found[q] + 16 <= range_cap(t.M)) next.push_back(q);
+            } else {
+                k[q] = found[q];
+            }
+        }
+        active.swap(next);
+        if (active.empty()) break;
+        // 32 columns (a tile's width in the products) at first; 16 later, where a
+        // wider core costs the SVD more than another block costs here
+        const int nc = c0 < 64 ? 32 : 16;
+        range_test_vectors_kernel<<<(maxM * nc + 255) / 256, 256, 0, s>>>(d_omega, maxM * nc, c0 * maxM);
+        DenseProducts y, b;
+        y.slice_limit = b.slice_limit = (size_t)384 << 20;   // few tiles a product: fill the GPU instead
+        y.stage(DenseProducts::kNoBalance);
+        auto out = [](DenseProducts &p, const DenseWork &w, int M, int N, double *cd) {
+            const size_t first = p.jobs.size();
+            p.add_tile({p.add(w, M, N)});
+            for (size_t j = first; j < p.jobs.size(); ++j) {
+                p.jobs[j].cd = cd;
+                p.jobs[j].ldcd = M;
+            }
+        };
+        auto product = [](const double *P, int ldp, const double *Q, int ldq, int kk, double coef, double beta,
+                          int tr) {
+            DenseWork w{};
+            w.P = P; w.ldp = ldp; w.Q = Q; w.ldq = ldq; w.kk = kk; w.coef = coef; w.beta = beta; w.tr = tr;
+            return w;
+        };
+        for (int q : active) {
+            const RangeTile &t = tiles[q];
+            out(y, product(t.E, t.M, d_omega, maxM, t.M, 1.0, 0.0, 2), t.M, nc, t.Q + (size_t)c0 * t.M);
+        }
+        b.stage(DenseProducts::kNoBalance);
+        for (int q : active) {
+            const RangeTile &t = tiles[q];
+            out(b, product(t.E, t.M, t.Q + (size_t)c0 * t.M, t.M, t.M, 1.0, 0.0, 3), t.M, nc,
+                t.B + (size_t)c0 * t.M);
+        }
+        b.stage(DenseProducts::kNoBalance);
+        for (int q : active) {
+            const RangeTile &t = tiles[q];
+            out(b, product(t.Q + (size_t)c0 * t.M, t.M, t.B + (size_t)c0 * t.M, t.M, nc, -1.0, 1.0, 0), t.M, t.M,
+                t.E);
+        }
+        e = products(y);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(d_list, active.data(), active.size() * sizeof(int), cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) {
+            const unsigned g = (unsigned)active.size();
+            if (maxM <= 512) range_orth_kernel<16><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
+            else if (maxM <= 1024) range_orth_kernel<32><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
+            else range_orth_kernel<64><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
+            e = cudaGetLastError();
+        }
+        // (both lists use one arena: the second's layout is copied after the
+        // first's launches in stream order)
+        if (e == cudaSuccess) e = products(b);
+        c0 += nc;
+        for (int q : active) found[q] = c0;
+        if (e == cudaSuccess) e = norms(false);
+    }
+    cudaStreamSynchronize(s);
+    cudaFree(arena);
+    cudaFree(buf);
+    return e;
+}
 
 // Compress tasks [0, n) (device-accessible pointers, validated) in chunks
 // whose QR workspaces fit `budget` bytes.
@@ -244,22 +539,27 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
         int i1 = i0;
         while (i1 < n) {
             const size_t M = tasks[i1].M;
-            const size_t need = al256c(M * M * 8) + 3 * al256c(M * 8) + al256c(kMaxK * 8);
+            const size_t need = al256c(M * M * 8) + 3 * al256c(M * 8) + al256c(kMaxK * 8) +
+                                2 * al256c(M * range_cap((int)M) * 8);
             if (i1 > i0 && bytes + need > budget) break;
             bytes += need;
             ++i1;
         }
         const int nc = i1 - i0;
         std::vector<QrcpTask> qt(nc);
+        std::vector<RangeTile> rt;
+        std::vector<const hcore_compress_task *> rtask;
+        std::vector<int> rq;   // the range finder's tiles
         char *qa = nullptr;
-        const size_t b_meta = al256c(nc * sizeof(QrcpTask)) + 2 * al256c(nc * sizeof(int));
+        const size_t b_qt = al256c(nc * sizeof(QrcpTask)), b_rt = al256c(nc * sizeof(RangeTile));
+        const size_t b_meta = b_qt + b_rt + 2 * al256c(nc * sizeof(int));
         if (cudaMalloc(&qa, bytes + b_meta) != cudaSuccess) {
             cudaGetLastError();
             set_error("hcore_gpu_compress_batched: cudaMalloc of %zu bytes failed", bytes + b_meta);
             return HCORE_GPU_ENOMEM;
         }
         char *p = qa + b_meta;
-        int maxM = 1;
+        int maxM = 1, rangeM = 1;
         for (int q = 0; q < nc; ++q) {
             const hcore_compress_task &t = tasks[i0 + q];
             QrcpTask &u = qt[q];
@@ -272,27 +572,67 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             p += al256c(M * 8);
             u.tau = (double *)p; p += al256c(kMaxK * 8);
             maxM = std::max(maxM, t.M);
+            if (const int cap = range_cap(t.M)) {
+                RangeTile r{t.D, t.ldd, t.M, u.W, (double *)p, nullptr};
+                p += al256c(M * cap * 8);
+                r.B = (double *)p; p += al256c(M * cap * 8);
+                rt.push_back(r);
+                rtask.push_back(&t);
+                rq.push_back(q);
+                rangeM = std::max(rangeM, t.M);
+            }
         }
         QrcpTask *d_qt = (QrcpTask *)qa;
-        int *d_k = (int *)(qa + al256c(nc * sizeof(QrcpTask)));
+        RangeTile *d_rt = (RangeTile *)(qa + b_qt);
+        int *d_k = (int *)(qa + b_qt + b_rt);
         int *d_st = d_k + al256c(nc * sizeof(int)) / sizeof(int);
-        cudaError_t e = cudaMemcpyAsync(d_qt, qt.data(), nc * sizeof(QrcpTask),
-                                        cudaMemcpyHostToDevice, s);
-        const size_t smem = (size_t)maxM * sizeof(double);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(qrcp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)std::max<size_t>(smem, 1024));
+        cudaError_t e = cudaSuccess;
+        if (!rt.empty())
+            e = cudaMemcpyAsync(d_rt, rt.data(), rt.size() * sizeof(RangeTile), cudaMemcpyHostToDevice, s);
+        std::vector<int> rk, hk(nc, -1), hst(nc, HCORE_GPU_S_OK), slot(nc, -1);
+        if (e == cudaSuccess) e = find_ranges((int)rt.size(), rt.data(), rtask.data(), d_rt, rangeM, rk, s);
+        // the tiles it did not take: the pivoted QR
+        std::vector<QrcpTask> rest;
+        std::vector<int> rest_q;
         if (e == cudaSuccess) {
-            qrcp_kernel<<<nc, 256, smem, s>>>(d_qt, d_k, d_st);
-            e = cudaGetLastError();
+            for (size_t x = 0; x < rq.size(); ++x) {
+                hk[rq[x]] = rk[x];
+                slot[rq[x]] = (int)x;
+            }
+            for (int q = 0; q < nc; ++q)
+                if (hk[q] < 0) {
+                    rest.push_back(qt[q]);
+                    rest_q.push_back(q);
+                    slot[q] = -1;
+                }
         }
-        std::vector<int> hk(nc), hst(nc);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hk.data(), d_k, nc * sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hst.data(), d_st, nc * sizeof(int), cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        const int nq = (int)rest.size();
+        if (e == cudaSuccess && nq > 0) {
+            std::vector<int> k1(nq), st1(nq);
+            const size_t smem = (size_t)maxM * sizeof(double);
+            e = cudaMemcpyAsync(d_qt, rest.data(), nq * sizeof(QrcpTask), cudaMemcpyHostToDevice, s);
+            if (e == cudaSuccess)
+                e = cudaFuncSetAttribute(qrcp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)std::max<size_t>(smem, 1024));
+            if (e == cudaSuccess) {
+                qrcp_kernel<<<nq, 256, smem, s>>>(d_qt, d_k, d_st);
+                e = cudaGetLastError();
+            }
+            if (e == cudaSuccess) e = cudaMemcpyAsync(k1.data(), d_k, nq * sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(st1.data(), d_st, nq * sizeof(int), cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            for (int x = 0; x < nq && e == cudaSuccess; ++x) {
+                hk[rest_q[x]] = k1[x];
+                hst[rest_q[x]] = st1[x];
+            }
+        }
         if (e != cudaSuccess) {
             set_error("hcore_gpu_compress_batched: %s", cudaGetErrorString(e));
             cudaFree(qa);
+            if (e == cudaErrorMemoryAllocation) {
+                cudaGetLastError();
+                return HCORE_GPU_ENOMEM;
+            }
             return HCORE_GPU_ECUDA;
         }
         // the plan phases for the tiles with a range of k >= 1 columns,
@@ -320,7 +660,8 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
                 d.CUo = t.U; d.CVo = t.V; d.ldco = t.ldo;
                 d.rk = 0; d.max_rank = std::max(t.maxrank, 0); d.storage_rank = INT_MAX;
                 d.rank_start = 0;
-                d.rule = kRuleCapRank | (t.relative ? kRuleRelative : 0);
+                d.rule = kRuleCapRank | (t.relative ? kRuleRelative : 0) |
+                         (slot[q] >= 0 ? kRuleRange : 0);
                 d.status0 = 0;
                 d.idx = i0 + q;
                 d.ws = ws;
@@ -346,8 +687,10 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             for (int x = 0; x < nd; ++x) {
                 const int q = order[x];
                 const WsLayout L = ws_layout(descs[x]);
+                const RangeTile *r = slot[q] >= 0 ? &rt[slot[q]] : nullptr;
                 fw[x] = FormWork{qt[q].W, qt[q].tau, qt[q].perm, pws + descs[x].ws + L.UA,
-                                 pws + descs[x].ws + L.VB, descs[x].M, descs[x].k};
+                                 pws + descs[x].ws + L.VB, descs[x].M, descs[x].k,
+                                 r ? r->Q : nullptr, r ? r->B : nullptr};
             }
             LaunchShape shape;
             shape.maxM = pM;

@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "hc_host.h"
+#include "hc_products.h"
 #include "hc_zinternal.h"
 #include "hcore_d.h"
 #include "hcore_s.h"
@@ -497,26 +498,13 @@ struct DenseRun {
 // pointers): group by output tile (list order kept inside each group), the
 // rank-K' form of every task and the workspace layout.
 struct DensePrep {
-    // a batch's digit slices stay in the L2 (129 MB; the tiles pass through it
-    // too), and 96 MB more than that held costs 2.5%: 384 products of 1024 x
-    // 1024 x 17 took 2873, 2625, 2557, 2538 and 2493 us with limits of 16, 48,
-    // 96, 160 and 400 MB
-    static constexpr size_t kSliceBytes = (size_t)96 << 20;
-    int n = 0, maxM01 = 0;       // maxM01: largest syrk or gemmcd tile
-    std::vector<DenseWork> work; // the tasks', then the gemmbdcd tasks' Q = BD^T AV
-    std::vector<int> bdcd;       // the gemmbdcd tasks
-    int first_cols = 0, first_batches = 0;   // of the products that make Q
-    std::vector<int2> cols;      // the K axes of all tiles: (task, its column)
-    std::vector<int2> dims;      // M, N of each task
-    std::vector<DenseChunk> chunks;
-    std::vector<DenseJob> jobs;
-    std::vector<DenseBatch> batches;
-    long long ws = 0;            // doubles
-    size_t slice_bytes = 0, max_exps = 0;
-    // arena: what pack() writes, then the workspace, column shifts, row scales
-    // and slices
-    size_t o_work = 0, o_cols = 0, o_dims = 0, o_chunks = 0, o_jobs = 0, o_ws = 0,
-           o_shift = 0, o_exps = 0, o_slices = 0, b_all = 0;
+    int n = 0, maxM01 = 0;   // maxM01: largest syrk or gemmcd tile
+    std::vector<int> bdcd;   // the gemmbdcd tasks
+    DenseProducts pr;        // the tasks' products, then the gemmbdcd tasks' Q = BD^T AV
+    long long ws = 0;        // doubles
+    // arena: the tasks and the products' layout (what pack() writes), then the
+    // workspace and the products' device arrays
+    size_t o_ws = 0, b_all = 0;
     size_t bytes() const { return b_all; }
     size_t ws_offset() const { return o_ws; }
 
@@ -543,7 +531,6 @@ struct DensePrep {
         n = n_;
         std::map<const double *, int> gid;
         std::vector<std::vector<int>> groups;
-        work.assign(n, DenseWork{});
         ws = 0;
         for (int i = 0; i < n; ++i) {
             const hcore_dense_task &t = tasks[i];
@@ -564,8 +551,8 @@ struct DensePrep {
                 }
                 groups[it->second].push_back(i);
             }
-            dims.push_back(make_int2(t.M, N));
-            DenseWork &w = work[i];
+            pr.add(DenseWork{}, t.M, N);
+            DenseWork &w = pr.work[i];
             w.ws = ws;
             w.beta = 1.0;
             if (t.kind <= 1) {
@@ -590,33 +577,22 @@ struct DensePrep {
                 }
             }
         }
+        pr.stage(DenseProducts::kBalanceByThread);
         for (int i : bdcd) {
             const hcore_dense_task &t = tasks[i];
             DenseWork w{};
             w.kk = t.kdim ? t.kdim : t.M;
             w.coef = 1.0;
             w.tr = 3;
-            work.push_back(w);
-            dims.push_back(make_int2(t.N ? t.N : t.M, t.a));
-            add_tile({(int)work.size() - 1});
+            pr.add_tile({pr.add(w, t.N ? t.N : t.M, t.a)});
         }
-        first_cols = (int)cols.size();
-        first_batches = (int)batches.size();
-        for (const auto &g : groups) add_tile(g);
-        auto place = [&](size_t &o, size_t bytes_) {
-            o = b_all;
-            b_all += al256(std::max<size_t>(bytes_, 1));
-        };
+        pr.stage(DenseProducts::kBalanceByWarp);
+        for (const auto &g : groups) pr.add_tile(g);
         b_all = al256(n * sizeof(hcore_dense_task));
-        place(o_work, work.size() * sizeof(DenseWork));
-        place(o_cols, cols.size() * sizeof(int2));
-        place(o_dims, dims.size() * sizeof(int2));
-        place(o_chunks, chunks.size() * sizeof(DenseChunk));
-        place(o_jobs, jobs.size() * sizeof(DenseJob));
-        place(o_ws, (size_t)ws * sizeof(double));
-        place(o_shift, cols.size() * sizeof(int));
-        place(o_exps, max_exps * sizeof(int));
-        place(o_slices, slice_bytes);
+        pr.place_host(b_all);
+        o_ws = b_all;
+        b_all += al256((size_t)ws * sizeof(double));
+        pr.place_device(b_all);
         const cudaError_t e = configure_dense_tc();
         if (e != cudaSuccess) {
             set_error("dense tasks: %s", cudaGetErrorString(e));
@@ -625,74 +601,22 @@ struct DensePrep {
         return HCORE_GPU_OK;
     }
 
-    // lay a tile's tasks out along K: a chunk ends after 128 columns, where a
-    // task scales CD, and where syrk tasks change to others (a run of syrk
-    // tasks may zero the strict upper triangle at its end: it writes nothing
-    // else there)
-    void add_tile(const std::vector<int> &g) {
-        const int2 mn = dims[g[0]];
-        const int first = (int)chunks.size();
-        auto open = [&](double beta, int syrk) {
-            chunks.push_back(DenseChunk{0, 0, 0, 0, (int)cols.size(), 0, mn.x, mn.y, beta, syrk,
-                                        beta == 1.0 ? 0 : (beta == 0.0 ? 2 : 1)});
-        };
-        for (size_t x = 0; x < g.size(); ++x) {
-            const DenseWork &w = work[g[x]];
-            if (x == 0 || w.beta != 1.0 || w.syrk != chunks.back().zero_upper) open(w.beta, w.syrk);
-            for (int l = 0; l < w.kk; ++l) {
-                if (chunks.back().ncol == 128) open(1.0, w.syrk);
-                cols.push_back(make_int2(g[x], l));
-                ++chunks.back().ncol;
-            }
-        }
-        const int tiles = dense_tiles(mn.x, mn.y);
-        // jobs: the tile's chunks, split where a batch's slice buffer is full
-        for (int c = first; c < (int)chunks.size(); ++c) {
-            DenseChunk &ch = chunks[c];
-            const size_t need = dense_slice_bytes(mn.x, mn.y, ch.ncol);
-            if ((int)batches.size() == first_batches || (cur_slices > 0 && cur_slices + need > kSliceBytes) ||
-                batches.back().ntiles > INT_MAX - tiles || batches.back().nchunks == 65535) {
-                batches.push_back(DenseBatch{(int)jobs.size(), 0, 0, c, 0, 1, 1});
-                cur_slices = cur_exps = 0;
-            }
-            DenseBatch &b = batches.back();
-            if (c == first || b.nchunks == 0) {
-                jobs.push_back(DenseJob{nullptr, 0, g[0], mn.x, mn.y, c, 0, b.ntiles});
-                ++b.njobs;
-                b.ntiles += tiles;
-            }
-            ++jobs.back().nchunks;
-            ++b.nchunks;
-            b.maxM = std::max(b.maxM, mn.x);
-            b.maxN = std::max(b.maxN, mn.y);
-            ch.p = (long long)cur_slices;
-            ch.q = ch.p + (long long)dense_slice_q_offset(mn.x, ch.ncol);
-            ch.ep = (int)cur_exps;
-            ch.eq = ch.ep + mn.x;
-            cur_slices += need;
-            cur_exps += (size_t)mn.x + mn.y;
-            slice_bytes = std::max(slice_bytes, cur_slices);
-            max_exps = std::max(max_exps, cur_exps);
-        }
-    }
-    size_t cur_slices = 0, cur_exps = 0;
-
     // point each product's P/Q at its inputs or at a computed factor in the
     // workspace that starts at d_ws, and each job at its output
     void bind(const hcore_dense_task *tasks, double *d_ws) {
         for (size_t q = 0; q < bdcd.size(); ++q) {
             const hcore_dense_task &t = tasks[bdcd[q]];
-            DenseWork &w = work[n + q];
+            DenseWork &w = pr.work[n + q];
             w.P = t.Bd; w.ldp = t.ldb; w.Q = t.Av; w.ldq = t.lda;
         }
-        for (DenseJob &j : jobs) {
+        for (DenseJob &j : pr.jobs) {
             const bool aux = j.task >= n;
-            j.cd = aux ? d_ws + work[bdcd[j.task - n]].ws : tasks[j.task].CD;
+            j.cd = aux ? d_ws + pr.work[bdcd[j.task - n]].ws : tasks[j.task].CD;
             j.ldcd = aux ? j.M : tasks[j.task].ldcd;
         }
         for (int i = 0; i < n; ++i) {
             const hcore_dense_task &t = tasks[i];
-            DenseWork &w = work[i];
+            DenseWork &w = pr.work[i];
             const int N = t.N ? t.N : t.M;
             if (t.kind == 2) {
                 w.P = t.Au; w.ldp = t.lda; w.Q = t.Bv; w.ldq = t.ldb;
@@ -714,41 +638,19 @@ struct DensePrep {
         }
     }
 
-    // copy tasks, work, the gemmbdcd list and the products' layout into `host`
-    // (pinned or not) laid out as the device arena's first ws_offset() bytes
+    // copy the tasks and the products' layout into `host` (pinned or not) laid
+    // out as the device arena's first ws_offset() bytes
     void pack(char *host, const hcore_dense_task *tasks) const {
-        auto put = [host](size_t o, const void *src, size_t bytes_) {
-            if (bytes_) memcpy(host + o, src, bytes_);
-        };
-        put(0, tasks, n * sizeof(hcore_dense_task));
-        put(o_work, work.data(), work.size() * sizeof(DenseWork));
-        put(o_cols, cols.data(), cols.size() * sizeof(int2));
-        put(o_dims, dims.data(), dims.size() * sizeof(int2));
-        put(o_chunks, chunks.data(), chunks.size() * sizeof(DenseChunk));
-        put(o_jobs, jobs.data(), jobs.size() * sizeof(DenseJob));
+        memcpy(host, tasks, n * sizeof(hcore_dense_task));
+        pr.pack(host);
     }
 
     cudaError_t launch(char *arena, cudaStream_t s) const {
-        const hcore_dense_task *d_tasks = (const hcore_dense_task *)arena;
-        const DenseWork *d_work = (const DenseWork *)(arena + o_work);
-        const int2 *d_cols = (const int2 *)(arena + o_cols);
-        int *d_shift = (int *)(arena + o_shift);
-        double *d_ws = (double *)(arena + o_ws);
-        cudaError_t e = maxM01 > 0 ? launch_dense_prep(d_tasks, d_work, n, maxM01, d_ws, s) : cudaSuccess;
-        // the products that make gemmbdcd's Q, then the tiles themselves
-        const int nc = (int)cols.size(), nb = (int)batches.size();
-        for (int stage = 0; stage < 2; ++stage) {
-            const int c0 = stage ? first_cols : 0, c1 = stage ? nc : first_cols;
-            if (e == cudaSuccess)
-                e = launch_dense_balance(d_work, d_cols + c0, (const int2 *)(arena + o_dims), c1 - c0,
-                                         stage == 0, d_shift + c0, s);
-            for (int b = stage ? first_batches : 0; b < (stage ? nb : first_batches); ++b)
-                if (e == cudaSuccess)
-                    e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
-                                              (const DenseJob *)(arena + o_jobs), batches[b],
-                                              (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), s);
-        }
-        return e;
+        const cudaError_t e =
+            maxM01 > 0 ? launch_dense_prep((const hcore_dense_task *)arena, pr.device_work(arena), n,
+                                           maxM01, (double *)(arena + o_ws), s)
+                       : cudaSuccess;
+        return e == cudaSuccess ? pr.launch(arena, s) : e;
     }
 };
 

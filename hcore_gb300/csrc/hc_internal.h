@@ -1,6 +1,7 @@
 // hcore-gb300 internal definitions shared by the kernels and the host API.
 #pragma once
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdint.h>
 
 #include "hcore_gb300.h"
@@ -26,8 +27,22 @@ struct Desc {
     int rule;            // rank rule bits (kRule*): 0 for HCORE_dgemm's rule
 };
 // rank rule bits of a descriptor: cap the rank at max_rank instead of
-// reporting RANK_MAX; compare with acc * sigma_max instead of acc
-constexpr int kRuleCapRank = 1, kRuleRelative = 2;
+// reporting RANK_MAX; compare with acc * sigma_max instead of acc; the update
+// is a compressed tile's range, whose core is deflated with the compressor's
+// error budget (kRangeShare)
+constexpr int kRuleCapRank = 1, kRuleRelative = 2, kRuleRange = 4;
+// The compressor's error budget delta (Frobenius) is shared by the range's
+// residual (0.8 delta) and the core's deflation (0.6 delta): the two errors
+// are orthogonal, so together they stay below delta.
+constexpr double kRangeShare = 0.8, kCoreShare = 0.6;
+// delta for a tile of Frobenius norm fro and order M: 1e-3 of the truncation
+// threshold (for the relative rule its lower bound acc fro / sqrt(M)), at least
+// what the arithmetic resolves
+__host__ __device__ inline double range_delta(double fro, int M, bool relative, double acc) {
+    const double d1 = 1e-3 * (relative ? acc * fro / sqrt((double)M) : acc);
+    const double d2 = 64.0 * 2.220446049250313e-16 * fro;
+    return d1 > d2 ? d1 : d2;
+}
 
 // Workspace layout of one update (element offsets from Desc::ws), k = a + c:
 //   UA  M*k   stacked [beta CU | alpha AU], then its QR (R on top, reflectors below)

@@ -518,7 +518,7 @@ __global__ void __launch_bounds__(kSvdMaxThreads) gesvd_kernel(const Desc *__res
     if (tid == 0) {
         T f2 = 0;   // ||T||_F^2 of the scaled T
         for (int c = 0; c < k; ++c) f2 += s_nrm[c];
-        s_defl2 = deflation_bound2(f2, k, d.rk, d.rule, d.acc, sexp);
+        s_defl2 = deflation_bound2(f2, k, M, d.rk, d.rule, d.acc, sexp);
     }
     int kk = k;   // columns of R^T that the Jacobi rotates
     // (the rank search keeps its first rank_start columns whatever their size)

@@ -1,0 +1,158 @@
+// hcore-gb300 — host side of the tensor-core products (hc_dense_tc.cu): lists of
+// products CD = beta CD + coef P Q^T, laid out as chunks, jobs and batches in
+// one arena and launched stage after stage.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <climits>
+#include <cstring>
+#include <vector>
+
+#include "hc_internal.h"
+
+namespace hc {
+
+struct DenseProducts {
+    // a batch's digit slices stay in the L2 (129 MB; the tiles pass through it
+    // too), and 96 MB more than that held costs 2.5%: 384 products of 1024 x
+    // 1024 x 17 took 2873, 2625, 2557, 2538 and 2493 us with limits of 16, 48,
+    // 96, 160 and 400 MB
+    size_t slice_limit = (size_t)96 << 20;
+    // how the columns of a stage's products are balanced: not at all (the
+    // caller's operands need none), a warp per column, or a thread per column
+    // (both operands stored transposed)
+    enum Balance { kNoBalance, kBalanceByWarp, kBalanceByThread };
+
+    std::vector<DenseWork> work;
+    std::vector<int2> dims;      // M, N of each product
+    std::vector<int2> cols;      // the K axes of all tiles: (product, its column)
+    std::vector<DenseChunk> chunks;
+    std::vector<DenseJob> jobs;
+    std::vector<DenseBatch> batches;
+
+    // a product; its kk columns are laid out by add_tile
+    int add(const DenseWork &w, int M, int N) {
+        work.push_back(w);
+        dims.push_back(make_int2(M, N));
+        return (int)work.size() - 1;
+    }
+
+    // the tiles added from here on run after those before
+    void stage(Balance b) { stages.push_back(Stage{(int)cols.size(), (int)batches.size(), b}); }
+
+    // lay a tile's tasks out along K: a chunk ends after 128 columns, where a
+    // task scales CD, and where syrk tasks change to others (a run of syrk
+    // tasks may zero the strict upper triangle at its end: it writes nothing
+    // else there)
+    void add_tile(const std::vector<int> &g) {
+        const int2 mn = dims[g[0]];
+        const int first = (int)chunks.size();
+        auto open = [&](double beta, int syrk) {
+            chunks.push_back(DenseChunk{0, 0, 0, 0, (int)cols.size(), 0, mn.x, mn.y, beta, syrk,
+                                        beta == 1.0 ? 0 : (beta == 0.0 ? 2 : 1)});
+        };
+        for (size_t x = 0; x < g.size(); ++x) {
+            const DenseWork &w = work[g[x]];
+            if (x == 0 || w.beta != 1.0 || w.syrk != chunks.back().zero_upper) open(w.beta, w.syrk);
+            for (int l = 0; l < w.kk; ++l) {
+                if (chunks.back().ncol == 128) open(1.0, w.syrk);
+                cols.push_back(make_int2(g[x], l));
+                ++chunks.back().ncol;
+            }
+        }
+        const int tiles = dense_tiles(mn.x, mn.y);
+        // jobs: the tile's chunks, split where a batch's slice buffer is full
+        for (int c = first; c < (int)chunks.size(); ++c) {
+            DenseChunk &ch = chunks[c];
+            const size_t need = dense_slice_bytes(mn.x, mn.y, ch.ncol);
+            if ((int)batches.size() == stages.back().batches0 ||
+                (cur_slices > 0 && cur_slices + need > slice_limit) || batches.back().ntiles > INT_MAX - tiles ||
+                batches.back().nchunks == 65535) {
+                batches.push_back(DenseBatch{(int)jobs.size(), 0, 0, c, 0, 1, 1});
+                cur_slices = cur_exps = 0;
+            }
+            DenseBatch &b = batches.back();
+            if (c == first || b.nchunks == 0) {
+                jobs.push_back(DenseJob{nullptr, 0, g[0], mn.x, mn.y, c, 0, b.ntiles});
+                ++b.njobs;
+                b.ntiles += tiles;
+            }
+            ++jobs.back().nchunks;
+            ++b.nchunks;
+            b.maxM = std::max(b.maxM, mn.x);
+            b.maxN = std::max(b.maxN, mn.y);
+            ch.p = (long long)cur_slices;
+            ch.q = ch.p + (long long)dense_slice_q_offset(mn.x, ch.ncol);
+            ch.ep = (int)cur_exps;
+            ch.eq = ch.ep + mn.x;
+            cur_slices += need;
+            cur_exps += (size_t)mn.x + mn.y;
+            slice_bytes = std::max(slice_bytes, cur_slices);
+            max_exps = std::max(max_exps, cur_exps);
+        }
+    }
+
+    // the arena: what pack() writes at `at`, and the device's own arrays
+    void place_host(size_t &at) {
+        place(at, o_work, work.size() * sizeof(DenseWork));
+        place(at, o_cols, cols.size() * sizeof(int2));
+        place(at, o_dims, dims.size() * sizeof(int2));
+        place(at, o_chunks, chunks.size() * sizeof(DenseChunk));
+        place(at, o_jobs, jobs.size() * sizeof(DenseJob));
+    }
+    void place_device(size_t &at) {
+        place(at, o_shift, cols.size() * sizeof(int));
+        place(at, o_exps, max_exps * sizeof(int));
+        place(at, o_slices, slice_bytes);
+    }
+    void pack(char *host) const {
+        auto put = [host](size_t o, const void *src, size_t bytes) {
+            if (bytes) memcpy(host + o, src, bytes);
+        };
+        put(o_work, work.data(), work.size() * sizeof(DenseWork));
+        put(o_cols, cols.data(), cols.size() * sizeof(int2));
+        put(o_dims, dims.data(), dims.size() * sizeof(int2));
+        put(o_chunks, chunks.data(), chunks.size() * sizeof(DenseChunk));
+        put(o_jobs, jobs.data(), jobs.size() * sizeof(DenseJob));
+    }
+    const DenseWork *device_work(const char *arena) const { return (const DenseWork *)(arena + o_work); }
+
+    cudaError_t launch(char *arena, cudaStream_t s) const {
+        const DenseWork *d_work = device_work(arena);
+        const int2 *d_cols = (const int2 *)(arena + o_cols), *d_dims = (const int2 *)(arena + o_dims);
+        int *d_shift = (int *)(arena + o_shift);
+        cudaError_t e = cudaSuccess;
+        for (size_t q = 0; q < stages.size() && e == cudaSuccess; ++q) {
+            const bool last = q + 1 == stages.size();
+            const int c0 = stages[q].cols0, c1 = last ? (int)cols.size() : stages[q + 1].cols0;
+            const int b1 = last ? (int)batches.size() : stages[q + 1].batches0;
+            if (stages[q].balance != kNoBalance)
+                e = launch_dense_balance(d_work, d_cols + c0, d_dims, c1 - c0,
+                                         stages[q].balance == kBalanceByThread, d_shift + c0, s);
+            else if (c1 > c0)
+                e = cudaMemsetAsync(d_shift + c0, 0, (size_t)(c1 - c0) * sizeof(int), s);
+            for (int b = stages[q].batches0; b < b1 && e == cudaSuccess; ++b)
+                e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
+                                          (const DenseJob *)(arena + o_jobs), batches[b],
+                                          (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), s);
+        }
+        return e;
+    }
+
+private:
+    struct Stage {
+        int cols0, batches0;
+        Balance balance;
+    };
+    std::vector<Stage> stages;
+    size_t slice_bytes = 0, max_exps = 0, cur_slices = 0, cur_exps = 0;
+    size_t o_work = 0, o_cols = 0, o_dims = 0, o_chunks = 0, o_jobs = 0, o_shift = 0, o_exps = 0, o_slices = 0;
+
+    static void place(size_t &at, size_t &o, size_t bytes) {
+        o = at;
+        at += (std::max<size_t>(bytes, 1) + 255) & ~(size_t)255;
+    }
+};
+
+}  // namespace hc

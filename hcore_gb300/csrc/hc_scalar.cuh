@@ -43,15 +43,19 @@ __device__ __forceinline__ T mul_exp2(T x, int n) {
 
 // Squared deflation bound of the SVD kernel's QR (described there): delta^2
 // for an FP64 update ranked by accuracy, -1 (no deflation) otherwise.  f2 is
-// ||T||_F^2 of T scaled by 2^-sexp.  One thread computes it once per update
-// (a warp-wide sum there cost the Jacobi loops registers).
+// ||T||_F^2 of T scaled by 2^-sexp.
 template <typename T>
-__device__ __forceinline__ T deflation_bound2(T f2, int k, int rk, int rule, double acc, int sexp) {
+__device__ __forceinline__ T deflation_bound2(T f2, int k, int M, int rk, int rule, double acc, int sexp) {
     if constexpr (sizeof(T) != sizeof(double)) {
         return T(-1);
     } else {
-        if (rk != 0 || !(acc > 0.0)) return T(-1);
         const T fro = sqrt(f2);
+        if (rule & kRuleRange) {
+            const T dl = kCoreShare * range_delta(
+                fro, M, rule & kRuleRelative, (rule & kRuleRelative) ? acc : mul_exp2(acc, -sexp));
+            return isfinite(dl) ? dl * dl : T(-1);
+        }
+        if (rk != 0 || !(acc > 0.0)) return T(-1);
         const T thr = (rule & kRuleRelative) ? (T)acc * fro * rsqrt(T(k)) : mul_exp2((T)acc, -sexp);
         const T dl = min(T(1e-13) * thr, T(1e-16) * fro);
         return isfinite(dl) ? dl * dl : T(-1);

@@ -308,7 +308,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     // squared deflation bound (see gesvd_kernel), the same in every thread
     T f2 = 0;
     for (int c = lane; c < k; c += 32) f2 += X0[c];
-    const T defl2 = deflation_bound2(warp_sum(f2), k, d.rk, d.rule, d.acc, sexp);
+    const T defl2 = deflation_bound2(warp_sum(f2), k, M, d.rk, d.rule, d.acc, sexp);
     const int kfloor = d.rank_start < k ? (d.rank_start > 0 ? d.rank_start : 0) : k;
 
     // ---- QR with column pivoting, T P = Q R ------------------------------------
