@@ -118,8 +118,8 @@ struct LaunchShape {
     // FP64 plans: the rebuild of updates with k <= kTcMaxK on the tensor cores
     // (hc_rebuild_tc.cu); off: the DFMA reflector kernel for every update
     bool tc_rebuild = true;
-    // FP64 plans: the QR of updates with k <= kTcMaxK blocked, with the
-    // trailing updates on the tensor cores; off: the unblocked FP64 kernel
+    // FP64 plans: the QR blocked, with the trailing updates on the tensor
+    // cores; off: the unblocked FP64 kernel
     bool tc_qr = true;
     // FP64 plans, opt-in (HCORE_GPU_TC_STACK): the stack's products F and G on
     // the tensor cores for updates that stack_tc_eligible accepts
@@ -168,8 +168,8 @@ constexpr int kTcMaxK = 64;
 // kernel launches of the rebuild phase of one execute (hc_kernels.cu)
 int rebuild_launches(const LaunchShape &shape, bool fp64);
 
-// Blocked QR (FP64 plans, a + c <= kTcMaxK): 16-column panels factored by the
-// FP64 register kernel, the last panel taking the rest when it is at most 20
+// Blocked QR (FP64 plans): 16-column panels factored by the FP64 register
+// kernel, the last panel taking the rest when it is at most 20
 // columns wide (on the TLR panel workload the QR phase took 10.7, 10.1, 9.85
 // and 10.1 ms with limits 32, 24, 20 and 16); between panels the trailing
 // columns are updated on the tensor cores (hc_qr_tc.cu).  Returns false when
@@ -181,13 +181,13 @@ __host__ __device__ inline bool qr_panel_bounds(int k, int p, int &c0, int &c1) 
     c1 = p < q ? c0 + 16 : k;
     return true;
 }
-constexpr int kQrPanels = 4;  // panels of the widest blocked QR (k = 64)
+constexpr int kQrGroup = 48;  // trailing columns of one update CTA
 // tensor-core trailing update: variant by 16 + (columns right of the panel)
-// rounded up (32, 48 or 64; 0 above 64); launches only
+// rounded up (32, 48, or 64: groups of kQrGroup columns); launches only
 int qr_update_class(int rows);
 cudaError_t configure_qr_tc();
 void launch_qr_update_tc(const Desc *d_desc, int n, double *ws, int panel, int *d_status,
-                         int rclass, cudaStream_t s);
+                         int rclass, int groups, cudaStream_t s);
 // kernel launches of the QR phase of one execute (hc_kernels.cu)
 int qr_launches(const LaunchShape &shape, bool fp64);
 

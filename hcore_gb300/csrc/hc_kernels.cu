@@ -14,9 +14,10 @@
 //   4. apply  (hcore_dgemm.c:508-696) CU = Q_A [U_r; 0], CV = Q_B [V_r S_r; 0]
 //              written straight into the caller's output factors
 //
-// In FP64 plans with a + c <= 64 the QR runs blocked, its trailing updates on
-// the tensor cores (hc_qr_tc.cu), and the rebuild runs there too
-// (hc_rebuild_tc.cu); this file keeps the panels and every other case.
+// In FP64 plans the QR runs blocked, its trailing updates on the tensor cores
+// (hc_qr_tc.cu); the rebuild of updates with a + c <= 64 runs there too
+// (hc_rebuild_tc.cu), and the SVD of those whose core fits shared memory in
+// hc_svd.cu; this file keeps the panels and every other case.
 //
 // The scalar type T is double (HCORE_dgemm) or float (HCORE_sgemm); every
 // step computes in T, like the reference's two copies.  With the plan flag
@@ -55,71 +56,128 @@ __device__ __forceinline__ float flip_sign(float x) {
 // ---------------------------------------------------------------------------
 // phase 1: stack the factors
 // ---------------------------------------------------------------------------
-// tc_products: the products F and G of updates that stack_tc_eligible
-// accepts are left to the tensor-core kernel (hc_stack_tc.cu)
+// Two kernels: the copies [beta CU | alpha AU], [CV | .] and F = AV^T BV, then
+// G = BU F^T (or B AV for a dense B).  Both are bound by FP64 issue, so a warp
+// takes four entries of F at a time (one load of BV's column for four FMAs, six
+// shuffled additions for the four sums instead of twenty), and an update's
+// columns and rows are split over CTAs until the GPU is full.  On one CTA each,
+// and now: one update of M = 512 and ranks 32 405, 74 us; 384 of M = 1024,
+// ranks 6-34, 1648, 720 us; 24 of M = 1000, ranks 40-110, 6.7, 0.83 ms.
+// tc_products: the products F and G of updates that stack_tc_eligible accepts
+// are left to the tensor-core kernel (hc_stack_tc.cu).
 template <typename T, typename Tc>
-__global__ void __launch_bounds__(kThreads) stack_kernel(const Desc *__restrict__ descs,
-                                                         T *__restrict__ ws, bool tc_products) {
+__global__ void __launch_bounds__(kThreads) stack_inner_kernel(const Desc *__restrict__ descs,
+                                                               T *__restrict__ ws, bool tc_products) {
     const Desc d = descs[blockIdx.x];
     if (d.status0) return;
     const int M = d.M, a = d.a, b = d.b, c = d.c;
     const WsLayout L = ws_layout(d);
-    T *UA = ws + d.ws + L.UA;
-    T *VB = ws + d.ws + L.VB;
-    T *F = ws + d.ws + L.F;
+    T *UA = ws + d.ws + L.UA, *VB = ws + d.ws + L.VB, *F = ws + d.ws + L.F;
     const T alpha = (T)d.alpha, beta = (T)d.beta;
-    const T *CU = (const T *)d.CU, *CV = (const T *)d.CV;
-    const T *AU = (const T *)d.AU, *AV = (const T *)d.AV;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int lane = threadIdx.x & 31;
+    const int warp = blockIdx.y * kWarps + (threadIdx.x >> 5), nwarps = gridDim.y * kWarps;
 
-    // [beta*CU | alpha*AU] and [CV | .] (hcore_dgemm.c:106-114, :199-205).
-    // The Schur update's coefficients 1 and -1 are applied without an FP64
-    // instruction (a copy, a sign-bit flip on the integer pipe): same bits.
+    // [beta*CU | alpha*AU] and [CV | .] (hcore_dgemm.c:106-114, :199-205), a
+    // warp per column.  The Schur update's coefficients 1 and -1 are applied
+    // without an FP64 instruction (a copy, a sign-bit flip on the integer
+    // pipe): same bits.
     const bool beta_one = beta == T(1), alpha_minus_one = alpha == T(-1);
-    for (long long e = tid; e < (long long)M * c; e += kThreads) {
-        const int i = (int)(e % M), j = (int)(e / M);
-        const T x = CU[(size_t)j * d.ldc + i];
-        UA[(size_t)j * M + i] = beta_one ? x : beta * x;
-        VB[(size_t)j * M + i] = CV[(size_t)j * d.ldc + i];
-    }
-    for (long long e = tid; e < (long long)M * a; e += kThreads) {
-        const int i = (int)(e % M), j = (int)(e / M);
-        const T x = AU[(size_t)j * d.lda + i];
-        UA[(size_t)(c + j) * M + i] = alpha_minus_one ? flip_sign(x) : alpha * x;
-    }
-    if (a == 0 || (tc_products && stack_tc_eligible(d))) return;
-    T *G = VB + (size_t)c * M;
-    if (d.Bd) {
-        // dense B: G = B * AV (hcore_dgemm.c:262-271)
-        const T *B = (const T *)d.Bd;
-        for (long long e = tid; e < (long long)M * a; e += kThreads) {
-            const int i = (int)(e % M), j = (int)(e / M);
-            Tc s = 0;
-            for (int l = 0; l < M; ++l)
-                s += (Tc)B[(size_t)l * d.ldb + i] * (Tc)AV[(size_t)j * d.lda + l];
-            G[(size_t)j * M + i] = (T)s;
+    for (int q = warp; q < 2 * c + a; q += nwarps) {
+        const T *src;
+        T *dst;
+        if (q < c) {
+            src = (const T *)d.CU + (size_t)q * d.ldc;
+            dst = UA + (size_t)q * M;
+        } else if (q < 2 * c) {
+            src = (const T *)d.CV + (size_t)(q - c) * d.ldc;
+            dst = VB + (size_t)(q - c) * M;
+        } else {
+            src = (const T *)d.AU + (size_t)(q - 2 * c) * d.lda;
+            dst = UA + (size_t)(q - c) * M;
         }
-        return;
+        if (q >= c && q < 2 * c) {
+#pragma unroll 4
+            for (int i = lane; i < M; i += 32) dst[i] = src[i];
+        } else if (q < c) {
+#pragma unroll 4
+            for (int i = lane; i < M; i += 32) dst[i] = beta_one ? src[i] : beta * src[i];
+        } else {
+#pragma unroll 4
+            for (int i = lane; i < M; i += 32) dst[i] = alpha_minus_one ? flip_sign(src[i]) : alpha * src[i];
+        }
     }
-    const T *BU = (const T *)d.BU, *BV = (const T *)d.BV;
-    // F = AV^T BV, a x b, one warp per entry (hcore_dgemm.c:175-178)
-    for (int e = warp; e < a * b; e += kWarps) {
-        const int p = e % a, q = e / a;
-        const T *x = AV + (size_t)p * d.lda;
+    if (a == 0 || d.Bd || (tc_products && stack_tc_eligible(d))) return;
+    // F = AV^T BV, a x b (hcore_dgemm.c:175-178)
+    const T *AV = (const T *)d.AV, *BV = (const T *)d.BV;
+    const int quads = (a + 3) / 4;
+    for (int e = warp; e < quads * b; e += nwarps) {
+        const int p0 = e % quads * 4, q = e / quads;
         const T *y = BV + (size_t)q * d.ldb;
-        Tc s = 0;
-        for (int l = lane; l < M; l += 32) s += (Tc)x[l] * (Tc)y[l];
-        s = warp_sum(s);
-        if (lane == 0) F[(size_t)q * a + p] = (T)s;
+        const T *x[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) x[u] = AV + (size_t)min(p0 + u, a - 1) * d.lda;
+        Tc s[4] = {};
+#pragma unroll 2
+        for (int l = lane; l < M; l += 32) {
+            const Tc yv = (Tc)y[l];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) s[u] += (Tc)x[u][l] * yv;
+        }
+        // lanes 8 u .. 8 u + 7 end with sum u
+        const bool h16 = lane & 16, h8 = lane & 8;
+        const Tc s0 = (h16 ? s[2] : s[0]) + __shfl_xor_sync(0xffffffffu, h16 ? s[0] : s[2], 16);
+        const Tc s1 = (h16 ? s[3] : s[1]) + __shfl_xor_sync(0xffffffffu, h16 ? s[1] : s[3], 16);
+        Tc r = (h8 ? s1 : s0) + __shfl_xor_sync(0xffffffffu, h8 ? s0 : s1, 8);
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+        const int p = p0 + (lane >> 3);
+        if ((lane & 7) == 0 && p < a) F[(size_t)q * a + p] = (T)r;
     }
-    __syncthreads();
-    // G = BU F^T, M x a (hcore_dgemm.c:199-205)
-    for (long long e = tid; e < (long long)M * a; e += kThreads) {
-        const int i = (int)(e % M), p = (int)(e / M);
-        Tc s = 0;
-        for (int q = 0; q < b; ++q) s += (Tc)BU[(size_t)q * d.ldb + i] * (Tc)F[(size_t)q * a + p];
-        G[(size_t)p * M + i] = (T)s;
+}
+
+// G (M x a): a thread per row, four columns at a time
+template <typename T, typename Tc>
+__global__ void __launch_bounds__(128) stack_outer_kernel(const Desc *__restrict__ descs,
+                                                          T *__restrict__ ws, bool tc_products) {
+    const Desc d = descs[blockIdx.x];
+    if (d.status0) return;
+    const int M = d.M, a = d.a, b = d.b, i = blockIdx.y * 128 + threadIdx.x;
+    if (i >= M || a == 0 || (tc_products && stack_tc_eligible(d))) return;
+    const WsLayout L = ws_layout(d);
+    const T *F = ws + d.ws + L.F;
+    T *G = ws + d.ws + L.VB + (size_t)d.c * M;
+    for (int p0 = 0; p0 < a; p0 += 4) {
+        Tc s[4] = {};
+        if (d.Bd) {   // dense B: G = B * AV (hcore_dgemm.c:262-271)
+            const T *B = (const T *)d.Bd + i, *AV = (const T *)d.AV;
+#pragma unroll 4
+            for (int l = 0; l < M; ++l) {
+                const Tc x = (Tc)B[(size_t)l * d.ldb];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] += x * (Tc)AV[(size_t)min(p0 + u, a - 1) * d.lda + l];
+            }
+        } else {      // G = BU F^T (hcore_dgemm.c:199-205)
+            const T *BU = (const T *)d.BU + i;
+#pragma unroll 4
+            for (int q = 0; q < b; ++q) {
+                const Tc x = (Tc)BU[(size_t)q * d.ldb];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) s[u] += x * (Tc)F[(size_t)q * a + min(p0 + u, a - 1)];
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (p0 + u < a) G[(size_t)(p0 + u) * M + i] = (T)s[u];
     }
+}
+
+template <typename T, typename Tc>
+static void launch_stack(const Desc *d_desc, int n, T *ws, bool tc_products, int updates, int maxM,
+                         cudaStream_t s) {
+    // eight CTAs an SM's worth over the updates that share the GPU
+    const int split = std::max(1, std::min(32, 1216 / std::max(updates, 1)));
+    stack_inner_kernel<T, Tc><<<dim3(n, split), kThreads, 0, s>>>(d_desc, ws, tc_products);
+    stack_outer_kernel<T, Tc><<<dim3(n, (maxM + 127) / 128), 128, 0, s>>>(d_desc, ws, tc_products);
 }
 
 // ---------------------------------------------------------------------------
@@ -1048,34 +1106,39 @@ static void launch_geqrf_all(const Desc *d_desc, int n, T *ws, int warps, int rp
     else launch_geqrf<T, 64>(d_desc, n, ws, warps, panel, s);
 }
 
-// Launch plan of the blocked QR over a shape's k-sorted buckets: the
-// descriptors above kTcMaxK (a prefix) take the unblocked kernel; for the
-// rest, panel p runs over every descriptor that has one, and the trailing
-// update after panel p once per update-size class.  fn(kind, start, count,
-// panel, class): kind 0 unblocked QR, 1 panel, 2 trailing update.
+// Launch plan of the blocked QR over a shape's k-sorted buckets: panel p runs
+// over every descriptor that has one, and the trailing update after panel p
+// once per update-size class.  fn(kind, start, count, panel, class, groups):
+// kind 1 panel, 2 trailing update.
+//
+// Every rank sum takes it: a column's update by one reflector is 2 M FP64 FMAs
+// on the register kernel, while the update by a panel of 16 is a sixteenth of
+// one pass over the column on the tensor cores.  QR phase of 24 updates of M =
+// 1000 and k 80-220 25.5 ms unblocked, 5.4 blocked; of 384 of M = 1024 and k
+// 12-68 5.06 ms with k > 64 unblocked, 3.17 (one GB300, graph replay).
 template <typename F>
 static void qr_plan(const LaunchShape &shape, int n, F &&fn) {
-    int split = 0;  // first descriptor with k <= kTcMaxK
-    int b = 0;
-    while (b < shape.nbuckets && shape.buckets[b].K > kTcMaxK) split += shape.buckets[b++].count;
-    if (split > 0) fn(0, 0, split, -1, 0);
-    if (split >= n || b >= shape.nbuckets) return;
-    const int kmax = shape.buckets[b].K;
-    for (int p = 0; p < kQrPanels; ++p) {
+    if (n <= 0 || shape.nbuckets <= 0) return;
+    const int kmax = shape.buckets[0].K;
+    for (int p = 0;; ++p) {
         int c0, c1;
         if (!qr_panel_bounds(kmax, p, c0, c1)) break;
-        fn(1, split, n - split, p, 0);
+        // descriptors below the buckets that have this panel exit at once
+        int count = 0;
+        for (int b = 0; b < shape.nbuckets && qr_panel_bounds(shape.buckets[b].K, p, c0, c1); ++b)
+            count += shape.buckets[b].count;
+        fn(1, 0, count, p, 0, 1);
         // trailing updates: descriptors whose panel p is not their last
-        int bb = b, start = split;
+        int bb = 0, start = 0;
         while (bb < shape.nbuckets) {
             const int K = shape.buckets[bb].K;
             if (!qr_panel_bounds(K, p, c0, c1) || c1 >= K) break;  // sorted: none below
-            const int cls = qr_update_class(K - 16 * p);
-            int count = 0;
+            const int cls = qr_update_class(K - 16 * p), groups = (K - c1 + kQrGroup - 1) / kQrGroup;
+            count = 0;
             while (bb < shape.nbuckets && qr_panel_bounds(shape.buckets[bb].K, p, c0, c1) &&
                    c1 < shape.buckets[bb].K && qr_update_class(shape.buckets[bb].K - 16 * p) == cls)
                 count += shape.buckets[bb++].count;
-            if (count > 0) fn(2, start, count, p, cls);
+            if (count > 0) fn(2, start, count, p, cls, groups);
             start += count;
         }
     }
@@ -1086,7 +1149,7 @@ int qr_launches(const LaunchShape &shape, bool fp64) {
     int c = 0;
     int n = 0;
     for (int b = 0; b < shape.nbuckets; ++b) n += shape.buckets[b].count;
-    qr_plan(shape, n, [&](int, int, int count, int, int) { c += count > 0; });
+    qr_plan(shape, n, [&](int, int, int count, int, int, int) { c += count > 0; });
     return c;
 }
 
@@ -1173,20 +1236,20 @@ cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int
     const bool mixed = shape.mixed && sizeof(T) == sizeof(double);
     if (phases & kPhaseStack) {
         if (mixed) {
-            stack_kernel<T, float><<<n, kThreads, 0, s>>>(d_desc, ws, false);
+            launch_stack<T, float>(d_desc, n, ws, false, shape.updates, maxM, s);
         } else {
             const bool tcs = sizeof(T) == sizeof(double) && shape.tc_stack;
-            stack_kernel<T, T><<<n, kThreads, 0, s>>>(d_desc, ws, tcs);
+            launch_stack<T, T>(d_desc, n, ws, tcs, shape.updates, maxM, s);
             if (tcs) launch_stack_tc(d_desc, n, (double *)ws, d_status, s);
         }
     }
     if (phases & kPhaseQR) {
         const int qw = shape.qr_warps;
         if (sizeof(T) == sizeof(double) && shape.tc_qr && shape.nbuckets > 0) {
-            qr_plan(shape, n, [&](int kind, int start, int count, int p, int cls) {
+            qr_plan(shape, n, [&](int kind, int start, int count, int p, int cls, int groups) {
                 if (count <= 0) return;
                 if (kind == 2)
-                    launch_qr_update_tc(d_desc + start, count, (double *)ws, p, d_status, cls, s);
+                    launch_qr_update_tc(d_desc + start, count, (double *)ws, p, d_status, cls, groups, s);
                 else
                     launch_geqrf_all<T>(d_desc + start, count, ws, qw, rpl, p, s);
             });

@@ -828,8 +828,8 @@ extern "C" int hcore_gpu_plan_launches(hcore_gpu_plan p) {
     if (!p || p->n == 0) return 0;
     const bool fp64 = p->prec == HCORE_GPU_F64;
     auto count = [fp64](const LaunchShape &sh) {
-        // stack (and its tensor-core products), QR, SVD buckets, rebuild
-        int c = 1 + (fp64 && sh.tc_stack && !sh.mixed) + qr_launches(sh, fp64) +
+        // stack (two, and its tensor-core products), QR, SVD buckets, rebuild
+        int c = 2 + (fp64 && sh.tc_stack && !sh.mixed) + qr_launches(sh, fp64) +
                 rebuild_launches(sh, fp64);
         for (int b = 0; b < sh.nbuckets; ++b) c += sh.buckets[b].count > 0;
         return c;

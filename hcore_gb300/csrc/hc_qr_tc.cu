@@ -19,7 +19,8 @@
 // (hc_digits.cuh); the FP64 pipe does the 16-row forward substitution and one
 // subtraction per updated entry.
 //
-// One CTA (8 warps) per (update, side) and panel.  Scales: Householder
+// One CTA (8 warps) per (update, side), panel and group of up to 48 trailing
+// columns (each forms the panel's 16 x 16 Gram matrix for itself).  Scales: Householder
 // vectors take 2^1 (|y| <= 1), each trailing column of A_t and each column of
 // W' its own power of two.
 #include "hc_digits.cuh"
@@ -103,8 +104,10 @@ __global__ void __maxnreg__(128)
     if (d.status0) return;
     const int M = d.M, k = d.k;
     int c0, c1;
-    if (!qr_panel_bounds(k, panel, c0, c1) || c1 >= k) return;
-    const int nt = k - c1;                      // 5 .. 48 trailing columns
+    if (!qr_panel_bounds(k, panel, c0, c1)) return;
+    c1 += kQrGroup * blockIdx.z;                // this CTA's trailing columns: c1 ..
+    if (c1 >= k) return;
+    const int nt = min(kQrGroup, k - c1);
     const int side = blockIdx.y;
     const WsLayout L = ws_layout(d);
     double *A = ws + d.ws + (side ? L.VB : L.UA);
@@ -400,8 +403,7 @@ cudaError_t set_qr_smem() {
 int qr_update_class(int rows) {
     if (rows <= 32) return 32;
     if (rows <= 48) return 48;
-    if (rows <= 64) return 64;
-    return 0;
+    return 64;
 }
 
 cudaError_t configure_qr_tc() {
@@ -412,9 +414,9 @@ cudaError_t configure_qr_tc() {
 }
 
 void launch_qr_update_tc(const Desc *d_desc, int n, double *ws, int panel, int *d_status,
-                         int rclass, cudaStream_t s) {
+                         int rclass, int groups, cudaStream_t s) {
     if (n <= 0) return;
-    const dim3 grid(n, 2);
+    const dim3 grid(n, 2, groups);
     if (rclass == 32)
         qr_update_tc_kernel<32><<<grid, kQThreads, QrCfg<32>::kSmem, s>>>(d_desc, ws, panel,
                                                                          d_status);
