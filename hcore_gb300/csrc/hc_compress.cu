@@ -695,7 +695,7 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             LaunchShape shape;
             shape.maxM = pM;
             shape.maxK = maxK;
-            shape.updates = nd;
+            shape.updates = shape.big_updates = nd;
             fill_buckets(descs, shape);
             e = cudaMemcpyAsync(d_desc, descs.data(), nd * sizeof(Desc), cudaMemcpyHostToDevice, s);
             if (e == cudaSuccess)
@@ -704,7 +704,7 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
                 compress_form_kernel<<<nd, 256, 0, s>>>(d_fw);
                 e = cudaGetLastError();
             }
-            if (e == cudaSuccess) e = configure_recompress<double>(maxK, &shape.svd_smem_kmax, &shape.svd_half_kmax);
+            if (e == cudaSuccess) e = configure_recompress<double>(maxK, &shape.svd_smem_kmax);
             if (e == cudaSuccess)
                 e = launch_recompress<double>(d_desc, nd, pws, d_rank, d_status, nullptr, shape, s,
                                               kPhaseQR | kPhaseSVD | kPhaseApply);

@@ -260,7 +260,7 @@ struct Single {
         // one update alone: its latency is the call's, so the QR CTAs take
         // eight warps
         shape.qr_warps = 8;
-        cudaError_t e = configure_recompress<T>(k, &shape.svd_smem_kmax, &shape.svd_half_kmax);
+        cudaError_t e = configure_recompress<T>(k, &shape.svd_smem_kmax);
         if (e == cudaSuccess)
             e = launch_recompress<T>(d_desc, 1, ws, d_rs, d_rs + 1, nullptr, shape, tc.stream,
                                      phases);

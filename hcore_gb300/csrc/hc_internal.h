@@ -49,15 +49,16 @@ __host__ __device__ inline double range_delta(double fro, int M, bool relative, 
 //   VB  M*k   stacked [CV | G], then its QR
 //   tauA k, tauB k, sig k
 //   F   a*b   AV^T BV
-//   W   k*k   Jacobi working matrix (used when it does not fit shared memory)
-//   V   k*k   Jacobi right vectors (same)
+//   W   k*k   T, its QR, then V_J (when they do not fit shared memory)
+//   V   k*k   R^T, rotated (same)
+//   sv  4k+16 column norms and scales (same)
 //   Uo  k*k   U_r (k x r, ld k); the SVD's QR reflectors until U_r is written
 //   Vo  k*k   V_r S_r (k x r, ld k)
 // U_r and V_r S_r are kept for an update whose rank exceeds its storage
 // limit too, so that it can be rebuilt into larger storage without being
 // recompressed (hcore_gpu_plan_rebuild).
 struct WsLayout {
-    long long UA, VB, tauA, tauB, sig, F, W, V, Uo, Vo, total;
+    long long UA, VB, tauA, tauB, sig, F, W, V, sv, Uo, Vo, total;
 };
 
 __host__ __device__ inline long long hc_align32(long long x) { return (x + 31) & ~31LL; }
@@ -74,6 +75,7 @@ __host__ __device__ inline WsLayout ws_layout(int M, int a, int b, int k) {
     L.F = o; o = hc_align32(o + (long long)a * b);
     L.W = o; o = hc_align32(o + (long long)k * k);
     L.V = o; o = hc_align32(o + (long long)k * k);
+    L.sv = o; o = hc_align32(o + 4LL * k + 16);
     L.Uo = o; o = hc_align32(o + (long long)k * u);
     L.Vo = o; o = hc_align32(o + (long long)k * u);
     L.total = o;
@@ -101,9 +103,6 @@ struct Bucket {
 };
 struct LaunchShape {
     int maxM = 1, maxK = 1, svd_smem_kmax = 0;
-    // largest k whose R^T alone fits shared memory (the SVD's mode with V_J
-    // in the workspace); 0: that mode is not used
-    int svd_half_kmax = 0;
     // most output columns an accepted update may have, max of
     // min(k, storage_rank): the rebuild's grid (0: maxK)
     int maxR = 0;
@@ -112,6 +111,7 @@ struct LaunchShape {
     // share the GPU); rank-bucket edge spacing
     int svd_lanes[3] = {-1, -1, -1};
     int updates = 1;
+    int big_updates = 1;   // those whose SVD does not fit shared memory
     int bucket_width = 8;
     int qr_warps = 4;   // warps per QR CTA (2, 4 or 8)
     bool mixed = false;  // FP32 factor products and rebuild (HCORE_GPU_MIXED_FACTORS)
@@ -139,7 +139,7 @@ int bucket_edge(int k, int width);
 // (not capturable) and returns the largest k whose Jacobi matrices fit in
 // shared memory; launch_recompress only launches (capturable).
 template <typename T>
-cudaError_t configure_recompress(int maxK, int *svd_smem_kmax, int *svd_half_kmax = nullptr);
+cudaError_t configure_recompress(int maxK, int *svd_smem_kmax);
 template <typename T>
 cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status,
                               int *d_info, const LaunchShape &shape, cudaStream_t s,
@@ -153,6 +153,11 @@ cudaError_t configure_svd_smem(int optin, int *kmax);
 template <typename T>
 void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
                      int G, cudaStream_t s);
+// SVD of larger updates: a cluster of CTAs each, sized for `updates` of them on
+// the GPU (hc_svd.cu)
+template <typename T>
+cudaError_t launch_svd_cluster(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info,
+                               int K, int updates, cudaStream_t s);
 // rebuild phase only, for listed updates whose status is STORAGE (set to
 // OK; d_cap, if not null, caps their rank)
 template <typename T>

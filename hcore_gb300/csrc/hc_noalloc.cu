@@ -28,7 +28,7 @@ namespace hc {
 
 // workspace capacity in doubles: M = 1024 rows with a + c <= 128 and
 // a*b <= 128*128 fit (ws_layout(1024, 128, 128, 128, no storage limit) is
-// 344448 doubles)
+// 344992 doubles)
 constexpr long long kNoAllocWsElems = 393216;                // 3 MiB
 constexpr size_t kNoAllocDescOff = kNoAllocWsElems * sizeof(double);
 constexpr size_t kNoAllocRankOff = kNoAllocDescOff + 512;   // rank, status
@@ -51,8 +51,7 @@ __global__ void noalloc_setup_kernel(Desc d) {
 constexpr int kNoAllocMaxDevices = 64;
 struct NoAllocDevice {
     unsigned char *addr = nullptr;  // device address of g_noalloc_scratch
-    int svd_smem_kmax = 0;          // SVD shared-memory limits on this device
-    int svd_half_kmax = 0;
+    int svd_smem_kmax = 0;          // SVD shared-memory limit on this device
 };
 static std::mutex g_noalloc_mu;
 static NoAllocDevice g_noalloc_dev[kNoAllocMaxDevices];
@@ -71,11 +70,10 @@ static cudaError_t noalloc_device(NoAllocDevice *out) {
         void *p = nullptr;
         e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess) return e;
-        int kmax = 0, khalf = 0;
-        e = configure_recompress<double>(kMaxK, &kmax, &khalf);
+        int kmax = 0;
+        e = configure_recompress<double>(kMaxK, &kmax);
         if (e != cudaSuccess) return e;
         d.svd_smem_kmax = kmax;
-        d.svd_half_kmax = khalf;
         d.addr = static_cast<unsigned char *>(p);
     }
     *out = d;
@@ -155,7 +153,6 @@ extern "C" int hcore_gpu_dgemm_noalloc(int M, double alpha, const double *AU, co
     shape.nbuckets = 1;
     shape.buckets[0] = Bucket{0, 1, k};
     shape.svd_smem_kmax = nd.svd_smem_kmax;
-    shape.svd_half_kmax = nd.svd_half_kmax;
     noalloc_setup_kernel<<<1, 32, 0, s>>>(d);
     e = cudaGetLastError();
     int *rs = reinterpret_cast<int *>(base + kNoAllocRankOff);

@@ -642,6 +642,460 @@ size_t smem_bytes(int K) {
            (size_t)2 * (K + 1) * sizeof(short) + 16;
 }
 
+
+// ---- larger cores: a cluster per update ----------------------------------------
+// k beyond shared memory (119 in FP64, 168 in FP32) up to kMaxK.  The matrices
+// sit in the workspace (L2-resident), column-major, and the CTAs of a cluster
+// share an update: columns (QR with column pivoting, norms, U_r), column pairs
+// (Jacobi), rows (T).  What one of them writes the others read after a cluster
+// barrier, past the L1 (ld.global.cg).  The arithmetic is the shared-memory
+// kernel's.
+//
+// What bounds it: a Jacobi round is 5 k FP64 FMAs per pair, 22 instructions of
+// rotation parameters and a barrier, and the FP64 pipe of one SM made it 38 us
+// at k = 220 (one CTA, 440 threads); over eight SMs it is about 7.  G lanes
+// hold a pair's two columns of B and of V_J in registers, R rows each, loaded
+// once a round, so that L2 latency is paid once.
+// SVD phase with one CTA per update (1024 threads, R^T in shared memory up to k =
+// 167) and now: 3 updates of k 160-220 65.1, 9.8 ms; 24 of k 80-220 57.1, 11.8;
+// 40 of k 200-256 109, 60; 6 of k 360-500 508, 90; 200 of k 120-140, where one
+// CTA an update fills the GPU either way, 32.1, 34.6 (their whole plan 52.4,
+// 45.8).
+constexpr int kClThreads = 256, kClMax = 8;
+
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+template <typename T, int G, int R>
+__global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
+    svd_cluster_kernel(const Desc *__restrict__ descs, T *__restrict__ ws, int *__restrict__ rank,
+                       int *__restrict__ status, int *__restrict__ info) {
+    __shared__ T s_tau[kMaxK], s_rdiag[kMaxK], s_sig[kMaxK];
+    __shared__ short s_perm[kMaxK], s_pcol[kMaxK];
+    __shared__ T s_wmax[kClThreads / 32];
+    __shared__ int s_rank;
+    unsigned cr, cs;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(cr));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(cs));
+    const Desc d = descs[blockIdx.x / cs];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, lig = tid & (G - 1);
+    const bool first = cr == 0 && tid == 0;
+    if (d.status0) {
+        if (first) {
+            status[d.idx] = d.status0;
+            rank[d.idx] = 0;
+            if (info) info[d.idx] = 0;
+        }
+        return;
+    }
+    const int M = d.M, k = d.k;
+    const WsLayout L = ws_layout(d);
+    T *base = ws + d.ws;
+    const T *UA = base + L.UA, *VB = base + L.VB;
+    T *A = base + L.W, *B = base + L.V;   // T, its QR, V_J; R^T, rotated (ld k)
+    T *X0 = base + L.sv, *X1 = X0 + k, *s_d = X1 + k, *s_rd = s_d + k, *slots = s_rd + k;
+    T *Yg = base + L.Uo;
+    // this thread's warp and group among the cluster's
+    const int gw = (int)cr * (kClThreads / 32) + warp, ngw = (int)cs * (kClThreads / 32);
+    const int gg = ((int)cr * kClThreads + tid) / G, ngg = (int)cs * kClThreads / G;
+    auto sum_group = [](T v) {
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        return v;
+    };
+    // rows lig, lig + G, ... of a column, zero outside [lo, hi)
+    auto load = [&](T (&x)[R], const T *col, int lo, int hi, bool act) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = lig + G * r;
+            x[r] = act && i >= lo && i < hi ? __ldcg(col + i) : T(0);
+        }
+    };
+    auto store = [&](const T (&x)[R], T *col, int lo, int hi) {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+            const int i = lig + G * r;
+            if (i >= lo && i < hi) col[i] = x[r];
+        }
+    };
+    auto dot = [&](const T (&x)[R], const T (&y)[R]) {
+        T a0 = 0, a1 = 0;
+#pragma unroll
+        for (int r = 0; r < R; r += 2) {
+            a0 += x[r] * y[r];
+            a1 += x[r + 1] * y[r + 1];
+        }
+        return sum_group(a0 + a1);
+    };
+
+    // ---- T = triu(R_A) triu(R_B)^T: a warp per row, 32 columns at a time -----------
+    T amax = 0;
+    bool bad = false;
+    for (int i = gw; i < k; i += ngw)
+        for (int c = 0; c < k; c += 32) {
+            const int j = c + lane, jr = min(j, k - 1);
+            T s0 = 0, s1 = 0;
+            int l = max(i, c);
+#pragma unroll 4
+            for (; l + 1 < k; l += 2) {
+                s0 += UA[(size_t)l * M + i] * (l >= jr ? VB[(size_t)l * M + jr] : T(0));
+                s1 += UA[(size_t)(l + 1) * M + i] * (l + 1 >= jr ? VB[(size_t)(l + 1) * M + jr] : T(0));
+            }
+            if (l < k) s0 += UA[(size_t)l * M + i] * (l >= jr ? VB[(size_t)l * M + jr] : T(0));
+            s0 += s1;
+            if (j < k) {
+                A[(size_t)j * k + i] = s0;
+                amax = max(amax, abs(s0));
+                bad = bad || !isfinite(s0);
+            }
+        }
+    amax = warp_max(amax);
+    if (lane == 0) s_wmax[warp] = amax;
+    const bool cta_bad = __syncthreads_or(bad);
+    if (tid == 0) {
+        for (int w = 1; w < kClThreads / 32; ++w) amax = max(amax, s_wmax[w]);
+        slots[cr] = cta_bad ? T(-1) : amax;
+    }
+    cluster_sync();
+    amax = 0;
+    bad = false;
+    for (unsigned q = 0; q < cs; ++q) {
+        const T x = __ldcg(slots + q);
+        bad = bad || x < T(0);
+        amax = max(amax, x);
+    }
+    if (bad) {   // a NaN or infinity: no decomposition; the update is not written
+        if (cr == 0)
+            for (int t = tid; t < k; t += kClThreads) base[L.sig + t] = T(NAN);
+        if (first) {
+            int r = d.rk != 0 && d.rk < k ? d.rk : k;
+            if ((d.rule & kRuleCapRank) && r > d.max_rank) r = d.max_rank;
+            rank[d.idx] = r;
+            status[d.idx] = HCORE_GPU_S_NOCONV;
+            if (info) info[d.idx] = 0;
+        }
+        return;
+    }
+    const int sexp = amax > T(0) ? binary_exponent(amax) : 0;
+    // scaled columns, their squared norms
+    for (int c0 = 0; c0 < k; c0 += ngg) {
+        const int c = c0 + gg;
+        T x[R];
+        load(x, A + (size_t)c * k, 0, k, c < k);
+#pragma unroll
+        for (int r = 0; r < R; ++r) x[r] = mul_exp2(x[r], -sexp);
+        const T s = dot(x, x);
+        if (c < k) {
+            store(x, A + (size_t)c * k, 0, k);
+            if (lig == 0) {
+                X0[c] = s;
+                s_d[c] = s;
+            }
+        }
+    }
+    cluster_sync();
+    T f2 = 0;
+    for (int c = lane; c < k; c += 32) f2 += __ldcg(X0 + c);
+    const T defl2 = deflation_bound2(warp_sum(f2), k, M, d.rk, d.rule, d.acc, sexp);
+    const int kfloor = d.rank_start < k ? (d.rank_start > 0 ? d.rank_start : 0) : k;
+
+    // ---- QR with column pivoting (as in svd_smem_kernel) ---------------------------
+    int kk = k;
+    for (int j = 0; j < k; ++j) {
+        const T *nr = (j & 1) ? X1 : X0;
+        T *nr2 = (j & 1) ? X0 : X1;
+        auto best = key(T(-1));
+        int pv = 0;
+#pragma unroll 4
+        for (int c = lane; c < k; c += 32) {
+            const auto x = key(__ldcg(nr + c));
+            if (x > best) {
+                best = x;
+                pv = c;
+            }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const auto ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, pv, o);
+            if (ob > best || (ob == best && oi < pv)) {
+                best = ob;
+                pv = oi;
+            }
+        }
+        if (j >= kfloor && defl2 >= T(0) && best <= key(defl2)) {
+            T tail = 0;
+            for (int c = lane; c < k; c += 32) tail += max(__ldcg(nr + c), T(0));
+            if (warp_sum(tail) <= defl2) {
+                kk = j;
+                break;
+            }
+        }
+        T p[R];
+        load(p, A + (size_t)pv * k, j + 1, k, true);
+        const T alpha = __ldcg(A + (size_t)pv * k + j), ss = dot(p, p);
+        T beta = alpha, vj = 0, ginv = 0;
+        if (ss > SvLim<T>::safmin) {
+            const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
+            T nb = n2 * rs;
+            nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
+            beta = -copysign(nb, alpha);
+            vj = alpha - beta;
+            ginv = inv(fma(-alpha, beta, n2));
+        }
+        if (tid == 0) {
+            s_pcol[j] = (short)pv;
+            s_rdiag[j] = beta;
+            s_tau[j] = ginv;
+        }
+        for (int c0 = 0; c0 < k; c0 += ngg) {
+            const int c = c0 + gg;
+            const T nc = c < k ? __ldcg(nr + c) : T(-1);
+            const bool act = c < k && c != pv && key(nc) >= 0;
+            T *ac = A + (size_t)c * k;
+            T x[R];
+            load(x, ac, j + 1, k, act);
+            const T acj = act ? __ldcg(ac + j) : T(0);
+            const T s = ginv * fma(vj, acj, dot(x, p));
+            T nn = 0;
+            bool redo = false;
+            if (act) {
+                if (ginv != T(0)) {
+#pragma unroll
+                    for (int r = 0; r < R; ++r) x[r] -= s * p[r];
+                    store(x, ac, j + 1, k);
+                }
+                const T r = ginv != T(0) ? acj - s * vj : acj;
+                if (lig == 0 && ginv != T(0)) ac[j] = r;
+                nn = nc - r * r;
+                redo = !(key(nn) > 0) || below_pow2(nn, __ldcg(s_d + c), 10);
+            }
+            if (__any_sync(0xffffffffu, redo)) {
+                const T q = dot(x, x);
+                if (redo) {
+                    nn = q;
+                    if (lig == 0) s_d[c] = q;
+                }
+            }
+            if (c < k && lig == 0) nr2[c] = act ? nn : T(-1);
+        }
+        cluster_sync();
+    }
+    if (kk < k) {   // columns that the deflation left: positions kk.. in column order
+        const T *nr = (kk & 1) ? X1 : X0;
+        for (int c = tid; c < k; c += kClThreads)
+            if (key(__ldcg(nr + c)) >= 0) {
+                int pos = kk;
+                for (int q = 0; q < c; ++q) pos += key(__ldcg(nr + q)) >= 0;
+                s_pcol[pos] = (short)c;
+            }
+    }
+    __syncthreads();
+    for (int h = gw; h < k; h += ngw) {
+        const T *ah = A + (size_t)s_pcol[h] * k;
+        for (int i = lane; i < k; i += 32) {
+            const T x = __ldcg(ah + i);
+            if (h < kk) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rdiag[h] : T(0));
+            B[(size_t)i * k + h] = i < kk ? (i < h ? x : (i == h ? s_rdiag[h] : T(0))) : T(0);
+        }
+    }
+    cluster_sync();
+    for (int c = gw; c < k; c += ngw)
+        for (int i = lane; i < k; i += 32) A[(size_t)c * k + i] = i == c ? T(1) : T(0);
+    T *s_nrm = X0;
+    auto column_norms = [&](bool fold) {
+        for (int c0 = 0; c0 < k; c0 += ngg) {
+            const int c = c0 + gg;
+            T dj = fold && c < kk ? __ldcg(s_d + c) : T(1);
+            T x[R];
+            load(x, B + (size_t)c * k, 0, k, c < kk);
+            if (fold && c < kk && dj < SvLim<T>::tiny_scale) {   // fold a scale before it underflows
+                T v[R];
+                load(v, A + (size_t)c * k, 0, k, true);
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    x[r] *= dj;
+                    v[r] *= dj;
+                }
+                store(x, B + (size_t)c * k, 0, k);
+                store(v, A + (size_t)c * k, 0, k);
+                dj = 1;
+            }
+            const T s = dot(x, x);
+            if (c < k && lig == 0) {
+                s_nrm[c] = c < kk ? dj * dj * s : T(0);
+                s_d[c] = dj;
+                s_rd[c] = fold && c < kk ? inv(dj) : T(1);
+            }
+        }
+    };
+    column_norms(false);
+    cluster_sync();
+
+    // ---- one-sided Jacobi ------------------------------------------------------------
+    const int n = kk + (kk & 1), np = n / 2;
+    const float tol = (float)(k > 8 ? k : 8) * (sizeof(T) == 8 ? (float)DBL_EPSILON : FLT_EPSILON);
+    bool converged = kk <= 1;
+    int sweeps = 0;
+    for (; sweeps < kMaxSweeps && !converged; ++sweeps) {
+        bool big = false;
+        for (int round = 0; round < n - 1; ++round) {
+            for (int b0 = 0; b0 < np; b0 += ngg) {
+                const int pi = b0 + gg;
+                int p = round + pi, q = round - pi;
+                if (p >= n - 1) p -= n - 1;
+                if (q < 0) q += n - 1;
+                if (pi == 0) p = n - 1;
+                const bool valid = pi < np && p < kk && q < kk;
+                T *xp = B + (size_t)p * k, *xq = B + (size_t)q * k;
+                T *vp = A + (size_t)p * k, *vq = A + (size_t)q * k;
+                T x[R], y[R], v[R], w[R];
+                load(x, xp, 0, k, valid);
+                load(y, xq, 0, k, valid);
+                load(v, vp, 0, kk, valid);
+                load(w, vq, 0, kk, valid);
+                T app = 0, aqq = 0, dp = 1, dq = 1, rdp = 1, rdq = 1;
+                if (valid) {
+                    app = __ldcg(s_nrm + p);
+                    aqq = __ldcg(s_nrm + q);
+                    dp = __ldcg(s_d + p);
+                    dq = __ldcg(s_d + q);
+                    rdp = sizeof(T) == 8 ? __ldcg(s_rd + p) : T(1) / dp;
+                    rdq = sizeof(T) == 8 ? __ldcg(s_rd + q) : T(1) / dq;
+                }
+                const T dt = dot(x, y);
+                bool rot = false, redo_p = false, redo_q = false;
+                T np_ = 0, nq_ = 0, cs_ = 1, ics = 1;
+                if (valid) {
+                    const T apq = (dp * dq) * dt;
+                    bool bigp = false;
+                    rot = key(app) > key(SvLim<T>::safmin) && key(aqq) > key(SvLim<T>::safmin) &&
+                          pair_test(app, aqq, apq, tol, bigp);
+                    if (rot) {
+                        big |= bigp;
+                        const T t = tangent(app, aqq, apq);
+                        const T u = fma(t, t, T(1));
+                        cs_ = inv_sqrt(u);
+                        ics = u * cs_;
+                        const T f1 = t * (dq * rdp), f2 = t * (dp * rdq);
+                        np_ = app - t * apq;
+                        nq_ = aqq + t * apq;
+                        redo_p = below_pow2(np_, app, 6);
+                        redo_q = below_pow2(nq_, aqq, 6);
+#pragma unroll
+                        for (int r = 0; r < R; ++r) {
+                            const T a = x[r], c = v[r];
+                            x[r] = a - f1 * y[r];
+                            y[r] = y[r] + f2 * a;
+                            v[r] = c - f1 * w[r];
+                            w[r] = w[r] + f2 * c;
+                        }
+                        store(x, xp, 0, k);
+                        store(y, xq, 0, k);
+                        store(v, vp, 0, kk);
+                        store(w, vq, 0, kk);
+                    }
+                }
+                const T dp2 = dp * cs_, dq2 = dq * cs_;
+                if (__any_sync(0xffffffffu, redo_p || redo_q)) {
+                    const T sp = dot(x, x), sq = dot(y, y);
+                    if (redo_p) np_ = dp2 * dp2 * sp;
+                    if (redo_q) nq_ = dq2 * dq2 * sq;
+                }
+                if (rot && lig == 0) {
+                    s_nrm[p] = np_;
+                    s_nrm[q] = nq_;
+                    s_d[p] = dp2;
+                    s_d[q] = dq2;
+                    s_rd[p] = rdp * ics;
+                    s_rd[q] = rdq * ics;
+                }
+            }
+            cluster_sync();
+        }
+        column_norms(true);
+        const bool cta_big = __syncthreads_or(big);
+        if (tid == 0) slots[(sweeps & 1) * kClMax + cr] = cta_big ? T(1) : T(0);
+        cluster_sync();
+        converged = true;
+        for (unsigned q = 0; q < cs; ++q)
+            if (__ldcg(slots + (sweeps & 1) * kClMax + q) != T(0)) converged = false;
+    }
+
+    // singular values, order and rank (as in svd_smem_kernel, in every CTA)
+    bool nonfinite = false;
+    for (int j = tid; j < k; j += kClThreads) {
+        const T s = sqrt(__ldcg(s_nrm + j));
+        nonfinite = nonfinite || !isfinite(s);
+        s_sig[j] = s == s ? s : T(-1);
+    }
+    if (tid == 0) s_rank = k;
+    const bool finite = !__syncthreads_or(nonfinite);
+    for (int j = tid; j < k; j += kClThreads) {
+        const auto sj = key(s_sig[j]);
+        int pos = 0;
+        for (int i = 0; i < k; ++i) {
+            const auto si = key(s_sig[i]);
+            pos += (si > sj) || (si == sj && i < j);
+        }
+        s_perm[pos] = (short)j;
+    }
+    __syncthreads();
+    const T thr = (d.rule & kRuleRelative) ? (T)d.acc * mul_exp2(s_sig[s_perm[0]], sexp) : (T)d.acc;
+    for (int t = tid; t < k; t += kClThreads) {
+        const T s = s_sig[s_perm[t]];
+        const T v = key(s) < 0 ? T(NAN) : mul_exp2(s, sexp);
+        if (cr == 0) base[L.sig + t] = v;
+        if (d.rk == 0 && t >= d.rank_start && v < thr) atomicMin(&s_rank, t);
+    }
+    __syncthreads();
+    int r = d.rk != 0 ? (d.rk < k ? d.rk : k) : s_rank;
+    if ((d.rule & kRuleCapRank) && r > d.max_rank) r = d.max_rank;
+    int st = HCORE_GPU_S_OK;
+    if (!converged || !finite) st = HCORE_GPU_S_NOCONV;
+    else if (r > d.max_rank) st = HCORE_GPU_S_RANK_MAX;
+    else if (r > d.storage_rank) st = HCORE_GPU_S_STORAGE;
+    if (first) {
+        rank[d.idx] = r;
+        status[d.idx] = st;
+        if (info) info[d.idx] = sweeps;
+    }
+    if (st != HCORE_GPU_S_OK && st != HCORE_GPU_S_STORAGE) return;
+    T *Uo = base + L.Uo, *Vo = base + L.Vo;
+    for (int t = gw; t < r; t += ngw) {
+        const int j = s_perm[t];
+        const T f = __ldcg(s_d + j);
+        for (int i = lane; i < k; i += 32)
+            Vo[(size_t)t * k + s_pcol[i]] = mul_exp2(f * __ldcg(B + (size_t)j * k + i), sexp);
+    }
+    cluster_sync();
+    // the reflectors leave the slot that U_r is written to
+    for (int h = gw; h < kk; h += ngw)
+        for (int i = lane; i < k; i += 32) B[(size_t)h * k + i] = __ldcg(Yg + (size_t)h * k + i);
+    cluster_sync();
+    for (int t0 = 0; t0 < r; t0 += ngg) {
+        const int t = t0 + gg;
+        const bool act = t < r;
+        const int j = act ? s_perm[t] : 0;
+        T x[R], y[R];
+        load(x, A + (size_t)j * k, 0, k, act);
+        const T dj = act ? __ldcg(s_d + j) : T(0);
+#pragma unroll
+        for (int q = 0; q < R; ++q) x[q] *= dj;
+        for (int h = kk - 1; h >= 0; --h) {
+            const T gi = s_tau[h];
+            if (gi == T(0)) continue;
+            load(y, B + (size_t)h * k, h, k, true);
+            const T s = gi * dot(y, x);
+#pragma unroll
+            for (int q = 0; q < R; ++q) x[q] -= s * y[q];
+        }
+        if (act) store(x, Uo + (size_t)t * k, 0, k);
+    }
+}
+
 }  // namespace
 
 template <typename T>
@@ -683,11 +1137,43 @@ void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_statu
     else launch_svd_g<T, 1>(d_desc, n, ws, d_rank, d_status, d_info, K, s);
 }
 
+// One cluster per update: as many CTAs (a power of two, at most eight, the
+// portable limit) as give every update's cluster its own SMs.
+template <typename T>
+cudaError_t launch_svd_cluster(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info,
+                               int K, int updates, cudaStream_t s) {
+    unsigned cs = 1;
+    while (cs < kClMax && 2 * cs * (unsigned)(updates > n ? updates : n) <= 152) cs *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n * cs);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    // rows past k cost instructions: the smallest G x R that holds them
+    auto go = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, d_info); };
+    if (K <= 160) return go(svd_cluster_kernel<T, 16, 10>);
+    if (K <= 224) return go(svd_cluster_kernel<T, 16, 14>);
+    if (K <= 256) return go(svd_cluster_kernel<T, 32, 8>);
+    if (K <= 384) return go(svd_cluster_kernel<T, 32, 12>);
+    return go(svd_cluster_kernel<T, 32, 16>);
+}
+
 template cudaError_t configure_svd_smem<double>(int, int *);
 template cudaError_t configure_svd_smem<float>(int, int *);
 template void launch_svd_smem<double>(const Desc *, int, double *, int *, int *, int *, int, int,
                                       cudaStream_t);
 template void launch_svd_smem<float>(const Desc *, int, float *, int *, int *, int *, int, int,
                                      cudaStream_t);
+
+template cudaError_t launch_svd_cluster<double>(const Desc *, int, double *, int *, int *, int *, int, int,
+                                                cudaStream_t);
+template cudaError_t launch_svd_cluster<float>(const Desc *, int, float *, int *, int *, int *, int, int,
+                                               cudaStream_t);
 
 }  // namespace hc
