@@ -19,6 +19,11 @@ bool build_descs(int n, const hcore_lr_task *tasks, unsigned flags, bool transla
                  std::vector<Desc> &descs, long long &ws_elems, int &maxM, int &maxK,
                  std::vector<int> *status0);
 
+// hcore_gpu_plan_create_tuned (tuning may be null); without `groups` the plan
+// has no stream groups, for callers that only execute it directly
+int plan_create(hcore_gpu_plan *plan, int precision, int n, const hcore_lr_task *tasks, unsigned flags,
+                const hcore_gpu_tuning *tuning, bool groups);
+
 // Per-thread execution context of the drop-in entry points: a non-blocking
 // stream, a growable device arena and a growable pinned staging buffer.  The
 // reference is reentrant (every call mallocs its own buffers), so HiCMA calls

@@ -120,7 +120,7 @@ extern "C" int hcore_gpu_tlr_panel_step(const hcore_tlr_matrix *A, int k, double
         }
     hcore_gpu_plan plan = nullptr;
     if (!lr.empty()) {
-        rc = hcore_gpu_plan_create(&plan, HCORE_GPU_F64, (int)lr.size(), lr.data(), 0);
+        rc = plan_create(&plan, HCORE_GPU_F64, (int)lr.size(), lr.data(), 0, nullptr, false);
         if (rc) return rc;
         rc = hcore_gpu_plan_execute(plan, stream);
         if (rc) {

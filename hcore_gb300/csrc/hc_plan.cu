@@ -202,7 +202,8 @@ struct hcore_gpu_plan_s {
     };
     std::vector<Group> groups;
     cudaEvent_t gfork = nullptr;
-    Desc *d_desc = nullptr;
+    Desc *d_desc = nullptr;     // dealt into the groups
+    Desc *d_sorted = nullptr;   // by decreasing k (the same array without groups)
     int *d_rank = nullptr;
     int *d_status = nullptr;
     int *d_info = nullptr;  // Jacobi sweeps per task
@@ -430,6 +431,7 @@ static void plan_free(hcore_gpu_plan p) {
     if (p->gfork) cudaEventDestroy(p->gfork);
     for (cudaEvent_t ev : p->stacked)
         if (ev) cudaEventDestroy(ev);
+    if (p->d_sorted != p->d_desc) cudaFree(p->d_sorted);
     cudaFree(p->d_desc);
     cudaFree(p->d_rank);
     cudaFree(p->d_status);
@@ -468,12 +470,18 @@ static bool valid_tuning(const hcore_gpu_tuning &t) {
 
 extern "C" int hcore_gpu_plan_create(hcore_gpu_plan *plan, int precision, int n,
                                      const hcore_lr_task *tasks, unsigned flags) {
-    return hcore_gpu_plan_create_tuned(plan, precision, n, tasks, flags, nullptr);
+    return hc::plan_create(plan, precision, n, tasks, flags, nullptr, true);
 }
 
 extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, int n,
                                            const hcore_lr_task *tasks, unsigned flags,
                                            const hcore_gpu_tuning *tuning) {
+    return hc::plan_create(plan, precision, n, tasks, flags, tuning, true);
+}
+
+// `groups`: create the stream groups that a captured execute uses
+int hc::plan_create(hcore_gpu_plan *plan, int precision, int n, const hcore_lr_task *tasks,
+                    unsigned flags, const hcore_gpu_tuning *tuning, bool groups) {
     if (!plan || n < 0 || (n > 0 && !tasks) ||
         (precision != HCORE_GPU_F64 && precision != HCORE_GPU_F32)) {
         set_error("hcore_gpu_plan_create: invalid argument");
@@ -511,7 +519,8 @@ extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, 
     build_descs(n, tasks, flags, true, descs, ws_elems, p->maxM, p->maxK, nullptr);
     // stream groups (HCORE_GPU_STREAMS, default 16): deal the k-sorted
     // descriptors round-robin so every group gets the same mix of sizes
-    int ngroups = std::max(1, std::min(tune.stream_groups, n > 0 ? n : 1));
+    const int ngroups = groups ? std::max(1, std::min(tune.stream_groups, n > 0 ? n : 1)) : 1;
+    const std::vector<Desc> sorted = descs;
     p->phase_sync = tune.phase_sync != 0;
     auto set_shape_tuning = [&](LaunchShape &sh) {
         for (int q = 0; q < 3 && tuning; ++q) sh.svd_lanes[q] = tune.svd_lanes[q];
@@ -560,21 +569,20 @@ extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, 
             plan_free(p);
             return HCORE_GPU_ECUDA;
         }
-    } else {
-        fill_buckets(descs, p->shape);
-        p->shape.maxM = p->maxM;
-        p->shape.maxK = p->maxK;
-        if (p->shape.nbuckets > 1) {
-            bool ok = cudaEventCreateWithFlags(&p->shape.fork, cudaEventDisableTiming) == cudaSuccess;
-            for (int b = 0; ok && b < p->shape.nbuckets; ++b)
-                ok = cudaStreamCreateWithFlags(&p->shape.side[b], cudaStreamNonBlocking) ==
-                         cudaSuccess &&
-                     cudaEventCreateWithFlags(&p->shape.join[b], cudaEventDisableTiming) == cudaSuccess;
-            if (!ok) {
-                set_error("hcore_gpu_plan_create: cannot create bucket streams");
-                plan_free(p);
-                return HCORE_GPU_ECUDA;
-            }
+    }
+    // the plan as one group: its SVD buckets run concurrently
+    fill_buckets(sorted, p->shape);
+    p->shape.maxM = p->maxM;
+    p->shape.maxK = p->maxK;
+    if (p->shape.nbuckets > 1) {
+        bool ok = cudaEventCreateWithFlags(&p->shape.fork, cudaEventDisableTiming) == cudaSuccess;
+        for (int b = 0; ok && b < p->shape.nbuckets; ++b)
+            ok = cudaStreamCreateWithFlags(&p->shape.side[b], cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&p->shape.join[b], cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) {
+            set_error("hcore_gpu_plan_create: cannot create bucket streams");
+            plan_free(p);
+            return HCORE_GPU_ECUDA;
         }
     }
     p->ws_of_task.assign(n, -1);
@@ -622,6 +630,8 @@ extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, 
     p->ws_bytes = (size_t)ws_elems * esz;
     const size_t nn = (size_t)(n > 0 ? n : 1);
     cudaError_t e = cudaMalloc(&p->d_desc, nn * sizeof(Desc));
+    if (e == cudaSuccess && !p->groups.empty()) e = cudaMalloc(&p->d_sorted, nn * sizeof(Desc));
+    if (p->groups.empty()) p->d_sorted = p->d_desc;
     if (e == cudaSuccess) e = cudaMalloc(&p->d_rank, nn * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&p->d_status, nn * sizeof(int));
     if (e == cudaSuccess) e = cudaMalloc(&p->d_info, nn * sizeof(int));
@@ -635,6 +645,8 @@ extern "C" int hcore_gpu_plan_create_tuned(hcore_gpu_plan *plan, int precision, 
     }
     if (n > 0) {
         e = cudaMemcpy(p->d_desc, descs.data(), n * sizeof(Desc), cudaMemcpyHostToDevice);
+        if (e == cudaSuccess && p->d_sorted != p->d_desc)
+            e = cudaMemcpy(p->d_sorted, sorted.data(), n * sizeof(Desc), cudaMemcpyHostToDevice);
         if (e == cudaSuccess) e = cudaMemset(p->d_rank, 0, n * sizeof(int));
         if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, n * sizeof(int));
         if (e == cudaSuccess) e = cudaMemset(p->d_info, 0, n * sizeof(int));
@@ -671,8 +683,21 @@ extern "C" int hcore_gpu_plan_execute_phases(hcore_gpu_plan p, void *stream, uns
                    : launch_recompress<float>(dd, cnt, (float *)p->d_ws, p->d_rank, p->d_status,
                                               p->d_info, sh, st, ph & kPhaseAll);
     };
-    if (p->groups.empty()) {
-        e = launch(p->d_desc, p->n, p->shape, s, phases);
+    // Stream groups let a CUDA graph overlap one update's phases with another's.
+    // Launched directly they lose: the streams share a few hardware queues, in
+    // which one group's chain waits behind another's, and every group repeats
+    // the launches.  Direct and captured executes with 1 and 16 groups, us (one
+    // GB300): 16 updates of k 8-24 521, 731 and 504, 474; 200 of k 12-68 5918,
+    // 31926 and 5955, 4853; 1900 17473, 34184 and 17925, 15528; 24 of k 80-220
+    // 22639, 44163 and 25450, 20142.  So the groups are for captured executes.
+    bool capturing = false;
+    if (!p->groups.empty() && s != nullptr) {   // (the default stream is never captured)
+        cudaStreamCaptureStatus cst = cudaStreamCaptureStatusNone;
+        if (cudaStreamIsCapturing(s, &cst) != cudaSuccess) cudaGetLastError();
+        capturing = cst == cudaStreamCaptureStatusActive;
+    }
+    if (!capturing) {
+        e = launch(p->d_sorted, p->n, p->shape, s, phases);
     } else if (p->phase_sync) {
         // every group finishes a phase before any group starts the next
         const unsigned order[4] = {kPhaseStack, kPhaseQR, kPhaseSVD, kPhaseApply};
@@ -918,7 +943,7 @@ extern "C" int hcore_gpu_plan_destroy(hcore_gpu_plan p) {
 static int batched_once(int prec, int n, const hcore_lr_task *tasks, int *ranks, int *status,
                         void *stream) {
     hcore_gpu_plan p = nullptr;
-    int rc = hcore_gpu_plan_create(&p, prec, n, tasks, 0);
+    int rc = hc::plan_create(&p, prec, n, tasks, 0, nullptr, false);
     if (rc) return rc;
     rc = hcore_gpu_plan_execute(p, stream);
     if (!rc) rc = hcore_gpu_plan_results(p, ranks, status, stream);

@@ -151,8 +151,8 @@ int hcore_gpu_plan_rebuild(hcore_gpu_plan plan, int n, const int *task_idx, void
 int hcore_gpu_plan_sigma(hcore_gpu_plan plan, int i, double *sigma, int *k, void *stream);
 /* Jacobi sweeps each task's SVD took (diagnostics; valid after execute) */
 int hcore_gpu_plan_sweeps(hcore_gpu_plan plan, int *sweeps, void *stream);
-/* kernel launches one execute makes (stack, QR, one SVD launch per rank
- * bucket, rebuild; per stream group) */
+/* kernel launches one captured execute makes (stack, QR, one SVD launch per
+ * rank bucket, rebuild; per stream group) */
 int hcore_gpu_plan_launches(hcore_gpu_plan plan);
 /* bytes of device workspace the plan holds */
 size_t hcore_gpu_plan_workspace_bytes(hcore_gpu_plan plan);
@@ -164,7 +164,9 @@ size_t hcore_gpu_plan_zero_copy_bytes(hcore_gpu_plan plan);
 int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
 
 /* Launch-shape tuning of a plan (no counterpart in the reference).
- *   stream_groups      updates are dealt into this many concurrent groups
+ *   stream_groups      updates are dealt into this many concurrent groups when
+ *                      an execute is captured in a CUDA graph; a direct execute
+ *                      runs each phase over all updates at once
  *   svd_lanes[3]       lanes per column pair of the shared-memory SVD buckets
  *                      with <= 24, <= 64 and more column pairs (1..32, a
  *                      power of two; 0: as many as fit in the warps that one
