@@ -1,11 +1,39 @@
-// hcore-gb300 — the core SVD of an update whose two k x k Jacobi matrices fit
-// one SM's shared memory (k <= 119 in FP64, 168 in FP32): T = R_A R_B^T, QR
-// with column pivoting, one-sided Jacobi, rank rule, U_r and V_r S_r
-// (reference step: src/compute/hcore_dgemm.c:296-503, __svd).
+// hcore-gb300 — the core SVD of an update: T = R_A R_B^T (k x k), QR with column
+// pivoting, one-sided Jacobi, rank rule, U_r and V_r S_r (reference step:
+// src/compute/hcore_dgemm.c:296-503, __svd).  Two kernels: svd_smem_kernel, one
+// CTA, both k x k matrices in its shared memory (k <= 119 in FP64, 168 in FP32),
+// and svd_cluster_kernel for larger k.
 //
-// The method is the one of the workspace kernel (gesvd_kernel in
-// hc_kernels.cu: Drmac-Veselic preconditioning, scaled rotations, deflation);
-// this kernel is written for latency, because a CTA's serial chain of Jacobi
+// Method (QR-preconditioned one-sided Jacobi, Drmac and Veselic 2008): T P = Q R
+// with column pivoting, then one-sided Jacobi on R^T, whose columns are graded
+// by the pivoting, so the sweeps are few.  With R^T V_J = U' S (U' orthonormal),
+// T = (Q V_J) S (P U')^T, hence U_T = Q V_J (V_J accumulated by the rotations)
+// and V_T S = P (R^T V_J).  The rotations are scaled ("fast"): column j is d_j
+// x_j in both R^T and V_J, so a rotation costs two FMAs per row and matrix.
+// Squared norms are tracked (exact in exact arithmetic), recomputed on strong
+// cancellation and after every sweep.  A pair is rotated when a_pq^2 > tol^2 a_pp
+// a_qq, tol = k eps (LAPACK dgesvj's criterion); the sweeps stop after one whose
+// largest relative off-diagonal was at most sqrt(tol): cyclic Jacobi converges
+// quadratically, so the next would only rotate by angles near tol.
+//
+// Deflation (FP64 updates ranked by accuracy): the QR stops at the first step j
+// whose trailing block R22 = R(j:k, j:k) has ||R22||_F <= delta, and the Jacobi
+// runs on the first j rows of R only.  Dropping R22 moves every singular value
+// by at most delta (Weyl), with delta = min(1e-13 thr, 1e-16 ||T||_F), thr the
+// truncation threshold (acc, or for the relative rule its lower bound acc
+// ||T||_F / sqrt(k)): a rank decision can change only for a singular value within
+// 1e-13 of the threshold, relative, and every singular value stays within a few
+// eps sigma_max of the full one (the accuracy of dgesvd's small singular
+// values).  The dropped directions come out with singular value 0.  (The core
+// of a compressed tile's range has the compressor's larger budget, kCoreShare.)
+//
+// Range safety (as LAPACK's dgesvd scales the matrix first): T is scaled by 2^-e
+// so that its largest entry lies in [1, 2) (exact; the singular values and V S
+// are scaled back by 2^e), and a column whose squared norm is below safmin is
+// negligible (< 2^-485 relative in FP64, 2^-51 in FP32) and not rotated.  A
+// non-finite T or singular value marks the update NOCONV.
+//
+// svd_smem_kernel is written for latency, because a CTA's serial chain of Jacobi
 // rounds and QR steps is what the SVD phase waits for.  One FP64 warp
 // instruction holds a sub-partition's FP64 pipe for about 64 cycles and a
 // dependent one cannot start earlier, so what counts is the number of FP64
@@ -25,7 +53,8 @@
 //     finds the pivot and builds the reflector itself, so a step has one
 //     barrier; G lanes share a column there and in U_r = Q V_J as in the
 //     Jacobi.
-// SVD phase, before (two and, alone, four lanes per pair) and now, one GB300,
+// SVD phase, with the kernel before (its parameters about 65 FP64 instructions a
+// round, two and, alone, four lanes per pair) and now, one GB300,
 // us: one update of k = 64 2388 -> 1453; 16 of k 8-24 485 -> 250; 384 of k
 // 12-68 4524 -> 3220; 1900 of the same 7272 -> 5747; FP32, 256 of k 10-48
 // 1139 -> 1050.  What bounds it now is the FP64 pipe of the one SM: in a round
@@ -305,7 +334,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
         }
     }
     __syncthreads();
-    // squared deflation bound (see gesvd_kernel), the same in every thread
+    // squared deflation bound, the same in every thread
     T f2 = 0;
     for (int c = lane; c < k; c += 32) f2 += X0[c];
     const T defl2 = deflation_bound2(warp_sum(f2), k, M, d.rk, d.rule, d.acc, sexp);
@@ -457,8 +486,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     __syncthreads();
 
     // ---- one-sided Jacobi on B = R^T, rotations accumulated in A ----------------
-    // (stopping rule and scaled rotations as in gesvd_kernel; columns kk.. of B
-    // are zero and take no part, V_J's rows kk.. stay zero)
+    // (columns kk.. of B are zero and take no part, V_J's rows kk.. stay zero)
     const int n = kk + (kk & 1), np = n / 2;
     const float tol = (float)(k > 8 ? k : 8) * (sizeof(T) == 8 ? (float)DBL_EPSILON : FLT_EPSILON);
     bool converged = kk <= 1;

@@ -279,7 +279,7 @@ __global__ void __launch_bounds__(256, 1) zgesvd_kernel(const ZDesc *__restrict_
         s_pcol[c] = c;
     }
     __syncthreads();
-    // Deflation, as in the real kernel (gesvd_kernel): the QR stops at the
+    // Deflation, as in the real kernels (hc_svd.cu): the QR stops at the
     // first step j >= 1 (the rank search starts at 1) whose trailing block has
     // ||R(j:k, j:k)||_F <= delta = min(1e-13 acc, 1e-16 ||T||_F) and the
     // Jacobi works on the first j rows of R.  Every singular value moves by at
