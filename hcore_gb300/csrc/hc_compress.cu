@@ -473,36 +473,23 @@ static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compr
         range_test_vectors_kernel<<<(maxM * nc + 255) / 256, 256, 0, s>>>(d_omega, maxM * nc, c0 * maxM);
         DenseProducts y, b;
         y.slice_limit = b.slice_limit = (size_t)384 << 20;   // few tiles a product: fill the GPU instead
-        y.stage(DenseProducts::kNoBalance);
-        auto out = [](DenseProducts &p, const DenseWork &w, int M, int N, double *cd) {
-            const size_t first = p.jobs.size();
-            p.add_tile({p.add(w, M, N)});
-            for (size_t j = first; j < p.jobs.size(); ++j) {
-                p.jobs[j].cd = cd;
-                p.jobs[j].ldcd = M;
-            }
-        };
-        auto product = [](const double *P, int ldp, const double *Q, int ldq, int kk, double coef, double beta,
-                          int tr) {
-            DenseWork w{};
-            w.P = P; w.ldp = ldp; w.Q = Q; w.ldq = ldq; w.kk = kk; w.coef = coef; w.beta = beta; w.tr = tr;
-            return w;
-        };
+        y.stage(kNoBalance);
+        using DP = DenseProducts;
         for (int q : active) {
             const RangeTile &t = tiles[q];
-            out(y, product(t.E, t.M, d_omega, maxM, t.M, 1.0, 0.0, 2), t.M, nc, t.Q + (size_t)c0 * t.M);
+            y.add_one(DP::product(t.E, t.M, d_omega, maxM, 2, t.M, 1.0, 0.0), t.M, nc, t.Q + (size_t)c0 * t.M, t.M);
         }
-        b.stage(DenseProducts::kNoBalance);
+        b.stage(kNoBalance);
         for (int q : active) {
             const RangeTile &t = tiles[q];
-            out(b, product(t.E, t.M, t.Q + (size_t)c0 * t.M, t.M, t.M, 1.0, 0.0, 3), t.M, nc,
-                t.B + (size_t)c0 * t.M);
+            b.add_one(DP::product(t.E, t.M, t.Q + (size_t)c0 * t.M, t.M, 3, t.M, 1.0, 0.0), t.M, nc,
+                      t.B + (size_t)c0 * t.M, t.M);
         }
-        b.stage(DenseProducts::kNoBalance);
+        b.stage(kNoBalance);
         for (int q : active) {
             const RangeTile &t = tiles[q];
-            out(b, product(t.Q + (size_t)c0 * t.M, t.M, t.B + (size_t)c0 * t.M, t.M, nc, -1.0, 1.0, 0), t.M, t.M,
-                t.E);
+            b.add_one(DP::product(t.Q + (size_t)c0 * t.M, t.M, t.B + (size_t)c0 * t.M, t.M, 0, nc, -1.0, 1.0), t.M,
+                      t.M, t.E, t.M);
         }
         e = products(y);
         if (e == cudaSuccess)

@@ -69,23 +69,28 @@ constexpr int kSms = 152;
 // blocks of a chunk's columns; a chunk without columns takes one of zeros
 __host__ __device__ constexpr int dense_blocks(int ncol) { return ncol > 0 ? (ncol + kKb - 1) / kKb : 1; }
 
-// largest exponent field of P's and Q's column l (a warp per column); 0x7FF if
-// one of them is not finite
+// balance of P's and Q's column l from their largest exponent fields (a warp per
+// column), or of P's alone: 2^s brings its largest entry near 1; a zero column
+// or one with a non-finite entry is left as it is
 __global__ void __launch_bounds__(256) dense_balance_kernel(const DenseWork *work, const int2 *cols,
-                                                            const int2 *dims, int n, int *shift) {
+                                                            const int2 *dims, int n, bool p_only, int *shift) {
     const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (c >= n) return;
     const int2 tl = cols[c], mn = dims[tl.x];
     const DenseWork w = work[tl.x];
-    const double *p = w.P + (size_t)tl.y * w.ldp, *q = w.Q + (size_t)tl.y * w.ldq;
+    const bool tp = w.tr & 1, tq = w.tr & 2;
+    const double *p = w.P + (tp ? (size_t)tl.y : (size_t)tl.y * w.ldp);
+    const double *q = w.Q + (tq ? (size_t)tl.y : (size_t)tl.y * w.ldq);
+    const size_t sp = tp ? w.ldp : 1, sq = tq ? w.ldq : 1;
     int ep = 0, eq = 0;
 #pragma unroll 4
-    for (int i = lane; i < mn.x; i += 32) ep = max(ep, exp_field(p[i]));
+    for (int i = lane; i < mn.x; i += 32) ep = max(ep, exp_field(p[i * sp]));
 #pragma unroll 4
-    for (int i = lane; i < mn.y; i += 32) eq = max(eq, exp_field(q[i]));
+    for (int i = lane; i < mn.y && !p_only; i += 32) eq = max(eq, exp_field(q[i * sq]));
     ep = __reduce_max_sync(0xffffffffu, ep);
     eq = __reduce_max_sync(0xffffffffu, eq);
-    if (lane == 0) shift[c] = ep == 0 || eq == 0 || ep == 0x7FF || eq == 0x7FF ? 0 : (ep - eq) / 2;
+    if (lane == 0 && p_only) shift[c] = ep == 0 || ep == 0x7FF ? 0 : ep - 1023;
+    else if (lane == 0) shift[c] = ep == 0 || eq == 0 || ep == 0x7FF || eq == 0x7FF ? 0 : (ep - eq) / 2;
 }
 
 // the same for operands stored transposed: a thread per column (64 a block,
@@ -126,7 +131,7 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
     const int mb = (ch.M + kRowsA - 1) / kRowsA;
     const bool q = (int)blockIdx.x >= mb;
     const int rb = q ? blockIdx.x - mb : blockIdx.x, n = q ? ch.N : ch.M;
-    if (rb * kRowsA >= n) return;
+    if (rb * kRowsA >= n || (!q && ch.shared_p)) return;
     const int tid = threadIdx.x, lrow = tid & 127, half = tid >> 7;
     if (tid < ch.ncol) {
         const int2 tl = cols[ch.col0 + tid];
@@ -256,7 +261,8 @@ struct Unit {
     int kcol0, ncol;    // its columns of the K axis
     int flags;          // kFirst ...
 };
-constexpr int kFirst = 1, kLast = 2, kZeroUpper = 4, kFromZero = 8, kScale = 16, kBetaZero = 32, kStop = 64;
+constexpr int kFirst = 1, kLast = 2, kZeroUpper = 4, kFromZero = 8, kScale = 16, kBetaZero = 32, kStop = 64,
+              kKeepUpper = 128, kKeepLower = 256;
 constexpr int kRing = 8;
 
 // The producer's walk over a CTA's units: tiles blockIdx.x, blockIdx.x +
@@ -304,8 +310,15 @@ __device__ __noinline__ void poison_tiles(const DenseJob *jobs, int njobs, const
         walk_tile(w, jobs, njobs, chunks);
         const int row = w.row0 + lrow;
         for (int col = w.col0 + cw; col < min(w.col0 + cw + 8, w.job.N); ++col)
-            if (row < w.job.M) w.job.cd[(size_t)col * w.job.ldcd + row] = __longlong_as_double(-1LL);
+            if (row < w.job.M && !(w.job.mask == 1 && row < col) && !(w.job.mask == 2 && row > col))
+                w.job.cd[(size_t)col * w.job.ldcd + row] = __longlong_as_double(-1LL);
     }
+}
+
+// tiles that a job's mask or its skip word leaves out
+__device__ __forceinline__ bool tile_left_out(const Walk &w) {
+    return (w.job.mask == 1 && w.row0 + kRowsA <= w.col0) ||
+           (w.job.mask == 2 && w.row0 >= w.col0 + kRowsB) || (w.job.skip && *w.job.skip != 0);
 }
 
 // Two CTAs of 18 warps per SM: 16 workers (thread: one row, 8 columns), a
@@ -351,6 +364,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         bool ok = true;
         for (w.t = blockIdx.x; w.t < ntiles && ok; w.t += gridDim.x) {
             walk_tile(w, jobs, njobs, chunks);
+            if (tile_left_out(w)) continue;
             double *cd = w.job.cd + (size_t)w.col0 * w.job.ldcd + w.row0;
             const int ldcd = w.job.ldcd;
             for (; w.c < w.c1 && ok; ++w.c, ++u) {
@@ -379,7 +393,8 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                         x.ncol = ch.ncol;
                         x.flags = (w.first ? kFirst : 0) | (w.c + 1 == w.c1 ? kLast : 0) |
                                   (ch.zero_upper ? kZeroUpper : 0) | (w.from_zero ? kFromZero : 0) |
-                                  (ch.scale != 0 ? kScale : 0) | (ch.scale == 2 ? kBetaZero : 0);
+                                  (ch.scale != 0 ? kScale : 0) | (ch.scale == 2 ? kBetaZero : 0) |
+                                  (w.job.mask == 1 ? kKeepUpper : 0) | (w.job.mask == 2 ? kKeepLower : 0);
                         tc::mbar_arrive(info + u % kRing);
                         w.first = false;
                     }
@@ -520,9 +535,12 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             }
             if ((flags & kLast) && in) {
                 double *p = x.cd + (size_t)cw * x.ldcd + lrow;
+                // entry e lies e + up columns right of the diagonal; lo .. hi are written
+                const int up = x.col0 + cw - (x.row0 + lrow);
+                const int lo = flags & kKeepLower ? -up : 0, hi = flags & kKeepUpper ? min(nc, 1 - up) : nc;
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
-                    if (e < nc) *p = acc[e];
+                    if (e >= lo && e < hi) *p = acc[e];
                     p += x.ldcd;
                 }
             }
@@ -551,12 +569,14 @@ cudaError_t configure_dense_tc() {
 }
 
 cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, const int2 *d_dims, int ncols,
-                                 bool transposed, int *d_shift, cudaStream_t s) {
+                                 DenseBalance how, int *d_shift, cudaStream_t s) {
     if (ncols <= 0) return cudaSuccess;
-    if (transposed)
+    if (how == kNoBalance) return cudaMemsetAsync(d_shift, 0, (size_t)ncols * sizeof(int), s);
+    if (how == kBalanceByThread)
         dense_balance_t_kernel<<<(ncols + 63) / 64, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, d_shift);
     else
-        dense_balance_kernel<<<(ncols + 7) / 8, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, d_shift);
+        dense_balance_kernel<<<(ncols + 7) / 8, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, how == kBalanceP,
+                                                             d_shift);
     return cudaGetLastError();
 }
 

@@ -577,7 +577,7 @@ struct DensePrep {
                 }
             }
         }
-        pr.stage(DenseProducts::kBalanceByThread);
+        pr.stage(kBalanceByThread);
         for (int i : bdcd) {
             const hcore_dense_task &t = tasks[i];
             DenseWork w{};
@@ -586,7 +586,7 @@ struct DensePrep {
             w.tr = 3;
             pr.add_tile({pr.add(w, t.N ? t.N : t.M, t.a)});
         }
-        pr.stage(DenseProducts::kBalanceByWarp);
+        pr.stage(kBalanceByWarp);
         for (const auto &g : groups) pr.add_tile(g);
         b_all = al256(n * sizeof(hcore_dense_task));
         pr.place_host(b_all);

@@ -235,10 +235,13 @@ struct DenseChunk {
     double beta;      // CD is scaled by it before this chunk
     int zero_upper;   // the strict upper triangle is zero after this chunk
     int scale;        // 0: beta = 1, 1: another value, 2: zero
+    int shared_p;     // 1: P's slices and scales are another chunk's
 };
 struct DenseJob {     // one tile and chunks of its list
     double *cd;
+    const int *skip;  // the job is left out when this is not zero (may be null)
     int ldcd, task;   // task: one of the tile's products
+    int mask;         // 1: entries above the diagonal are not touched, 2: below it
     int M, N, chunk0, nchunks;
     int tile0;        // its first tile in the batch
 };
@@ -251,10 +254,13 @@ cudaError_t configure_dense_tc();
 size_t dense_slice_bytes(int M, int N, int ncol);
 size_t dense_slice_q_offset(int M, int ncol);
 int dense_tiles(int M, int N);   // tiles of one job
-// the balance of ncols columns (transposed: of products with both operands
-// stored transposed)
+// how the columns of a stage's products are balanced: not at all (the caller's
+// operands need none), by both operands (a warp per column, or a thread per
+// column where both are stored transposed), or by P alone (its slices then do
+// not depend on Q)
+enum DenseBalance { kNoBalance, kBalanceByWarp, kBalanceByThread, kBalanceP };
 cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, const int2 *d_dims, int ncols,
-                                 bool transposed, int *d_shift, cudaStream_t s);
+                                 DenseBalance how, int *d_shift, cudaStream_t s);
 cudaError_t launch_dense_tiles_tc(const DenseWork *d_work, const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
                                   const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
                                   int *d_exps, cudaStream_t s);

@@ -19,11 +19,6 @@ struct DenseProducts {
     // 1024 x 17 took 2873, 2625, 2557, 2538 and 2493 us with limits of 16, 48,
     // 96, 160 and 400 MB
     size_t slice_limit = (size_t)96 << 20;
-    // how the columns of a stage's products are balanced: not at all (the
-    // caller's operands need none), a warp per column, or a thread per column
-    // (both operands stored transposed)
-    enum Balance { kNoBalance, kBalanceByWarp, kBalanceByThread };
-
     std::vector<DenseWork> work;
     std::vector<int2> dims;      // M, N of each product
     std::vector<int2> cols;      // the K axes of all tiles: (product, its column)
@@ -39,7 +34,7 @@ struct DenseProducts {
     }
 
     // the tiles added from here on run after those before
-    void stage(Balance b) { stages.push_back(Stage{(int)cols.size(), (int)batches.size(), b}); }
+    void stage(DenseBalance b) { stages.push_back(Stage{(int)cols.size(), (int)batches.size(), b}); }
 
     // lay a tile's tasks out along K: a chunk ends after 128 columns, where a
     // task scales CD, and where syrk tasks change to others (a run of syrk
@@ -50,7 +45,7 @@ struct DenseProducts {
         const int first = (int)chunks.size();
         auto open = [&](double beta, int syrk) {
             chunks.push_back(DenseChunk{0, 0, 0, 0, (int)cols.size(), 0, mn.x, mn.y, beta, syrk,
-                                        beta == 1.0 ? 0 : (beta == 0.0 ? 2 : 1)});
+                                        beta == 1.0 ? 0 : (beta == 0.0 ? 2 : 1), 0});
         };
         for (size_t x = 0; x < g.size(); ++x) {
             const DenseWork &w = work[g[x]];
@@ -65,7 +60,13 @@ struct DenseProducts {
         // jobs: the tile's chunks, split where a batch's slice buffer is full
         for (int c = first; c < (int)chunks.size(); ++c) {
             DenseChunk &ch = chunks[c];
-            const size_t need = dense_slice_bytes(mn.x, mn.y, ch.ncol);
+            // P's slices serve the next product too if it has the same P (and they
+            // do not depend on Q)
+            const size_t p_bytes = dense_slice_q_offset(mn.x, ch.ncol);
+            size_t need = dense_slice_bytes(mn.x, mn.y, ch.ncol);
+            const DenseChunk *same = last_p(g[0], c, first);
+            if (same && cur_slices + need - p_bytes <= slice_limit) need -= p_bytes;
+            else same = nullptr;
             if ((int)batches.size() == stages.back().batches0 ||
                 (cur_slices > 0 && cur_slices + need > slice_limit) || batches.back().ntiles > INT_MAX - tiles ||
                 batches.back().nchunks == 65535) {
@@ -74,7 +75,7 @@ struct DenseProducts {
             }
             DenseBatch &b = batches.back();
             if (c == first || b.nchunks == 0) {
-                jobs.push_back(DenseJob{nullptr, 0, g[0], mn.x, mn.y, c, 0, b.ntiles});
+                jobs.push_back(DenseJob{nullptr, nullptr, 0, g[0], 0, mn.x, mn.y, c, 0, b.ntiles});
                 ++b.njobs;
                 b.ntiles += tiles;
             }
@@ -82,12 +83,13 @@ struct DenseProducts {
             ++b.nchunks;
             b.maxM = std::max(b.maxM, mn.x);
             b.maxN = std::max(b.maxN, mn.y);
-            ch.p = (long long)cur_slices;
-            ch.q = ch.p + (long long)dense_slice_q_offset(mn.x, ch.ncol);
-            ch.ep = (int)cur_exps;
-            ch.eq = ch.ep + mn.x;
+            ch.shared_p = same != nullptr;
+            ch.p = same ? same->p : (long long)cur_slices;
+            ch.ep = same ? same->ep : (int)cur_exps;
+            ch.q = (long long)(cur_slices + (same ? 0 : p_bytes));
+            ch.eq = (int)cur_exps + (same ? 0 : mn.x);
             cur_slices += need;
-            cur_exps += (size_t)mn.x + mn.y;
+            cur_exps += (size_t)(same ? 0 : mn.x) + mn.y;
             slice_bytes = std::max(slice_bytes, cur_slices);
             max_exps = std::max(max_exps, cur_exps);
         }
@@ -118,32 +120,67 @@ struct DenseProducts {
     }
     const DenseWork *device_work(const char *arena) const { return (const DenseWork *)(arena + o_work); }
 
-    cudaError_t launch(char *arena, cudaStream_t s) const {
+    // the chunk before chunk c, if c is its product's only one and has the same P
+    // in the same batch
+    const DenseChunk *last_p(int prod, int c, int first) const {
+        if (c == 0 || c != first || c + 1 != (int)chunks.size() || stages.back().balance == kBalanceByWarp ||
+            stages.back().balance == kBalanceByThread || (int)batches.size() == stages.back().batches0)
+            return nullptr;
+        const DenseBatch &b = batches.back();
+        if (b.nchunks == 0 || b.chunk0 + b.nchunks != c || b.nchunks == 65535) return nullptr;
+        const DenseChunk &q = chunks[c - 1], &x = chunks[c];
+        if (q.ncol != x.ncol || q.M != x.M || q.ncol == 0) return nullptr;
+        const int2 l = cols[q.col0], m = cols[x.col0];
+        const DenseWork &w = work[l.x], &v = work[prod];
+        const bool same = l.y == 0 && m.y == 0 && w.kk == v.kk && w.kk == x.ncol && w.P == v.P && w.P != nullptr &&
+                          w.ldp == v.ldp && (w.tr & 1) == (v.tr & 1) && w.coef == v.coef;
+        return same ? &q : nullptr;
+    }
+
+    int nstages() const { return (int)stages.size(); }
+    cudaError_t launch_stage(char *arena, int q, cudaStream_t s) const {
         const DenseWork *d_work = device_work(arena);
         const int2 *d_cols = (const int2 *)(arena + o_cols), *d_dims = (const int2 *)(arena + o_dims);
         int *d_shift = (int *)(arena + o_shift);
-        cudaError_t e = cudaSuccess;
-        for (size_t q = 0; q < stages.size() && e == cudaSuccess; ++q) {
-            const bool last = q + 1 == stages.size();
-            const int c0 = stages[q].cols0, c1 = last ? (int)cols.size() : stages[q + 1].cols0;
-            const int b1 = last ? (int)batches.size() : stages[q + 1].batches0;
-            if (stages[q].balance != kNoBalance)
-                e = launch_dense_balance(d_work, d_cols + c0, d_dims, c1 - c0,
-                                         stages[q].balance == kBalanceByThread, d_shift + c0, s);
-            else if (c1 > c0)
-                e = cudaMemsetAsync(d_shift + c0, 0, (size_t)(c1 - c0) * sizeof(int), s);
-            for (int b = stages[q].batches0; b < b1 && e == cudaSuccess; ++b)
-                e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
-                                          (const DenseJob *)(arena + o_jobs), batches[b],
-                                          (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), s);
-        }
+        const bool last = q + 1 == nstages();
+        const int c0 = stages[q].cols0, c1 = last ? (int)cols.size() : stages[q + 1].cols0;
+        const int b1 = last ? (int)batches.size() : stages[q + 1].batches0;
+        cudaError_t e = launch_dense_balance(d_work, d_cols + c0, d_dims, c1 - c0, stages[q].balance,
+                                             d_shift + c0, s);
+        for (int b = stages[q].batches0; b < b1 && e == cudaSuccess; ++b)
+            e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
+                                      (const DenseJob *)(arena + o_jobs), batches[b],
+                                      (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), s);
         return e;
+    }
+    cudaError_t launch(char *arena, cudaStream_t s) const {
+        cudaError_t e = cudaSuccess;
+        for (int q = 0; q < nstages() && e == cudaSuccess; ++q) e = launch_stage(arena, q, s);
+        return e;
+    }
+
+    // a product alone on its output
+    void add_one(const DenseWork &w, int M, int N, double *cd, int ldcd, int mask = 0, const int *skip = nullptr) {
+        const size_t first = jobs.size();
+        add_tile({add(w, M, N)});
+        for (size_t j = first; j < jobs.size(); ++j) {
+            jobs[j].cd = cd;
+            jobs[j].ldcd = ldcd;
+            jobs[j].mask = mask;
+            jobs[j].skip = skip;
+        }
+    }
+    static DenseWork product(const double *P, int ldp, const double *Q, int ldq, int tr, int kk, double coef,
+                             double beta) {
+        DenseWork w{};
+        w.P = P; w.ldp = ldp; w.Q = Q; w.ldq = ldq; w.tr = tr; w.kk = kk; w.coef = coef; w.beta = beta;
+        return w;
     }
 
 private:
     struct Stage {
         int cols0, batches0;
-        Balance balance;
+        DenseBalance balance;
     };
     std::vector<Stage> stages;
     size_t slice_bytes = 0, max_exps = 0, cur_slices = 0, cur_exps = 0;

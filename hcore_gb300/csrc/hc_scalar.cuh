@@ -1,5 +1,6 @@
 // hcore-gb300: small device helpers shared by the recompression kernels
-// (warp reductions, exact scaling by powers of two, the SVD's deflation bound).
+// (warp reductions, exact scaling by powers of two, reciprocals and square roots
+// from FP32 seeds, the SVD's deflation bound).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -61,6 +62,54 @@ __device__ __forceinline__ T deflation_bound2(T f2, int k, int M, int rk, int ru
         return isfinite(dl) ? dl * dl : T(-1);
     }
 }
+
+// ---- numbers from their bits -------------------------------------------------
+// x = m 2^(e - 1023), m in [1, 2) as FP32 (truncated); e = 0 for zero and
+// subnormals (their m is meaningless and not used)
+__device__ __forceinline__ void split(double x, float &m, int &e) {
+    const unsigned hi = (unsigned)__double2hiint(x), lo = (unsigned)__double2loint(x);
+    e = (int)((hi >> 20) & 0x7FFu);
+    m = __uint_as_float(0x3F800000u | ((hi & 0xFFFFFu) << 3) | (lo >> 29));
+}
+// q 2^d as FP64 for a positive normal FP32 q; 0 when the result is not normal
+__device__ __forceinline__ double widen(float q, int d) {
+    const unsigned b = __float_as_uint(q);
+    const int e = (int)(b >> 23) + (1023 - 127) + d;
+    if (e <= 0) return 0.0;
+    return __hiloint2double((int)(((unsigned)e << 20) | ((b & 0x7FFFFFu) >> 3)), (int)(b << 29));
+}
+__device__ __forceinline__ float fsqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float frsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1 / sqrt(x), x normal and positive: y (1 + e/2 + 3 e^2/8), e = 1 - x y^2
+__device__ __forceinline__ double inv_sqrt(double x) {
+    float m;
+    int e;
+    split(x, m, e);
+    const int ex = e - 1023, odd = ex & 1, half = (ex - odd) >> 1;
+    const double y = widen(frsqrt_fast(odd ? 2.f * m : m), -half);
+    const double r = fma(-x * y, y, 1.0);
+    return fma(y * r, fma(0.375, r, 0.5), y);
+}
+__device__ __forceinline__ float inv_sqrt(float x) { return 1.f / sqrtf(x); }
+// 1 / x, x normal and positive: y (1 + e + e^2), e = 1 - x y
+__device__ __forceinline__ double inv(double x) {
+    float m;
+    int e;
+    split(x, m, e);
+    const double y = widen(__fdividef(1.f, m), 1023 - e);
+    const double r = fma(-x, y, 1.0);
+    return fma(y, fma(r, r, r), y);
+}
+__device__ __forceinline__ float inv(float x) { return 1.f / x; }
 
 // odd leading dimension of a k x k matrix in shared memory
 __host__ __device__ inline int svd_ld(int k) { return k | 1; }

@@ -16,17 +16,18 @@
 // are updated with the block's 32 solved values, 64 rows at a time through a
 // shared-memory tile of T' that every vector of the CTA reuses.  Tiles are
 // read along A's contiguous dimension, so a transposed A is read coalesced
-// too.  A task's groups share A, which stays in L2.
+// too.  A task's groups share A, which stays in L2.  Large triangles are solved
+// that way block by block, with products on the tensor cores between the blocks
+// (trsm_block_step).
 //
 // POTRF.  Blocked right-looking Cholesky on the lower view of the tile (the
-// transposed view for uplo 'U'), 64 columns per block, three launches per
-// block: the diagonal block (left-looking columns in shared memory, the
-// reference LAPACK's pivot test: a pivot that is not > 0, or is NaN, stops
-// the factorization and is left in place), the panel below it
-// (A_ik = A_ik L_kk^-T, 64 rows per CTA, the 64 components of a row spread
-// over 4 threads), and the trailing lower triangle (A_ij -= A_ik A_jk^T,
-// 32 x 32 tiles, 2 x 2 register blocks).  Every launch first reads the
-// task's info and returns once a pivot has failed.
+// transposed view for uplo 'U'), 64 columns per block, three parts per block:
+// the diagonal block (sub-blocks of 16 columns; the reference LAPACK's pivot
+// test: a pivot that is not > 0, or is NaN, stops the factorization and is left
+// in place), the panel below it (A_ik = A_ik L_kk^-T, 32 rows per CTA, four lanes
+// a row), and the trailing lower triangle (A_ij -= A_ik A_jk^T: products on the
+// tensor cores while it is large, else 32 x 32 tiles with 2 x 2 register blocks).
+// Every launch first reads the task's info and returns once a pivot has failed.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -36,6 +37,8 @@
 #include <vector>
 
 #include "hc_host.h"
+#include "hc_products.h"
+#include "hc_scalar.cuh"
 #include "hcore.h"
 #include "hcore_d.h"
 
@@ -167,18 +170,47 @@ struct PotrfView {
     }
 };
 
-__device__ __forceinline__ double warp_sum_d(double v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    return v;
+// Columns [j0, j0 + 16) of the 64 x 64 block S: the diagonal 16 x 16 block by one
+// warp (lane i holds row i in registers; one reciprocal square root and one
+// scaling a column, no barrier), rows below it by four lanes a row.
+constexpr int kSb = 16;
+
+// 1 / sqrt(d) and sqrt(d) of a positive pivot
+__device__ __forceinline__ void pivot_root(double d, double &r, double &l) {
+    if (d < 2.2250738585072014e-308) {   // subnormal
+        l = sqrt(d);
+        r = 1.0 / l;
+        return;
+    }
+    r = inv_sqrt(d);
+    l = d * r;
+    l = fma(fma(-l, l, d) * 0.5, r, l);
 }
 
-// diagonal block [kb, kb + bs): left-looking columns (LAPACK dpotf2 order);
-// a failing pivot is stored in place and ends the task (info = column + 1)
+// Solve rows of X L16^T = A16 in place: four lanes a row (lane q of the four
+// holds columns q, q + 4, ... of the sixteen), L16's rows and reciprocal
+// pivots in shared memory.  x_j goes around the four lanes by a shuffle.
+__device__ __forceinline__ void solve16(double (&a)[4], const double (*L)[kPb + 1], int j0, const double *rL,
+                                        int q) {
+#pragma unroll
+    for (int j = 0; j < kSb; ++j) {
+        double x = a[j / 4] * rL[j0 + j];
+        x = __shfl_sync(0xffffffffu, x, j & 3, 4);
+        if (q == (j & 3)) a[j / 4] = x;
+#pragma unroll
+        for (int m = j / 4; m < 4; ++m)
+            if (q + 4 * m > j) a[m] -= x * L[j0 + q + 4 * m][j0 + j];
+    }
+}
+
+// diagonal block [kb, kb + bs): right-looking over sub-blocks of 16 columns; a
+// failing pivot is stored in place and ends the task (info = column + 1).  Bound
+// by the chain of pivots and the FP64 instructions between them: 121 us per
+// block with two barriers a column, 102 us now.
 __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task *tasks, int *info,
                                                          int kb) {
     __shared__ double S[kPb][kPb + 1];
-    __shared__ double rpiv;
+    __shared__ double rL[kPb];
     __shared__ int fail;
     const hcore_potrf_task t = tasks[blockIdx.x];
     if (info[blockIdx.x] != 0 || kb >= t.n) return;
@@ -186,104 +218,147 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task 
     const PotrfView V{t.A, t.lda, t.uplo == 'U' || t.uplo == 'u'};
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int e = tid; e < kPb * kPb; e += 256) {
-        const int i = e % kPb, j = e / kPb;
+        const int i = V.up ? e / kPb : e % kPb, j = V.up ? e % kPb : e / kPb;
         S[i][j] = (i < bs && j <= i) ? V.at(kb + i, kb + j) : 0.0;
     }
     if (tid == 0) fail = -1;
     __syncthreads();
-    const int row = tid >> 2, part = tid & 3;  // 4 threads per row
-    for (int j = 0; j < bs; ++j) {
+    for (int j0 = 0; j0 < bs; j0 += kSb) {
         if (warp == 0) {
-            double s = 0.0;
-            for (int l = lane; l < j; l += 32) s += S[j][l] * S[j][l];
-            s = warp_sum_d(s);
-            if (lane == 0) {
-                const double d = S[j][j] - s;
-                if (!(d > 0.0)) {  // not positive, or NaN
-                    S[j][j] = d;
-                    fail = j;
-                } else {
-                    const double l = sqrt(d);
-                    S[j][j] = l;
-                    rpiv = 1.0 / l;  // the column is scaled by the reciprocal, as dpotf2 does
+            double a[kSb];
+            const int i = lane & (kSb - 1);
+#pragma unroll
+            for (int j = 0; j < kSb; ++j) a[j] = S[j0 + i][j0 + j];
+            int bad = -1;
+#pragma unroll
+            for (int j = 0; j < kSb; ++j) {
+                const double d = __shfl_sync(0xffffffffu, a[j], j);
+                if (bad < 0 && j0 + j < bs) {   // uniform in the warp
+                    if (!(d > 0.0)) {           // not positive, or NaN
+                        bad = j;
+                    } else {
+                        double r, l;
+                        pivot_root(d, r, l);
+                        if (lane == 0) rL[j0 + j] = r;
+                        a[j] = i == j ? l : a[j] * r;
+                    }
+                }
+#pragma unroll
+                for (int c = j + 1; c < kSb; ++c) {
+                    const double lc = __shfl_sync(0xffffffffu, a[j], c);
+                    if (bad < 0 && i >= c) a[c] -= a[j] * lc;
                 }
             }
+            if (lane < kSb)
+#pragma unroll
+                for (int j = 0; j < kSb; ++j)
+                    if (j <= i) S[j0 + i][j0 + j] = a[j];
+            if (lane == 0 && bad >= 0) fail = j0 + bad;
         }
         __syncthreads();
         if (fail >= 0) break;
-        double s = 0.0;
-        if (row > j && row < bs)
-            for (int l = part; l < j; l += 4) s += S[row][l] * S[j][l];
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        if (part == 0 && row > j && row < bs) S[row][j] = (S[row][j] - s) * rpiv;
+        const int below = j0 + kSb;
+        if (below >= bs) break;
+        // rows below (64 rows a pass, four lanes each; all lanes take part in the shuffles)
+        {
+            const int row = below + (tid >> 2), q = tid & 3;
+            const bool in = row < kPb;
+            double a[4];
+#pragma unroll
+            for (int m = 0; m < 4; ++m) a[m] = in ? S[row][j0 + q + 4 * m] : 0.0;
+            solve16(a, S, j0, rL, q);
+#pragma unroll
+            for (int m = 0; m < 4; ++m)
+                if (in) S[row][j0 + q + 4 * m] = a[m];
+        }
+        __syncthreads();
+        const int nr = bs - below;
+        for (int e = tid; e < nr * nr; e += 256) {
+            const int i = below + e % nr, c = below + e / nr;
+            if (c > i) continue;
+            double s0 = S[i][c], s1 = 0.0;
+#pragma unroll
+            for (int l = 0; l < kSb; l += 2) {
+                s0 -= S[i][j0 + l] * S[c][j0 + l];
+                s1 -= S[i][j0 + l + 1] * S[c][j0 + l + 1];
+            }
+            S[i][c] = s0 + s1;
+        }
         __syncthreads();
     }
     for (int e = tid; e < kPb * kPb; e += 256) {
-        const int i = e % kPb, j = e / kPb;
+        const int i = V.up ? e / kPb : e % kPb, j = V.up ? e % kPb : e / kPb;
         if (i < bs && j <= i) V.at(kb + i, kb + j) = S[i][j];
     }
     if (tid == 0 && fail >= 0) info[blockIdx.x] = kb + fail + 1;
 }
 
-// panel rows [r0, r0 + 64) below the diagonal block: X L_kk^T = A_ik.
-// Thread (r, q) holds components q, q + 4, ... of row r in registers; the
-// solve runs over the columns c in order, one barrier per column.
-__global__ void __launch_bounds__(256) potrf_panel_kernel(const hcore_potrf_task *tasks,
-                                                          const int *info, int kb) {
+// panel rows below the diagonal block: X L_kk^T = A_ik, 32 rows a CTA, four
+// lanes a row.  Sixteen columns at a time are solved in registers and taken
+// out of the columns on their right (64 steps with a barrier each, 64 rows a
+// CTA, took 126 us a block, eight tiles of order 1024; this 47 us).
+constexpr int kPr = 32;
+__global__ void __launch_bounds__(4 * kPr) potrf_panel_kernel(const hcore_potrf_task *tasks,
+                                                              const int *info, int kb) {
     __shared__ double Ls[kPb][kPb + 1];
-    __shared__ double Xs[kPb][kPb + 1];
+    __shared__ double Xs[kPr][kPb + 1];
     __shared__ double rL[kPb];
     const hcore_potrf_task t = tasks[blockIdx.y];
     if (info[blockIdx.y] != 0 || kb >= t.n) return;
     const int bs = min(kPb, t.n - kb);
-    const int r0 = kb + bs + blockIdx.x * kPb;
-    if (r0 >= t.n) return;
-    const int rows = min(kPb, t.n - r0);
+    const int r0 = kb + bs + blockIdx.x * kPr;
+    if (r0 >= t.n) return;   // (rows below exist, so bs = kPb)
+    const int rows = min(kPr, t.n - r0);
     const PotrfView V{t.A, t.lda, t.uplo == 'U' || t.uplo == 'u'};
     const int tid = threadIdx.x;
-    for (int e = tid; e < kPb * kPb; e += 256) {
-        const int i = e % kPb, j = e / kPb;
-        Ls[i][j] = (i < bs && j <= i) ? V.at(kb + i, kb + j) : 0.0;
+    for (int e = tid; e < kPb * kPb; e += 4 * kPr) {
+        const int i = V.up ? e / kPb : e % kPb, j = V.up ? e % kPb : e / kPb;
+        Ls[i][j] = j <= i ? V.at(kb + i, kb + j) : 0.0;
     }
-    const int r = tid & 63, q = tid >> 6;
-    double a[kPb / 4];
-#pragma unroll
-    for (int m = 0; m < kPb / 4; ++m) {
-        const int c = q + 4 * m;
-        a[m] = (r < rows && c < bs) ? V.at(r0 + r, kb + c) : 0.0;
+    for (int e = tid; e < kPr * kPb; e += 4 * kPr) {
+        const int i = V.up ? e / kPb : e % kPr, j = V.up ? e % kPb : e / kPr;
+        Xs[i][j] = i < rows ? V.at(r0 + i, kb + j) : 0.0;
     }
-    if (tid < bs) rL[tid] = 1.0 / V.at(kb + tid, kb + tid);
+    if (tid < kPb) rL[tid] = 1.0 / V.at(kb + tid, kb + tid);
     __syncthreads();
-    for (int c = 0; c < bs; ++c) {
-        if (q == (c & 3)) {
+    const int r = tid >> 2, q = tid & 3;
+#pragma unroll 1
+    for (int j0 = 0; j0 < kPb; j0 += kSb) {
+        double a[4];
 #pragma unroll
-            for (int m = 0; m < kPb / 4; ++m)
-                if (q + 4 * m == c) {
-                    a[m] *= rL[c];
-                    Xs[r][c] = a[m];
-                }
-        }
-        __syncthreads();
-        const double xc = Xs[r][c];
+        for (int m = 0; m < 4; ++m) a[m] = Xs[r][j0 + q + 4 * m];
+        solve16(a, Ls, j0, rL, q);
 #pragma unroll
-        for (int m = 0; m < kPb / 4; ++m) {
-            const int l = q + 4 * m;
-            if (l > c && l < bs) a[m] -= xc * Ls[l][c];
+        for (int m = 0; m < 4; ++m) Xs[r][j0 + q + 4 * m] = a[m];
+        __syncwarp();   // a row's four lanes share a warp
+        for (int c = j0 + kSb + q; c < kPb; c += 4) {
+            double s0 = Xs[r][c], s1 = 0.0;
+#pragma unroll
+            for (int l = 0; l < kSb; l += 2) {
+                s0 -= Xs[r][j0 + l] * Ls[c][j0 + l];
+                s1 -= Xs[r][j0 + l + 1] * Ls[c][j0 + l + 1];
+            }
+            Xs[r][c] = s0 + s1;
         }
+        __syncwarp();
     }
     __syncthreads();
-    for (int e = tid; e < kPb * kPb; e += 256) {
-        const int i = e % kPb, j = e / kPb;
-        if (i < rows && j < bs) V.at(r0 + i, kb + j) = Xs[i][j];
+    for (int e = tid; e < kPr * kPb; e += 4 * kPr) {
+        const int i = V.up ? e / kPb : e % kPr, j = V.up ? e % kPb : e / kPr;
+        if (i < rows) V.at(r0 + i, kb + j) = Xs[i][j];
     }
 }
 
-// trailing lower triangle from row/column t0 = kb + bs: A_ij -= A_ik A_jk^T,
+// small trailing lower triangle from row/column t0 = kb + bs: A_ij -= A_ik A_jk^T,
 // one CTA per 32 x 32 tile (bi >= bj), 2 x 2 outputs per thread, K = bs
 // staged 16 at a time.  Small tiles keep each CTA short: the update is on the
 // factorization's critical path once per block.
 constexpr int kUt = 32;
+// From this many tiles in a step (two for each SM) the products go to the tensor
+// cores: about 25 us a step with their slicing, where potrf_update_kernel takes 17
+// us per tile and SM (all updates of eight tiles of order 1024: 2.6 ms, then 0.9).
+// Their error is half that of FP64 FMAs.
+constexpr int kTcUpdateTiles = 304;
 __global__ void __launch_bounds__(256) potrf_update_kernel(const hcore_potrf_task *tasks,
                                                            const int *info, int kb, int tiles) {
     __shared__ double sP[16][kUt + 1];
@@ -356,9 +431,50 @@ static bool trsm_valid(const hcore_trsm_task &t) {
     return t.A && t.B && t.lda >= std::max(1, na) && t.ldb >= std::max(1, t.M);
 }
 
+// Triangles from this order on are solved by blocks: the vectors against a
+// diagonal block of kTrTb (trsm_kernel), then one product on the tensor cores
+// takes them out of all rows (columns) that follow.  The whole solve in one CTA
+// per eight vectors is bound by FP64 issue and, with few vectors, by its chain
+// of n / 32 blocks; a block step costs about 55 us however few the vectors.
+// Whole and by blocks, us (one GB300): order 384, 16 vectors 301, 318; 512 492,
+// 430; 1024 1747, 889; eight of order 384 with 240 vectors each 481, 434; 1024
+// 2720, 1286.
+constexpr int kTrTcOrder = 448, kTrTb = 64;
+
+// Step `blk` of a task solved by blocks: the diagonal block's task, and the
+// product that follows (false when it is the last block).
+static bool trsm_block_step(const hcore_trsm_task &t, int blk, hcore_trsm_task &diag, DenseProducts *pr) {
+    const bool left = t.side == HCORE_Left, notrans = t.trans == HCORE_NoTrans;
+    const int n = left ? t.M : t.N;
+    // op(A)'s triangle: lower is solved forwards, upper backwards (left side; the
+    // other way round on the right)
+    const bool lower = (t.uplo == HCORE_Lower) == notrans, forward = left == lower;
+    const int b0 = blk * kTrTb, b1 = std::min(n, b0 + kTrTb);
+    const int p0 = forward ? b0 : n - b1, p1 = forward ? b1 : n - b0;
+    const int r0 = forward ? p1 : 0, nr = forward ? n - p1 : p0;   // what is not solved yet
+    const size_t lda = t.lda, ldb = t.ldb;
+    diag = t;
+    diag.alpha = blk == 0 ? t.alpha : 1.0;
+    diag.A = t.A + p0 * (lda + 1);
+    diag.B = t.B + (left ? (size_t)p0 : p0 * ldb);
+    (left ? diag.M : diag.N) = p1 - p0;
+    if (nr == 0) return false;
+    if (!pr) return true;
+    const double beta = blk == 0 ? t.alpha : 1.0;
+    using DP = DenseProducts;
+    const double *Ablk = notrans == left ? t.A + p0 * lda + r0 : t.A + r0 * lda + p0;
+    const int trA = notrans == left ? 0 : 1;   // op(A)(rest, block), or its transpose on the right
+    if (left)
+        pr->add_one(DP::product(Ablk, t.lda, t.B + p0, t.ldb, trA | 2, p1 - p0, -1.0, beta), nr, t.N, t.B + r0,
+                    t.ldb);
+    else
+        pr->add_one(DP::product(t.B + p0 * ldb, t.ldb, Ablk, t.lda, trA << 1, p1 - p0, -1.0, beta), t.M, nr,
+                    t.B + r0 * ldb, t.ldb);
+    return true;
+}
+
 // Run n TRSM tasks (device-accessible pointers) on stream s and wait.
 static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
-    std::vector<TrsmWork> work;
     int maxn = 1;
     for (int i = 0; i < n; ++i) {
         const hcore_trsm_task &t = tasks[i];
@@ -369,41 +485,93 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
         if (t.M == 0 || t.N == 0) continue;
         maxn = std::max(maxn, t.side == HCORE_Left ? t.M : t.N);
     }
-    const int S = trsm_stride(maxn);
-    if (S == 0) {
+    if (trsm_stride(maxn) == 0) {
         set_error("hcore_gpu_trsm_batched: triangle of order %d does not fit shared memory", maxn);
         return HCORE_GPU_EINVAL;
     }
-    for (int i = 0; i < n; ++i) {
-        const hcore_trsm_task &t = tasks[i];
-        if (t.M == 0 || t.N == 0) continue;
-        const int nvec = t.side == HCORE_Left ? t.N : t.M;
-        for (int v0 = 0; v0 < nvec; v0 += S) work.push_back({i, v0, std::min(S, nvec - v0), 0});
+    // the launches of trsm_kernel: the small triangles, then the diagonal blocks
+    // of the others, step by step, each followed by a stage of products
+    struct Launch {
+        size_t work0, count;
+        int S, maxn, stage;
+    };
+    std::vector<hcore_trsm_task> solve;
+    std::vector<TrsmWork> work;
+    std::vector<Launch> launches;
+    DenseProducts pr;
+    int steps = 0;
+    auto by_blocks = [](const hcore_trsm_task &t) {
+        return t.alpha != 0.0 && t.M > 0 && t.N > 0 && (t.side == HCORE_Left ? t.M : t.N) >= kTrTcOrder;
+    };
+    for (int blk = -1; blk < steps; ++blk) {
+        Launch l{work.size(), 0, 0, 1, -1};
+        std::vector<int> todo;
+        const size_t first = solve.size();
+        bool any = false;
+        for (int i = 0; i < n; ++i) {
+            const hcore_trsm_task &t = tasks[i];
+            if (t.M == 0 || t.N == 0) continue;
+            const int order = t.side == HCORE_Left ? t.M : t.N;
+            hcore_trsm_task d = t;
+            if (by_blocks(t)) {
+                steps = std::max(steps, (order + kTrTb - 1) / kTrTb);
+                if (blk < 0 || blk * kTrTb >= order) continue;
+                any = trsm_block_step(t, blk, d, nullptr) || any;
+                todo.push_back(i);
+            } else if (blk >= 0) {
+                continue;
+            }
+            l.maxn = std::max(l.maxn, d.side == HCORE_Left ? d.M : d.N);
+            solve.push_back(d);
+        }
+        l.S = trsm_stride(l.maxn);
+        for (size_t q = first; q < solve.size(); ++q) {
+            const int nvec = solve[q].side == HCORE_Left ? solve[q].N : solve[q].M;
+            for (int v0 = 0; v0 < nvec; v0 += l.S) work.push_back({(int)q, v0, std::min(l.S, nvec - v0), 0});
+        }
+        l.count = work.size() - l.work0;
+        if (any) {
+            l.stage = pr.nstages();
+            pr.stage(kBalanceP);   // (many right-hand sides share a triangle)
+            for (int i : todo) {
+                hcore_trsm_task d;
+                trsm_block_step(tasks[i], blk, d, &pr);
+            }
+        }
+        if (l.count) launches.push_back(l);
     }
     if (work.empty()) return HCORE_GPU_OK;
-    if (work.size() > (size_t)INT_MAX) {
+    if (work.size() > (size_t)INT_MAX || solve.size() > (size_t)INT_MAX) {
         set_error("hcore_gpu_trsm_batched: too many vector groups");
         return HCORE_GPU_EINVAL;
     }
     ThreadCtx &tc = thread_ctx();
-    const size_t bt = al256(n * sizeof(hcore_trsm_task)), bw = al256(work.size() * sizeof(TrsmWork));
-    char *arena = (char *)tc.dev_ensure(bt + bw);
-    char *pin = (char *)tc.pin_ensure(bt + bw);
+    const size_t bt = al256(solve.size() * sizeof(hcore_trsm_task)), bw = al256(work.size() * sizeof(TrsmWork));
+    size_t up = bt + bw;
+    pr.place_host(up);
+    size_t all = up;
+    pr.place_device(all);
+    char *arena = (char *)tc.dev_ensure(all);
+    char *pin = (char *)tc.pin_ensure(up);
     if (!arena || !pin) {
         set_error("hcore_gpu_trsm_batched: out of memory");
         return HCORE_GPU_ENOMEM;
     }
     cudaStreamSynchronize(s);  // the previous call may still read the pinned buffer
-    memcpy(pin, tasks, n * sizeof(hcore_trsm_task));
+    memcpy(pin, solve.data(), solve.size() * sizeof(hcore_trsm_task));
     memcpy(pin + bt, work.data(), work.size() * sizeof(TrsmWork));
-    cudaMemcpyAsync(arena, pin, bt + bw, cudaMemcpyHostToDevice, s);
-    const size_t smem = (size_t)maxn * S * sizeof(double);
-    cudaError_t e = cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e == cudaSuccess) {
-        trsm_kernel<<<(unsigned)work.size(), 256, smem, s>>>(
-            (const hcore_trsm_task *)arena, (const TrsmWork *)(arena + bt), S);
+    pr.pack(pin);
+    cudaMemcpyAsync(arena, pin, up, cudaMemcpyHostToDevice, s);
+    cudaError_t e = configure_dense_tc();
+    for (const Launch &l : launches) {
+        const size_t smem = (size_t)l.maxn * l.S * sizeof(double);
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) break;
+        trsm_kernel<<<(unsigned)l.count, 256, smem, s>>>((const hcore_trsm_task *)arena,
+                                                         (const TrsmWork *)(arena + bt) + l.work0, l.S);
         e = cudaGetLastError();
+        if (e == cudaSuccess && l.stage >= 0) e = pr.launch_stage(arena, l.stage, s);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
@@ -446,28 +614,66 @@ static int run_potrf(int n, const hcore_potrf_task *tasks, int *info, cudaStream
     }
     ThreadCtx &tc = thread_ctx();
     const size_t bt = al256(nr * sizeof(hcore_potrf_task)), bi = al256(nr * sizeof(int));
-    char *arena = (char *)tc.dev_ensure(bt + bi);
-    char *pin = (char *)tc.pin_ensure(bt + bi);
+    // The trailing updates of a block step, A_ij -= A_ik A_jk^T, run as products
+    // on the tensor cores (hc_dense_tc.cu) while they are large.  Their rounding is
+    // relative to the rows' largest entries, at most sqrt(a_ii) and sqrt(a_jj):
+    // the backward error of a Cholesky factorization.
+    DenseProducts pr;
+    std::vector<int> stage_of;   // per block step: its stage of pr, or -1
+    size_t up = bt + bi;
+    std::vector<int> tile_of_job;
+    {
+        for (int kb = 0; kb < maxn; kb += kPb) {
+            long long tiles = 0;
+            for (const auto &t : run) {
+                const long long x = t.n > kb + kPb ? (t.n - kb - kPb + kUt - 1) / kUt : 0;
+                tiles += x * (x + 1) / 2;
+            }
+            stage_of.push_back(tiles >= kTcUpdateTiles ? pr.nstages() : -1);
+            if (tiles < kTcUpdateTiles) continue;
+            pr.stage(kNoBalance);   // (P and Q are the same rows)
+            for (int q = 0; q < nr; ++q) {
+                const hcore_potrf_task &t = run[q];
+                const int n1 = t.n - kb - kPb;
+                if (n1 <= 0) continue;
+                const size_t ld = t.lda, k1 = kb + kPb;
+                const bool up_ = t.uplo == 'U' || t.uplo == 'u';
+                const double *p = up_ ? t.A + k1 * ld + kb : t.A + (size_t)kb * ld + k1;
+                pr.add_one(DenseProducts::product(p, t.lda, p, t.lda, up_ ? 3 : 0, kPb, -1.0, 1.0), n1, n1,
+                           t.A + k1 * (ld + 1), t.lda, up_ ? 2 : 1);
+                tile_of_job.resize(pr.jobs.size(), q);
+            }
+        }
+    }
+    pr.place_host(up);
+    size_t all = up;
+    pr.place_device(all);
+    char *arena = (char *)tc.dev_ensure(all);
+    char *pin = (char *)tc.pin_ensure(up);
     if (!arena || !pin) {
         set_error("hcore_gpu_potrf_batched: out of memory");
         return HCORE_GPU_ENOMEM;
     }
+    const hcore_potrf_task *d_t = (const hcore_potrf_task *)arena;
+    int *d_info = (int *)(arena + bt);
+    for (size_t j = 0; j < pr.jobs.size(); ++j) pr.jobs[j].skip = d_info + tile_of_job[j];
     cudaStreamSynchronize(s);
     memcpy(pin, run.data(), nr * sizeof(hcore_potrf_task));
     memset(pin + bt, 0, nr * sizeof(int));
-    cudaMemcpyAsync(arena, pin, bt + bi, cudaMemcpyHostToDevice, s);
-    const hcore_potrf_task *d_t = (const hcore_potrf_task *)arena;
-    int *d_info = (int *)(arena + bt);
-    cudaError_t e = cudaSuccess;
+    pr.pack(pin);
+    cudaMemcpyAsync(arena, pin, up, cudaMemcpyHostToDevice, s);
+    cudaError_t e = configure_dense_tc();
     for (int kb = 0; kb < maxn && e == cudaSuccess; kb += kPb) {
         potrf_diag_kernel<<<nr, 256, 0, s>>>(d_t, d_info, kb);
-        const int below = maxn - std::min(maxn, kb + kPb);
+        const int below = maxn - std::min(maxn, kb + kPb), stage = stage_of[kb / kPb];
         if (below > 0) {
-            const int panels = (below + kPb - 1) / kPb, tiles = (below + kUt - 1) / kUt;
-            potrf_panel_kernel<<<dim3(panels, nr), 256, 0, s>>>(d_t, d_info, kb);
-            potrf_update_kernel<<<dim3(tiles * tiles, nr), 256, 0, s>>>(d_t, d_info, kb, tiles);
+            const int panels = (below + kPr - 1) / kPr, tiles = (below + kUt - 1) / kUt;
+            potrf_panel_kernel<<<dim3(panels, nr), 4 * kPr, 0, s>>>(d_t, d_info, kb);
+            if (stage < 0)
+                potrf_update_kernel<<<dim3(tiles * tiles, nr), 256, 0, s>>>(d_t, d_info, kb, tiles);
         }
         e = cudaGetLastError();
+        if (e == cudaSuccess && stage >= 0) e = pr.launch_stage(arena, stage, s);
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(pin + bt, d_info, nr * sizeof(int), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
