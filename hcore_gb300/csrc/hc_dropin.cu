@@ -1473,8 +1473,10 @@ __global__ void __launch_bounds__(256) zextract_kernel(const ZExtractTask *__res
 // packed on the host into pinned staging and copied to the device in one
 // transfer, because the stack kernel reads every factor column many times
 // (F = AV^T BV, G = BU F^T), which over the host link would cost each read
-// again.  The new factors are written to a device buffer and copied to the
-// tasks' CU/CV.
+// again.  A task whose CU and CV are both in device memory gets its new factors
+// there from the last kernel (by then every input of the batch has been read);
+// for the others they go through a device buffer and the staging.  (48 updates of
+// order 512: the download, two uploads a task and their threads took 2.5 of 17.9 ms.)
 static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<int> &run,
                                 int *ranks, int *status, cudaStream_t s) {
     const int nr = (int)run.size();
@@ -1487,9 +1489,10 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
     std::vector<size_t> pack_off;
     std::vector<long long> ws_off(nr);
     std::vector<size_t> out_off(nr);
+    std::vector<char> direct(nr);
     size_t n_pack = 0, n_out = 0;
     long long n_ws = 0;
-    int maxM = 1, maxK = 1;
+    int maxM = 1, maxK = 1, maxB = 1;
     for (int x = 0; x < nr; ++x) {
         const hcore_zlr_task &t = tasks[run[x]];
         const Src f[6] = {{t.AU, t.M, t.a, t.lda}, {t.AV, t.M, t.a, t.lda},
@@ -1505,10 +1508,12 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
         const int k = t.a + t.c;
         ws_off[x] = n_ws;
         n_ws += zlayout(t.M, t.a, t.b, k).total;
+        direct[x] = is_device_memory(t.CU) && is_device_memory(t.CV);
         out_off[x] = n_out;
-        n_out += 2 * (size_t)t.M * k;
+        if (!direct[x]) n_out += 2 * (size_t)t.M * k;
         maxM = std::max(maxM, t.M);
         maxK = std::max(maxK, k);
+        maxB = std::max(maxB, t.b);
     }
     ThreadCtx &tc = thread_ctx();
     const size_t stage = std::max(n_pack, n_out) * sizeof(zd);
@@ -1527,7 +1532,7 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
     ZDesc *ddesc = (ZDesc *)(arena + b_ws + b_out + b_in);
     int *drank = (int *)(arena + b_ws + b_out + b_in + b_desc), *dstat = drank + nr;
     cudaStreamSynchronize(tc.stream);   // the staging may still feed an earlier copy
-    parallel_for((int)src.size(), [&](int bi) {
+    if (n_pack > 0) parallel_for((int)src.size(), [&](int bi) {
         if (pack_off[bi] == SIZE_MAX) return;
         const Src &b = src[bi];
         zd *dst = pin + pack_off[bi];
@@ -1550,9 +1555,9 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
         d.ldau = ldv[0]; d.ldav = ldv[1]; d.ldbu = ldv[2];
         d.ldbv = ldv[3]; d.ldcu = ldv[4]; d.ldcv = ldv[5];
         const int k = t.a + t.c;
-        d.CUo = dout + out_off[x];
-        d.CVo = d.CUo + (size_t)t.M * k;
-        d.ldco = t.M;
+        d.CUo = direct[x] ? (zd *)t.CU : dout + out_off[x];
+        d.CVo = direct[x] ? (zd *)t.CV : d.CUo + (size_t)t.M * k;
+        d.ldco = direct[x] ? t.ldc : t.M;
         d.ws = ws_off[x];
         d.alpha = zd{t.alpha.re, t.alpha.im};
         d.beta = zd{t.beta.re, t.beta.im};
@@ -1570,23 +1575,26 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
              cudaSuccess) ||
         cudaMemcpyAsync(ddesc, desc.data(), nr * sizeof(ZDesc), cudaMemcpyHostToDevice, s) !=
             cudaSuccess ||
-        launch_zrecompress(ddesc, nr, dws, drank, dstat, maxM, maxK, s) != cudaSuccess ||
+        launch_zrecompress(ddesc, nr, dws, drank, dstat, maxM, maxK, maxB, s) != cudaSuccess ||
         cudaMemcpyAsync(rs.data(), drank, 2 * nr * sizeof(int), cudaMemcpyDeviceToHost, s) !=
             cudaSuccess ||
-        cudaMemcpyAsync(pin, dout, n_out * sizeof(zd), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+        (n_out > 0 &&
+         cudaMemcpyAsync(pin, dout, n_out * sizeof(zd), cudaMemcpyDeviceToHost, s) != cudaSuccess) ||
         cudaStreamSynchronize(s) != cudaSuccess) {
         set_error("hcore_gpu_zgemm_batched: %s", cudaGetErrorString(cudaGetLastError()));
         rc = HCORE_GPU_ECUDA;
     }
     cudaFree(arena);
     if (rc) return rc;
+    for (int x = 0; x < nr; ++x) {
+        status[run[x]] = rs[nr + x];
+        if (rs[nr + x] == HCORE_GPU_S_OK) ranks[run[x]] = rs[x];
+    }
     std::vector<int> copy_failed(nr, 0);
-    parallel_for(nr, [&](int x) {
+    if (n_out > 0) parallel_for(nr, [&](int x) {
         const hcore_zlr_task &t = tasks[run[x]];
-        const int q = run[x], r = rs[x], st = rs[nr + x];
-        status[q] = st;
-        if (st) return;
-        const int M = t.M, k = t.a + t.c;
+        if (direct[x] || rs[nr + x]) return;
+        const int M = t.M, k = t.a + t.c, r = rs[x];
         const zd *pU = pin + out_off[x], *pV = pU + (size_t)M * k;
         if (r > 0) {
             if (is_device_memory(t.CU) || is_device_memory(t.CV)) {
@@ -1602,7 +1610,6 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
                 }
             }
         }
-        ranks[q] = r;
     });
     for (int x = 0; x < nr; ++x)
         if (copy_failed[x]) {

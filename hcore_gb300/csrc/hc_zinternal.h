@@ -72,6 +72,6 @@ constexpr int kZApplyChunk = 4;   // reflectors staged per pass of the complex r
 int zsvd_kmax();
 // the four complex phases over n descriptors (M <= 1024, k <= zsvd_kmax())
 cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status,
-                               int maxM, int maxK, cudaStream_t s);
+                               int maxM, int maxK, int maxB, cudaStream_t s);
 
 }  // namespace hc

@@ -9,7 +9,7 @@
 // transpose puts conj(W) next to Q_B.)  Four phases, one grid each, as the
 // real kernels (hc_kernels.cu):
 //
-//   zstack_kernel   UA = [beta CU | alpha AU], F = AV^T BV, G = BU F^T, VB = [CV | G]
+//   zstack kernels  UA = [beta CU | alpha AU], F = AV^T BV, G = BU F^T, VB = [CV | G]
 //   zgeqrf_kernel   Householder QR of UA and VB (zlarfg conventions: beta real,
 //                   tau complex, H = I - tau v v^H, Q^H applied to the trailing columns)
 //   zgesvd_kernel   T = R_A R_B^T, QR with column pivoting T P = Q R (deflated
@@ -23,6 +23,7 @@
 // keeps both Jacobi matrices in shared memory (the embedding's 128 does not).
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cfloat>
 
 #include "hc_zinternal.h"
@@ -73,40 +74,68 @@ __device__ __forceinline__ double dmul_exp2(double x, int n) {
 // ---------------------------------------------------------------------------
 // phase 1: stack (hcore_zgemm.c:79-225 in complex arithmetic)
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) zstack_kernel(const ZDesc *__restrict__ descs,
-                                                     zd *__restrict__ ws) {
+// Two launches: F = AV^T BV, a warp for one column of F and a group of its rows
+// (the column of BV read once for kZf columns of AV), then row blocks of UA and
+// VB.  FP64 work, 4 M b (a + 1) multiply-adds an update: with one CTA per update
+// the whole phase took 1.10 ms for 48 updates of order 512, ranks 16-32, 0.44 now.
+constexpr int kZf = 4, kZsRows = 64;
+
+__global__ void __launch_bounds__(256) zstack_inner_kernel(const ZDesc *__restrict__ descs, zd *__restrict__ ws) {
     const ZDesc d = descs[blockIdx.x];
-    if (d.status0) return;
+    const int lane = threadIdx.x & 31, q = blockIdx.y * 8 + (threadIdx.x >> 5);
+    if (d.status0 || q >= d.b) return;
+    const int M = d.M, a = d.a;
+    zd *F = ws + d.ws + zlayout(M, a, d.b, d.k).F;
+    const zd *y = d.BV + (size_t)q * d.ldbv;
+    for (int p0 = blockIdx.z * kZf; p0 < a; p0 += gridDim.z * kZf) {
+        const zd *x[kZf];
+        zd s[kZf];
+#pragma unroll
+        for (int h = 0; h < kZf; ++h) {
+            x[h] = d.AV + (size_t)min(p0 + h, a - 1) * d.ldav;
+            s[h] = zmk(0, 0);
+        }
+        for (int l = lane; l < M; l += 32) {
+            const zd v = y[l];
+#pragma unroll
+            for (int h = 0; h < kZf; ++h) s[h] = zfma(x[h][l], v, s[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < kZf; ++h) {
+            s[h] = zwarp_sum(s[h]);
+            if (lane == 0 && p0 + h < a) F[(size_t)q * a + p0 + h] = s[h];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(256) zstack_outer_kernel(const ZDesc *__restrict__ descs, zd *__restrict__ ws) {
+    const ZDesc d = descs[blockIdx.x];
+    const int i = blockIdx.y * kZsRows + threadIdx.x % kZsRows, grp = threadIdx.x / kZsRows;
+    constexpr int NG = 256 / kZsRows;
+    if (d.status0 || i >= d.M) return;
     const int M = d.M, a = d.a, b = d.b, c = d.c;
     const ZLayout L = zlayout(M, a, b, d.k);
-    zd *UA = ws + d.ws + L.UA, *VB = ws + d.ws + L.VB, *F = ws + d.ws + L.F;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    for (long long e = tid; e < (long long)M * c; e += 256) {
-        const int i = (int)(e % M), j = (int)(e / M);
+    zd *UA = ws + d.ws + L.UA, *VB = ws + d.ws + L.VB;
+    const zd *F = ws + d.ws + L.F;
+    for (int j = grp; j < c; j += NG) {
         UA[(size_t)j * M + i] = zmul(d.beta, d.CU[(size_t)j * d.ldcu + i]);
         VB[(size_t)j * M + i] = d.CV[(size_t)j * d.ldcv + i];
     }
-    for (long long e = tid; e < (long long)M * a; e += 256) {
-        const int i = (int)(e % M), j = (int)(e / M);
-        UA[(size_t)(c + j) * M + i] = zmul(d.alpha, d.AU[(size_t)j * d.ldau + i]);
-    }
-    // F = AV^T BV (a x b), one warp per entry
-    for (int e = warp; e < a * b; e += 8) {
-        const int p = e % a, q = e / a;
-        const zd *x = d.AV + (size_t)p * d.ldav, *y = d.BV + (size_t)q * d.ldbv;
-        zd s = zmk(0, 0);
-        for (int l = lane; l < M; l += 32) s = zfma(x[l], y[l], s);
-        s = zwarp_sum(s);
-        if (lane == 0) F[(size_t)q * a + p] = s;
-    }
-    __syncthreads();
-    // G = BU F^T (M x a) after CV in VB
-    zd *G = VB + (size_t)c * M;
-    for (long long e = tid; e < (long long)M * a; e += 256) {
-        const int i = (int)(e % M), p = (int)(e / M);
-        zd s = zmk(0, 0);
-        for (int q = 0; q < b; ++q) s = zfma(d.BU[(size_t)q * d.ldbu + i], F[(size_t)q * a + p], s);
-        G[(size_t)p * M + i] = s;
+    UA += (size_t)c * M;
+    VB += (size_t)c * M;   // G = BU F^T (M x a) after CV
+    for (int j = grp; j < a; j += NG) UA[(size_t)j * M + i] = zmul(d.alpha, d.AU[(size_t)j * d.ldau + i]);
+    for (int p0 = grp * kZf; p0 < a; p0 += NG * kZf) {
+        zd s[kZf];
+#pragma unroll
+        for (int h = 0; h < kZf; ++h) s[h] = zmk(0, 0);
+        for (int q = 0; q < b; ++q) {
+            const zd u = d.BU[(size_t)q * d.ldbu + i];
+#pragma unroll
+            for (int h = 0; h < kZf; ++h) s[h] = zfma(u, F[(size_t)q * a + min(p0 + h, a - 1)], s[h]);
+        }
+#pragma unroll
+        for (int h = 0; h < kZf; ++h)
+            if (p0 + h < a) VB[(size_t)(p0 + h) * M + i] = s[h];
     }
 }
 
@@ -619,6 +648,7 @@ __global__ void __launch_bounds__(256, 1) zapply_kernel(const ZDesc *__restrict_
     const zd *tau = base + (side ? L.tauB : L.tauA);
     const zd *X0 = base + (side ? L.Vo : L.Uo);
     zd *out = side ? d.CVo : d.CUo;
+    const int ldo = d.ldco;
     const int tid = threadIdx.x, lane = tid & 31;
     const bool active = col < r;
     constexpr int ROWS = 32 * RPL;
@@ -658,7 +688,7 @@ __global__ void __launch_bounds__(256, 1) zapply_kernel(const ZDesc *__restrict_
 #pragma unroll
         for (int t = 0; t < RPL; ++t) {
             const int i = lane + 32 * t;
-            if (i < M) out[(size_t)col * d.ldco + i] = x[t];
+            if (i < M) out[(size_t)col * ldo + i] = x[t];
         }
     }
 }
@@ -685,11 +715,18 @@ int zsvd_kmax() {
 }
 
 cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status,
-                               int maxM, int maxK, cudaStream_t s) {
+                               int maxM, int maxK, int maxB, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int rpl = (maxM + 31) / 32;
-    if (rpl > 32 || maxK > zsvd_kmax()) return cudaErrorInvalidValue;
-    zstack_kernel<<<n, 256, 0, s>>>(d_desc, ws);
+    if (rpl > 32 || maxK > zsvd_kmax() || maxB > 8 * 65535) return cudaErrorInvalidValue;
+    int dev = 0, sms = 1, optin = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    // F: the z axis splits a column's rows while the grid is below two CTAs an SM
+    const int fy = (maxB + 7) / 8, fz = std::max(1, std::min((maxK + kZf - 1) / kZf, 2 * sms / std::max(1, n * fy)));
+    zstack_inner_kernel<<<dim3(n, fy, fz), 256, 0, s>>>(d_desc, ws);
+    zstack_outer_kernel<<<dim3(n, (maxM + kZsRows - 1) / kZsRows), 256, 0, s>>>(d_desc, ws);
     const size_t qsm = (size_t)maxM * sizeof(zd);
     zgeqrf_kernel<<<dim3(n, 2), 256, qsm, s>>>(d_desc, ws);
     // lanes per column pair: as many as fit in 256 threads, at most 4
@@ -700,10 +737,6 @@ cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, 
     // both Jacobi matrices in shared memory, unless that leaves one CTA per
     // SM while the batch has more updates than SMs: then V_J moves to the
     // workspace and three CTAs share an SM
-    int dev = 0, sms = 1, optin = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const bool aglobal = n > sms && 2 * zsvd_smem_bytes(maxK) > (size_t)optin;
     const size_t ssm = aglobal ? zsvd_smem_bytes_half(maxK) : zsvd_smem_bytes(maxK);
     cudaError_t e;
