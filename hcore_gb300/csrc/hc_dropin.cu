@@ -1568,6 +1568,11 @@ static int zgemm_batched_native(const hcore_zlr_task *tasks, const std::vector<i
         d.idx = x;
         d.status0 = 0;
     }
+    // the large updates first: a phase then ends with small ones
+    std::sort(desc.begin(), desc.end(), [](const ZDesc &x, const ZDesc &y) {
+        const double wx = (double)x.M * x.k * x.k, wy = (double)y.M * y.k * y.k;
+        return wx != wy ? wx > wy : x.idx < y.idx;
+    });
     int rc = HCORE_GPU_OK;
     std::vector<int> rs(2 * nr);
     if ((n_pack > 0 &&

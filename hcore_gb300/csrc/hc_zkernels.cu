@@ -10,7 +10,7 @@
 // real kernels (hc_kernels.cu):
 //
 //   zstack kernels  UA = [beta CU | alpha AU], F = AV^T BV, G = BU F^T, VB = [CV | G]
-//   zgeqrf_kernel   Householder QR of UA and VB (zlarfg conventions: beta real,
+//   zgeqrf_kernel   Householder QR of UA and VB, rows over a cluster (zlarfg conventions: beta real,
 //                   tau complex, H = I - tau v v^H, Q^H applied to the trailing columns)
 //   zgesvd_kernel   T = R_A R_B^T, QR with column pivoting T P = Q R (deflated
 //                   as the real kernel's), one-sided Jacobi on B = R^H with
@@ -26,6 +26,7 @@
 #include <algorithm>
 #include <cfloat>
 
+#include "hc_scalar.cuh"
 #include "hc_zinternal.h"
 
 namespace hc {
@@ -140,7 +141,7 @@ __global__ void __launch_bounds__(256) zstack_outer_kernel(const ZDesc *__restri
 }
 
 // ---------------------------------------------------------------------------
-// phase 2: Householder QR, one CTA (8 warps) per (update, side)
+// phase 2: Householder QR, a cluster of CTAs per (update, side)
 // ---------------------------------------------------------------------------
 // zlarfg on (alpha, ||x||^2): beta = -sign(Re alpha) sqrt(|alpha|^2 + ||x||^2),
 // tau = (beta - alpha) / beta, x scaled by 1 / (alpha - beta); tau = 0 when
@@ -152,66 +153,163 @@ __device__ __forceinline__ void zlarfg(zd alpha, double xn2, double &beta, zd &t
         scal = zmk(1, 0);
         return;
     }
-    beta = -copysign(sqrt(zabs2(alpha) + xn2), alpha.re);
+    const double n2 = zabs2(alpha) + xn2;
+    if (n2 > 1e-280 && n2 < 1e280) {   // the short square root and reciprocal (hc_scalar.cuh)
+        const double rs = inv_sqrt(n2);
+        double nb = n2 * rs;
+        nb = fma(fma(-nb, nb, n2) * 0.5, rs, nb);
+        beta = -copysign(nb, alpha.re);
+        const double ib = -copysign(rs, alpha.re), dr = alpha.re - beta;
+        tau = zmk(-dr * ib, -alpha.im * ib);
+        const double id = inv(fma(dr, dr, alpha.im * alpha.im));
+        scal = zmk(dr * id, -alpha.im * id);
+        return;
+    }
+    beta = -copysign(sqrt(n2), alpha.re);
     tau = zmk((beta - alpha.re) / beta, -alpha.im / beta);
     scal = zinv(zmk(alpha.re - beta, alpha.im));
 }
 
-__global__ void __launch_bounds__(256) zgeqrf_kernel(const ZDesc *__restrict__ descs,
-                                                     zd *__restrict__ ws) {
-    extern __shared__ unsigned char zsm[];
-    zd *sv = reinterpret_cast<zd *>(zsm);   // reflector v (M), zero above row j
-    __shared__ double red[8];
-    __shared__ zd s_tau, s_scal;
-    const ZDesc d = descs[blockIdx.x];
-    if (d.status0) return;
-    const int M = d.M, k = d.k, side = blockIdx.y;
+// The rows are split over the CTAs of a cluster (R each, a multiple of 32), which
+// keep them in shared memory from the first column to the last.  A step has one
+// exchange: every CTA sends its part of x^H y for x, the rows below j of column j
+// (not yet scaled), and every remaining column y, and the owner of row j that row,
+// to all CTAs; then each of them forms the reflector and its coefficients and
+// updates its rows.  Bound by FP64 issue (8 k^2 M / 2 multiply-adds a side), which
+// one SM per side made 2.95 ms for 48 updates of order 512, ranks 16-32; 1.71 now.
+// A warp takes four columns at a time, so that x is read once for them and their
+// eight sums share the shuffles (9 additions instead of 40).
+constexpr int kZqThreads = 256, kZqMaxCluster = 8;
+
+// shared memory of a CTA: slab k x R | partial sums 2 x 8 x k | row j 2 x k |
+// coefficients k | scales k | diagonal k
+__host__ __device__ inline size_t zqr_smem_bytes(int K, int R) {
+    return ((size_t)K * R + (size_t)(2 * kZqMaxCluster + 5) * K) * sizeof(zd);
+}
+
+__device__ __forceinline__ void zq_send(zd *local, int cta, int word, double v) {
+    unsigned at;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(at) : "r"((unsigned)__cvta_generic_to_shared(local) + 8u * word), "r"(cta));
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+__global__ void __launch_bounds__(kZqThreads) zgeqrf_kernel(const ZDesc *__restrict__ descs, zd *__restrict__ ws,
+                                                            int cs, int R, int K) {
+    extern __shared__ __align__(16) unsigned char zsm[];
+    const ZDesc d = descs[blockIdx.x / cs];
+    if (d.status0) return;   // (the whole cluster)
+    const int M = d.M, k = d.k, side = blockIdx.y, cta = blockIdx.x % cs, r0 = cta * R;
     const ZLayout L = zlayout(M, d.a, d.b, k);
     zd *A = ws + d.ws + (side ? L.VB : L.UA);
     zd *tau = ws + d.ws + (side ? L.tauB : L.tauA);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    zd *Y = reinterpret_cast<zd *>(zsm);                 // column c, row i: Y[c R + i]
+    zd *part = Y + (size_t)K * R;                        // [parity][source CTA][column]
+    zd *rowj = part + (size_t)2 * kZqMaxCluster * K;     // [parity][column]
+    zd *coef = rowj + 2 * (size_t)K, *scale = coef + K, *diag = scale + K;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nr = R / 32;
+    for (int c = warp; c < k; c += kZqThreads / 32)
+        for (int i = lane; i < R; i += 32) Y[(size_t)c * R + i] = r0 + i < M ? A[(size_t)c * M + r0 + i] : zmk(0, 0);
+    __syncthreads();
     for (int j = 0; j < k; ++j) {
-        zd *x = A + (size_t)j * M;
-        double ss = 0;
-        for (int i = j + 1 + tid; i < M; i += 256) ss += zabs2(x[i]);
-        ss = zwarp_sum(ss);
-        if (lane == 0) red[warp] = ss;
-        __syncthreads();
-        if (tid == 0) {
-            double t = 0;
-            for (int w = 0; w < 8; ++w) t += red[w];
+        const int par = j & 1, jl = j - r0;   // row j here if 0 <= jl < R
+        const bool owner = jl >= 0 && jl < R;
+        const int t0 = max(0, jl + 1) >> 5;   // 32-row pieces above are done
+        const zd *x = Y + (size_t)j * R;
+        zd *pt = part + (size_t)(par * kZqMaxCluster + cta) * K, *rj = rowj + par * K;
+        for (int g = j + 4 * warp; g < k; g += kZqThreads / 8) {
+            double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+            const zd *y[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) y[h] = Y + (size_t)min(g + h, k - 1) * R;
+            for (int t = t0; t < nr; ++t) {
+                const int i = lane + 32 * t;
+                const zd xi = i > jl ? x[i] : zmk(0, 0);
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    const zd s = zcfma(xi, y[h][i], zmk(v[2 * h], v[2 * h + 1]));
+                    v[2 * h] = s.re;
+                    v[2 * h + 1] = s.im;
+                }
+            }
+            // lane l comes to hold sum l >> 2
+#pragma unroll
+            for (int n = 4, o = 16; n >= 1; n /= 2, o /= 2) {
+                const bool up = lane & o;
+#pragma unroll
+                for (int e = 0; e < n; ++e) {
+                    const double keep = up ? v[e + n] : v[e], send = up ? v[e] : v[e + n];
+                    v[e] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                }
+            }
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+            const int c = g + (lane >> 3);
+            if (c < k)
+                for (int to = lane & 3; to < cs; to += 4) zq_send(pt + c, to, (lane >> 2) & 1, v[0]);
+        }
+        if (owner)
+            for (int e = tid; e < (k - j) * cs; e += kZqThreads) {
+                const int c = j + e / cs, to = e % cs;
+                const zd y = Y[(size_t)c * R + jl];
+                zq_send(rj + c, to, 0, y.re);
+                zq_send(rj + c, to, 1, y.im);
+            }
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        // two lanes a column (real and imaginary part); every warp with columns forms
+        // the reflector itself
+        const double *ps = reinterpret_cast<const double *>(part + (size_t)par * kZqMaxCluster * K);
+        for (int c0 = j + 16 * warp; c0 < k; c0 += kZqThreads / 2) {
+            double ss = lane < cs ? ps[((size_t)lane * K + j) * 2] : 0.0;
+#pragma unroll
+            for (int o = kZqMaxCluster / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            ss = __shfl_sync(0xffffffffu, ss, 0);
+            const int c = min(c0 + (lane >> 1), k - 1), im = lane & 1;
+            double w = 0;
+            for (int q = 0; q < cs; ++q) w += ps[((size_t)q * K + c) * 2 + im];
+            const double ow = __shfl_xor_sync(0xffffffffu, w, 1);
             double beta;
             zd tj, scal;
-            zlarfg(x[j], t, beta, tj, scal);
-            s_tau = tj;
-            tau[j] = tj;
-            s_scal = scal;
-            x[j] = zmk(beta, 0);          // R(j, j)
+            zlarfg(rj[j], ss, beta, tj, scal);
+            if (im == 0 && c0 + (lane >> 1) < k) {
+                if (c == j) {
+                    scale[j] = scal;
+                    diag[j] = zmk(beta, 0);
+                    if (cta == 0) tau[j] = tj;
+                } else {
+                    // conj(tau) v^H y, v = (1, scal x); then y -= that times v
+                    const zd s = zmul(zconj(tj), zadd(rj[c], zcmul(scal, zmk(w, ow))));
+                    coef[c] = zmul(s, scal);
+                    if (owner) Y[(size_t)c * R + jl] = zsub(rj[c], s);
+                }
+            }
         }
         __syncthreads();
-        const zd scal = s_scal;
-        for (int i = tid; i < M; i += 256) {
-            zd v = zmk(0, 0);
-            if (i > j) {
-                v = zmul(x[i], scal);
-                x[i] = v;
-            } else if (i == j) {
-                v = zmk(1, 0);
+        for (int g = j + 1 + 4 * warp; g < k; g += kZqThreads / 8) {
+            zd *y[4], s[4];
+#pragma unroll
+            for (int h = 0; h < 4; ++h) {
+                y[h] = Y + (size_t)min(g + h, k - 1) * R;
+                s[h] = coef[min(g + h, k - 1)];
             }
-            sv[i] = v;
+            for (int t = t0; t < nr; ++t) {
+                const int i = lane + 32 * t;
+                if (i <= jl) continue;
+                const zd xi = x[i];
+#pragma unroll
+                for (int h = 0; h < 4; ++h)
+                    if (g + h < k) y[h][i] = zfms(s[h], xi, y[h][i]);
+            }
         }
         __syncthreads();
-        // trailing columns: c <- c - conj(tau) (v^H c) v, one warp per column
-        const zd tc = zconj(s_tau);
-        if (s_tau.re != 0.0 || s_tau.im != 0.0)
-            for (int col = j + 1 + warp; col < k; col += 8) {
-                zd *y = A + (size_t)col * M;
-                zd s = zmk(0, 0);
-                for (int i = j + lane; i < M; i += 32) s = zcfma(sv[i], y[i], s);
-                s = zmul(tc, zwarp_sum(s));
-                for (int i = j + lane; i < M; i += 32) y[i] = zfms(s, sv[i], y[i]);
-            }
-        __syncthreads();
+    }
+    for (int c = warp; c < k; c += kZqThreads / 32) {
+        const zd sc = scale[c];
+        for (int i = lane; i < R && r0 + i < M; i += 32) {
+            const zd y = Y[(size_t)c * R + i];
+            A[(size_t)c * M + r0 + i] = r0 + i > c ? zmul(y, sc) : (r0 + i == c ? diag[c] : y);
+        }
     }
 }
 
@@ -703,6 +801,35 @@ static void launch_zapply(const ZDesc *d_desc, int n, const zd *ws, const int *d
                                                                       d_status);
 }
 
+// CTAs per cluster: enough that two CTAs share an SM, and more while SMs are idle
+// and every CTA keeps 64 rows (48 updates of order 512, ranks 16-32: four 1.75,
+// eight 1.72 ms)
+static cudaError_t launch_zgeqrf(const ZDesc *d_desc, int n, zd *ws, int maxM, int maxK, int sms, int optin,
+                                 cudaStream_t s) {
+    auto rows = [&](int cs) { return (maxM + 32 * cs - 1) / (32 * cs) * 32; };
+    int cs = 1;
+    while (cs < kZqMaxCluster && (2 * (zqr_smem_bytes(maxK, rows(cs)) + 1024) > (size_t)optin ||
+                                  (4 * n * cs <= 2 * sms && rows(2 * cs) >= 64)))
+        cs *= 2;
+    const int R = rows(cs);
+    const size_t smem = zqr_smem_bytes(maxK, R);
+    cudaError_t e = cudaFuncSetAttribute(zgeqrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n * cs, 2);
+    cfg.blockDim = dim3(kZqThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, zgeqrf_kernel, d_desc, ws, cs, R, maxK);
+}
+
 int zsvd_kmax() {
     int dev = 0, optin = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
@@ -727,8 +854,7 @@ cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, 
     const int fy = (maxB + 7) / 8, fz = std::max(1, std::min((maxK + kZf - 1) / kZf, 2 * sms / std::max(1, n * fy)));
     zstack_inner_kernel<<<dim3(n, fy, fz), 256, 0, s>>>(d_desc, ws);
     zstack_outer_kernel<<<dim3(n, (maxM + kZsRows - 1) / kZsRows), 256, 0, s>>>(d_desc, ws);
-    const size_t qsm = (size_t)maxM * sizeof(zd);
-    zgeqrf_kernel<<<dim3(n, 2), 256, qsm, s>>>(d_desc, ws);
+    if (cudaError_t e = launch_zgeqrf(d_desc, n, ws, maxM, maxK, sms, optin, s)) return e;
     // lanes per column pair: as many as fit in 256 threads, at most 4
     const int np = (maxK + 1) / 2;
     int G = 1;
