@@ -153,6 +153,10 @@ cudaError_t configure_svd_smem(int optin, int *kmax);
 template <typename T>
 void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
                      int G, cudaStream_t s);
+// the same with a cluster of cs CTAs per update
+template <typename T>
+cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
+                              int cs, cudaStream_t s);
 // SVD of larger updates: a cluster of CTAs each, sized for `updates` of them on
 // the GPU (hc_svd.cu)
 template <typename T>

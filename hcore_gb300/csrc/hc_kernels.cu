@@ -402,6 +402,22 @@ static int svd_smem_lanes(int K, const int *lanes, int updates) {
     return g;
 }
 
+// CTAs per update of the shared-memory SVD, the same bits whatever their number:
+// as many as leave each eight column pairs (one warp a sub-partition at 16 lanes a
+// pair), within the SMs that the plan's updates leave idle; one where that gives
+// fewer than four or the update has at most 24 pairs, since an exchange costs 0.8 us
+// of a round, about as much as it saves there.  FP32 rounds wait for latency, not
+// for a pipe.  SVD phase, one CTA and a cluster, us: one update of k = 40 550, 589;
+// 64 1403, 1175; 116 6241, 3556; 24 of k 80-116 5725, 4680 (six); 36 of k 16-56 913,
+// 841 (four); 48 of k 32-64 1355, 1389 (three).
+template <typename T>
+static int svd_spread(int K, const int *lanes, int updates) {
+    const int np = (K + 1) / 2;
+    if (sizeof(T) != sizeof(double) || np <= 24 || (np <= 64 ? lanes[1] : lanes[2]) >= 0) return 1;
+    const int cs = std::min({8, (np + 7) / 8, 152 / std::max(1, updates)});
+    return cs >= 4 ? cs : 1;
+}
+
 // ---------------------------------------------------------------------------
 // phase 4: CU = Q_A [U_r; 0], CV = Q_B [V_r S_r; 0]   (dormqr 'L','N')
 // ---------------------------------------------------------------------------
@@ -684,7 +700,12 @@ cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int
             const int K = bk.K;
             cudaStream_t sb = forked ? shape.side[b] : s;
             if (forked) cudaStreamWaitEvent(sb, shape.fork, 0);
-            if (K <= shape.svd_smem_kmax) {
+            const int cs = K <= shape.svd_smem_kmax ? svd_spread<T>(K, shape.svd_lanes, shape.updates) : 1;
+            if (cs > 1) {
+                const cudaError_t e =
+                    launch_svd_spread<T>(d_desc + bk.start, bk.count, ws, d_rank, d_status, d_info, K, cs, sb);
+                if (e != cudaSuccess) return e;
+            } else if (K <= shape.svd_smem_kmax) {
                 launch_svd_smem<T>(d_desc + bk.start, bk.count, ws, d_rank, d_status, d_info, K,
                                    svd_smem_lanes(K, shape.svd_lanes, shape.updates), sb);
             } else {

@@ -50,17 +50,20 @@
 //   * the scales keep their reciprocals, so no rotation divides;
 //   * comparisons of non-negative values run on the integer pipe;
 //   * the pivoted QR moves no column (a permutation instead), every warp
-//     finds the pivot and builds the reflector itself, so a step has one
-//     barrier; G lanes share a column there and in U_r = Q V_J as in the
-//     Jacobi.
+//     finds the pivot itself, and the inner products with the remaining
+//     columns run beside the reflector's parameters (which only warp 0 forms:
+//     every warp doing so took 1453 us, not 1403, below); up to eight lanes
+//     share a column there, G lanes in U_r = Q V_J as in the Jacobi.
 // SVD phase, with the kernel before (its parameters about 65 FP64 instructions a
 // round, two and, alone, four lanes per pair) and now, one GB300,
-// us: one update of k = 64 2388 -> 1453; 16 of k 8-24 485 -> 250; 384 of k
-// 12-68 4524 -> 3220; 1900 of the same 7272 -> 5747; FP32, 256 of k 10-48
-// 1139 -> 1050.  What bounds it now is the FP64 pipe of the one SM: in a round
+// us: one update of k = 64 2388 -> 1403; 16 of k 8-24 485 -> 249; 384 of k
+// 12-68 4524 -> 3200; 1900 of the same 7272 -> 5747; FP32, 256 of k 10-48
+// 1139 -> 1069.  What bounds it with one CTA is the FP64 pipe of the one SM: in a round
 // at k = 64 each of eight warps issues about 8 instructions of inner product,
 // 22 of rotation parameters and 32 of rows, two warps a sub-partition, at 64
-// cycles each (4.0 us of the 4.3 us measured).
+// cycles each (4.0 us of the 4.3 us measured).  Few updates of k > 48 therefore run
+// on a cluster of CTAs each (CL): 2.6 us a round at k = 64 with four CTAs, 0.8 of
+// them the exchange; the phase 1175 us.
 #include <cfloat>
 #include <climits>
 
@@ -175,21 +178,57 @@ __device__ __forceinline__ T group_sum(bool act, int start, int k, int lig, F f)
     return v;
 }
 
+// ---- a cluster of CTAs on one update -------------------------------------------
+__device__ __forceinline__ void cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// what to add to a shared-memory address here for the same place in CTA `to`
+__device__ __forceinline__ unsigned peer_delta(const void *any, int to) {
+    const unsigned here = (unsigned)__cvta_generic_to_shared(any);
+    unsigned there;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(to));
+    return there - here;
+}
+__device__ __forceinline__ void peer_store(double *p, unsigned delta, double v) {
+    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p) + delta), "d"(v)
+                 : "memory");
+}
+__device__ __forceinline__ void peer_store(float *p, unsigned delta, float v) {
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p) + delta), "f"(v)
+                 : "memory");
+}
+
 constexpr int kSvThreads = 512;
 constexpr int kSvRows = 6;   // 32-row pieces of the largest k (168)
+template <typename T>
+constexpr int kSvMaxK = sizeof(T) == 8 ? 119 : 168;
 
-template <typename T, int G>
+// CL: cs CTAs (a cluster) per update.  Each of them computes T and its pivoted QR
+// (the same bits), then takes a share of the pairs of every Jacobi round, pairs pi0
+// .. pi1 - 1 of the tournament, and so holds the current values of those pairs'
+// columns only.  From one round to the next a column moves by one pair, so a CTA
+// sends two columns to its neighbours' shared memory and one cluster barrier ends
+// the round.  Sums and rotations are the same as with one CTA, bit for bit: sums
+// over a column take up to eight lanes (D), rows G.
+template <typename T, int G, bool CL>
 __global__ void __launch_bounds__(kSvThreads, 1)
     svd_smem_kernel(const Desc *__restrict__ descs, T *__restrict__ ws, int *__restrict__ rank,
-                    int *__restrict__ status, int *__restrict__ info, int maxK) {
+                    int *__restrict__ status, int *__restrict__ info, int maxK, int cs) {
+    static_assert(CL || G <= 8, "a column's sum has eight parts");
+    constexpr int D = G < 8 ? G : 8;
+    __shared__ int s_big[2][CL ? 8 : 1];
+    __shared__ unsigned char s_own[CL ? kSvMaxK<T> : 1];   // (static: every byte takes from k <= 119)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ T s_wmax[kSvThreads / 32];
+    __shared__ T s_vj;
     __shared__ int s_rank;
-    const Desc d = descs[blockIdx.x];
+    const Desc d = descs[CL ? blockIdx.x / cs : blockIdx.x];
+    const int cr = CL ? blockIdx.x % cs : 0;   // this CTA's rank in the cluster
     const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5;
     const int nw = nthr >> 5;
     if (d.status0) {
-        if (tid == 0) {
+        if (tid == 0 && cr == 0) {
             status[d.idx] = d.status0;
             rank[d.idx] = 0;
             if (info) info[d.idx] = 0;
@@ -213,6 +252,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     short *s_pcol = s_perm + (maxK + 1);
     T *Yg = base + L.Uo;   // reflectors of Q (k x k, ld k) in the Uo slot until U_r is written
     const int grp = tid / G, lig = tid & (G - 1), ngrp = nthr / G;
+    const int qgrp = tid / D, dlig = tid & (D - 1), nqgrp = nthr / D;   // the QR's groups
 
     // ---- T = triu(R_A) triu(R_B)^T (hcore_dgemm.c:330-387): a warp per row,
     // the row of T replaces the row of R_A that only it reads --------------------
@@ -256,6 +296,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     if (lane == 0) s_wmax[warp] = amax;
     if (__syncthreads_or(bad)) {
         // a NaN or infinity: no decomposition; the update is not written
+        if (cr != 0) return;
         for (int t = tid; t < k; t += nthr) base[L.sig + t] = T(NAN);
         if (tid == 0) {
             int r = d.rk != 0 && d.rk < k ? d.rk : k;
@@ -275,11 +316,10 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     for (int c0 = 0; c0 < k; c0 += ngrp) {
         const int c = c0 + grp;
         T *ac = A + (size_t)c * ld;
-        const T s = group_sum<G, T>(c < k, 0, k, lig, [&](int i) {
-            const T x = sexp != 0 ? mul_exp2(ac[i], -sexp) : ac[i];
-            ac[i] = x;
-            return x * x;
-        });
+        if (c < k && sexp != 0)
+            for (int i = lig; i < k; i += G) ac[i] = mul_exp2(ac[i], -sexp);
+        if (G > D) __syncwarp();
+        const T s = group_sum<D, T>(c < k, 0, k, dlig, [&](int i) { return ac[i] * ac[i]; });
         if (c < k && lig == 0) {
             X0[c] = s;    // norms of rows j.. of column c, squared; -1: pivoted already
             s_d[c] = s;   // the same at the last exact computation
@@ -325,45 +365,60 @@ __global__ void __launch_bounds__(kSvThreads, 1)
             }
         }
         // the reflector of column pv, rows j.., unscaled: v = (alpha - beta, x),
-        // beta = -sign(alpha) ||(alpha, x)|| (dlarfg's), g = beta (beta - alpha)
+        // beta = -sign(alpha) ||(alpha, x)|| (dlarfg's), g = beta (beta - alpha),
+        // by warp 0 while the others form x^T y for the remaining columns y
         const T *ap = A + (size_t)pv * ld;
-        const T alpha = ap[j];
-        T ss = 0;
-        for (int i = j + 1 + lane; i < k; i += 32) ss += ap[i] * ap[i];
-        ss = warp_sum(ss);
-        T beta = alpha, vj = 0, ginv = 0;
-        if (ss > SvLim<T>::safmin) {
-            const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
-            T nb = n2 * rs;
-            nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
-            beta = -copysign(nb, alpha);
-            vj = alpha - beta;
-            ginv = inv(fma(-alpha, beta, n2));
+        if (warp == 0) {
+            const T alpha = ap[j];
+            T ss = 0;
+            for (int i = j + 1 + lane; i < k; i += 32) ss += ap[i] * ap[i];
+            ss = warp_sum(ss);
+            T beta = alpha, vj = 0, ginv = 0;
+            if (ss > SvLim<T>::safmin) {
+                const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
+                T nb = n2 * rs;
+                nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
+                beta = -copysign(nb, alpha);
+                vj = alpha - beta;
+                ginv = inv(fma(-alpha, beta, n2));
+            }
+            if (lane == 0) {
+                s_pcol[j] = (short)pv;
+                s_rd[j] = beta;
+                s_tau[j] = ginv;
+                s_vj = vj;
+            }
         }
-        if (tid == 0) {
-            s_pcol[j] = (short)pv;
-            s_rd[j] = beta;
-            s_tau[j] = ginv;
+        for (int c0 = 0; c0 < k; c0 += nqgrp) {
+            const int c = c0 + qgrp;
+            const bool act = c < k && c != pv && key(nr[c]) >= 0;
+            const T *ac = A + (size_t)c * ld;
+            const T w = group_sum<D, T>(act, j + 1, k, dlig, [&](int i) { return ap[i] * ac[i]; });
+            if (act && dlig == 0) nr2[c] = w;   // (kept where the column's new norm goes)
         }
-        // apply it to the other remaining columns and downdate their norms
-        // (dlaqp2's rule), G lanes per column
-        const int i0 = j + 1 + ((lig - (j + 1)) & (G - 1));
-        for (int c0 = 0; c0 < k; c0 += ngrp) {
-            const int c = c0 + grp;
+        __syncthreads();
+        // apply it to them and downdate their norms (dlaqp2's rule), D lanes per column
+        const T ginv = s_tau[j], vj = s_vj;
+        const int i0 = j + 1 + ((dlig - (j + 1)) & (D - 1));
+        for (int c0 = 0; c0 < k; c0 += nqgrp) {
+            const int c = c0 + qgrp;
             const T nc = c < k ? nr[c] : T(-1);
             const bool act = c < k && c != pv && key(nc) >= 0;
             T *ac = A + (size_t)c * ld;
             const bool upd = act && ginv != T(0);
-            const T acj = upd && lig == 0 ? ac[j] : T(0);
             // (row j's term, in lane 0's hands, is added to the sum of the rows below)
-            T s = group_sum<G, T>(upd, j + 1, k, lig, [&](int i) { return ap[i] * ac[i]; });
-            s = ginv * fma(vj, __shfl_sync(0xffffffffu, acj, lane & ~(G - 1)), s);
+            T acj = 0, s = 0;
+            if (upd && dlig == 0) {
+                acj = ac[j];
+                s = ginv * fma(vj, acj, nr2[c]);
+            }
+            s = __shfl_sync(0xffffffffu, s, lane & ~(D - 1));
             T nn = 0;
             bool redo = false;
             if (act) {
                 if (upd)
-                    for (int i = i0; i < k; i += G) ac[i] -= s * ap[i];
-                if (lig == 0) {
+                    for (int i = i0; i < k; i += D) ac[i] -= s * ap[i];
+                if (dlig == 0) {
                     const T r = upd ? acj - s * vj : ac[j];
                     ac[j] = r;
                     nn = nc - r * r;
@@ -371,14 +426,14 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 }
             }
             if (__any_sync(0xffffffffu, redo)) {
-                redo = __shfl_sync(0xffffffffu, (int)redo, lane & ~(G - 1)) != 0;
-                const T q = group_sum<G, T>(redo, j + 1, k, lig, [&](int i) { return ac[i] * ac[i]; });
-                if (redo && lig == 0) {
+                redo = __shfl_sync(0xffffffffu, (int)redo, lane & ~(D - 1)) != 0;
+                const T q = group_sum<D, T>(redo, j + 1, k, dlig, [&](int i) { return ac[i] * ac[i]; });
+                if (redo && dlig == 0) {
                     nn = q;
                     s_d[c] = q;
                 }
             }
-            if (c < k && lig == 0) nr2[c] = act ? nn : T(-1);
+            if (c < k && dlig == 0) nr2[c] = act ? nn : T(-1);
         }
         __syncthreads();
     }
@@ -399,7 +454,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
         const T *ah = A + (size_t)s_pcol[h] * ld;
         for (int i = lane; i < k; i += 32) {
             const T x = ah[i];
-            if (h < kk) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rd[h] : T(0));
+            if (h < kk && cr == 0) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rd[h] : T(0));
             // R(i, h)
             B[(size_t)i * ld + h] = i < kk ? (i < h ? x : (i == h ? s_rd[h] : T(0))) : T(0);
         }
@@ -408,45 +463,49 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     for (int c = warp; c < k; c += nw)
         for (int i = lane; i < k; i += 32) A[(size_t)c * ld + i] = i == c ? T(1) : T(0);
     T *s_nrm = X0, *s_sig = X1;
-    auto column_norms = [&](bool fold) {
-        for (int c0 = 0; c0 < k; c0 += ngrp) {
-            const int c = c0 + grp;
-            T dj = 1;
-            T *xj = B + (size_t)c * ld;
-            if (c < kk) {
-                if (fold) {
-                    dj = s_d[c];
-                    if (dj < SvLim<T>::tiny_scale) {   // fold a scale before it underflows
-                        T *vj = A + (size_t)c * ld;
-                        for (int i = lig; i < k; i += G) {
-                            xj[i] *= dj;
-                            vj[i] *= dj;
-                        }
-                        dj = 1;
-                    }
+    auto column_norm = [&](int c, bool fold) {   // of column c, by its group
+        T dj = 1;
+        T *xj = B + (size_t)c * ld;
+        if (c < kk && fold) {
+            dj = s_d[c];
+            if (dj < SvLim<T>::tiny_scale) {   // fold a scale before it underflows
+                T *vj = A + (size_t)c * ld;
+                for (int i = lig; i < k; i += G) {
+                    xj[i] *= dj;
+                    vj[i] *= dj;
                 }
-            }
-            const T s = group_sum<G, T>(c < kk, 0, k, lig, [&](int i) { return xj[i] * xj[i]; });
-            if (c < k && lig == 0) {
-                s_nrm[c] = c < kk ? dj * dj * s : T(0);
-                s_d[c] = dj;
-                s_rd[c] = fold && c < kk ? inv(dj) : T(1);
+                dj = 1;
             }
         }
+        __syncwarp();
+        const T s = group_sum<D, T>(c < kk, 0, k, dlig, [&](int i) { return xj[i] * xj[i]; });
+        if (c < k && lig == 0) {
+            s_nrm[c] = c < kk ? dj * dj * s : T(0);
+            s_d[c] = dj;
+            s_rd[c] = fold && c < kk ? inv(dj) : T(1);
+        }
+    };
+    auto column_norms = [&](bool fold) {
+        for (int c0 = 0; c0 < k; c0 += ngrp) column_norm(c0 + grp, fold);
     };
     column_norms(false);
-    __syncthreads();
+    if constexpr (CL) cluster_sync(); else __syncthreads();
 
     // ---- one-sided Jacobi on B = R^T, rotations accumulated in A ----------------
     // (columns kk.. of B are zero and take no part, V_J's rows kk.. stay zero)
     const int n = kk + (kk & 1), np = n / 2;
+    // this CTA's pairs (a CTA without any only takes part in the barriers)
+    const int active = CL ? max(1, min(cs, np)) : 1;
+    const int pi0 = CL ? min(cr, active) * np / active : 0, pi1 = CL ? min(cr + 1, active) * np / active : np;
+    const unsigned left = CL && pi0 > 0 && cr < active ? peer_delta(A, cr - 1) : 0;
+    const unsigned right = CL && pi1 < np ? peer_delta(A, cr + 1) : 0;
     const float tol = (float)(k > 8 ? k : 8) * (sizeof(T) == 8 ? (float)DBL_EPSILON : FLT_EPSILON);
     bool converged = kk <= 1;
     int sweeps = 0;
     for (; sweeps < kMaxSweeps && !converged; ++sweeps) {
         bool big = false;   // this thread rotated a pair above sqrt(tol)
         for (int round = 0; round < n - 1; ++round) {
-            for (int b0 = 0; b0 < np; b0 += ngrp) {
+            for (int b0 = pi0; b0 < pi1; b0 += ngrp) {
                 // circle-method tournament: pair 0 is (n - 1, round), pair i
                 // (round + i, round - i) mod n - 1
                 const int pi = b0 + grp;
@@ -454,7 +513,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 if (p >= n - 1) p -= n - 1;
                 if (q < 0) q += n - 1;
                 if (pi == 0) p = n - 1;
-                const bool valid = pi < np && p < kk && q < kk;
+                const bool valid = pi < pi1 && p < kk && q < kk;
                 T *xp = B + (size_t)p * ld, *xq = B + (size_t)q * ld;
                 T app = 0, aqq = 0, dp = 1, dq = 1;
                 if (valid) {
@@ -463,7 +522,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                     dp = s_d[p];
                     dq = s_d[q];
                 }
-                const T dot = group_sum<G, T>(valid, 0, k, lig, [&](int i) { return xp[i] * xq[i]; });
+                const T dot = group_sum<D, T>(valid, 0, k, dlig, [&](int i) { return xp[i] * xq[i]; });
                 bool rot = false, redo_p = false, redo_q = false;
                 T np_ = 0, nq_ = 0, dp2 = 1, dq2 = 1, rdp2 = 1, rdq2 = 1;
                 if (valid) {
@@ -509,8 +568,9 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 }
                 // strong cancellation in a tracked norm: recompute
                 if (__any_sync(0xffffffffu, redo_p || redo_q)) {
-                    const T sp = group_sum<G, T>(redo_p, 0, k, lig, [&](int i) { return xp[i] * xp[i]; });
-                    const T sq = group_sum<G, T>(redo_q, 0, k, lig, [&](int i) { return xq[i] * xq[i]; });
+                    if (G > D) __syncwarp();
+                    const T sp = group_sum<D, T>(redo_p, 0, k, dlig, [&](int i) { return xp[i] * xp[i]; });
+                    const T sq = group_sum<D, T>(redo_q, 0, k, dlig, [&](int i) { return xq[i] * xq[i]; });
                     if (redo_p) np_ = dp2 * dp2 * sp;
                     if (redo_q) nq_ = dq2 * dq2 * sq;
                 }
@@ -522,11 +582,61 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                     s_rd[p] = rdp2;
                     s_rd[q] = rdq2;
                 }
+                if constexpr (CL) {
+                    // the next round has p in pair pi - 1 and q in pair pi + 1
+                    auto send = [&](int c, unsigned to) {
+                        T *x = B + (size_t)c * ld, *v = A + (size_t)c * ld;
+                        for (int i = lig; i < k; i += G) {
+                            peer_store(x + i, to, x[i]);
+                            if (i < kk) peer_store(v + i, to, v[i]);
+                        }
+                        if (lig == 0) {
+                            peer_store(s_nrm + c, to, s_nrm[c]);
+                            peer_store(s_d + c, to, s_d[c]);
+                            peer_store(s_rd + c, to, s_rd[c]);
+                        }
+                    };
+                    if (pi == pi0 && pi > 0 && p < kk) send(p, left);
+                    if (pi == pi1 - 1 && pi1 < np && q < kk) send(q, right);
+                    __syncwarp();
+                }
             }
-            __syncthreads();
+            if constexpr (CL) cluster_sync(); else __syncthreads();
         }
-        column_norms(true);   // exact norms once per sweep
-        converged = !__syncthreads_or(big);
+        // exact norms once per sweep (every column is back in its first pair)
+        if constexpr (CL) {
+            for (int b0 = pi0; b0 < pi1; b0 += ngrp) {
+                const int pi = b0 + grp;
+                column_norm(pi < pi1 ? (pi == 0 ? n - 1 : pi) : k, true);
+                column_norm(pi < pi1 ? (pi == 0 ? 0 : n - 1 - pi) : k, true);
+            }
+            const int any = __syncthreads_or(big);
+            if (tid < cs)
+                asm volatile("st.shared::cluster.u32 [%0], %1;" ::
+                             "r"((unsigned)__cvta_generic_to_shared(&s_big[sweeps & 1][cr]) + peer_delta(A, tid)),
+                             "r"(any) : "memory");
+            cluster_sync();
+            converged = true;
+            for (int t = 0; t < cs; ++t) converged = converged && !s_big[sweeps & 1][t];
+        } else {
+            column_norms(true);
+            converged = !__syncthreads_or(big);
+        }
+    }
+    auto owner = [&](int j) {   // the CTA that holds column j
+        const int pi = j == n - 1 ? 0 : (j < np ? j : n - 1 - j);
+        int o = 0;
+        while (o + 1 < active && (o + 1) * np / active <= pi) ++o;
+        return j < kk ? o : 0;
+    };
+    if constexpr (CL) {
+        for (int j = warp; j < kk; j += nw)
+            if (owner(j) == cr && lane < cs && lane != cr) {
+                const unsigned to = peer_delta(A, lane);
+                peer_store(s_nrm + j, to, s_nrm[j]);
+                peer_store(s_d + j, to, s_d[j]);
+            }
+        cluster_sync();
     }
 
     // singular values = true column norms of B (of the scaled T), descending,
@@ -556,7 +666,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     for (int t = tid; t < k; t += nthr) {
         const T s = s_sig[s_perm[t]];
         const T v = key(s) < 0 ? T(NAN) : mul_exp2(s, sexp);
-        base[L.sig + t] = v;
+        if (cr == 0) base[L.sig + t] = v;
         if (d.rk == 0 && t >= d.rank_start && v < thr) atomicMin(&s_rank, t);
     }
     __syncthreads();
@@ -575,9 +685,19 @@ __global__ void __launch_bounds__(kSvThreads, 1)
         T *Uo = base + L.Uo, *Vo = base + L.Vo;
         for (int t = warp; t < r; t += nw) {
             const int j = s_perm[t];
+            if (CL && owner(j) != cr) continue;
             const T f = s_d[j];
             for (int i = lane; i < k; i += 32)
                 Vo[(size_t)t * k + s_pcol[i]] = mul_exp2(f * B[(size_t)j * ld + i], sexp);
+        }
+        int nown = r;   // the columns of U_r that this CTA forms
+        if constexpr (CL) {
+            nown = 0;
+            for (int t = 0; t < r; ++t) {
+                const bool mine = owner(s_perm[t]) == cr;
+                if (mine && tid == 0) s_own[nown] = (unsigned char)t;
+                nown += mine;
+            }
         }
         __syncthreads();
         // U_r = Q (V_J's true columns), Q = H_0 ... H_{kk-1}: the reflectors
@@ -585,10 +705,10 @@ __global__ void __launch_bounds__(kSvThreads, 1)
         // columns of V_J
         for (int h = warp; h < kk; h += nw)
             for (int i = lane; i < k; i += 32) B[(size_t)h * ld + i] = Yg[(size_t)h * k + i];
-        __syncthreads();
-        for (int t0 = 0; t0 < r; t0 += ngrp) {
-            const int t = t0 + grp;
-            const bool act = t < r;
+        if constexpr (CL) cluster_sync(); else __syncthreads();   // Yg is Uo's place
+        for (int t0 = 0; t0 < nown; t0 += ngrp) {
+            const bool act = t0 + grp < nown;
+            const int t = !act ? 0 : (CL ? s_own[t0 + grp] : t0 + grp);
             const int j = act ? s_perm[t] : 0;
             T *x = A + (size_t)j * ld;   // each group owns the column of its own j
             if (act) {
@@ -600,7 +720,8 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 if (gi == T(0)) continue;
                 const T *y = B + (size_t)h * ld;
                 const int i0 = h + ((lig - h) & (G - 1));
-                const T s = gi * group_sum<G, T>(act, h, k, lig, [&](int i) { return y[i] * x[i]; });
+                if (G > D) __syncwarp();
+                const T s = gi * group_sum<D, T>(act, h, k, dlig, [&](int i) { return y[i] * x[i]; });
                 if (act)
                     for (int i = i0; i < k; i += G) x[i] -= s * y[i];
             }
@@ -608,7 +729,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 for (int i = lig; i < k; i += G) Uo[(size_t)t * k + i] = x[i];
         }
     }
-    if (tid == 0) {
+    if (tid == 0 && cr == 0) {
         rank[d.idx] = r;
         status[d.idx] = st;
         if (info) info[d.idx] = sweeps;
@@ -642,11 +763,6 @@ size_t smem_bytes(int K) {
 // CTA an update fills the GPU either way, 32.1, 34.6 (their whole plan 52.4,
 // 45.8).
 constexpr int kClThreads = 256, kClMax = 8;
-
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <typename T, int G, int R>
 __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
@@ -1080,9 +1196,9 @@ __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
 
 template <typename T>
 cudaError_t configure_svd_smem(int optin, int *kmax) {
-    using K = void (*)(const Desc *, T *, int *, int *, int *, int);
-    const K kernels[] = {svd_smem_kernel<T, 1>, svd_smem_kernel<T, 2>, svd_smem_kernel<T, 4>,
-                         svd_smem_kernel<T, 8>};
+    using K = void (*)(const Desc *, T *, int *, int *, int *, int, int);
+    const K kernels[] = {svd_smem_kernel<T, 1, false>, svd_smem_kernel<T, 2, false>, svd_smem_kernel<T, 4, false>,
+                         svd_smem_kernel<T, 8, false>, svd_smem_kernel<T, 8, true>, svd_smem_kernel<T, 16, true>};
     int dyn = optin;
     for (K f : kernels) {
         cudaFuncAttributes fa;
@@ -1091,7 +1207,7 @@ cudaError_t configure_svd_smem(int optin, int *kmax) {
         dyn = dyn < optin - (int)fa.sharedSizeBytes ? dyn : optin - (int)fa.sharedSizeBytes;
     }
     int k = 0;
-    while (k < 32 * kSvRows && smem_bytes<T>(k + 1) <= (size_t)dyn) ++k;
+    while (k < kSvMaxK<T> && smem_bytes<T>(k + 1) <= (size_t)dyn) ++k;
     *kmax = k;
     for (K f : kernels) {
         const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn);
@@ -1104,8 +1220,29 @@ template <typename T, int G>
 static void launch_svd_g(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info,
                          int K, cudaStream_t s) {
     const int np = (K + 1) / 2, t = (np * G + 31) / 32 * 32;
-    svd_smem_kernel<T, G><<<n, t < kSvThreads ? t : kSvThreads, smem_bytes<T>(K), s>>>(
-        d_desc, ws, d_rank, d_status, d_info, K);
+    svd_smem_kernel<T, G, false><<<n, t < kSvThreads ? t : kSvThreads, smem_bytes<T>(K), s>>>(
+        d_desc, ws, d_rank, d_status, d_info, K, 1);
+}
+
+// cs CTAs per update
+template <typename T>
+cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
+                              int cs, cudaStream_t s) {
+    const int pairs = ((K + 1) / 2 + cs - 1) / cs;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n * cs);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem_bytes<T>(K);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    auto go = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, d_info, K, cs); };
+    return pairs <= 8 ? go(svd_smem_kernel<T, 16, true>) : go(svd_smem_kernel<T, 8, true>);
 }
 
 template <typename T>
@@ -1150,6 +1287,11 @@ template void launch_svd_smem<double>(const Desc *, int, double *, int *, int *,
                                       cudaStream_t);
 template void launch_svd_smem<float>(const Desc *, int, float *, int *, int *, int *, int, int,
                                      cudaStream_t);
+
+template cudaError_t launch_svd_spread<double>(const Desc *, int, double *, int *, int *, int *, int, int,
+                                               cudaStream_t);
+template cudaError_t launch_svd_spread<float>(const Desc *, int, float *, int *, int *, int *, int, int,
+                                              cudaStream_t);
 
 template cudaError_t launch_svd_cluster<double>(const Desc *, int, double *, int *, int *, int *, int, int,
                                                 cudaStream_t);
