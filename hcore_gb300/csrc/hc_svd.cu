@@ -118,35 +118,6 @@ __device__ __forceinline__ bool pair_test(float app, float aqq, float apq, float
     return apq != 0.f && x > tol * tol * y;
 }
 
-// t = v / (|w| + sqrt(w^2 + v^2)) with the sign of w v (w = 0: of v), the
-// tangent of the rotation that makes the pair orthogonal, w = a_qq - a_pp,
-// v = 2 a_pq
-__device__ __forceinline__ double tangent(double app, double aqq, double apq) {
-    const double w = aqq - app;
-    float mw, mv;
-    int ew, ev;
-    split(w, mw, ew);
-    split(apq, mv, ev);
-    ev += 1;
-    if (ew == 0) {   // equal norms: 45 degrees
-        mw = 0.f;
-        ew = ev;
-    }
-    const int em = max(ew, ev), dv = ev - em;
-    const float fw = mw * __int_as_float((max(ew - em, -60) + 127) << 23);
-    const float fv = mv * __int_as_float((max(dv, -60) + 127) << 23);
-    const float q = __fdividef(mv, fw + fsqrt_fast(fmaf(fw, fw, fv * fv)));
-    const double t = widen(q, dv);
-    const int sgn = ((ew == ev && mw == 0.f ? 0 : __double2hiint(w)) ^ __double2hiint(apq)) & (int)0x80000000;
-    return __hiloint2double(__double2hiint(t) | sgn, __double2loint(t));
-}
-__device__ __forceinline__ float tangent(float app, float aqq, float apq) {
-    const float w = aqq - app, v = 2.f * apq;
-    const float h = sqrtf(fmaf(w, w, v * v));
-    const float t = fabsf(v) / (fabsf(w) + h);
-    return (w < 0.f) != (v < 0.f) ? -t : t;
-}
-
 // Sum of f(i) over start <= i < k by a group of G lanes (rows i = lig mod G
 // each): eight partial sums by i mod 8, added in one fixed tree, so the result
 // does not depend on G.
@@ -176,27 +147,6 @@ __device__ __forceinline__ T group_sum(bool act, int start, int k, int lig, F f)
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// ---- a cluster of CTAs on one update -------------------------------------------
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// what to add to a shared-memory address here for the same place in CTA `to`
-__device__ __forceinline__ unsigned peer_delta(const void *any, int to) {
-    const unsigned here = (unsigned)__cvta_generic_to_shared(any);
-    unsigned there;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(here), "r"(to));
-    return there - here;
-}
-__device__ __forceinline__ void peer_store(double *p, unsigned delta, double v) {
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p) + delta), "d"(v)
-                 : "memory");
-}
-__device__ __forceinline__ void peer_store(float *p, unsigned delta, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(p) + delta), "f"(v)
-                 : "memory");
 }
 
 constexpr int kSvThreads = 512;
@@ -611,10 +561,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 column_norm(pi < pi1 ? (pi == 0 ? 0 : n - 1 - pi) : k, true);
             }
             const int any = __syncthreads_or(big);
-            if (tid < cs)
-                asm volatile("st.shared::cluster.u32 [%0], %1;" ::
-                             "r"((unsigned)__cvta_generic_to_shared(&s_big[sweeps & 1][cr]) + peer_delta(A, tid)),
-                             "r"(any) : "memory");
+            if (tid < cs) peer_store(&s_big[sweeps & 1][cr], peer_delta(A, tid), any);
             cluster_sync();
             converged = true;
             for (int t = 0; t < cs; ++t) converged = converged && !s_big[sweeps & 1][t];

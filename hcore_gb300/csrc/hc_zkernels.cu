@@ -14,7 +14,7 @@
 //                   tau complex, H = I - tau v v^H, Q^H applied to the trailing columns)
 //   zgesvd_kernel   T = R_A R_B^T, QR with column pivoting T P = Q R (deflated
 //                   as the real kernel's), one-sided Jacobi on B = R^H with
-//                   complex column scales, rank rule;
+//                   real column scales, rank rule;
 //                   U_r = Q V_J, conj(W_r S_r) = conj(P (rotated B))
 //   zapply_kernel   CU = Q_A [U_r; 0], CV = Q_B [conj(W_r S_r); 0]
 //
@@ -67,11 +67,6 @@ __device__ __forceinline__ double zwarp_sum(double v) {
     return v;
 }
 __device__ __forceinline__ zd zwarp_sum(zd v) { return zd{zwarp_sum(v.re), zwarp_sum(v.im)}; }
-__device__ __forceinline__ double dmul_exp2(double x, int n) {
-    return (x * __longlong_as_double((long long)(n / 2 + 1023) << 52)) *
-           __longlong_as_double((long long)(n - n / 2 + 1023) << 52);
-}
-
 // ---------------------------------------------------------------------------
 // phase 1: stack (hcore_zgemm.c:79-225 in complex arithmetic)
 // ---------------------------------------------------------------------------
@@ -316,406 +311,531 @@ __global__ void __launch_bounds__(kZqThreads) zgeqrf_kernel(const ZDesc *__restr
 // ---------------------------------------------------------------------------
 // phase 3: SVD of T = R_A R_B^T, both Jacobi matrices in shared memory
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void zrr_pair(int round, int pi, int n, int &p, int &q) {
-    if (pi == 0) {
-        p = n - 1;
-        q = round;
-    } else {
-        p = (round + pi) % (n - 1);
-        q = (round - pi + (n - 1)) % (n - 1);
-    }
+// Written as the real kernel (hc_svd.cu): the same pivoted QR, deflation, tournament
+// of column pairs, FP32 tangents and short reciprocals.  Bound by the FP64 FMAs of
+// the rotations' rows (16 a pair of rows and matrix column, four times the real
+// kernel's), so few updates take a cluster of CTAs each (CL), which share a round's
+// pairs and pass columns on as there.
+//
+// Rotations: column j is sqrt(w_j) x_j in B = R^H and in V_J, w_j real (a common
+// phase of a column of both cancels in U_r conj(W_r S_r)^T, so none is kept).  With
+// s = x_p^H x_q, m = |a_pq| = sqrt(w_p w_q) |s| and t the real Jacobi tangent of
+// (a_pp, a_qq, m): x_p -= (t / m) w_q conj(s) x_q, x_q += (t / m) w_p s x_p, w_p and
+// w_q divided by 1 + t^2: no square root but 1 / m, no complex scale.
+// SVD phase of 48 updates of order 512, ranks 16-32 (k 32-64): 4.87 ms with one CTA
+// an update, four lanes a pair, complex scales, a thread per column in the QR and in
+// U_r; 2.77 now.
+constexpr int kZvThreads = 384, kZvRows = 3;   // (k <= 96)
+
+// sum over a group of G lanes: real and imaginary part take half of the lanes each
+template <int G>
+__device__ __forceinline__ zd zgroup_add(zd v, int lig) {
+    const bool up = lig & (G / 2);
+    double r = up ? v.im : v.re;
+    r += __shfl_xor_sync(0xffffffffu, up ? v.re : v.im, G / 2);
+#pragma unroll
+    for (int o = G / 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+    const double other = __shfl_xor_sync(0xffffffffu, r, G / 2);
+    return up ? zmk(other, r) : zmk(r, other);
+}
+// sum of conj(x_i) y_i, start <= i < k, by a group of G lanes
+template <int G>
+__device__ __forceinline__ zd zgroup_dot(bool act, const zd *x, const zd *y, int start, int k, int lig) {
+    zd v = zmk(0, 0);
+    if (act)
+        for (int i = start + ((lig - start) & (G - 1)); i < k; i += G) v = zcfma(x[i], y[i], v);
+    return zgroup_add<G>(v, lig);
+}
+// sum of |x_i|^2, start <= i < k, by a group of G lanes
+template <int G>
+__device__ __forceinline__ double zgroup_norm(bool act, const zd *x, int start, int k, int lig) {
+    double v = 0, w = 0;
+    if (act)
+        for (int i = start + ((lig - start) & (G - 1)); i < k; i += G) {
+            v = fma(x[i].re, x[i].re, v);
+            w = fma(x[i].im, x[i].im, w);
+        }
+    v += w;
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+}
+// is the pair to be rotated, m2 > tol^2 app aqq, and above the stopping level (big)?
+__device__ __forceinline__ bool zpair_test(double app, double aqq, double m2, float tol, bool &big) {
+    float mp, mq, mm;
+    int ep, eq, em;
+    split(app, mp, ep);
+    split(aqq, mq, eq);
+    split(m2, mm, em);
+    const int ex = em - ep - eq + 1023;
+    if (em == 0 || ex < -110) return false;
+    const float x = mm * __int_as_float((min(ex, 60) + 127) << 23), y = mp * mq;
+    big = x > tol * y;
+    return x > tol * tol * y;
+}
+__device__ __forceinline__ long long zkey(double x) { return __double_as_longlong(x); }
+__device__ __forceinline__ bool zbelow_pow2(double x, double y, int n) {   // x < y 2^-n, y >= 0
+    return __double2hiint(x) < __double2hiint(y) - (n << 20);
 }
 
-// Shared memory: A (V_J, then the QRCP's working matrix) and B (R^H), each
-// K x ld column-major (ld = K | 1), then per-column complex scales d,
-// squared norms, complex QRCP taus, and two index arrays.
-// (one CTA per SM at k near 64: its shared memory is the limit, so the
-// registers need not be)
-template <bool AGLOBAL>
-__global__ void __launch_bounds__(256, 1) zgesvd_kernel(const ZDesc *__restrict__ descs,
-                                                     zd *__restrict__ ws, int *__restrict__ rank,
-                                                     int *__restrict__ status, int maxK, int G) {
-    extern __shared__ unsigned char zsm[];
-    __shared__ int s_piv, s_exp, s_conv, s_rot, s_bad;
-    __shared__ double s_wmax[8];
-    __shared__ double s_defl2;
-    const ZDesc d = descs[blockIdx.x];
-    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31;
+template <int G, bool CL>
+__global__ void __launch_bounds__(kZvThreads, 1)
+    zgesvd_kernel(const ZDesc *__restrict__ descs, zd *__restrict__ ws, int *__restrict__ rank,
+                  int *__restrict__ status, int maxK, int cs) {
+    extern __shared__ __align__(16) unsigned char zsm[];
+    __shared__ double s_wmax[kZvThreads / 32];
+    __shared__ zd s_vj;
+    __shared__ int s_big[2][8], s_rank;
+    __shared__ short s_own[128];
+    const ZDesc d = descs[CL ? blockIdx.x / cs : blockIdx.x];
+    const int cr = CL ? blockIdx.x % cs : 0;
+    const int tid = threadIdx.x, nthr = blockDim.x, lane = tid & 31, warp = tid >> 5, nw = nthr >> 5;
     if (d.status0) {
-        if (tid == 0) {
+        if (tid == 0 && cr == 0) {
             status[d.idx] = d.status0;
             rank[d.idx] = 0;
         }
         return;
     }
-    const int M = d.M, k = d.k;
+    const int M = d.M, k = d.k, ld = zsvd_ld(k);
     const ZLayout L = zlayout(M, d.a, d.b, k);
     zd *base = ws + d.ws;
     const zd *UA = base + L.UA, *VB = base + L.VB;
-    const int ld = zsvd_ld(maxK);
-    // AGLOBAL: A (the QRCP's matrix, then V_J) in the workspace, only B in
-    // shared memory, so that three CTAs fit an SM at k near 64
-    zd *B = reinterpret_cast<zd *>(zsm) + (AGLOBAL ? 0 : (size_t)maxK * ld);
-    zd *A = AGLOBAL ? base + L.W : reinterpret_cast<zd *>(zsm);
-    const int ldA = AGLOBAL ? k : ld;
-    zd *s_d = B + (size_t)maxK * ld;
-    zd *s_tau = s_d + (maxK + 1);
-    double *s_nrm = reinterpret_cast<double *>(s_tau + (maxK + 1));
-    double *s_dn = s_nrm + (maxK + 1);   // norms at the last exact computation
-    int *s_perm = reinterpret_cast<int *>(s_dn + (maxK + 1));
-    int *s_pcol = s_perm + (maxK + 1);
-    zd *Yg = base + L.Y;   // the QRCP's reflectors (k x k, ld k)
-    auto ix = [ld](int i, int j) { return (size_t)j * ld + i; };
-    auto ixA = [ldA](int i, int j) { return (size_t)j * ldA + i; };
+    const size_t mat = (size_t)maxK * zsvd_ld(maxK);
+    zd *A = reinterpret_cast<zd *>(zsm);   // R_A, T, its QR, then V_J
+    zd *B = A + mat;                       // R_B, then R^H; at the end Q's reflectors
+    zd *s_tau = B + mat, *s_rd = s_tau + (maxK + 1);   // reflector j's conj(tau) |scale|^2, R's diagonal
+    double *X0 = reinterpret_cast<double *>(s_rd + (maxK + 1)), *X1 = X0 + (maxK + 1);
+    double *s_w = X1 + (maxK + 1);
+    short *s_perm = reinterpret_cast<short *>(s_w + (maxK + 1)), *s_pcol = s_perm + (maxK + 1);
+    zd *Yg = base + L.Y;   // reflectors of Q (k x k, ld k)
+    const int grp = tid / G, lig = tid & (G - 1), ngrp = nthr / G;
+    constexpr int D = G < 8 ? G : 8;   // lanes per column in the QR
+    const int qgrp = tid / D, qlig = tid & (D - 1), nqgrp = nthr / D;
 
-    // T = triu(R_A) triu(R_B)^T
+    // ---- T = triu(R_A) triu(R_B)^T: a warp per row, the row of T replaces the row
+    // of R_A that only it reads
+    for (int l = warp; l < k; l += nw)
+        for (int i = lane; i < k; i += 32) {
+            A[(size_t)l * ld + i] = i <= l ? UA[(size_t)l * M + i] : zmk(0, 0);
+            B[(size_t)l * ld + i] = i <= l ? VB[(size_t)l * M + i] : zmk(0, 0);
+        }
+    __syncthreads();
     double amax = 0;
-    for (int e = tid; e < k * k; e += nthr) {
-        const int i = e % k, j = e / k;
-        zd s = zmk(0, 0);
-        for (int l = max(i, j); l < k; ++l)
-            s = zfma(UA[(size_t)l * M + i], VB[(size_t)l * M + j], s);
-        A[ixA(i, j)] = s;
-        amax = max(amax, max(fabs(s.re), fabs(s.im)));
-    }
-    for (int o = 16; o > 0; o >>= 1) amax = max(amax, __shfl_xor_sync(0xffffffffu, amax, o));
-    if (lane == 0) s_wmax[tid >> 5] = amax;
-    __syncthreads();
-    if (tid == 0) {
-        double m = 0;
-        for (int w = 0; w < nthr / 32; ++w) m = max(m, s_wmax[w]);
-        s_exp = (m > 0 && isfinite(m)) ? ilogb(m) : 0;
-        s_bad = 0;
-    }
-    __syncthreads();
-    const int sexp = s_exp;
-    if (sexp != 0)
-        for (int e = tid; e < k * k; e += nthr) {
-            const int i = e % k, j = e / k;
-            const zd v = A[ixA(i, j)];
-            A[ixA(i, j)] = zmk(dmul_exp2(v.re, -sexp), dmul_exp2(v.im, -sexp));
+    bool bad = false;
+    for (int i = warp; i < k; i += nw) {
+        zd acc[kZvRows];
+#pragma unroll
+        for (int c = 0; c < kZvRows; ++c) {
+            acc[c] = zmk(0, 0);
+            if (32 * c < k) {
+                const zd *b = B + min(lane + 32 * c, k - 1);
+                for (int l = max(i, 32 * c); l < k; ++l)
+                    acc[c] = zfma(A[(size_t)l * ld + i], b[(size_t)l * ld], acc[c]);
+            }
         }
+        __syncwarp();
+#pragma unroll
+        for (int c = 0; c < kZvRows; ++c) {
+            const int j = lane + 32 * c;
+            if (j < k) {
+                A[(size_t)j * ld + i] = acc[c];
+                amax = max(amax, max(fabs(acc[c].re), fabs(acc[c].im)));
+                bad = bad || !isfinite(acc[c].re) || !isfinite(acc[c].im);
+            }
+        }
+    }
+    amax = warp_max(amax);
+    if (lane == 0) s_wmax[warp] = amax;
+    if (__syncthreads_or(bad)) {   // a NaN or infinity: the update is not written
+        if (cr != 0) return;
+        for (int t = tid; t < k; t += nthr) base[L.sig + t] = zmk(NAN, 0);
+        if (tid == 0) {
+            rank[d.idx] = d.rk != 0 && d.rk < k ? d.rk : k;
+            status[d.idx] = HCORE_GPU_S_NOCONV;
+        }
+        return;
+    }
+    amax = 0;
+    for (int w = 0; w < nw; ++w) amax = max(amax, s_wmax[w]);
+    const int sexp = amax > 0 ? binary_exponent(amax) : 0;
+    for (int c0 = 0; c0 < k; c0 += nqgrp) {
+        const int c = c0 + qgrp;
+        zd *ac = A + (size_t)c * ld;
+        if (c < k && sexp != 0)
+            for (int i = qlig; i < k; i += D) ac[i] = zmk(mul_exp2(ac[i].re, -sexp), mul_exp2(ac[i].im, -sexp));
+        const double s = zgroup_norm<D>(c < k, ac, 0, k, qlig);
+        if (c < k && qlig == 0) {
+            X0[c] = s;    // norms of rows j.. of column c, squared; -1: pivoted already
+            s_w[c] = s;   // the same at the last exact computation
+        }
+    }
     __syncthreads();
+    double f2 = 0;
+    for (int c = lane; c < k; c += 32) f2 += X0[c];
+    const double defl2 = deflation_bound2(warp_sum(f2), k, M, d.rk, 0, d.acc, sexp);
 
-    // QR with column pivoting, T P = Q R (lane per trailing column)
-    for (int c = tid; c < k; c += nthr) {
-        double s = 0;
-        for (int i = 0; i < k; ++i) s += zabs2(A[ixA(i, c)]);
-        s_nrm[c] = s;
-        s_dn[c] = s;
-        s_pcol[c] = c;
-    }
-    __syncthreads();
-    // Deflation, as in the real kernels (hc_svd.cu): the QR stops at the
-    // first step j >= 1 (the rank search starts at 1) whose trailing block has
-    // ||R(j:k, j:k)||_F <= delta = min(1e-13 acc, 1e-16 ||T||_F) and the
-    // Jacobi works on the first j rows of R.  Every singular value moves by at
-    // most delta (Weyl); the dropped directions come out with singular value 0.
-    if (tid == 0) {
-        double f2 = 0;   // ||T||_F^2 of the scaled T
-        for (int c = 0; c < k; ++c) f2 += s_nrm[c];
-        double dl = -1.0;
-        if (d.rk == 0 && d.acc > 0.0) dl = fmin(1e-13 * dmul_exp2(d.acc, -sexp), 1e-16 * sqrt(f2));
-        s_defl2 = (dl >= 0.0 && isfinite(dl)) ? dl * dl : -1.0;
-    }
-    int kk = k;   // columns of R^H that the Jacobi rotates
+    // ---- QR with column pivoting, T P = Q R (columns stay in place) -----------------
+    int kk = k;
     for (int j = 0; j < k; ++j) {
-        if (tid < 32) {
-            double best = -1, tail = 0;
-            int bi = j;
-            for (int c = j + lane; c < k; c += 32) {
-                tail += s_nrm[c];
-                if (s_nrm[c] > best) {
-                    best = s_nrm[c];
-                    bi = c;
-                }
-            }
-            for (int o = 16; o > 0; o >>= 1) {
-                const double ob = __shfl_xor_sync(0xffffffffu, best, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                tail += __shfl_xor_sync(0xffffffffu, tail, o);
-                if (ob > best || (ob == best && oi < bi)) {
-                    best = ob;
-                    bi = oi;
-                }
-            }
-            if (lane == 0) s_piv = (j >= 1 && tail <= s_defl2) ? -1 : bi;
-        }
-        __syncthreads();
-        const int pv = s_piv;
-        if (pv < 0) {
-            kk = j;
-            break;
-        }
-        if (pv != j) {
-            for (int i = tid; i < k; i += nthr) {
-                const zd x = A[ixA(i, j)];
-                A[ixA(i, j)] = A[ixA(i, pv)];
-                A[ixA(i, pv)] = x;
-            }
-            if (tid == 0) {
-                double x = s_nrm[j]; s_nrm[j] = s_nrm[pv]; s_nrm[pv] = x;
-                x = s_dn[j]; s_dn[j] = s_dn[pv]; s_dn[pv] = x;
-                const int ci = s_pcol[j]; s_pcol[j] = s_pcol[pv]; s_pcol[pv] = ci;
+        const double *nr = (j & 1) ? X1 : X0;
+        double *nr2 = (j & 1) ? X0 : X1;
+        long long best = zkey(-1.0);
+        int pv = 0;
+        for (int c = lane; c < k; c += 32) {
+            const long long x = zkey(nr[c]);
+            if (x > best) {
+                best = x;
+                pv = c;
             }
         }
-        __syncthreads();
-        if (tid < 32) {   // reflector of column j, rows j..k-1
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const long long ob = __shfl_xor_sync(0xffffffffu, best, o);
+            const int oi = __shfl_xor_sync(0xffffffffu, pv, o);
+            if (ob > best || (ob == best && oi < pv)) {
+                best = ob;
+                pv = oi;
+            }
+        }
+        if (j >= 1 && defl2 >= 0.0 && best <= zkey(defl2)) {
+            double tail = 0;
+            for (int c = lane; c < k; c += 32) tail += max(nr[c], 0.0);
+            if (warp_sum(tail) <= defl2) {
+                kk = j;
+                break;
+            }
+        }
+        // reflector of column pv, rows j.., unscaled: v = (alpha - beta, x), H^H y =
+        // y - g (v^H y) v, g = 1 / (beta (beta - alpha)), by warp 0 while the others
+        // form x^H y for the remaining columns y
+        const zd *ap = A + (size_t)pv * ld;
+        if (warp == 0) {
+            const zd alpha = ap[j];
             double ss = 0;
-            for (int i = j + 1 + lane; i < k; i += 32) ss += zabs2(A[ixA(i, j)]);
-            ss = zwarp_sum(ss);
-            double beta;
-            zd tj, scal;
-            zlarfg(A[ixA(j, j)], ss, beta, tj, scal);
-            for (int i = j + 1 + lane; i < k; i += 32) A[ixA(i, j)] = zmul(A[ixA(i, j)], scal);
-            __syncwarp();
+            for (int i = j + 1 + lane; i < k; i += 32) ss += zabs2(ap[i]);
+            ss = warp_sum(ss);
+            zd beta = alpha, vj = zmk(0, 0), g = zmk(0, 0);
+            if (ss > DBL_MIN / DBL_EPSILON) {
+                const double n2 = zabs2(alpha) + ss, rs = inv_sqrt(n2);
+                double nb = n2 * rs;
+                nb = fma(fma(-nb, nb, n2) * 0.5, rs, nb);
+                beta = zmk(-copysign(nb, alpha.re), 0);
+                vj = zsub(alpha, beta);
+                const double ib = -copysign(rs, alpha.re), iv = inv(zabs2(vj)) * ib;
+                g = zmk(-vj.re * iv, vj.im * iv);   // -1 / (beta vj)
+            }
             if (lane == 0) {
-                A[ixA(j, j)] = zmk(beta, 0);
-                s_tau[j] = tj;
+                s_pcol[j] = (short)pv;
+                s_rd[j] = beta;
+                s_tau[j] = g;
+                s_vj = vj;
             }
         }
-        __syncthreads();
-        // apply H_j^H to the trailing columns and downdate their norms
-        const zd tc = zconj(s_tau[j]);
-        for (int c = j + 1 + tid; c < k; c += nthr) {
-            if (tc.re != 0.0 || tc.im != 0.0) {
-                zd dot = A[ixA(j, c)];
-                for (int i = j + 1; i < k; ++i) dot = zcfma(A[ixA(i, j)], A[ixA(i, c)], dot);
-                const zd s = zmul(tc, dot);
-                A[ixA(j, c)] = zsub(A[ixA(j, c)], s);
-                for (int i = j + 1; i < k; ++i) A[ixA(i, c)] = zfms(s, A[ixA(i, j)], A[ixA(i, c)]);
-            }
-            double nn = s_nrm[c] - zabs2(A[ixA(j, c)]);
-            if (nn <= s_dn[c] * (1.0 / 1024) || nn <= 0.0) {
-                double s = 0;
-                for (int i = j + 1; i < k; ++i) s += zabs2(A[ixA(i, c)]);
-                nn = s;
-                s_dn[c] = s;
-            }
-            s_nrm[c] = nn;
+        zd *dots = B;   // (free until R^H is formed)
+        for (int c0 = 0; c0 < k; c0 += nqgrp) {
+            const int c = c0 + qgrp;
+            const bool act = c < k && c != pv && zkey(nr[c]) >= 0;
+            const zd w = zgroup_dot<D>(act, ap, A + (size_t)c * ld, j + 1, k, qlig);
+            if (act && qlig == 0) dots[c] = w;
         }
         __syncthreads();
-    }
-    // reflectors to the workspace; B = R^H (rows kk.. of R dropped: B's
-    // columns kk.. are zero; reflectors kk.. were never formed); A = I
-    for (int h = kk + tid; h < k; h += nthr) s_tau[h] = zmk(0, 0);
-    for (int e = tid; e < k * k; e += nthr) {
-        const int i = e % k, j = e / k;
-        const zd x = A[ixA(i, j)];
-        Yg[(size_t)j * k + i] = (i > j && j < kk) ? x : zmk(0, 0);
-        B[ix(j, i)] = (i <= j && i < kk) ? zconj(x) : zmk(0, 0);   // B(j, i) = conj(R(i, j))
-    }
-    __syncthreads();
-    for (int e = tid; e < k * k; e += nthr) {
-        const int i = e % k, j = e / k;
-        A[ixA(i, j)] = zmk(i == j ? 1.0 : 0.0, 0);
-    }
-    for (int c = tid; c < k; c += nthr) {
-        double s = 0;
-        if (c < kk)
-            for (int i = 0; i < k; ++i) s += zabs2(B[ix(i, c)]);
-        s_nrm[c] = s;
-        s_d[c] = zmk(1, 0);
-    }
-    __syncthreads();
-
-    // one-sided Jacobi on B with complex column scales: true column j is
-    // d_j x_j in B and in V_J (A).  For a pair with a_pq = P^H Q = |a_pq|
-    // e^{i phi}: P' = c (P - t e^{-i phi} Q), Q' = c (e^{-i phi} Q + t P),
-    // t the real Jacobi tangent of (a_pp, a_qq, |a_pq|); in scaled form
-    // x_p -= f1 x_q, x_q += f2 x_p with f1 = t e^{-i phi} d_q / d_p,
-    // f2 = t e^{i phi} d_p / d_q, d_p <- c d_p, d_q <- c e^{-i phi} d_q
-    // (columns kk.. of B are zero and take no part; V_J's rows kk.. stay zero)
-    const int n = kk + (kk & 1), np = n / 2;
-    const int grp = tid / G, lig = tid % G, ngrp = nthr / G;
-    const double tol = (double)(k > 8 ? k : 8) * DBL_EPSILON;
-    const double tol2 = tol * tol, stop2 = tol;
-    const double safmin = DBL_MIN / DBL_EPSILON;
-    bool converged = (kk <= 1);
-    for (int sweep = 0; sweep < kMaxSweeps && !converged; ++sweep) {
-        if (tid == 0) s_rot = 0;
-        bool big = false;
-        __syncthreads();
-        for (int round = 0; round < n - 1; ++round) {
-            for (int bs = 0; bs < np; bs += ngrp) {
-                const int pi = bs + grp;
-                int p = 0, q = 0;
-                if (pi < np) zrr_pair(round, pi, n, p, q);
-                const bool valid = pi < np && p < kk && q < kk;
-                zd *xp = B + ix(0, p), *xq = B + ix(0, q);
-                zd dot = zmk(0, 0);
-                if (valid)
-                    for (int i = lig; i < k; i += G) dot = zcfma(xp[i], xq[i], dot);
-                for (int o = G / 2; o > 0; o >>= 1) {
-                    dot.re += __shfl_xor_sync(0xffffffffu, dot.re, o);
-                    dot.im += __shfl_xor_sync(0xffffffffu, dot.im, o);
+        const zd g = s_tau[j], vj = s_vj;
+        const bool none = g.re == 0.0 && g.im == 0.0;
+        for (int c0 = 0; c0 < k; c0 += nqgrp) {
+            const int c = c0 + qgrp;
+            const double nc = c < k ? nr[c] : -1.0;
+            const bool act = c < k && c != pv && zkey(nc) >= 0, upd = act && !none;
+            zd *ac = A + (size_t)c * ld;
+            zd acj = zmk(0, 0), s = zmk(0, 0);
+            if (upd && qlig == 0) {
+                acj = ac[j];
+                s = zmul(g, zcfma(vj, acj, dots[c]));
+            }
+            s.re = __shfl_sync(0xffffffffu, s.re, lane & ~(D - 1));
+            s.im = __shfl_sync(0xffffffffu, s.im, lane & ~(D - 1));
+            double nn = 0;
+            bool redo = false;
+            if (act) {
+                if (upd)
+                    for (int i = j + 1 + ((qlig - (j + 1)) & (D - 1)); i < k; i += D) ac[i] = zfms(s, ap[i], ac[i]);
+                if (qlig == 0) {
+                    const zd r = upd ? zfms(s, vj, acj) : ac[j];
+                    ac[j] = r;
+                    nn = nc - zabs2(r);
+                    redo = !(zkey(nn) > 0) || zbelow_pow2(nn, s_w[c], 10);
                 }
-                zd dp = zmk(1, 0), dq = zmk(1, 0);
-                double app = 0, aqq = 0, amag2 = 0;
-                zd apq = zmk(0, 0);
+            }
+            if (__any_sync(0xffffffffu, redo)) {
+                redo = __shfl_sync(0xffffffffu, (int)redo, lane & ~(D - 1)) != 0;
+                const double q = zgroup_norm<D>(redo, ac, j + 1, k, qlig);
+                if (redo && qlig == 0) {
+                    nn = q;
+                    s_w[c] = q;
+                }
+            }
+            if (c < k && qlig == 0) nr2[c] = act ? nn : -1.0;
+        }
+        __syncthreads();
+    }
+    {
+        // columns that the deflation left: positions kk.. in column order
+        const double *nr = (kk & 1) ? X1 : X0;
+        if (kk < k)
+            for (int c = tid; c < k; c += nthr)
+                if (zkey(nr[c]) >= 0) {
+                    int pos = kk;
+                    for (int q = 0; q < c; ++q) pos += zkey(nr[q]) >= 0;
+                    s_pcol[pos] = (short)c;
+                }
+    }
+    __syncthreads();
+    // Q's reflectors to the workspace, B = R^H (its columns kk.. are zero), A = I
+    for (int h = warp; h < k; h += nw) {
+        const zd *ah = A + (size_t)s_pcol[h] * ld;
+        for (int i = lane; i < k; i += 32) {
+            const zd x = ah[i], rd = h < kk ? s_rd[h] : zmk(0, 0);
+            if (h < kk && cr == 0) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? zsub(x, rd) : zmk(0, 0));
+            B[(size_t)i * ld + h] = i < kk ? (i < h ? zconj(x) : (i == h ? zconj(rd) : zmk(0, 0))) : zmk(0, 0);
+        }
+    }
+    __syncthreads();
+    for (int c = warp; c < k; c += nw)
+        for (int i = lane; i < k; i += 32) A[(size_t)c * ld + i] = zmk(i == c ? 1.0 : 0.0, 0);
+    double *s_nrm = X0, *s_sig = X1;
+    auto column_norm = [&](int c, bool fold) {   // of column c, by its group
+        double w = 1;
+        zd *xj = B + (size_t)c * ld;
+        if (c < kk && fold) {
+            w = s_w[c];
+            if (w < 1e-120) {   // fold a scale before it underflows
+                const double f = sqrt(w);
+                zd *vj = A + (size_t)c * ld;
+                for (int i = lig; i < k; i += G) {
+                    xj[i] = zscal(f, xj[i]);
+                    vj[i] = zscal(f, vj[i]);
+                }
+                w = 1;
+            }
+        }
+        const double s = zgroup_norm<G>(c < kk, xj, 0, k, lig);
+        if (c < k && lig == 0) {
+            s_nrm[c] = c < kk ? w * s : 0.0;
+            s_w[c] = w;
+        }
+    };
+    for (int c0 = 0; c0 < k; c0 += ngrp) column_norm(c0 + grp, false);
+    if constexpr (CL) cluster_sync(); else __syncthreads();
+
+    // ---- one-sided Jacobi on B, rotations accumulated in A ---------------------------
+    // (columns kk.. of B are zero and take no part, V_J's rows kk.. stay zero)
+    const int n = kk + (kk & 1), np = n / 2;
+    const int active = CL ? max(1, min(cs, np)) : 1;
+    const int pi0 = CL ? min(cr, active) * np / active : 0, pi1 = CL ? min(cr + 1, active) * np / active : np;
+    const unsigned left = CL && pi0 > 0 && cr < active ? peer_delta(zsm, cr - 1) : 0;
+    const unsigned right = CL && pi1 < np ? peer_delta(zsm, cr + 1) : 0;
+    const float tol = (float)(k > 8 ? k : 8) * (float)DBL_EPSILON;
+    bool converged = kk <= 1;
+    for (int sweep = 0; sweep < kMaxSweeps && !converged; ++sweep) {
+        bool big = false;   // this thread rotated a pair above sqrt(tol)
+        for (int round = 0; round < n - 1; ++round) {
+            for (int b0 = pi0; b0 < pi1; b0 += ngrp) {
+                const int pi = b0 + grp;
+                int p = round + pi, q = round - pi;
+                if (p >= n - 1) p -= n - 1;
+                if (q < 0) q += n - 1;
+                if (pi == 0) p = n - 1;
+                const bool valid = pi < pi1 && p < kk && q < kk;
+                zd *xp = B + (size_t)p * ld, *xq = B + (size_t)q * ld;
+                double app = 0, aqq = 0, wp = 1, wq = 1;
                 if (valid) {
-                    dp = s_d[p];
-                    dq = s_d[q];
                     app = s_nrm[p];
                     aqq = s_nrm[q];
-                    apq = zmul(zcmul(dp, dq), dot);   // conj(dp) dq x_p^H x_q
-                    amag2 = zabs2(apq);
+                    wp = s_w[p];
+                    wq = s_w[q];
                 }
-                const double pq = app * aqq;
-                const bool rot = valid && app > safmin && aqq > safmin && amag2 > 0.0 &&
-                                 amag2 > tol2 * pq;
-                double t = 0, cs = 1;
-                zd ph = zmk(1, 0);
-                if (rot) {
-                    big |= amag2 > stop2 * pq;
-                    const double am = sqrt(amag2);
-                    ph = zscal(1.0 / am, apq);                // e^{i phi}
-                    const double w = aqq - app, v = 2.0 * am;
-                    const double h = sqrt(fma(w, w, v * v));
-                    t = v / (fabs(w) + h);
-                    if (w < 0.0) t = -t;
-                    cs = rsqrt(fma(t, t, 1.0));
-                    const zd f1 = zscal(t / zabs2(dp), zmul(zconj(ph), zmul(dq, zconj(dp))));
-                    const zd f2 = zscal(t / zabs2(dq), zmul(ph, zmul(dp, zconj(dq))));
-                    zd *vp = A + ixA(0, p), *vq = A + ixA(0, q);
-                    int i = lig;
-                    for (; i < kk; i += G) {
-                        const zd a = xp[i], b = xq[i];
-                        xp[i] = zfms(f1, b, a);
-                        xq[i] = zfma(f2, a, b);
-                        const zd u = vp[i], vv = vq[i];
-                        vp[i] = zfms(f1, vv, u);
-                        vq[i] = zfma(f2, u, vv);
-                    }
-                    for (; i < k; i += G) {   // V_J's rows kk.. are zero
-                        const zd a = xp[i], b = xq[i];
-                        xp[i] = zfms(f1, b, a);
-                        xq[i] = zfma(f2, a, b);
-                    }
-                }
-                double np_ = app - t * sqrt(amag2), nq_ = aqq + t * sqrt(amag2);
-                const bool redo_p = rot && np_ < app * (1.0 / 64);
-                const bool redo_q = rot && nq_ < aqq * (1.0 / 64);
-                const zd dp2 = zscal(cs, dp), dq2 = zscal(cs, zcmul(ph, dq));   // c e^{-i phi} dq
-                if (__any_sync(0xffffffffu, redo_p || redo_q)) {
-                    double sp = 0, sq = 0;
-                    if (redo_p || redo_q)
-                        for (int i = lig; i < k; i += G) {
-                            sp += zabs2(xp[i]);
-                            sq += zabs2(xq[i]);
+                const zd dot = zgroup_dot<G>(valid, xp, xq, 0, k, lig);
+                bool rot = false, redo_p = false, redo_q = false;
+                double np_ = 0, nq_ = 0, wp2 = 1, wq2 = 1;
+                if (valid) {
+                    const double m2 = (wp * wq) * zabs2(dot);
+                    bool bigp = false;
+                    rot = zkey(app) > zkey(DBL_MIN / DBL_EPSILON) && zkey(aqq) > zkey(DBL_MIN / DBL_EPSILON) &&
+                          zpair_test(app, aqq, m2, tol, bigp);
+                    if (rot) {
+                        big |= bigp;
+                        const double rm = inv_sqrt(m2), m = m2 * rm, t = tangent(app, aqq, m), tm = t * rm;
+                        const zd f1 = zscal(tm * wq, zconj(dot)), f2_ = zscal(tm * wp, dot);
+                        np_ = fma(-t, m, app);
+                        nq_ = fma(t, m, aqq);
+                        redo_p = zbelow_pow2(np_, app, 6);
+                        redo_q = zbelow_pow2(nq_, aqq, 6);
+                        zd *vp = A + (size_t)p * ld, *vq = A + (size_t)q * ld;
+                        int i = lig;
+                        for (; i < kk; i += G) {
+                            const zd a = xp[i], b = xq[i], u = vp[i], v = vq[i];
+                            xp[i] = zfms(f1, b, a);
+                            xq[i] = zfma(f2_, a, b);
+                            vp[i] = zfms(f1, v, u);
+                            vq[i] = zfma(f2_, u, v);
                         }
-                    for (int o = G / 2; o > 0; o >>= 1) {
-                        sp += __shfl_xor_sync(0xffffffffu, sp, o);
-                        sq += __shfl_xor_sync(0xffffffffu, sq, o);
+                        for (; i < k; i += G) {
+                            const zd a = xp[i], b = xq[i];
+                            xp[i] = zfms(f1, b, a);
+                            xq[i] = zfma(f2_, a, b);
+                        }
+                        const double c2 = inv(fma(t, t, 1.0));
+                        wp2 = wp * c2;
+                        wq2 = wq * c2;
                     }
-                    if (redo_p) np_ = zabs2(dp2) * sp;
-                    if (redo_q) nq_ = zabs2(dq2) * sq;
+                }
+                if (__any_sync(0xffffffffu, redo_p || redo_q)) {   // strong cancellation in a tracked norm
+                    const double sp = zgroup_norm<G>(redo_p, xp, 0, k, lig);
+                    const double sq = zgroup_norm<G>(redo_q, xq, 0, k, lig);
+                    if (redo_p) np_ = wp2 * sp;
+                    if (redo_q) nq_ = wq2 * sq;
                 }
                 if (rot && lig == 0) {
                     s_nrm[p] = np_;
                     s_nrm[q] = nq_;
-                    s_d[p] = dp2;
-                    s_d[q] = dq2;
-                    s_rot = 1;
+                    s_w[p] = wp2;
+                    s_w[q] = wq2;
+                }
+                if constexpr (CL) {
+                    // the next round has p in pair pi - 1 and q in pair pi + 1
+                    auto send = [&](int c, unsigned to) {
+                        zd *x = B + (size_t)c * ld, *v = A + (size_t)c * ld;
+                        for (int i = lig; i < k; i += G) {
+                            peer_store(&x[i].re, to, x[i].re);
+                            peer_store(&x[i].im, to, x[i].im);
+                            if (i < kk) {
+                                peer_store(&v[i].re, to, v[i].re);
+                                peer_store(&v[i].im, to, v[i].im);
+                            }
+                        }
+                        if (lig == 0) {
+                            peer_store(s_nrm + c, to, s_nrm[c]);
+                            peer_store(s_w + c, to, s_w[c]);
+                        }
+                    };
+                    if (pi == pi0 && pi > 0 && p < kk) send(p, left);
+                    if (pi == pi1 - 1 && pi1 < np && q < kk) send(q, right);
+                    __syncwarp();
                 }
             }
-            __syncthreads();
+            if constexpr (CL) cluster_sync(); else __syncthreads();
         }
-        // exact norms once per sweep; fold scales before they underflow
-        for (int j = tid; j < kk; j += nthr) {
-            zd *xj = B + ix(0, j);
-            zd dj = s_d[j];
-            if (zabs2(dj) < 1e-120) {
-                zd *vj = A + ixA(0, j);
-                for (int i = 0; i < k; ++i) {
-                    xj[i] = zmul(dj, xj[i]);
-                    vj[i] = zmul(dj, vj[i]);
-                }
-                dj = zmk(1, 0);
-                s_d[j] = dj;
+        // exact norms once per sweep (every column is back in its first pair)
+        if constexpr (CL) {
+            for (int b0 = pi0; b0 < pi1; b0 += ngrp) {
+                const int pi = b0 + grp;
+                column_norm(pi < pi1 ? (pi == 0 ? n - 1 : pi) : k, true);
+                column_norm(pi < pi1 ? (pi == 0 ? 0 : n - 1 - pi) : k, true);
             }
-            double s2 = 0;
-            for (int i = 0; i < k; ++i) s2 += zabs2(xj[i]);
-            s_nrm[j] = zabs2(dj) * s2;
+            const int any = __syncthreads_or(big);
+            if (tid < cs) peer_store(&s_big[sweep & 1][cr], peer_delta(zsm, tid), any);
+            cluster_sync();
+            converged = true;
+            for (int t = 0; t < cs; ++t) converged = converged && !s_big[sweep & 1][t];
+        } else {
+            for (int c0 = 0; c0 < k; c0 += ngrp) column_norm(c0 + grp, true);
+            converged = !__syncthreads_or(big);
         }
-        const bool anybig = __any_sync(0xffffffffu, big);
-        if (lane == 0) s_wmax[tid >> 5] = anybig ? 1.0 : 0.0;
-        __syncthreads();
-        if (tid == 0) {
-            double m = 0;
-            for (int w = 0; w < nthr / 32; ++w) m = max(m, s_wmax[w]);
-            s_conv = (s_rot == 0 || m == 0.0) ? 1 : 0;
-        }
-        __syncthreads();
-        converged = s_conv != 0;
-        __syncthreads();
+    }
+    auto owner = [&](int j) {   // the CTA that holds column j
+        const int pi = j == n - 1 ? 0 : (j < np ? j : n - 1 - j);
+        int o = 0;
+        while (o + 1 < active && (o + 1) * np / active <= pi) ++o;
+        return j < kk ? o : 0;
+    };
+    if constexpr (CL) {
+        for (int j = warp; j < kk; j += nw)
+            if (owner(j) == cr && lane < cs && lane != cr) {
+                const unsigned to = peer_delta(zsm, lane);
+                peer_store(s_nrm + j, to, s_nrm[j]);
+                peer_store(s_w + j, to, s_w[j]);
+            }
+        cluster_sync();
     }
 
-    // singular values, sorted descending (ties by index, NaN last)
-    double *s_sig = s_dn;
+    // singular values, sorted descending (ties by index, NaN last), rank rule
+    bool nonfinite = false;
     for (int j = tid; j < k; j += nthr) {
         const double s = sqrt(s_nrm[j]);
-        s_sig[j] = s;
-        if (!isfinite(s)) s_bad = 1;
+        nonfinite = nonfinite || !isfinite(s);
+        s_sig[j] = s == s ? s : -1.0;
     }
-    __syncthreads();
+    if (tid == 0) s_rank = k;
+    const bool finite = !__syncthreads_or(nonfinite);
     for (int j = tid; j < k; j += nthr) {
-        const double sj = s_sig[j] == s_sig[j] ? s_sig[j] : -1.0;
+        const long long sj = zkey(s_sig[j]);
         int pos = 0;
         for (int i = 0; i < k; ++i) {
-            const double si = s_sig[i] == s_sig[i] ? s_sig[i] : -1.0;
+            const long long si = zkey(s_sig[i]);
             pos += (si > sj) || (si == sj && i < j);
         }
-        s_perm[pos] = j;
+        s_perm[pos] = (short)j;
     }
     __syncthreads();
-    zd *sig_out = base + L.sig;
-    for (int t = tid; t < k; t += nthr) sig_out[t] = zmk(dmul_exp2(s_sig[s_perm[t]], sexp), 0);
-    int r;
-    if (d.rk != 0) {
-        r = d.rk < k ? d.rk : k;
-    } else {
-        r = k;
-        for (int i = 1; i < k; ++i)
-            if (dmul_exp2(s_sig[s_perm[i]], sexp) < d.acc) {
-                r = i;
-                break;
-            }
+    for (int t = tid; t < k; t += nthr) {
+        const double s = s_sig[s_perm[t]], v = s < 0 ? NAN : mul_exp2(s, sexp);
+        if (cr == 0) base[L.sig + t] = zmk(v, 0);
+        if (d.rk == 0 && t >= 1 && v < d.acc) atomicMin(&s_rank, t);
     }
+    __syncthreads();
+    const int r = d.rk != 0 ? (d.rk < k ? d.rk : k) : s_rank;
     int st = HCORE_GPU_S_OK;
-    if (!converged || s_bad) st = HCORE_GPU_S_NOCONV;
+    if (!converged || !finite) st = HCORE_GPU_S_NOCONV;
     else if (r > d.max_rank) st = HCORE_GPU_S_RANK_MAX;
     if (st == HCORE_GPU_S_OK) {
-        // U_r = Q (true V_J columns), Q = H_0 ... H_{k-1}: lane per output
-        // column, reflectors from last to first, H_h x = x - tau_h v_h (v_h^H x)
-        for (int t = tid; t < r; t += nthr) {
+        // Vo = conj(W_r S_r), W S = P (B's columns), scaled back
+        zd *Uo = base + L.Uo, *Vo = base + L.Vo;
+        for (int t = warp; t < r; t += nw) {
             const int j = s_perm[t];
-            zd *x = A + ixA(0, j);
-            const zd dj = s_d[j];
-            for (int i = 0; i < k; ++i) x[i] = zmul(dj, x[i]);
-            for (int h = k - 1; h >= 0; --h) {
-                const zd th = s_tau[h];
-                if (th.re == 0.0 && th.im == 0.0) continue;
-                const zd *y = Yg + (size_t)h * k;
-                zd dot = x[h];
-                for (int i = h + 1; i < k; ++i) dot = zcfma(y[i], x[i], dot);
-                const zd s = zmul(th, dot);
-                x[h] = zsub(x[h], s);
-                for (int i = h + 1; i < k; ++i) x[i] = zfms(s, y[i], x[i]);
+            if (CL && owner(j) != cr) continue;
+            const double f = sqrt(s_w[j]);
+            for (int i = lane; i < k; i += 32) {
+                const zd w = zscal(f, B[(size_t)j * ld + i]);
+                Vo[(size_t)t * k + s_pcol[i]] = zmk(mul_exp2(w.re, sexp), -mul_exp2(w.im, sexp));
+            }
+        }
+        int nown = r;   // the columns of U_r that this CTA forms
+        if constexpr (CL) {
+            nown = 0;
+            for (int t = 0; t < r; ++t) {
+                const bool mine = owner(s_perm[t]) == cr;
+                if (mine && tid == 0) s_own[nown] = (short)t;
+                nown += mine;
             }
         }
         __syncthreads();
-        // Uo = U_r; Vo = conj(W_r S_r) with W S = P (rotated B), scaled back
-        zd *Uo = base + L.Uo, *Vo = base + L.Vo;
-        for (int e = tid; e < k * r; e += nthr) {
-            const int i = e % k, t = e / k;
-            const int j = s_perm[t];
-            const zd w = zmul(s_d[j], B[ix(i, j)]);
-            Vo[(size_t)t * k + s_pcol[i]] = zmk(dmul_exp2(w.re, sexp), -dmul_exp2(w.im, sexp));
-            Uo[(size_t)t * k + i] = A[ixA(i, j)];
+        // U_r = Q (V_J's columns), Q = H_0 ... H_{kk-1}: the reflectors come into B's
+        // place, each group applies them, last to first, to its columns
+        for (int h = warp; h < kk; h += nw)
+            for (int i = lane; i < k; i += 32) B[(size_t)h * ld + i] = Yg[(size_t)h * k + i];
+        __syncthreads();
+        for (int t0 = 0; t0 < nown; t0 += ngrp) {
+            const bool act = t0 + grp < nown;
+            const int t = !act ? 0 : (CL ? s_own[t0 + grp] : t0 + grp);
+            const int j = act ? s_perm[t] : 0;
+            zd *x = A + (size_t)j * ld;   // each group owns the column of its own j
+            if (act) {
+                const double f = sqrt(s_w[j]);
+                for (int i = lig; i < k; i += G) x[i] = zscal(f, x[i]);
+            }
+            for (int h = kk - 1; h >= 0; --h) {
+                const zd g = s_tau[h];
+                if (g.re == 0.0 && g.im == 0.0) continue;
+                const zd *y = B + (size_t)h * ld;
+                const zd s = zmul(zconj(g), zgroup_dot<G>(act, y, x, h, k, lig));
+                if (act)
+                    for (int i = h + ((lig - h) & (G - 1)); i < k; i += G) x[i] = zfms(s, y[i], x[i]);
+            }
+            if (act)
+                for (int i = lig; i < k; i += G) Uo[(size_t)t * k + i] = x[i];
         }
     }
-    if (tid == 0) {
+    if (tid == 0 && cr == 0) {
         rank[d.idx] = r;
         status[d.idx] = st;
     }
@@ -841,6 +961,39 @@ int zsvd_kmax() {
     return kmax;
 }
 
+// While SMs are idle, a cluster per update of more than 12 column pairs: up to eight
+// pairs a CTA (16 lanes each, a warp a sub-partition), else eight lanes a pair.  SVD
+// phase, one CTA and a cluster, us: one update of k = 17 324, 337, of 64 4182, 2266;
+// 20 of k 24-32 779, 655 (two CTAs); 48 of k 32-64 3422, 2870 (three); 70 3416, 2899
+// (two).  Eight lanes also with more updates than SMs: 600 of k 16-32 1.44 ms, four
+// lanes 1.63; 600 of k 32-64 8.07, four lanes with V_J in the workspace, so that
+// three CTAs share an SM, 9.01.
+static cudaError_t launch_zgesvd(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status, int K, int sms,
+                                 cudaStream_t s) {
+    const int np = (K + 1) / 2, cs = np > 12 ? std::max(1, std::min({8, (np + 7) / 8, sms / n})) : 1;
+    const int pairs = (np + cs - 1) / cs;
+    const size_t smem = zsvd_smem_bytes(K);
+    auto go = [&](auto kernel, int G) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)n * cs);
+        cfg.blockDim = dim3(std::max(n > sms ? 32 : 256, (pairs * G + 31) / 32 * 32));
+        cfg.dynamicSmemBytes = smem;
+        cfg.stream = s;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = cs;
+        at[0].val.clusterDim.y = 1;
+        at[0].val.clusterDim.z = 1;
+        cfg.attrs = at;
+        cfg.numAttrs = cs > 1 ? 1 : 0;
+        return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, K, cs);
+    };
+    if (cs > 1) return pairs <= 8 ? go(zgesvd_kernel<16, true>, 16) : go(zgesvd_kernel<8, true>, 8);
+    return pairs <= 8 && n <= sms ? go(zgesvd_kernel<16, false>, 16) : go(zgesvd_kernel<8, false>, 8);
+}
+
 cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status,
                                int maxM, int maxK, int maxB, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
@@ -855,28 +1008,7 @@ cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, 
     zstack_inner_kernel<<<dim3(n, fy, fz), 256, 0, s>>>(d_desc, ws);
     zstack_outer_kernel<<<dim3(n, (maxM + kZsRows - 1) / kZsRows), 256, 0, s>>>(d_desc, ws);
     if (cudaError_t e = launch_zgeqrf(d_desc, n, ws, maxM, maxK, sms, optin, s)) return e;
-    // lanes per column pair: as many as fit in 256 threads, at most 4
-    const int np = (maxK + 1) / 2;
-    int G = 1;
-    while (G < 4 && 2 * G * np <= 256) G *= 2;
-    const int nt = ((np * G + 31) / 32) * 32;
-    // both Jacobi matrices in shared memory, unless that leaves one CTA per
-    // SM while the batch has more updates than SMs: then V_J moves to the
-    // workspace and three CTAs share an SM
-    const bool aglobal = n > sms && 2 * zsvd_smem_bytes(maxK) > (size_t)optin;
-    const size_t ssm = aglobal ? zsvd_smem_bytes_half(maxK) : zsvd_smem_bytes(maxK);
-    cudaError_t e;
-    if (aglobal) {
-        e = cudaFuncSetAttribute(zgesvd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ssm);
-        if (e != cudaSuccess) return e;
-        zgesvd_kernel<true><<<n, nt < 32 ? 32 : nt, ssm, s>>>(d_desc, ws, d_rank, d_status, maxK, G);
-    } else {
-        e = cudaFuncSetAttribute(zgesvd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)ssm);
-        if (e != cudaSuccess) return e;
-        zgesvd_kernel<false><<<n, nt < 32 ? 32 : nt, ssm, s>>>(d_desc, ws, d_rank, d_status, maxK, G);
-    }
+    if (cudaError_t e = launch_zgesvd(d_desc, n, ws, d_rank, d_status, maxK, sms, s)) return e;
     if (rpl <= 4) launch_zapply<4>(d_desc, n, ws, d_rank, d_status, maxK, s);
     else if (rpl <= 8) launch_zapply<8>(d_desc, n, ws, d_rank, d_status, maxK, s);
     else if (rpl <= 16) launch_zapply<16>(d_desc, n, ws, d_rank, d_status, maxK, s);
