@@ -170,43 +170,98 @@ struct PotrfView {
     }
 };
 
-// Columns [j0, j0 + 16) of the 64 x 64 block S: the diagonal 16 x 16 block by one
-// warp (lane i holds row i in registers; one reciprocal square root and one
-// scaling a column, no barrier), rows below it by four lanes a row.
 constexpr int kSb = 16;
 
-// 1 / sqrt(d) and sqrt(d) of a positive pivot
-__device__ __forceinline__ void pivot_root(double d, double &r, double &l) {
-    if (d < 2.2250738585072014e-308) {   // subnormal
-        l = sqrt(d);
-        r = 1.0 / l;
-        return;
-    }
-    r = inv_sqrt(d);
-    l = d * r;
-    l = fma(fma(-l, l, d) * 0.5, r, l);
+// 1 / sqrt(d) of a positive pivot, and sqrt(d) from both
+__device__ __forceinline__ double pivot_rsqrt(double d) {
+    return d < 2.2250738585072014e-308 ? 1.0 / sqrt(d) : inv_sqrt(d);   // (subnormal)
+}
+__device__ __forceinline__ double pivot_sqrt(double d, double r) {
+    if (d < 2.2250738585072014e-308) return sqrt(d);
+    const double l = d * r;
+    return fma(fma(-l, l, d) * 0.5, r, l);
 }
 
-// Solve rows of X L16^T = A16 in place: four lanes a row (lane q of the four
-// holds columns q, q + 4, ... of the sixteen), L16's rows and reciprocal
-// pivots in shared memory.  x_j goes around the four lanes by a shuffle.
-__device__ __forceinline__ void solve16(double (&a)[4], const double (*L)[kPb + 1], int j0, const double *rL,
+// The 16 x 16 block at (j0, j0) of S, by one warp in registers: lanes i and i + 16
+// hold the even and the odd columns of row i.  One reciprocal square root and one
+// scaling a column, no barrier; the pivots' square roots together at the end.
+__device__ __forceinline__ void factor16(double (*S)[kPb + 1], int j0, int bs, double *rL, int *fail) {
+    const int lane = threadIdx.x & 31, i = lane & 15, h = lane >> 4;
+    double a[8], dd = 1.0, rr = 1.0;
+#pragma unroll
+    for (int m = 0; m < 8; ++m) a[m] = S[j0 + i][j0 + 2 * m + h];
+    int bad = -1;
+#pragma unroll
+    for (int j = 0; j < kSb; ++j) {
+        const double d = __shfl_sync(0xffffffffu, a[j / 2], j + 16 * (j & 1));
+        double v = 0.0;
+        if (bad < 0 && j0 + j < bs) {   // uniform in the warp
+            if (!(d > 0.0)) {           // not positive, or NaN
+                bad = j;
+            } else {
+                const double r = pivot_rsqrt(d);
+                if (i == j) {
+                    dd = d;
+                    rr = r;
+                }
+                v = a[j / 2] * r;
+                if (h == (j & 1) && i > j) a[j / 2] = v;
+            }
+        }
+        v = __shfl_sync(0xffffffffu, v, i + 16 * (j & 1));   // L(i, j)
+#pragma unroll
+        for (int m = j / 2; m < 8; ++m) {
+            const int c = 2 * m + h;
+            const double lc = __shfl_sync(0xffffffffu, v, c);
+            if (bad < 0 && c > j && i >= c) a[m] -= v * lc;
+        }
+    }
+    const double l = pivot_sqrt(dd, rr);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+        const int c = 2 * m + h;
+        const bool done = c == i && j0 + i < bs && (bad < 0 || i < bad);
+        if (c <= i) S[j0 + i][j0 + c] = done ? l : a[m];
+    }
+    if (h == 0) rL[j0 + i] = rr;
+    if (lane == 0 && bad >= 0) *fail = j0 + bad;
+}
+
+// Solve rows of X L16^T = A16 in place: Q lanes a row (lane q of them holds
+// columns q, q + Q, ... of the sixteen), L16's rows and reciprocal pivots in
+// shared memory.  x_j goes around the lanes by a shuffle.
+template <int Q>
+__device__ __forceinline__ void solve16(double (&a)[kSb / Q], const double (*L)[kPb + 1], int j0, const double *rL,
                                         int q) {
 #pragma unroll
     for (int j = 0; j < kSb; ++j) {
-        double x = a[j / 4] * rL[j0 + j];
-        x = __shfl_sync(0xffffffffu, x, j & 3, 4);
-        if (q == (j & 3)) a[j / 4] = x;
+        double x = a[j / Q] * rL[j0 + j];
+        x = __shfl_sync(0xffffffffu, x, j % Q, Q);
+        if (q == j % Q) a[j / Q] = x;
 #pragma unroll
-        for (int m = j / 4; m < 4; ++m)
-            if (q + 4 * m > j) a[m] -= x * L[j0 + q + 4 * m][j0 + j];
+        for (int m = j / Q; m < kSb / Q; ++m)
+            if (q + Q * m > j) a[m] -= x * L[j0 + q + Q * m][j0 + j];
     }
 }
 
+// S(i, c) less the products of columns [l0, l0 + 16) of rows i and c
+__device__ __forceinline__ void update16(double (*S)[kPb + 1], int i, int c, int l0) {
+    double s0 = S[i][c], s1 = 0.0;
+#pragma unroll
+    for (int l = 0; l < kSb; l += 2) {
+        s0 -= S[i][l0 + l] * S[c][l0 + l];
+        s1 -= S[i][l0 + l + 1] * S[c][l0 + l + 1];
+    }
+    S[i][c] = s0 + s1;
+}
+
 // diagonal block [kb, kb + bs): right-looking over sub-blocks of 16 columns; a
-// failing pivot is stored in place and ends the task (info = column + 1).  Bound
-// by the chain of pivots and the FP64 instructions between them: 121 us per
-// block with two barriers a column, 102 us now.
+// failing pivot is stored in place and ends the task (info = column + 1).  Bound by
+// the chain of pivots: an FP64 instruction takes a warp 65 cycles, and a column 6
+// of them and its updates.  So only the next sub-block's diagonal part is updated
+// before its factorization (warp 0), the rest beside it (six warps that share no
+// sub-partition with warp 0).  A block took 121 us with two barriers a column, 102
+// with sub-blocks one after the other; 60 now.
 __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task *tasks, int *info,
                                                          int kb) {
     __shared__ double S[kPb][kPb + 1];
@@ -217,6 +272,7 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task 
     const int bs = min(kPb, t.n - kb);
     const PotrfView V{t.A, t.lda, t.uplo == 'U' || t.uplo == 'u'};
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+#pragma unroll 16
     for (int e = tid; e < kPb * kPb; e += 256) {
         const int i = V.up ? e / kPb : e % kPb, j = V.up ? e % kPb : e / kPb;
         S[i][j] = (i < bs && j <= i) ? V.at(kb + i, kb + j) : 0.0;
@@ -225,35 +281,21 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task 
     __syncthreads();
     for (int j0 = 0; j0 < bs; j0 += kSb) {
         if (warp == 0) {
-            double a[kSb];
-            const int i = lane & (kSb - 1);
-#pragma unroll
-            for (int j = 0; j < kSb; ++j) a[j] = S[j0 + i][j0 + j];
-            int bad = -1;
-#pragma unroll
-            for (int j = 0; j < kSb; ++j) {
-                const double d = __shfl_sync(0xffffffffu, a[j], j);
-                if (bad < 0 && j0 + j < bs) {   // uniform in the warp
-                    if (!(d > 0.0)) {           // not positive, or NaN
-                        bad = j;
-                    } else {
-                        double r, l;
-                        pivot_root(d, r, l);
-                        if (lane == 0) rL[j0 + j] = r;
-                        a[j] = i == j ? l : a[j] * r;
-                    }
-                }
-#pragma unroll
-                for (int c = j + 1; c < kSb; ++c) {
-                    const double lc = __shfl_sync(0xffffffffu, a[j], c);
-                    if (bad < 0 && i >= c) a[c] -= a[j] * lc;
+            factor16(S, j0, bs, rL, &fail);
+        } else if (warp != 4 && j0 > 0) {
+            // rows from j0 + 16 on, columns from j0 on: 16 columns, then a triangle
+            const int r0 = j0 + kSb, nr = max(0, bs - r0), box = kSb * nr;
+            for (int e = (warp - 1 - (warp > 4)) * 32 + lane; e < box + nr * (nr + 1) / 2; e += 192) {
+                if (e < box) {
+                    update16(S, r0 + e % nr, j0 + e / nr, j0 - kSb);
+                } else {
+                    const int x = e - box;
+                    int i = (int)((sqrtf(8.f * x + 1.f) - 1.f) * 0.5f);
+                    i += (i + 1) * (i + 2) / 2 <= x;
+                    i -= i * (i + 1) / 2 > x;
+                    update16(S, r0 + i, r0 + x - i * (i + 1) / 2, j0 - kSb);
                 }
             }
-            if (lane < kSb)
-#pragma unroll
-                for (int j = 0; j < kSb; ++j)
-                    if (j <= i) S[j0 + i][j0 + j] = a[j];
-            if (lane == 0 && bad >= 0) fail = j0 + bad;
         }
         __syncthreads();
         if (fail >= 0) break;
@@ -266,23 +308,15 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task 
             double a[4];
 #pragma unroll
             for (int m = 0; m < 4; ++m) a[m] = in ? S[row][j0 + q + 4 * m] : 0.0;
-            solve16(a, S, j0, rL, q);
+            solve16<4>(a, S, j0, rL, q);
 #pragma unroll
             for (int m = 0; m < 4; ++m)
                 if (in) S[row][j0 + q + 4 * m] = a[m];
         }
         __syncthreads();
-        const int nr = bs - below;
-        for (int e = tid; e < nr * nr; e += 256) {
-            const int i = below + e % nr, c = below + e / nr;
-            if (c > i) continue;
-            double s0 = S[i][c], s1 = 0.0;
-#pragma unroll
-            for (int l = 0; l < kSb; l += 2) {
-                s0 -= S[i][j0 + l] * S[c][j0 + l];
-                s1 -= S[i][j0 + l + 1] * S[c][j0 + l + 1];
-            }
-            S[i][c] = s0 + s1;
+        {
+            const int i = below + (tid >> 4), c = below + (tid & 15);   // the next diagonal part
+            if (c <= i && i < bs) update16(S, i, c, j0);
         }
         __syncthreads();
     }
@@ -293,45 +327,52 @@ __global__ void __launch_bounds__(256) potrf_diag_kernel(const hcore_potrf_task 
     if (tid == 0 && fail >= 0) info[blockIdx.x] = kb + fail + 1;
 }
 
-// panel rows below the diagonal block: X L_kk^T = A_ik, 32 rows a CTA, four
-// lanes a row.  Sixteen columns at a time are solved in registers and taken
-// out of the columns on their right (64 steps with a barrier each, 64 rows a
-// CTA, took 126 us a block, eight tiles of order 1024; this 47 us).
-constexpr int kPr = 32;
-__global__ void __launch_bounds__(4 * kPr) potrf_panel_kernel(const hcore_potrf_task *tasks,
-                                                              const int *info, int kb) {
+// panel rows below the diagonal block: X L_kk^T = A_ik, Q lanes a row, 128 / Q
+// rows a CTA.  Sixteen columns at a time are solved in registers and taken out of
+// the columns on their right (64 steps with a barrier each, 64 rows a CTA, took 126
+// us a block, eight tiles of order 1024; this 48 us).  Bound by FP64 issue: about
+// 630 instructions a warp with four lanes a row, 360 with eight, which do the same
+// for half as many rows and so serve while all CTAs have an SM of their own (one
+// tile of order 300: 40 and 28 us).
+constexpr int kPrThreads = 128;
+template <int Q>
+__global__ void __launch_bounds__(kPrThreads) potrf_panel_kernel(const hcore_potrf_task *tasks,
+                                                                 const int *info, int kb) {
+    constexpr int PR = kPrThreads / Q;
     __shared__ double Ls[kPb][kPb + 1];
-    __shared__ double Xs[kPr][kPb + 1];
+    __shared__ double Xs[PR][kPb + 1];
     __shared__ double rL[kPb];
     const hcore_potrf_task t = tasks[blockIdx.y];
     if (info[blockIdx.y] != 0 || kb >= t.n) return;
     const int bs = min(kPb, t.n - kb);
-    const int r0 = kb + bs + blockIdx.x * kPr;
+    const int r0 = kb + bs + blockIdx.x * PR;
     if (r0 >= t.n) return;   // (rows below exist, so bs = kPb)
-    const int rows = min(kPr, t.n - r0);
+    const int rows = min(PR, t.n - r0);
     const PotrfView V{t.A, t.lda, t.uplo == 'U' || t.uplo == 'u'};
     const int tid = threadIdx.x;
-    for (int e = tid; e < kPb * kPb; e += 4 * kPr) {
+#pragma unroll 16
+    for (int e = tid; e < kPb * kPb; e += kPrThreads) {
         const int i = V.up ? e / kPb : e % kPb, j = V.up ? e % kPb : e / kPb;
         Ls[i][j] = j <= i ? V.at(kb + i, kb + j) : 0.0;
     }
-    for (int e = tid; e < kPr * kPb; e += 4 * kPr) {
-        const int i = V.up ? e / kPb : e % kPr, j = V.up ? e % kPb : e / kPr;
+#pragma unroll 16
+    for (int e = tid; e < PR * kPb; e += kPrThreads) {
+        const int i = V.up ? e / kPb : e % PR, j = V.up ? e % kPb : e / PR;
         Xs[i][j] = i < rows ? V.at(r0 + i, kb + j) : 0.0;
     }
     if (tid < kPb) rL[tid] = 1.0 / V.at(kb + tid, kb + tid);
     __syncthreads();
-    const int r = tid >> 2, q = tid & 3;
+    const int r = tid / Q, q = tid % Q;
 #pragma unroll 1
     for (int j0 = 0; j0 < kPb; j0 += kSb) {
-        double a[4];
+        double a[kSb / Q];
 #pragma unroll
-        for (int m = 0; m < 4; ++m) a[m] = Xs[r][j0 + q + 4 * m];
-        solve16(a, Ls, j0, rL, q);
+        for (int m = 0; m < kSb / Q; ++m) a[m] = Xs[r][j0 + q + Q * m];
+        solve16<Q>(a, Ls, j0, rL, q);
 #pragma unroll
-        for (int m = 0; m < 4; ++m) Xs[r][j0 + q + 4 * m] = a[m];
-        __syncwarp();   // a row's four lanes share a warp
-        for (int c = j0 + kSb + q; c < kPb; c += 4) {
+        for (int m = 0; m < kSb / Q; ++m) Xs[r][j0 + q + Q * m] = a[m];
+        __syncwarp();   // a row's lanes share a warp
+        for (int c = j0 + kSb + q; c < kPb; c += Q) {
             double s0 = Xs[r][c], s1 = 0.0;
 #pragma unroll
             for (int l = 0; l < kSb; l += 2) {
@@ -343,8 +384,8 @@ __global__ void __launch_bounds__(4 * kPr) potrf_panel_kernel(const hcore_potrf_
         __syncwarp();
     }
     __syncthreads();
-    for (int e = tid; e < kPr * kPb; e += 4 * kPr) {
-        const int i = V.up ? e / kPb : e % kPr, j = V.up ? e % kPb : e / kPr;
+    for (int e = tid; e < PR * kPb; e += kPrThreads) {
+        const int i = V.up ? e / kPb : e % PR, j = V.up ? e % kPb : e / PR;
         if (i < rows) V.at(r0 + i, kb + j) = Xs[i][j];
     }
 }
@@ -667,8 +708,11 @@ static int run_potrf(int n, const hcore_potrf_task *tasks, int *info, cudaStream
         potrf_diag_kernel<<<nr, 256, 0, s>>>(d_t, d_info, kb);
         const int below = maxn - std::min(maxn, kb + kPb), stage = stage_of[kb / kPb];
         if (below > 0) {
-            const int panels = (below + kPr - 1) / kPr, tiles = (below + kUt - 1) / kUt;
-            potrf_panel_kernel<<<dim3(panels, nr), 4 * kPr, 0, s>>>(d_t, d_info, kb);
+            const int tiles = (below + kUt - 1) / kUt;
+            if ((below + 15) / 16 * (long long)nr <= 152)
+                potrf_panel_kernel<8><<<dim3((below + 15) / 16, nr), kPrThreads, 0, s>>>(d_t, d_info, kb);
+            else
+                potrf_panel_kernel<4><<<dim3((below + 31) / 32, nr), kPrThreads, 0, s>>>(d_t, d_info, kb);
             if (stage < 0)
                 potrf_update_kernel<<<dim3(tiles * tiles, nr), 256, 0, s>>>(d_t, d_info, kb, tiles);
         }
