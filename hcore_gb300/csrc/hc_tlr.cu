@@ -13,7 +13,7 @@
 // triangular T' (transposing and/or reversing the index order of A).  T' is
 // walked in 32-column blocks: the block's diagonal part is solved by one warp
 // per vector (lane i holds x_i; 32 steps with a shuffle), then the rows below
-// are updated with the block's 32 solved values, 64 rows at a time through a
+// are updated with the block's 32 solved values, 64 or 128 rows at a time through a
 // shared-memory tile of T' that every vector of the CTA reuses.  Tiles are
 // read along A's contiguous dimension, so a transposed A is read coalesced
 // too.  A task's groups share A, which stays in L2.  Large triangles are solved
@@ -45,7 +45,7 @@
 namespace hc {
 
 constexpr int kTrBs = 32;  // diagonal block of T'
-constexpr int kTrRc = 64;  // rows per trailing chunk
+constexpr int kTrThreads = 256;
 
 struct TrsmWork {
     int task, v0, nv, pad;
@@ -68,7 +68,8 @@ struct TrsmView {
 template <int R>
 __device__ __forceinline__ void trsm_tile(double (*T)[kTrBs + 1], const TrsmView &v, int r0, int rows, int c0,
                           int cols) {
-    for (int e = threadIdx.x; e < R * kTrBs; e += blockDim.x) {
+#pragma unroll 8
+    for (int e = threadIdx.x; e < R * kTrBs; e += kTrThreads) {
         int r, c;
         if (v.tflag) {  // A(q, p): contiguous in q, i.e. along a row of T'
             c = e % kTrBs; r = e / kTrBs;
@@ -79,10 +80,12 @@ __device__ __forceinline__ void trsm_tile(double (*T)[kTrBs + 1], const TrsmView
     }
 }
 
-__global__ void __launch_bounds__(256) trsm_kernel(const hcore_trsm_task *tasks,
-                                                   const TrsmWork *work, int S) {
+// RC rows of T' per trailing chunk
+template <int RC>
+__global__ void __launch_bounds__(kTrThreads) trsm_kernel(const hcore_trsm_task *tasks,
+                                                          const TrsmWork *work, int S) {
     extern __shared__ double X[];  // X[i * S + v]
-    __shared__ double Tt[kTrRc][kTrBs + 1];
+    __shared__ double Tt[RC][kTrBs + 1];
     __shared__ double Td[kTrBs][kTrBs + 1];
     const TrsmWork w = work[blockIdx.x];
     const hcore_trsm_task t = tasks[w.task];
@@ -99,13 +102,13 @@ __global__ void __launch_bounds__(256) trsm_kernel(const hcore_trsm_task *tasks,
     const size_t es = left ? 1 : (size_t)t.ldb, vs = left ? (size_t)t.ldb : 1;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (t.alpha == 0.0) {  // B = 0 without reading A (BLAS convention)
-        for (int e = tid; e < n * w.nv; e += blockDim.x) {
+        for (int e = tid; e < n * w.nv; e += kTrThreads) {
             const int i = left ? e % n : e / w.nv, u = left ? e / n : e % w.nv;
             t.B[(size_t)i * es + (size_t)(w.v0 + u) * vs] = 0.0;
         }
         return;
     }
-    for (int e = tid; e < n * S; e += blockDim.x) {
+    for (int e = tid; e < n * S; e += kTrThreads) {
         const int i = left ? e % n : e / S, u = left ? e / n : e % S;
         double x = 0.0;
         if (u < w.nv) {
@@ -132,11 +135,11 @@ __global__ void __launch_bounds__(256) trsm_kernel(const hcore_trsm_task *tasks,
             if (lane < bs) X[(b0 + lane) * S + warp] = x;
         }
         __syncthreads();
-        for (int r0 = b0 + bs; r0 < n; r0 += kTrRc) {
-            const int rc = min(kTrRc, n - r0);
-            trsm_tile<kTrRc>(Tt, v, r0, rc, b0, bs);
+        for (int r0 = b0 + bs; r0 < n; r0 += RC) {
+            const int rc = min(RC, n - r0);
+            trsm_tile<RC>(Tt, v, r0, rc, b0, bs);
             __syncthreads();
-            for (int o = tid; o < kTrRc * S; o += blockDim.x) {
+            for (int o = tid; o < RC * S; o += kTrThreads) {
                 const int u = o % S, r = o / S;
                 if (r < rc && u < w.nv) {
                     double acc = X[(r0 + r) * S + u];
@@ -148,7 +151,7 @@ __global__ void __launch_bounds__(256) trsm_kernel(const hcore_trsm_task *tasks,
             __syncthreads();
         }
     }
-    for (int e = tid; e < n * w.nv; e += blockDim.x) {
+    for (int e = tid; e < n * w.nv; e += kTrThreads) {
         const int i = left ? e % n : e / w.nv, u = left ? e / n : e % w.nv;
         const int ia = v.rev ? n - 1 - i : i;
         t.B[(size_t)ia * es + (size_t)(w.v0 + u) * vs] = X[i * S + u];
@@ -447,19 +450,25 @@ __global__ void __launch_bounds__(256) potrf_update_kernel(const hcore_potrf_tas
 // ---------------------------------------------------------------------------
 static size_t al256(size_t x) { return (x + 255) & ~(size_t)255; }
 
-// vectors per CTA: up to 8 while the CTA's vectors take at most 64 KB of
-// shared memory (two or more CTAs per SM), fewer for longer vectors, 0 if
-// not even one fits
-static int trsm_stride(int maxn) {
+// Vectors per CTA for `vectors` of them in all (tasks' last groups aside): up to 8
+// while the CTA's vectors take at most 64 KB of shared memory (two or more CTAs per
+// SM), fewer for longer vectors and while the CTAs do not outnumber the SMs: a
+// CTA's time is its vectors' FP64 multiply-adds (order 300, 16 vectors: 214 us with
+// eight a CTA, 131 with one; order 1024, 100 vectors: 1742, 803).  0 if not even one fits.
+static int trsm_stride(int maxn, long long vectors) {
     int dev = 0, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-    const long long stat = (kTrRc + kTrBs) * (kTrBs + 1) * (long long)sizeof(double);
+    const long long stat = (64 + kTrBs) * (kTrBs + 1) * (long long)sizeof(double);
     const long long per = (long long)maxn * (long long)sizeof(double);
-    for (int S = 8; S >= 1; S >>= 1)
-        if (per * S <= 65536 && per * S + stat <= optin) return S;
-    return per + stat <= optin ? 1 : 0;
+    if (per + stat > optin) return 0;
+    int S = 8;
+    while (S > 1 && (per * S > 65536 || 2 * vectors <= 152LL * S)) S >>= 1;
+    return S;
 }
+
+static int order_of(const hcore_trsm_task &t) { return t.side == HCORE_Left ? t.M : t.N; }
+static int vectors_of(const hcore_trsm_task &t) { return t.side == HCORE_Left ? t.N : t.M; }
 
 static bool trsm_valid(const hcore_trsm_task &t) {
     const bool side = t.side == HCORE_Left || t.side == HCORE_Right;
@@ -472,14 +481,16 @@ static bool trsm_valid(const hcore_trsm_task &t) {
     return t.A && t.B && t.lda >= std::max(1, na) && t.ldb >= std::max(1, t.M);
 }
 
-// Triangles from this order on are solved by blocks: the vectors against a
+// Triangles from this order on may be solved by blocks: the vectors against a
 // diagonal block of kTrTb (trsm_kernel), then one product on the tensor cores
 // takes them out of all rows (columns) that follow.  The whole solve in one CTA
-// per eight vectors is bound by FP64 issue and, with few vectors, by its chain
-// of n / 32 blocks; a block step costs about 55 us however few the vectors.
-// Whole and by blocks, us (one GB300): order 384, 16 vectors 301, 318; 512 492,
-// 430; 1024 1747, 889; eight of order 384 with 240 vectors each 481, 434; 1024
-// 2720, 1286.
+// is bound by the FP64 issue of its vectors and its chain of n / 32 blocks; a block
+// step costs about 45 us however few the vectors.  Both ways, whole and by blocks,
+// us (one GB300), by the vectors of all such tasks: order 448: 16 210, 356; 800 390,
+// 414; 1920 615, 510; order 512: 160 278, 444; 800 487, 477; 1920 773, 589; order
+// 1024: 160 879, 926; 480 1147, 901; 1920 2744, 1297.  So by blocks where CTAs of
+// eight vectors outnumber the SMs, or where order and vectors a CTA (trsm_stride)
+// make the whole solve as long as at order 512 with eight.
 constexpr int kTrTcOrder = 448, kTrTb = 64;
 
 // Step `blk` of a task solved by blocks: the diagonal block's task, and the
@@ -526,7 +537,7 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
         if (t.M == 0 || t.N == 0) continue;
         maxn = std::max(maxn, t.side == HCORE_Left ? t.M : t.N);
     }
-    if (trsm_stride(maxn) == 0) {
+    if (trsm_stride(maxn, 0) == 0) {
         set_error("hcore_gpu_trsm_batched: triangle of order %d does not fit shared memory", maxn);
         return HCORE_GPU_EINVAL;
     }
@@ -534,6 +545,7 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
     // of the others, step by step, each followed by a stage of products
     struct Launch {
         size_t work0, count;
+        long long vectors;
         int S, maxn, stage;
     };
     std::vector<hcore_trsm_task> solve;
@@ -541,18 +553,24 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
     std::vector<Launch> launches;
     DenseProducts pr;
     int steps = 0;
-    auto by_blocks = [](const hcore_trsm_task &t) {
-        return t.alpha != 0.0 && t.M > 0 && t.N > 0 && (t.side == HCORE_Left ? t.M : t.N) >= kTrTcOrder;
+    long long large = 0;   // vectors of the tasks that may go by blocks
+    for (int i = 0; i < n; ++i)
+        if (tasks[i].M > 0 && tasks[i].N > 0 && order_of(tasks[i]) >= kTrTcOrder)
+            large += vectors_of(tasks[i]);
+    const int large_S = trsm_stride(kTrTcOrder, large);
+    auto by_blocks = [&](const hcore_trsm_task &t) {
+        return t.alpha != 0.0 && t.M > 0 && t.N > 0 && order_of(t) >= kTrTcOrder &&
+               (large > 8 * 152 || (long long)order_of(t) * large_S >= 8 * 512);
     };
     for (int blk = -1; blk < steps; ++blk) {
-        Launch l{work.size(), 0, 0, 1, -1};
+        Launch l{work.size(), 0, 0, 0, 1, -1};
         std::vector<int> todo;
         const size_t first = solve.size();
         bool any = false;
         for (int i = 0; i < n; ++i) {
             const hcore_trsm_task &t = tasks[i];
             if (t.M == 0 || t.N == 0) continue;
-            const int order = t.side == HCORE_Left ? t.M : t.N;
+            const int order = order_of(t);
             hcore_trsm_task d = t;
             if (by_blocks(t)) {
                 steps = std::max(steps, (order + kTrTb - 1) / kTrTb);
@@ -562,12 +580,13 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
             } else if (blk >= 0) {
                 continue;
             }
-            l.maxn = std::max(l.maxn, d.side == HCORE_Left ? d.M : d.N);
+            l.maxn = std::max(l.maxn, order_of(d));
+            l.vectors += vectors_of(d);
             solve.push_back(d);
         }
-        l.S = trsm_stride(l.maxn);
+        l.S = trsm_stride(l.maxn, l.vectors);
         for (size_t q = first; q < solve.size(); ++q) {
-            const int nvec = solve[q].side == HCORE_Left ? solve[q].N : solve[q].M;
+            const int nvec = vectors_of(solve[q]);
             for (int v0 = 0; v0 < nvec; v0 += l.S) work.push_back({(int)q, v0, std::min(l.S, nvec - v0), 0});
         }
         l.count = work.size() - l.work0;
@@ -606,11 +625,13 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
     cudaError_t e = configure_dense_tc();
     for (const Launch &l : launches) {
         const size_t smem = (size_t)l.maxn * l.S * sizeof(double);
+        // (few vectors: larger chunks, fewer barriers)
+        auto kernel = l.S <= 2 && smem <= 65536 ? trsm_kernel<128> : trsm_kernel<64>;
         if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(trsm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) break;
-        trsm_kernel<<<(unsigned)l.count, 256, smem, s>>>((const hcore_trsm_task *)arena,
-                                                         (const TrsmWork *)(arena + bt) + l.work0, l.S);
+        kernel<<<(unsigned)l.count, kTrThreads, smem, s>>>((const hcore_trsm_task *)arena,
+                                                           (const TrsmWork *)(arena + bt) + l.work0, l.S);
         e = cudaGetLastError();
         if (e == cudaSuccess && l.stage >= 0) e = pr.launch_stage(arena, l.stage, s);
     }
