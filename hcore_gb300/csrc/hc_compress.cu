@@ -39,6 +39,7 @@
 
 #include "hc_host.h"
 #include "hc_products.h"
+#include "hc_scalar.cuh"
 
 namespace hc {
 
@@ -112,81 +113,124 @@ __global__ void range_test_vectors_kernel(double *omega, int n, int base) {
 }
 
 // Columns c0 .. c0 + nc of each listed tile's Q made orthonormal among
-// themselves (modified Gram-Schmidt; a warp keeps the column it updates in
-// registers, RPL rows per lane).  Twice: a block spans several decades of
-// singular values, and what one pass leaves (about 1e-9) would stay in E far
-// above delta and be found again as new directions (160 columns instead of 80
+// themselves (Gram-Schmidt, column by column).  Twice: a block spans several
+// decades of singular values, and what one pass leaves (about 1e-9) would stay in E
+// far above delta and be found again as new directions (160 columns instead of 80
 // for 1024-tiles of rank 40 at 1e-8).  They need not be orthogonal to the
 // earlier ones to rounding: E = D - Q B holds whatever Q is, and the plan
 // factors Q.
-template <int RPL>
-__global__ void __launch_bounds__(256, 1) range_orth_kernel(const RangeTile *tiles, const int *list, int c0,
-                                                            int nc) {
-    __shared__ double s_q[2][32 * RPL];
-    const RangeTile t = tiles[list[blockIdx.x]];
-    double *Q = t.Q + (size_t)c0 * t.M;
-    const int M = t.M, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    double x[RPL];
-    auto load = [&](int col) {
-#pragma unroll
-        for (int r = 0; r < RPL; ++r) {
-            const int i = lane + 32 * r;
-            x[r] = i < M ? Q[(size_t)col * M + i] : 0.0;
-        }
-    };
-    auto store = [&](int col) {
-#pragma unroll
-        for (int r = 0; r < RPL; ++r) {
-            const int i = lane + 32 * r;
-            if (i < M) Q[(size_t)col * M + i] = x[r];
-        }
-    };
-    auto publish = [&](double *q) {   // x / ||x|| (a zero column stays zero)
-        double s0 = 0.0, s1 = 0.0;
-#pragma unroll
-        for (int r = 0; r < RPL; r += 2) {
-            s0 += x[r] * x[r];
-            s1 += x[r + 1] * x[r + 1];
-        }
-        s0 += s1;
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s0 += __shfl_xor_sync(0xffffffffu, s0, o);
-        const double f = s0 > 0.0 ? rsqrt(s0) : 0.0;
-#pragma unroll
-        for (int r = 0; r < RPL; ++r) {
-            x[r] *= f;
-            q[lane + 32 * r] = x[r];
-        }
-    };
+// A cluster of CTAs per tile, R rows each in shared memory; a column's products
+// with itself and the later ones are summed over the cluster in one exchange, then
+// every CTA updates its rows (the arithmetic is bound by FP64 issue: one CTA per
+// tile, its columns in registers, took 670 us for 32 columns of 48 tiles of order
+// 1024; 340 now, three CTAs a tile).
+constexpr int kOrCols = 32, kOrMaxCluster = 8;
+static size_t orth_smem(int R) { return ((size_t)kOrCols * R + (2 * kOrMaxCluster + 2) * kOrCols) * sizeof(double); }
+
+__global__ void __launch_bounds__(256) range_orth_kernel(const RangeTile *tiles, const int *list, int c0,
+                                                         int nc, int cs, int R) {
+    extern __shared__ __align__(16) double or_sm[];
+    const RangeTile t = tiles[list[blockIdx.x / cs]];
+    const int cta = blockIdx.x % cs, M = t.M, r0 = cta * R, nr = R / 32;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    double *Q = t.Q + (size_t)c0 * M;
+    double *Y = or_sm;                                          // column c, row i: Y[c R + i]
+    double *part = Y + (size_t)kOrCols * R;                     // [parity][source CTA][column]
+    double *coef = part + 2 * kOrMaxCluster * kOrCols, *scale = coef + kOrCols;
+    for (int c = warp; c < nc; c += 8)
+        for (int i = lane; i < R; i += 32) Y[c * R + i] = r0 + i < M ? Q[(size_t)c * M + r0 + i] : 0.0;
+    cluster_sync();   // (every CTA has started before the first remote store)
+    int par = 0;
     for (int pass = 0; pass < 2; ++pass) {
-        if (warp == 0) {
-            load(0);
-            publish(s_q[0]);
-            store(0);
-        }
-        __syncthreads();
-        for (int j = 0; j + 1 < nc; ++j) {
-            const double *q = s_q[j & 1];
-            for (int col = j + 1 + warp; col < nc; col += 8) {
-                load(col);
-                double d0 = 0.0, d1 = 0.0;
+        for (int j = 0; j < nc; ++j, par ^= 1) {
+            const double *x = Y + j * R;
+            for (int g = j + 4 * warp; g < nc; g += 32) {
+                double v[4] = {0.0, 0.0, 0.0, 0.0};
+                const double *y[4];
 #pragma unroll
-                for (int r = 0; r < RPL; r += 2) {
-                    d0 += q[lane + 32 * r] * x[r];
-                    d1 += q[lane + 32 * (r + 1)] * x[r + 1];
+                for (int h = 0; h < 4; ++h) y[h] = Y + min(g + h, nc - 1) * R + lane;
+                for (int r = 0; r < nr; ++r) {
+                    const double xi = x[lane + 32 * r];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) v[h] = fma(xi, y[h][32 * r], v[h]);
                 }
-                d0 += d1;
+                // lane l comes to hold sum l >> 3
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) d0 += __shfl_xor_sync(0xffffffffu, d0, o);
-                const volatile double *qv = q;   // re-read rather than held in registers
+                for (int n = 2, o = 16; n >= 1; n /= 2, o /= 2) {
+                    const bool up = lane & o;
 #pragma unroll
-                for (int r = 0; r < RPL; ++r) x[r] -= d0 * qv[lane + 32 * r];
-                if (col == j + 1) publish(s_q[(j + 1) & 1]);
-                store(col);
+                    for (int e = 0; e < n; ++e) {
+                        const double keep = up ? v[e + n] : v[e], send = up ? v[e] : v[e + n];
+                        v[e] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+                    }
+                }
+#pragma unroll
+                for (int o = 4; o > 0; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+                const int c = g + (lane >> 3), to = lane & 7;
+                if (c < nc && to < cs)
+                    peer_store(part + (par * kOrMaxCluster + cta) * kOrCols + c, peer_delta(or_sm, to), v[0]);
+            }
+            cluster_sync();
+            if (warp == 0) {   // lane c: column c
+                double ss = 0.0, w = 0.0;
+                for (int q = 0; q < cs; ++q) {
+                    const double *p = part + (par * kOrMaxCluster + q) * kOrCols;
+                    ss += p[j];
+                    w += p[lane];
+                }
+                const double f = ss > 0.0 ? rsqrt(ss) : 0.0;   // (a zero column stays zero)
+                if (lane > j && lane < nc) coef[lane] = f * (f * w);
+                if (lane == j) scale[j] = f;
+            }
+            __syncthreads();
+            for (int g = j + 1 + 4 * warp; g < nc; g += 32) {
+                double *y[4], s[4];
+#pragma unroll
+                for (int h = 0; h < 4; ++h) {
+                    y[h] = Y + min(g + h, nc - 1) * R + lane;
+                    s[h] = coef[min(g + h, nc - 1)];
+                }
+                for (int r = 0; r < nr; ++r) {
+                    const double xi = x[lane + 32 * r];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h)
+                        if (g + h < nc) y[h][32 * r] -= s[h] * xi;
+                }
             }
             __syncthreads();
         }
+        for (int c = warp; c < nc; c += 8)
+            for (int i = lane; i < R; i += 32) Y[c * R + i] *= scale[c];
+        __syncthreads();
     }
+    for (int c = warp; c < nc; c += 8)
+        for (int i = lane; i < R && r0 + i < M; i += 32) Q[(size_t)c * M + r0 + i] = Y[c * R + i];
+}
+
+// CTAs per tile: at least two CTAs an SM, and as many as leave every tile's cluster
+// SMs of its own
+static cudaError_t launch_range_orth(const RangeTile *tiles, const int *list, int n, int c0, int nc, int maxM,
+                                     cudaStream_t s) {
+    auto rows = [&](int cs) { return (maxM + 32 * cs - 1) / (32 * cs) * 32; };
+    int cs = 1;
+    while (cs < kOrMaxCluster && (orth_smem(rows(cs)) > 110 * 1024 || (n * (cs + 1) <= 152 && rows(cs + 1) >= 64))) ++cs;
+    const size_t smem = orth_smem(rows(cs));
+    const cudaError_t e =
+        cudaFuncSetAttribute(range_orth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)n * cs);
+    cfg.blockDim = dim3(256);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = cs;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, range_orth_kernel, tiles, list, c0, nc, cs, rows(cs));
 }
 
 // ---- the range by a pivoted QR ---------------------------------------------------
@@ -495,11 +539,7 @@ static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compr
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_list, active.data(), active.size() * sizeof(int), cudaMemcpyHostToDevice, s);
         if (e == cudaSuccess) {
-            const unsigned g = (unsigned)active.size();
-            if (maxM <= 512) range_orth_kernel<16><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
-            else if (maxM <= 1024) range_orth_kernel<32><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
-            else range_orth_kernel<64><<<g, 256, 0, s>>>(d_tiles, d_list, c0, nc);
-            e = cudaGetLastError();
+            e = launch_range_orth(d_tiles, d_list, (int)active.size(), c0, nc, maxM, s);
         }
         // (both lists use one arena: the second's layout is copied after the
         // first's launches in stream order)

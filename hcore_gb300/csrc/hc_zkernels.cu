@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(kZqThreads) zgeqrf_kernel(const ZDesc *__restr
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nr = R / 32;
     for (int c = warp; c < k; c += kZqThreads / 32)
         for (int i = lane; i < R; i += 32) Y[(size_t)c * R + i] = r0 + i < M ? A[(size_t)c * M + r0 + i] : zmk(0, 0);
-    __syncthreads();
+    cluster_sync();   // (every CTA has started before the first remote store)
     for (int j = 0; j < k; ++j) {
         const int par = j & 1, jl = j - r0;   // row j here if 0 <= jl < R
         const bool owner = jl >= 0 && jl < R;
@@ -250,8 +250,7 @@ __global__ void __launch_bounds__(kZqThreads) zgeqrf_kernel(const ZDesc *__restr
                 zq_send(rj + c, to, 0, y.re);
                 zq_send(rj + c, to, 1, y.im);
             }
-        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_sync();
         // two lanes a column (real and imaginary part); every warp with columns forms
         // the reflector itself
         const double *ps = reinterpret_cast<const double *>(part + (size_t)par * kZqMaxCluster * K);
