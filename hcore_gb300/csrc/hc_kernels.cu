@@ -389,10 +389,14 @@ __global__ void __launch_bounds__(NW * 32, (RPL <= 32 ? 2 : 1) * (8 / NW))
 // phase with 2, 4 and 8 lanes (us): 16 updates of k 8-24 410, 287, 250; one
 // of k = 64 2839, 1753, 1453; 24 of k 80-116 8262, 5794, 6099; 384 of k
 // 12-68 4120, 3220, 3205 (whole plan 10787, 9669, 10455); 1900 of the same
-// 6216, 5747, 6881.
+// 6216, 5747, 6881.  FP32 (no pipe to wait for, so eight lanes up to two updates an
+// SM and 16 warps), the whole plan with 4 and 8 lanes: 256 of k 10-48 570, 535; 1000
+// of the same 933, 991; 20 of k 60-120 2611, 2276.
+template <typename T>
 static int svd_smem_lanes(int K, const int *lanes, int updates) {
     const int np = (K + 1) / 2;
     int g = np <= 24 ? lanes[0] : (np <= 64 ? lanes[1] : lanes[2]);
+    if (g < 0 && sizeof(T) == 4) g = updates <= 304 && 8 * np <= 512 ? 8 : 4;
     if (g < 0) g = updates <= 152 && 8 * np <= 256 ? 8 : 4;
     if (g == 0) {
         const int w = (np + 31) / 32;
@@ -707,7 +711,7 @@ cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int
                 if (e != cudaSuccess) return e;
             } else if (K <= shape.svd_smem_kmax) {
                 launch_svd_smem<T>(d_desc + bk.start, bk.count, ws, d_rank, d_status, d_info, K,
-                                   svd_smem_lanes(K, shape.svd_lanes, shape.updates), sb);
+                                   svd_smem_lanes<T>(K, shape.svd_lanes, shape.updates), sb);
             } else {
                 const cudaError_t e = launch_svd_cluster<T>(d_desc + bk.start, bk.count, ws, d_rank, d_status,
                                                             d_info, K, shape.big_updates, sb);

@@ -99,7 +99,10 @@ __device__ __forceinline__ double inv_sqrt(double x) {
     const double r = fma(-x * y, y, 1.0);
     return fma(y * r, fma(0.375, r, 0.5), y);
 }
-__device__ __forceinline__ float inv_sqrt(float x) { return 1.f / sqrtf(x); }
+__device__ __forceinline__ float inv_sqrt(float x) {   // one Newton step
+    const float y = frsqrt_fast(x), h = 0.5f * y;
+    return fmaf(h, fmaf(-x * y, y, 1.f), y);
+}
 // 1 / x, x normal and positive: y (1 + e + e^2), e = 1 - x y
 __device__ __forceinline__ double inv(double x) {
     float m;
@@ -109,7 +112,10 @@ __device__ __forceinline__ double inv(double x) {
     const double r = fma(-x, y, 1.0);
     return fma(y, fma(r, r, r), y);
 }
-__device__ __forceinline__ float inv(float x) { return 1.f / x; }
+__device__ __forceinline__ float inv(float x) {   // one Newton step
+    const float y = __fdividef(1.f, x);
+    return fmaf(y, fmaf(-x, y, 1.f), y);
+}
 
 // ---- Jacobi rotations ----------------------------------------------------------
 // t = v / (|w| + sqrt(w^2 + v^2)) with the sign of w v (w = 0: of v), the
@@ -136,8 +142,8 @@ __device__ __forceinline__ double tangent(double app, double aqq, double apq) {
 }
 __device__ __forceinline__ float tangent(float app, float aqq, float apq) {
     const float w = aqq - app, v = 2.f * apq;
-    const float h = sqrtf(fmaf(w, w, v * v));
-    const float t = fabsf(v) / (fabsf(w) + h);
+    const float h = fsqrt_fast(fmaf(w, w, v * v));
+    const float t = __fdividef(fabsf(v), fabsf(w) + h);
     return (w < 0.f) != (v < 0.f) ? -t : t;
 }
 

@@ -487,8 +487,8 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                         const T t = tangent(app, aqq, apq);
                         // (FP32 divides: it is cheap there, and the tracked
                         // reciprocals' drift of one rounding a rotation is not)
-                        const T rdp = sizeof(T) == 8 ? s_rd[p] : T(1) / dp;
-                        const T rdq = sizeof(T) == 8 ? s_rd[q] : T(1) / dq;
+                        const T rdp = sizeof(T) == 8 ? s_rd[p] : inv(dp);
+                        const T rdq = sizeof(T) == 8 ? s_rd[q] : inv(dq);
                         const T u = fma(t, t, T(1)), cs = inv_sqrt(u);
                         const T f1 = t * (dq * rdp), f2 = t * (dp * rdq);
                         np_ = app - t * apq;
@@ -1005,8 +1005,8 @@ __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
                     aqq = __ldcg(s_nrm + q);
                     dp = __ldcg(s_d + p);
                     dq = __ldcg(s_d + q);
-                    rdp = sizeof(T) == 8 ? __ldcg(s_rd + p) : T(1) / dp;
-                    rdq = sizeof(T) == 8 ? __ldcg(s_rd + q) : T(1) / dq;
+                    rdp = sizeof(T) == 8 ? __ldcg(s_rd + p) : inv(dp);
+                    rdq = sizeof(T) == 8 ? __ldcg(s_rd + q) : inv(dq);
                 }
                 const T dt = dot(x, y);
                 bool rot = false, redo_p = false, redo_q = false;
