@@ -242,8 +242,22 @@ __device__ __forceinline__ void make_reflector(T (&x)[RPL], int j, int M, int la
     }
     const T alpha = __shfl_sync(0xffffffffu, alpha_l, j & 31);
     ss = warp_sum(ss);
-    T xnorm;
-    if (ss > NormLim<T>::lo && ss < NormLim<T>::hi) {
+    T xnorm = 0, tj = 0, beta = alpha, scal = 1;
+    bool rescale = false;
+    const T n2 = fma(alpha, alpha, ss);
+    const bool plain = sizeof(T) == sizeof(double) && ss > NormLim<T>::lo && n2 < NormLim<T>::hi;
+    if (plain) {
+        // the short square root and reciprocals (hc_scalar.cuh): hypot, a square root
+        // and two divisions take about 100 FP64 instructions of 65 cycles in the
+        // chain of every column (QR panels of one update of order 512, k = 64: 432 us
+        // with them, 388 so)
+        const T rs = inv_sqrt(n2);
+        T nb = n2 * rs;
+        nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
+        beta = -copysign(nb, alpha);
+        tj = (beta - alpha) * -copysign(rs, alpha);
+        scal = copysign(inv(abs(alpha - beta)), alpha);
+    } else if (ss > NormLim<T>::lo && ss < NormLim<T>::hi) {
         xnorm = sqrt(ss);
     } else {  // scaled recomputation (dnrm2's guard against under/overflow)
         T amax = 0;
@@ -270,9 +284,7 @@ __device__ __forceinline__ void make_reflector(T (&x)[RPL], int j, int M, int la
         }
         xnorm = mul_exp2(sqrt(warp_sum(s2)), -sc);
     }
-    T tj = 0, beta = alpha, scal = 1;
-    bool rescale = false;
-    if (xnorm > T(0)) {
+    if (!plain && xnorm > T(0)) {
         beta = -copysign(hypot(alpha, xnorm), alpha);
         if (abs(beta) >= NormLim<T>::safmin) {
             tj = (beta - alpha) / beta;
