@@ -153,7 +153,10 @@ cudaError_t configure_svd_smem(int optin, int *kmax);
 template <typename T>
 void launch_svd_smem(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
                      int G, cudaStream_t s);
-// the same with a cluster of cs CTAs per update
+// the same with a cluster of cs CTAs per update; svd_spread_fit is how many such
+// clusters the GPU runs at once
+template <typename T>
+int svd_spread_fit(int K, int cs);
 template <typename T>
 cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
                               int cs, cudaStream_t s);

@@ -420,18 +420,22 @@ static int svd_smem_lanes(int K, const int *lanes, int updates) {
 
 // CTAs per update of the shared-memory SVD, the same bits whatever their number:
 // as many as leave each eight column pairs (one warp a sub-partition at 16 lanes a
-// pair), within the SMs that the plan's updates leave idle; one where that gives
-// fewer than four or the update has at most 24 pairs, since an exchange costs 0.8 us
-// of a round, about as much as it saves there.  FP32 rounds wait for latency, not
-// for a pipe.  SVD phase, one CTA and a cluster, us: one update of k = 40 550, 589;
-// 64 1403, 1175; 116 6241, 3556; 24 of k 80-116 5725, 4680 (six); 36 of k 16-56 913,
-// 841 (four); 48 of k 32-64 1355, 1389 (three).
+// pair) and as run at once for all of the plan's updates (a cluster's CTAs share a
+// GPC: 48 clusters of three fill 152 SMs, and the two left over of 50 ran alone
+// after them, 7.2 ms with one CTA, 7.7 so).  One where the update has at most 24
+// pairs, or where that gives too few, since an exchange costs 0.8 us of a round,
+// about as much as it saves there.  FP32 rounds wait for latency, not for a pipe.
+// SVD phase, one CTA and a cluster, us: one update of k = 40 550, 589; 64 1403,
+// 1175; 116 6241, 3556; 24 of k 80-116 5725, 4680 (six); 36 of k 16-56 913, 841
+// (four); 40 of k 80-116 5780, 4182, 48 of k 60-80 2801, 2168, of k 32-64 1355, 1389
+// (three).
 template <typename T>
 static int svd_spread(int K, const int *lanes, int updates) {
     const int np = (K + 1) / 2;
     if (sizeof(T) != sizeof(double) || np <= 24 || (np <= 64 ? lanes[1] : lanes[2]) >= 0) return 1;
-    const int cs = std::min({8, (np + 7) / 8, 152 / std::max(1, updates)});
-    return cs >= 4 ? cs : 1;
+    for (int cs = std::min({8, (np + 7) / 8, 152 / std::max(1, updates)}); cs >= (np > 32 ? 3 : 4); --cs)
+        if (svd_spread_fit<T>(K, cs) >= updates) return cs;
+    return 1;
 }
 
 // ---------------------------------------------------------------------------

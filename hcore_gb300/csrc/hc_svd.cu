@@ -1172,12 +1172,11 @@ static void launch_svd_g(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_s
 }
 
 // cs CTAs per update
-template <typename T>
-cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
-                              int cs, cudaStream_t s) {
+template <typename T, typename F>
+static auto with_spread(int K, int cs, unsigned grid, cudaStream_t s, F f) {
     const int pairs = ((K + 1) / 2 + cs - 1) / cs;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)n * cs);
+    cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem_bytes<T>(K);
     cfg.stream = s;
@@ -1188,8 +1187,24 @@ cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int
     at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    auto go = [&](auto kernel) { return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, d_info, K, cs); };
-    return pairs <= 8 ? go(svd_smem_kernel<T, 16, true>) : go(svd_smem_kernel<T, 8, true>);
+    return pairs <= 8 ? f(cfg, svd_smem_kernel<T, 16, true>) : f(cfg, svd_smem_kernel<T, 8, true>);
+}
+template <typename T>
+int svd_spread_fit(int K, int cs) {
+    int n = 0;
+    const cudaError_t e = with_spread<T>(K, cs, (unsigned)cs, nullptr, [&](const cudaLaunchConfig_t &cfg, auto kernel) {
+        return cudaOccupancyMaxActiveClusters(&n, kernel, &cfg);
+    });
+    if (e == cudaSuccess) return n;
+    cudaGetLastError();
+    return 0;
+}
+template <typename T>
+cudaError_t launch_svd_spread(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status, int *d_info, int K,
+                              int cs, cudaStream_t s) {
+    return with_spread<T>(K, cs, (unsigned)n * cs, s, [&](const cudaLaunchConfig_t &cfg, auto kernel) {
+        return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, d_info, K, cs);
+    });
 }
 
 template <typename T>
@@ -1235,6 +1250,8 @@ template void launch_svd_smem<double>(const Desc *, int, double *, int *, int *,
 template void launch_svd_smem<float>(const Desc *, int, float *, int *, int *, int *, int, int,
                                      cudaStream_t);
 
+template int svd_spread_fit<double>(int, int);
+template int svd_spread_fit<float>(int, int);
 template cudaError_t launch_svd_spread<double>(const Desc *, int, double *, int *, int *, int *, int, int,
                                                cudaStream_t);
 template cudaError_t launch_svd_spread<float>(const Desc *, int, float *, int *, int *, int *, int, int,

@@ -969,10 +969,10 @@ int zsvd_kmax() {
 // three CTAs share an SM, 9.01.
 static cudaError_t launch_zgesvd(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status, int K, int sms,
                                  cudaStream_t s) {
-    const int np = (K + 1) / 2, cs = np > 12 ? std::max(1, std::min({8, (np + 7) / 8, sms / n})) : 1;
-    const int pairs = (np + cs - 1) / cs;
+    const int np = (K + 1) / 2;
+    int cs = np > 12 ? std::max(1, std::min({8, (np + 7) / 8, sms / n})) : 1;
     const size_t smem = zsvd_smem_bytes(K);
-    auto go = [&](auto kernel, int G) {
+    auto go = [&](auto kernel, int G, int pairs, int *fit) {
         cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
@@ -987,10 +987,21 @@ static cudaError_t launch_zgesvd(const ZDesc *d_desc, int n, zd *ws, int *d_rank
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = cs > 1 ? 1 : 0;
+        if (fit) return cudaOccupancyMaxActiveClusters(fit, kernel, &cfg);
         return cudaLaunchKernelEx(&cfg, kernel, d_desc, ws, d_rank, d_status, K, cs);
     };
-    if (cs > 1) return pairs <= 8 ? go(zgesvd_kernel<16, true>, 16) : go(zgesvd_kernel<8, true>, 8);
-    return pairs <= 8 && n <= sms ? go(zgesvd_kernel<16, false>, 16) : go(zgesvd_kernel<8, false>, 8);
+    for (; cs > 1; --cs) {   // all clusters at once, or smaller ones
+        const int pairs = (np + cs - 1) / cs;
+        int fit = 0;
+        const cudaError_t e = pairs <= 8 ? go(zgesvd_kernel<16, true>, 16, pairs, &fit)
+                                         : go(zgesvd_kernel<8, true>, 8, pairs, &fit);
+        if (e != cudaSuccess) return e;
+        if (fit < n) continue;
+        return pairs <= 8 ? go(zgesvd_kernel<16, true>, 16, pairs, nullptr)
+                          : go(zgesvd_kernel<8, true>, 8, pairs, nullptr);
+    }
+    return np <= 8 && n <= sms ? go(zgesvd_kernel<16, false>, 16, np, nullptr)
+                               : go(zgesvd_kernel<8, false>, 8, np, nullptr);
 }
 
 cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, int *d_status,
