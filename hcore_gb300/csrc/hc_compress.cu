@@ -21,7 +21,7 @@
 // columns.  A truncated Householder QR with column pivoting (qrcp_kernel) does
 // the same one column at a time; it applies 3 M^2 FP64 FMAs per column on one
 // SM (98 ms for 48 tiles of 1024 and ranks 8-40 at 1e-8, where the blocks take
-// 7 ms and the whole call went from 120.7 to 19.3 ms), so it is kept for what
+// 5 ms and the whole call went from 120.7 to 13.9 ms), so it is kept for what
 // the blocks leave: small tiles, wide ranges, non-finite tiles.
 //
 // qrcp_kernel: one CTA per tile; the tile is copied into a workspace and

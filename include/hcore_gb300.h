@@ -82,9 +82,9 @@ extern "C" {
  * hc_rebuild_tc.cu).  This flag keeps the FP64 (DFMA) reflector kernel for
  * every update instead. */
 #define HCORE_GPU_DFMA_REBUILD 0x8
-/* FP64 plans factor the stacked matrices of updates with a + c <= 64 as a
- * blocked Householder QR: 16-column panels in FP64, the trailing columns
- * updated between panels on the tensor cores, FP64-accurate (hc_qr_tc.cu).
+/* FP64 plans factor the stacked matrices as a blocked Householder QR:
+ * 16-column panels in FP64, the trailing columns updated between panels on the
+ * tensor cores, FP64-accurate (hc_qr_tc.cu).
  * This flag keeps the unblocked FP64 QR for every update instead. */
 #define HCORE_GPU_UNBLOCKED_QR 0x10
 /* FP64 plans: form the stack's products F = AV^T BV and G = BU F^T of updates
@@ -169,8 +169,8 @@ int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
  *                      runs each phase over all updates at once
  *   svd_lanes[3]       lanes per column pair of the shared-memory SVD buckets
  *                      with <= 24, <= 64 and more column pairs (1..32, a
- *                      power of two; 0: as many as fit in the warps that one
- *                      lane per pair needs)
+ *                      power of two, above 8 as 8; 0: as many as fit in the
+ *                      warps that one lane per pair needs)
  *   bucket_width       rank-bucket edges every 8 (fine) or 16 (coarse)
  *   phase_sync         0: each group runs its four phases as soon as it can
  *                      (phases of different groups overlap); 1: every group
@@ -181,7 +181,7 @@ int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
  * pair, width 8, no phase sync, 4 QR warps: the autotuner's pick on a TLR
  * panel of 1953 updates; HCORE_GPU_STREAMS overrides the groups; a plan
  * created without a tuning also gives a short list of small updates eight
- * lanes).  hcore_gpu_autotune
+ * lanes, and the SVDs of few wide ones a cluster of CTAs each).  hcore_gpu_autotune
  * times plans of the given tasks over a search of these parameters
  * (coordinate descent; each candidate's execute captured in a CUDA graph on
  * a private stream and replayed `reps` times) and returns the fastest; the
@@ -284,8 +284,9 @@ int hcore_gpu_potrf_batched(int n, const hcore_potrf_task *tasks, int *info, voi
  * in testing/testing_dgemm.c:119-236): a dense M x M tile D (ld ldd) becomes
  * U and V (M x r each, ld ldo) with D ~ U V^T, U the first r left singular
  * vectors, V = (S V^T)^T, r the number of leading singular values >= acc
- * (relative = 1: >= acc * sigma_max), capped at maxrank; r may be 0.  A
- * truncated pivoted QR finds the tile's range first, so ranks agree with a
+ * (relative = 1: >= acc * sigma_max), capped at maxrank; r may be 0.  The
+ * tile's range is found first (by blocks of test vectors, or a truncated pivoted
+ * QR where those do not apply), so ranks agree with a
  * full SVD's except for singular values within 1e-3 * threshold of it.
  * Status per tile: OK, NOCONV (non-finite input), RANK_MAX (the range needs
  * more than min(M, 512) columns).  M <= 2048.  Synchronous. */
