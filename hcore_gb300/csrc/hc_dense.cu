@@ -41,6 +41,7 @@ namespace hc {
 // diagonal only.  Tasks are split over CTAs (entries of S, rows of the factor)
 // so that uneven ranks and short lists fill the GPU.  768 tasks of ranks 8-32,
 // M = 1024: 2097 us in one kernel of a CTA per task, 825 + 723 us in these two.
+// Long lists form the factors as products on the tensor cores instead (DensePrep).
 __global__ void __launch_bounds__(256) dense_inner_kernel(const hcore_dense_task *tasks,
                                                           const DenseWork *work, double *ws) {
     const hcore_dense_task t = tasks[blockIdx.x];
@@ -115,12 +116,12 @@ __global__ void __launch_bounds__(128) dense_factor_kernel(const hcore_dense_tas
 
 
 cudaError_t launch_dense_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work, int n,
-                              int maxM, double *ws, cudaStream_t s) {
+                              int maxM, bool factors, double *ws, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     // about four CTAs an SM and more: a task's entries over up to eight CTAs
     const int split = std::max(1, std::min(8, 1216 / n));
     dense_inner_kernel<<<dim3(n, split), 256, 0, s>>>(d_tasks, d_work, ws);
-    dense_factor_kernel<<<dim3(n, (maxM + 127) / 128), 128, 0, s>>>(d_tasks, d_work, ws);
+    if (factors) dense_factor_kernel<<<dim3(n, (maxM + 127) / 128), 128, 0, s>>>(d_tasks, d_work, ws);
     return cudaGetLastError();
 }
 

@@ -500,7 +500,8 @@ struct DenseRun {
 struct DensePrep {
     int n = 0, maxM01 = 0;   // maxM01: largest syrk or gemmcd tile
     std::vector<int> bdcd;   // the gemmbdcd tasks
-    DenseProducts pr;        // the tasks' products, then the gemmbdcd tasks' Q = BD^T AV
+    std::vector<int> factor; // the syrk and gemmcd tasks whose factor is a product too
+    DenseProducts pr;        // the tasks' products, the gemmbdcd tasks' Q = BD^T AV, the factors
     long long ws = 0;        // doubles
     // arena: the tasks and the products' layout (what pack() writes), then the
     // workspace and the products' device arrays
@@ -577,6 +578,20 @@ struct DensePrep {
                 }
             }
         }
+        // Factors M x cols of the syrk and gemmcd tasks: as products where they take
+        // more than 40 million multiply-adds, 75 us at the FP64 pipe's rate, since three
+        // launches stand against one.  The whole call with FP64 factors and with
+        // products, us: 768 tasks of ranks 8-32, M = 1024 2907, 2628; 46 of ranks 17-52,
+        // M = 773 537, 414
+        double fma = 0.0;
+        for (int i = 0; i < n; ++i) {
+            const hcore_dense_task &t = tasks[i];
+            const int q = t.kind == 0 ? t.a : t.b;
+            if (t.kind > 1 || t.a == 0 || q == 0) continue;
+            factor.push_back(i);
+            fma += (double)t.M * t.a * q;
+        }
+        if (fma < 4e7) factor.clear();
         pr.stage(kBalanceByThread);
         for (int i : bdcd) {
             const hcore_dense_task &t = tasks[i];
@@ -585,6 +600,17 @@ struct DensePrep {
             w.coef = 1.0;
             w.tr = 3;
             pr.add_tile({pr.add(w, t.N ? t.N : t.M, t.a)});
+        }
+        pr.stage(kBalanceByWarp);
+        for (int i : factor) {
+            const hcore_dense_task &t = tasks[i];
+            const int q = t.kind == 0 ? t.a : t.b;
+            const bool left = t.kind == 0 || t.a > t.b;   // F S, or F S^T
+            DenseWork w{};
+            w.kk = left ? t.a : q;
+            w.coef = 1.0;
+            w.tr = left ? 2 : 0;
+            pr.add_tile({pr.add(w, t.M, left ? q : t.a)});
         }
         pr.stage(kBalanceByWarp);
         for (const auto &g : groups) pr.add_tile(g);
@@ -609,9 +635,22 @@ struct DensePrep {
             DenseWork &w = pr.work[n + q];
             w.P = t.Bd; w.ldp = t.ldb; w.Q = t.Av; w.ldq = t.lda;
         }
+        const int nb = n + (int)bdcd.size();
+        for (size_t q = 0; q < factor.size(); ++q) {
+            const hcore_dense_task &t = tasks[factor[q]];
+            DenseWork &w = pr.work[nb + q];
+            const bool left = t.kind == 0 || t.a > t.b;
+            w.P = left ? t.Au : t.Bu; w.ldp = t.kind == 0 ? t.lda : t.M;
+            w.Q = d_ws + pr.work[factor[q]].ws; w.ldq = t.a;   // S
+        }
         for (DenseJob &j : pr.jobs) {
             const bool aux = j.task >= n;
-            j.cd = aux ? d_ws + pr.work[bdcd[j.task - n]].ws : tasks[j.task].CD;
+            if (j.task >= nb) {
+                const hcore_dense_task &t = tasks[factor[j.task - nb]];
+                j.cd = d_ws + pr.work[factor[j.task - nb]].ws + (long long)t.a * (t.kind == 0 ? t.a : t.b);
+            } else {
+                j.cd = aux ? d_ws + pr.work[bdcd[j.task - n]].ws : tasks[j.task].CD;
+            }
             j.ldcd = aux ? j.M : tasks[j.task].ldcd;
         }
         for (int i = 0; i < n; ++i) {
@@ -648,7 +687,7 @@ struct DensePrep {
     cudaError_t launch(char *arena, cudaStream_t s) const {
         const cudaError_t e =
             maxM01 > 0 ? launch_dense_prep((const hcore_dense_task *)arena, pr.device_work(arena), n,
-                                           maxM01, (double *)(arena + o_ws), s)
+                                           maxM01, factor.empty(), (double *)(arena + o_ws), s)
                        : cudaSuccess;
         return e == cudaSuccess ? pr.launch(arena, s) : e;
     }

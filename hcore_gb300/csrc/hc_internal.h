@@ -231,7 +231,7 @@ struct DenseWork {
 };
 // S and the computed factor of the syrk and gemmcd tasks (of n tasks of all kinds)
 cudaError_t launch_dense_prep(const hcore_dense_task *d_tasks, const DenseWork *d_work, int n,
-                              int maxM, double *ws, cudaStream_t s);
+                              int maxM, bool factors, double *ws, cudaStream_t s);
 // the products on the tensor cores (hc_dense_tc.cu): the tasks of a tile laid
 // out along K in chunks of up to 128 columns.  cols[c] = (task, its column l).
 struct DenseChunk {
