@@ -249,6 +249,7 @@ __device__ __forceinline__ void combine4(long long (&acc)[4], uint32_t taddr) {
     constexpr unsigned long long C = 0x4B400000ull;
     constexpr unsigned long long K0 = (C * 257ull << 33) + (C * 257ull << 17) + (C * 257ull << 1);
     auto bits = [](float v) { return __float_as_uint(v + 12582912.f); };
+    __syncwarp();   // (the loads are .aligned, and what comes before branches by lane)
 #pragma unroll
     for (int m = 0; m < 4; ++m) {
         float v0[4], v1[4];

@@ -63,7 +63,8 @@ __device__ __forceinline__ long long pair_term(float v0, float v1) {
 }
 
 // add the eight planes of 8 columns (taddr: lane base + first column; plane
-// d sits d * stride columns further) into the running sums
+// d sits d * stride columns further) into the running sums.  The loads are .aligned:
+// combine_planes brings the warp together first, and nothing after that branches.
 template <int S, int PM>
 __device__ __forceinline__ void add_pair(long long (&acc)[8], uint32_t taddr, int stride) {
     float v0[8], v1[8];
@@ -75,6 +76,7 @@ __device__ __forceinline__ void add_pair(long long (&acc)[8], uint32_t taddr, in
 }
 template <int S>
 __device__ __forceinline__ void combine_planes(long long (&acc)[8], uint32_t taddr, int stride) {
+    __syncwarp();
     add_pair<S, 0>(acc, taddr, stride);
     add_pair<S, 1>(acc, taddr, stride);
     add_pair<S, 2>(acc, taddr, stride);

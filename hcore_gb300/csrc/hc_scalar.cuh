@@ -148,7 +148,10 @@ __device__ __forceinline__ float tangent(float app, float aqq, float apq) {
 }
 
 // ---- a cluster of CTAs on one update -------------------------------------------
+// (.aligned wants the whole warp at the barrier together, and callers come from loops
+// and branches that lanes leave at different times)
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }

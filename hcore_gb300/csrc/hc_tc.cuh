@@ -46,7 +46,9 @@ __host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
 
 // ---- tensor memory --------------------------------------------------------
 // One full warp allocates; the column base is written to *slot (shared).
+// (.aligned wants the whole warp at the instruction together)
 __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
                      smem_u32(slot)),
                  "r"(ncols)
@@ -54,6 +56,7 @@ __device__ __forceinline__ void tmem_alloc(uint32_t *slot, uint32_t ncols) {
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
 }
 __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+    __syncwarp();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
                  : "memory");
 }
