@@ -255,7 +255,7 @@ __device__ __forceinline__ void make_reflector(T (&x)[RPL], int j, int M, int la
         T nb = n2 * rs;
         nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
         beta = -copysign(nb, alpha);
-        tj = (beta - alpha) * -copysign(rs, alpha);
+        tj = fma(abs(alpha), rs, T(1));   // (beta - alpha) / beta; 2 where x is small
         scal = copysign(inv(abs(alpha - beta)), alpha);
     } else if (ss > NormLim<T>::lo && ss < NormLim<T>::hi) {
         xnorm = sqrt(ss);

@@ -149,6 +149,27 @@ __device__ __forceinline__ T group_sum(bool act, int start, int k, int lig, F f)
     return v;
 }
 
+// dlarfg's reflector of (alpha, x), ss = ||x||^2.  The scaled form, with tau as a sum
+// and v's first entry 1, because of what it does to row j when x is small beside
+// alpha (most columns of a graded T): tau is 2 and y_j becomes -y_j with one
+// rounding.  With an unscaled v = (alpha - beta, x) and 1 / (beta (beta - alpha)) the
+// factor 2 comes out of four rounded operations, and the QR's backward error was four
+// times as large (products of FP32 updates 1.83e-7 from their 64-bit values, 1.41e-7
+// so).
+template <typename T>
+__device__ __forceinline__ T reflector_scal(T alpha, T beta) {
+    return copysign(inv(abs(alpha - beta)), alpha);
+}
+template <typename T>
+__device__ __forceinline__ void reflector(T alpha, T ss, T &beta, T &tau, T &scal) {
+    const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
+    T nb = n2 * rs;
+    nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
+    beta = -copysign(nb, alpha);
+    tau = fma(abs(alpha), rs, T(1));
+    scal = reflector_scal(alpha, beta);
+}
+
 constexpr int kSvThreads = 512;
 constexpr int kSvRows = 6;   // 32-row pieces of the largest k (168)
 template <typename T>
@@ -171,7 +192,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     __shared__ unsigned char s_own[CL ? kSvMaxK<T> : 1];   // (static: every byte takes from k <= 119)
     extern __shared__ __align__(16) unsigned char smem_raw[];
     __shared__ T s_wmax[kSvThreads / 32];
-    __shared__ T s_vj;
+    __shared__ T s_scal;
     __shared__ int s_rank;
     const Desc d = descs[CL ? blockIdx.x / cs : blockIdx.x];
     const int cr = CL ? blockIdx.x % cs : 0;   // this CTA's rank in the cluster
@@ -197,7 +218,7 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     T *B = A + mat;                           // R_B, then R^T, rotated; at the end Q's reflectors
     T *X0 = B + mat, *X1 = X0 + (maxK + 1), *s_d = X1 + (maxK + 1);
     T *s_rd = s_d + (maxK + 1);               // R's diagonal, then 1 / s_d
-    T *s_tau = s_rd + (maxK + 1);             // 1 / g of reflector j, H = I - v v^T / g
+    T *s_tau = s_rd + (maxK + 1);             // of reflector j, H = I - tau v v^T
     short *s_perm = reinterpret_cast<short *>(s_tau + (maxK + 1));
     short *s_pcol = s_perm + (maxK + 1);
     T *Yg = base + L.Uo;   // reflectors of Q (k x k, ld k) in the Uo slot until U_r is written
@@ -314,29 +335,23 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 break;
             }
         }
-        // the reflector of column pv, rows j.., unscaled: v = (alpha - beta, x),
-        // beta = -sign(alpha) ||(alpha, x)|| (dlarfg's), g = beta (beta - alpha),
-        // by warp 0 while the others form x^T y for the remaining columns y
+        // the reflector of column pv, rows j.., dlarfg's: beta = -sign(alpha) ||(alpha,
+        // x)||, v = (1, scal x) (x itself stays as it is), scal = 1 / (alpha - beta),
+        // tau = (beta - alpha) / beta = 1 + |alpha| / ||(alpha, x)||, by warp 0 while the
+        // others form x^T y for the remaining columns y
         const T *ap = A + (size_t)pv * ld;
         if (warp == 0) {
             const T alpha = ap[j];
             T ss = 0;
             for (int i = j + 1 + lane; i < k; i += 32) ss += ap[i] * ap[i];
             ss = warp_sum(ss);
-            T beta = alpha, vj = 0, ginv = 0;
-            if (ss > SvLim<T>::safmin) {
-                const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
-                T nb = n2 * rs;
-                nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
-                beta = -copysign(nb, alpha);
-                vj = alpha - beta;
-                ginv = inv(fma(-alpha, beta, n2));
-            }
+            T beta = alpha, scal = 0, tau = 0;
+            if (ss > SvLim<T>::safmin) reflector(alpha, ss, beta, tau, scal);
             if (lane == 0) {
                 s_pcol[j] = (short)pv;
                 s_rd[j] = beta;
-                s_tau[j] = ginv;
-                s_vj = vj;
+                s_tau[j] = tau;
+                s_scal = scal;
             }
         }
         for (int c0 = 0; c0 < k; c0 += nqgrp) {
@@ -348,19 +363,21 @@ __global__ void __launch_bounds__(kSvThreads, 1)
         }
         __syncthreads();
         // apply it to them and downdate their norms (dlaqp2's rule), D lanes per column
-        const T ginv = s_tau[j], vj = s_vj;
+        const T tau = s_tau[j], scal = s_scal;
         const int i0 = j + 1 + ((dlig - (j + 1)) & (D - 1));
         for (int c0 = 0; c0 < k; c0 += nqgrp) {
             const int c = c0 + qgrp;
             const T nc = c < k ? nr[c] : T(-1);
             const bool act = c < k && c != pv && key(nc) >= 0;
             T *ac = A + (size_t)c * ld;
-            const bool upd = act && ginv != T(0);
-            // (row j's term, in lane 0's hands, is added to the sum of the rows below)
-            T acj = 0, s = 0;
+            const bool upd = act && tau != T(0);
+            // (row j's term, in lane 0's hands, is added to the sum of the rows below;
+            // s = tau v^T y itself leaves row j, s scal times x the rows below)
+            T r = act && dlig == 0 ? ac[j] : T(0), s = 0;
             if (upd && dlig == 0) {
-                acj = ac[j];
-                s = ginv * fma(vj, acj, nr2[c]);
+                s = tau * fma(scal, nr2[c], r);
+                r -= s;
+                s *= scal;
             }
             s = __shfl_sync(0xffffffffu, s, lane & ~(D - 1));
             T nn = 0;
@@ -369,7 +386,6 @@ __global__ void __launch_bounds__(kSvThreads, 1)
                 if (upd)
                     for (int i = i0; i < k; i += D) ac[i] -= s * ap[i];
                 if (dlig == 0) {
-                    const T r = upd ? acj - s * vj : ac[j];
                     ac[j] = r;
                     nn = nc - r * r;
                     redo = !(key(nn) > 0) || below_pow2(nn, s_d[c], 10);
@@ -402,9 +418,11 @@ __global__ void __launch_bounds__(kSvThreads, 1)
     // Q's reflectors to the workspace, B = R^T (its columns kk.. are zero)
     for (int h = warp; h < k; h += nw) {
         const T *ah = A + (size_t)s_pcol[h] * ld;
+        // v = (1, scal x); scal once more (no use without a reflector)
+        const T scal = h < kk && s_tau[h] != T(0) ? reflector_scal(ah[h], s_rd[h]) : T(0);
         for (int i = lane; i < k; i += 32) {
             const T x = ah[i];
-            if (h < kk && cr == 0) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rd[h] : T(0));
+            if (h < kk && cr == 0) Yg[(size_t)h * k + i] = i > h ? x * scal : (i == h ? T(1) : T(0));
             // R(i, h)
             B[(size_t)i * ld + h] = i < kk ? (i < h ? x : (i == h ? s_rd[h] : T(0))) : T(0);
         }
@@ -879,19 +897,12 @@ __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
         T p[R];
         load(p, A + (size_t)pv * k, j + 1, k, true);
         const T alpha = __ldcg(A + (size_t)pv * k + j), ss = dot(p, p);
-        T beta = alpha, vj = 0, ginv = 0;
-        if (ss > SvLim<T>::safmin) {
-            const T n2 = fma(alpha, alpha, ss), rs = inv_sqrt(n2);
-            T nb = n2 * rs;
-            nb = fma(fma(-nb, nb, n2) * T(0.5), rs, nb);
-            beta = -copysign(nb, alpha);
-            vj = alpha - beta;
-            ginv = inv(fma(-alpha, beta, n2));
-        }
+        T beta = alpha, scal = 0, tau = 0;
+        if (ss > SvLim<T>::safmin) reflector(alpha, ss, beta, tau, scal);
         if (tid == 0) {
             s_pcol[j] = (short)pv;
             s_rdiag[j] = beta;
-            s_tau[j] = ginv;
+            s_tau[j] = tau;
         }
         for (int c0 = 0; c0 < k; c0 += ngg) {
             const int c = c0 + gg;
@@ -901,17 +912,18 @@ __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
             T x[R];
             load(x, ac, j + 1, k, act);
             const T acj = act ? __ldcg(ac + j) : T(0);
-            const T s = ginv * fma(vj, acj, dot(x, p));
+            const T s = tau * fma(scal, dot(x, p), acj);
             T nn = 0;
             bool redo = false;
             if (act) {
-                if (ginv != T(0)) {
+                if (tau != T(0)) {
+                    const T sx = s * scal;
 #pragma unroll
-                    for (int r = 0; r < R; ++r) x[r] -= s * p[r];
+                    for (int r = 0; r < R; ++r) x[r] -= sx * p[r];
                     store(x, ac, j + 1, k);
                 }
-                const T r = ginv != T(0) ? acj - s * vj : acj;
-                if (lig == 0 && ginv != T(0)) ac[j] = r;
+                const T r = acj - s;
+                if (lig == 0 && tau != T(0)) ac[j] = r;
                 nn = nc - r * r;
                 redo = !(key(nn) > 0) || below_pow2(nn, __ldcg(s_d + c), 10);
             }
@@ -938,9 +950,10 @@ __global__ void __launch_bounds__(kClThreads, R <= 10 ? 2 : 1)
     __syncthreads();
     for (int h = gw; h < k; h += ngw) {
         const T *ah = A + (size_t)s_pcol[h] * k;
+        const T scal = h < kk && s_tau[h] != T(0) ? reflector_scal(__ldcg(ah + h), s_rdiag[h]) : T(0);
         for (int i = lane; i < k; i += 32) {
             const T x = __ldcg(ah + i);
-            if (h < kk) Yg[(size_t)h * k + i] = i > h ? x : (i == h ? x - s_rdiag[h] : T(0));
+            if (h < kk) Yg[(size_t)h * k + i] = i > h ? x * scal : (i == h ? T(1) : T(0));
             B[(size_t)i * k + h] = i < kk ? (i < h ? x : (i == h ? s_rdiag[h] : T(0))) : T(0);
         }
     }

@@ -155,7 +155,7 @@ __device__ __forceinline__ void zlarfg(zd alpha, double xn2, double &beta, zd &t
         nb = fma(fma(-nb, nb, n2) * 0.5, rs, nb);
         beta = -copysign(nb, alpha.re);
         const double ib = -copysign(rs, alpha.re), dr = alpha.re - beta;
-        tau = zmk(-dr * ib, -alpha.im * ib);
+        tau = zmk(fma(fabs(alpha.re), rs, 1.0), -alpha.im * ib);
         const double id = inv(fma(dr, dr, alpha.im * alpha.im));
         scal = zmk(dr * id, -alpha.im * id);
         return;
