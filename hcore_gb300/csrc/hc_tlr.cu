@@ -175,12 +175,17 @@ struct PotrfView {
 
 constexpr int kSb = 16;
 
-// 1 / sqrt(d) of a positive pivot, and sqrt(d) from both
+// 1 / sqrt(d) of a positive pivot, and sqrt(d) from both.  The short forms hold for
+// finite normal d; +Inf passes LAPACK's pivot test (not d <= 0, not NaN) and gives
+// L_jj = Inf and a column of zeros, as there.
+__device__ __forceinline__ bool plain_pivot(double d) {
+    return d >= 2.2250738585072014e-308 && d <= 1.7976931348623157e308;
+}
 __device__ __forceinline__ double pivot_rsqrt(double d) {
-    return d < 2.2250738585072014e-308 ? 1.0 / sqrt(d) : inv_sqrt(d);   // (subnormal)
+    return plain_pivot(d) ? inv_sqrt(d) : 1.0 / sqrt(d);
 }
 __device__ __forceinline__ double pivot_sqrt(double d, double r) {
-    if (d < 2.2250738585072014e-308) return sqrt(d);
+    if (!plain_pivot(d)) return sqrt(d);
     const double l = d * r;
     return fma(fma(-l, l, d) * 0.5, r, l);
 }
