@@ -215,8 +215,7 @@ static cudaError_t launch_range_orth(const RangeTile *tiles, const int *list, in
     int cs = 1;
     while (cs < kOrMaxCluster && (orth_smem(rows(cs)) > 110 * 1024 || (n * (cs + 1) <= 152 && rows(cs + 1) >= 64))) ++cs;
     const size_t smem = orth_smem(rows(cs));
-    const cudaError_t e =
-        cudaFuncSetAttribute(range_orth_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem(range_orth_kernel);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n * cs);
@@ -638,10 +637,7 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             std::vector<int> k1(nq), st1(nq);
             const size_t smem = (size_t)maxM * sizeof(double);
             e = cudaMemcpyAsync(d_qt, rest.data(), nq * sizeof(QrcpTask), cudaMemcpyHostToDevice, s);
-            if (e == cudaSuccess)
-                e = cudaFuncSetAttribute(qrcp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)std::max<size_t>(smem, 1024));
-            if (e == cudaSuccess) {
+            if (e == cudaSuccess) {   // (at most 16 KB of shared memory)
                 qrcp_kernel<<<nq, 256, smem, s>>>(d_qt, d_k, d_st);
                 e = cudaGetLastError();
             }

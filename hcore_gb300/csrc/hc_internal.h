@@ -144,6 +144,15 @@ template <typename T>
 cudaError_t launch_recompress(const Desc *d_desc, int n, T *ws, int *d_rank, int *d_status,
                               int *d_info, const LaunchShape &shape, cudaStream_t s,
                               unsigned phases);
+// Lets `kernel` be launched on the current device with all the dynamic shared memory
+// that its static part leaves of a CTA's.  The attribute belongs to the process,
+// not to the call: a call that set its own size would take another thread's away
+// between that one's setting and its launch, so it is set once per device, to the most.
+cudaError_t allow_smem(const void *kernel);
+template <typename... A>
+cudaError_t allow_smem(void (*kernel)(A...)) {
+    return allow_smem((const void *)kernel);
+}
 // SVD of updates whose two Jacobi matrices fit shared memory (hc_svd.cu):
 // configure sets the kernel's shared-memory attribute (not capturable) and
 // returns the largest such k; launch runs n updates of k <= K with G lanes

@@ -28,6 +28,8 @@
 #include <cfloat>
 #include <climits>
 #include <mutex>
+#include <set>
+#include <utility>
 
 #include "hc_internal.h"
 #include "hc_scalar.cuh"
@@ -617,6 +619,23 @@ int qr_launches(const LaunchShape &shape, bool fp64) {
     for (int b = 0; b < shape.nbuckets; ++b) n += shape.buckets[b].count;
     qr_plan(shape, n, [&](int, int, int count, int, int, int) { c += count > 0; });
     return c;
+}
+
+cudaError_t allow_smem(const void *kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void *>> done;
+    int dev = 0, optin = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count({dev, kernel})) return cudaSuccess;
+    cudaFuncAttributes fa;
+    e = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+    if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, optin - (int)fa.sharedSizeBytes);
+    if (e == cudaSuccess) done.insert({dev, kernel});
+    return e;
 }
 
 template <typename T>

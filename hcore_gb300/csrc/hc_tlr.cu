@@ -632,8 +632,7 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
         const size_t smem = (size_t)l.maxn * l.S * sizeof(double);
         // (few vectors: larger chunks, fewer barriers)
         auto kernel = l.S <= 2 && smem <= 65536 ? trsm_kernel<128> : trsm_kernel<64>;
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e == cudaSuccess) e = allow_smem(kernel);
         if (e != cudaSuccess) break;
         kernel<<<(unsigned)l.count, kTrThreads, smem, s>>>((const hcore_trsm_task *)arena,
                                                            (const TrsmWork *)(arena + bt) + l.work0, l.S);

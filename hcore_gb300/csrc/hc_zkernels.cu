@@ -914,8 +914,7 @@ template <int RPL>
 static void launch_zapply(const ZDesc *d_desc, int n, const zd *ws, const int *d_rank,
                           const int *d_status, int maxR, cudaStream_t s) {
     const size_t smem = (size_t)kZApplyChunk * 32 * RPL * sizeof(zd);
-    cudaFuncSetAttribute(zapply_kernel<RPL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem);
+    allow_smem(zapply_kernel<RPL>);
     zapply_kernel<RPL><<<dim3(n, 2, (maxR + 7) / 8), 256, smem, s>>>(d_desc, ws, d_rank,
                                                                       d_status);
 }
@@ -932,7 +931,7 @@ static cudaError_t launch_zgeqrf(const ZDesc *d_desc, int n, zd *ws, int maxM, i
         cs *= 2;
     const int R = rows(cs);
     const size_t smem = zqr_smem_bytes(maxK, R);
-    cudaError_t e = cudaFuncSetAttribute(zgeqrf_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = allow_smem(zgeqrf_kernel);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)n * cs, 2);
@@ -973,7 +972,7 @@ static cudaError_t launch_zgesvd(const ZDesc *d_desc, int n, zd *ws, int *d_rank
     int cs = np > 12 ? std::max(1, std::min({8, (np + 7) / 8, sms / n})) : 1;
     const size_t smem = zsvd_smem_bytes(K);
     auto go = [&](auto kernel, int G, int pairs, int *fit) {
-        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaError_t e = allow_smem(kernel);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3((unsigned)n * cs);
