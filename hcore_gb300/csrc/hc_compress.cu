@@ -598,7 +598,9 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
             p += al256c(M * 8);
             u.tau = (double *)p; p += al256c(kMaxK * 8);
             maxM = std::max(maxM, t.M);
-            if (const int cap = range_cap(t.M)) {
+            // (without a threshold every column of the range counts: the pivoted QR
+            // finds no more of them than there are)
+            if (const int cap = t.acc > 0.0 ? range_cap(t.M) : 0) {
                 RangeTile r{t.D, t.ldd, t.M, u.W, (double *)p, nullptr};
                 p += al256c(M * cap * 8);
                 r.B = (double *)p; p += al256c(M * cap * 8);
