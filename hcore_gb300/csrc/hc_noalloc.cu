@@ -28,8 +28,10 @@ namespace hc {
 
 // workspace capacity in doubles: M = 1024 rows with a + c <= 128 and
 // a*b <= 128*128 fit (ws_layout(1024, 128, 128, 128, no storage limit) is
-// 344992 doubles)
-constexpr long long kNoAllocWsElems = 393216;                // 3 MiB
+// 344992 doubles).  The limit that a call is checked against leaves the SVD's small
+// arrays out (ws_layout's sv): room for the largest of them stands beside it.
+constexpr long long kNoAllocLimit = 393216;                  // 3 MiB
+constexpr long long kNoAllocWsElems = kNoAllocLimit + (4LL * kMaxK + 16 + 31) / 32 * 32;
 constexpr size_t kNoAllocDescOff = kNoAllocWsElems * sizeof(double);
 constexpr size_t kNoAllocRankOff = kNoAllocDescOff + 512;   // rank, status
 constexpr size_t kNoAllocBytes = kNoAllocRankOff + 256;
@@ -120,11 +122,12 @@ extern "C" int hcore_gpu_dgemm_noalloc(int M, double alpha, const double *AU, co
         set_error("hcore_gpu_dgemm_noalloc: task rejected (status %d)", st0);
         return HCORE_GPU_ETASK;
     }
-    const long long need = ws_layout(d).total;
-    if (need > kNoAllocWsElems) {
+    const WsLayout lay = ws_layout(d);
+    const long long need = lay.total - (lay.Uo - lay.sv);
+    if (need > kNoAllocLimit) {
         set_error("hcore_gpu_dgemm_noalloc: M=%d, a+c=%d, a*b=%d needs %lld doubles of "
                   "workspace; the fixed scratch holds %lld (e.g. M=1024 with a+c <= 128)",
-                  M, k, a * b, need, kNoAllocWsElems);
+                  M, k, a * b, need, kNoAllocLimit);
         return HCORE_GPU_EINVAL;
     }
     // an error left pending by the caller's own earlier work stays the
