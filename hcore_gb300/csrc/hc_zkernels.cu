@@ -78,28 +78,29 @@ constexpr int kZf = 4, kZsRows = 64;
 
 __global__ void __launch_bounds__(256) zstack_inner_kernel(const ZDesc *__restrict__ descs, zd *__restrict__ ws) {
     const ZDesc d = descs[blockIdx.x];
-    const int lane = threadIdx.x & 31, q = blockIdx.y * 8 + (threadIdx.x >> 5);
-    if (d.status0 || q >= d.b) return;
-    const int M = d.M, a = d.a;
+    if (d.status0) return;
+    const int lane = threadIdx.x & 31, M = d.M, a = d.a;
     zd *F = ws + d.ws + zlayout(M, a, d.b, d.k).F;
-    const zd *y = d.BV + (size_t)q * d.ldbv;
-    for (int p0 = blockIdx.z * kZf; p0 < a; p0 += gridDim.z * kZf) {
-        const zd *x[kZf];
-        zd s[kZf];
+    for (int q = blockIdx.y * 8 + (threadIdx.x >> 5); q < d.b; q += gridDim.y * 8) {
+        const zd *y = d.BV + (size_t)q * d.ldbv;
+        for (int p0 = blockIdx.z * kZf; p0 < a; p0 += gridDim.z * kZf) {
+            const zd *x[kZf];
+            zd s[kZf];
 #pragma unroll
-        for (int h = 0; h < kZf; ++h) {
-            x[h] = d.AV + (size_t)min(p0 + h, a - 1) * d.ldav;
-            s[h] = zmk(0, 0);
-        }
-        for (int l = lane; l < M; l += 32) {
-            const zd v = y[l];
+            for (int h = 0; h < kZf; ++h) {
+                x[h] = d.AV + (size_t)min(p0 + h, a - 1) * d.ldav;
+                s[h] = zmk(0, 0);
+            }
+            for (int l = lane; l < M; l += 32) {
+                const zd v = y[l];
 #pragma unroll
-            for (int h = 0; h < kZf; ++h) s[h] = zfma(x[h][l], v, s[h]);
-        }
+                for (int h = 0; h < kZf; ++h) s[h] = zfma(x[h][l], v, s[h]);
+            }
 #pragma unroll
-        for (int h = 0; h < kZf; ++h) {
-            s[h] = zwarp_sum(s[h]);
-            if (lane == 0 && p0 + h < a) F[(size_t)q * a + p0 + h] = s[h];
+            for (int h = 0; h < kZf; ++h) {
+                s[h] = zwarp_sum(s[h]);
+                if (lane == 0 && p0 + h < a) F[(size_t)q * a + p0 + h] = s[h];
+            }
         }
     }
 }
@@ -1007,13 +1008,14 @@ cudaError_t launch_zrecompress(const ZDesc *d_desc, int n, zd *ws, int *d_rank, 
                                int maxM, int maxK, int maxB, cudaStream_t s) {
     if (n <= 0) return cudaSuccess;
     const int rpl = (maxM + 31) / 32;
-    if (rpl > 32 || maxK > zsvd_kmax() || maxB > 8 * 65535) return cudaErrorInvalidValue;
+    if (rpl > 32 || maxK > zsvd_kmax()) return cudaErrorInvalidValue;
     int dev = 0, sms = 1, optin = 0;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     // F: the z axis splits a column's rows while the grid is below two CTAs an SM
-    const int fy = (maxB + 7) / 8, fz = std::max(1, std::min((maxK + kZf - 1) / kZf, 2 * sms / std::max(1, n * fy)));
+    const int fy = std::min((maxB + 7) / 8, 65535);
+    const int fz = (int)std::max(1LL, std::min<long long>((maxK + kZf - 1) / kZf, 2 * sms / std::max(1LL, (long long)n * fy)));
     zstack_inner_kernel<<<dim3(n, fy, fz), 256, 0, s>>>(d_desc, ws);
     zstack_outer_kernel<<<dim3(n, (maxM + kZsRows - 1) / kZsRows), 256, 0, s>>>(d_desc, ws);
     if (cudaError_t e = launch_zgeqrf(d_desc, n, ws, maxM, maxK, sms, optin, s)) return e;
