@@ -202,7 +202,10 @@ def lib() -> C.CDLL:
     L.hcore_gpu_dense_batched.argtypes = [C.c_int, C.POINTER(DenseTask), vp]
     L.hcore_gpu_dense_plan_create.argtypes = [C.POINTER(vp), C.c_int, C.POINTER(DenseTask)]
     L.hcore_gpu_dense_plan_execute.argtypes = [vp, vp]
+    L.hcore_gpu_dense_plan_status.argtypes = [vp, vp]
     L.hcore_gpu_dense_plan_destroy.argtypes = [vp]
+    L.hcore_gpu_test_wait_cycles.argtypes = [C.c_longlong]
+    L.hcore_gpu_test_wait_cycles.restype = None
     L.hcore_gpu_trsm_batched.argtypes = [C.c_int, C.POINTER(TrsmTask), vp]
     L.hcore_gpu_compress_batched.argtypes = [C.c_int, C.POINTER(CompressTask),
                                              C.POINTER(C.c_int), C.POINTER(C.c_int), vp]
@@ -483,6 +486,11 @@ class DensePlan:
     def execute(self, stream=None):
         _check(lib().hcore_gpu_dense_plan_execute(self._plan, stream or None),
                "hcore_gpu_dense_plan_execute")
+
+    def status(self, stream=None):
+        """Waits for the stream; raises if a bounded wait inside an execute gave up."""
+        _check(lib().hcore_gpu_dense_plan_status(self._plan, stream or None),
+               "hcore_gpu_dense_plan_status")
 
     def close(self):
         if self._plan:

@@ -447,6 +447,11 @@ static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compr
     int *d_list = (int *)buf;
     double *d_part = (double *)(buf + b_list), *d_omega = (double *)(buf + b_list + b_part);
     std::vector<double> part((size_t)nt * kSumParts), limit(nt);
+    int *word = thread_ctx().wait_word();
+    if (!word) {
+        cudaFree(buf);
+        return cudaErrorMemoryAllocation;
+    }
     auto norms = [&](bool load) -> cudaError_t {
         cudaError_t r = cudaMemcpyAsync(d_list, active.data(), active.size() * sizeof(int),
                                         cudaMemcpyHostToDevice, s);
@@ -457,7 +462,9 @@ static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compr
         }
         if (r == cudaSuccess)
             r = cudaMemcpyAsync(part.data(), d_part, part.size() * sizeof(double), cudaMemcpyDeviceToHost, s);
-        return r == cudaSuccess ? cudaStreamSynchronize(s) : r;
+        if (r == cudaSuccess) r = cudaStreamSynchronize(s);
+        // a product whose wait gave up left NaN: an error, not a tile for the pivoted QR
+        return r == cudaSuccess && *(volatile int *)word ? cudaErrorLaunchTimeout : r;
     };
     auto sum_of = [&](int q) {
         double x = 0.0;
@@ -484,6 +491,7 @@ static cudaError_t find_ranges(int nt, const RangeTile *tiles, const hcore_compr
         }
         host.resize(up);
         p.pack(host.data());
+        p.gave_up = word;
         // (from pageable memory: the copy has left `host` when it returns)
         const cudaError_t r = cudaMemcpyAsync(arena, host.data(), up, cudaMemcpyHostToDevice, s);
         return r == cudaSuccess ? p.launch(arena, s) : r;
@@ -650,6 +658,10 @@ static int run_compress(int n, const hcore_compress_task *tasks, int *ranks, int
                 hk[rest_q[x]] = k1[x];
                 hst[rest_q[x]] = st1[x];
             }
+        }
+        if (e == cudaErrorLaunchTimeout && thread_ctx().word && *(volatile int *)thread_ctx().word) {
+            cudaFree(qa);
+            return check_waits(thread_ctx().word, "hcore_gpu_compress_batched");
         }
         if (e != cudaSuccess) {
             set_error("hcore_gpu_compress_batched: %s", cudaGetErrorString(e));

@@ -321,14 +321,22 @@ __device__ __forceinline__ void walk_tile(Walk &w, const DenseJob *jobs, int njo
             }
 }
 
-// A wait gave up: NaN in every tile of this CTA, never stale or half-summed
-// ones (thread: one row, 8 columns).
+// tiles that a job's mask or its skip word leaves out
+__device__ __forceinline__ bool tile_left_out(const Walk &w) {
+    return (w.job.mask == 1 && w.row0 + kRowsA <= w.col0) ||
+           (w.job.mask == 2 && w.row0 >= w.col0 + kRowsB) || (w.job.skip && *w.job.skip != 0);
+}
+
+// A wait gave up: NaN in every tile of this CTA, never stale or half-summed ones
+// (thread: one row, 8 columns), and a word that the host reads (in its pinned memory).
 __device__ __noinline__ void poison_tiles(const DenseJob *jobs, int njobs, const DenseChunk *chunks,
-                                          int ntiles, int lrow, int cw) {
+                                          int ntiles, int lrow, int cw, int *gave_up) {
+    *gave_up = 1;
     Walk w;
     w.j = 0;
     for (w.t = blockIdx.x; w.t < ntiles; w.t += gridDim.x) {
         walk_tile(w, jobs, njobs, chunks);
+        if (tile_left_out(w)) continue;
         const int row = w.row0 + lrow;
         for (int col = w.col0 + cw; col < min(w.col0 + cw + 8, w.job.N); ++col)
             if (row < w.job.M && !(w.job.mask == 1 && row < col) && !(w.job.mask == 2 && row > col))
@@ -336,19 +344,16 @@ __device__ __noinline__ void poison_tiles(const DenseJob *jobs, int njobs, const
     }
 }
 
-// tiles that a job's mask or its skip word leaves out
-__device__ __forceinline__ bool tile_left_out(const Walk &w) {
-    return (w.job.mask == 1 && w.row0 + kRowsA <= w.col0) ||
-           (w.job.mask == 2 && w.row0 >= w.col0 + kRowsB) || (w.job.skip && *w.job.skip != 0);
-}
-
 // Two CTAs of 18 warps per SM: 16 workers (thread: one row, 8 columns), a
 // producer that walks the units, fetches their blocks and describes them, and
-// an issuer of MMAs.  All waits are bounded.
+// an issuer of MMAs.  All waits are bounded: after `limit` clock cycles a role gives
+// up, and so in turn do those that wait for it; the workers are the last, and fill
+// the tiles with NaN.  What a role has in flight by then, copies or MMAs, it waits
+// for with the full limit, whatever `limit` is.
 __global__ void __launch_bounds__(kThreadsTc, 2)
     dense_tile_tc_kernel(const DenseWork *work, const int2 *cols, const DenseChunk *chunks,
                          const DenseJob *jobs, int njobs, int ntiles, const unsigned char *slices,
-                         const int *exps) {
+                         const int *exps, int *gave_up, long long limit) {
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *misc = sm + kStages * kStage;
     uint64_t *full = reinterpret_cast<uint64_t *>(misc), *empty = full + kStages;
@@ -395,7 +400,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 for (int kb = 0; kb < nblocks && ok; ++kb, ++b) {
                     const int s = b % kStages;
                     if (b >= kStages)
-                        ok = tc::mbar_wait(empty + s, (b / kStages - 1) & 1, kTcWaitCycles);
+                        ok = tc::mbar_wait(empty + s, (b / kStages - 1) & 1, limit);
                     if (!ok) break;
                     if (kb == 0) {
                         // slot u % kRing is free: three blocks back the unit before
@@ -432,26 +437,29 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         }
         // the end, for the issuer and the workers
         const int s = b % kStages;
-        if (ok && b >= kStages) ok = tc::mbar_wait(empty + s, (b / kStages - 1) & 1, kTcWaitCycles);
+        if (ok && b >= kStages) ok = tc::mbar_wait(empty + s, (b / kStages - 1) & 1, limit);
         if (ok) {
             s_block[s] = kStop;
             tc::mbar_arrive(full + s);
             s_unit[u % kRing].flags = kStop;
             tc::mbar_arrive(info + u % kRing);
-        } else {   // copies in flight land before the CTA gives its memory up
-            for (int k = b > kStages ? b - kStages : 0; k < b; ++k)
-                tc::mbar_wait(full + k % kStages, (k / kStages) & 1, kTcWaitCycles);
         }
+        // copies in flight land before the CTA gives its memory up, also where the issuer
+        // no longer waits for them (after the stop, block b - kStages has been read and
+        // its barrier serves the stop)
+        const int flight = ok ? kStages - 1 : kStages;
+        for (int k = max(0, b - flight); k < b; ++k)
+            tc::mbar_wait(full + k % kStages, (k / kStages) & 1, kTcWaitCycles);
     } else if (tid == kWorkers + 32) {
         // ---- issuer --------------------------------------------------------------
         int u = 0;
         bool first_block = true;
         for (int b = 0;; ++b) {
             const int s = b % kStages;
-            bool ok = tc::mbar_wait(full + s, (b / kStages) & 1, kTcWaitCycles);
+            bool ok = tc::mbar_wait(full + s, (b / kStages) & 1, limit);
             const int fl = ok ? s_block[s] : kStop;
             if (ok && (fl & kFirst) && u > 0) {   // the accumulators are free again
-                ok = tc::mbar_wait(drained, (u - 1) & 1, kTcWaitCycles);
+                ok = tc::mbar_wait(drained, (u - 1) & 1, limit);
                 tc::fence_after_sync();
             }
             if (!ok || (fl & kStop)) {
@@ -479,10 +487,10 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
         double acc[8];
         bool unset = true;   // the first product is stored as it is, without an FP64 addition
         for (int u = 0;; ++u) {
-            bool ok = tc::mbar_wait(info + u % kRing, (u / kRing) & 1, kTcWaitCycles);
+            bool ok = tc::mbar_wait(info + u % kRing, (u / kRing) & 1, limit);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {
-                poison_tiles(jobs, njobs, chunks, ntiles, lrow, cw);
+                poison_tiles(jobs, njobs, chunks, ntiles, lrow, cw, gave_up);
                 break;
             }
             const Unit &x = s_unit[u % kRing];
@@ -507,9 +515,13 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             }
             const int Er = in ? x.ep[lrow] + kShift - 110 : 0;
             const int Ecl = (lane & 7) < nc ? x.eq[cw + (lane & 7)] : 0;
-            ok = tc::mbar_wait(done, u & 1, kTcWaitCycles);
+            ok = tc::mbar_wait(done, u & 1, limit);
             ok = __all_sync(0xffffffffu, ok);
-            if (ok) tc::fence_after_sync();
+            if (!ok) {   // (no later unit: its phase of `done` would be taken for this one's)
+                poison_tiles(jobs, njobs, chunks, ntiles, lrow, cw, gave_up);
+                break;
+            }
+            tc::fence_after_sync();
             unsigned slow = 0;   // entries that a NaN, an infinity or a subnormal result needs
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -550,10 +562,6 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 for (int e = 0; e < 8; ++e)
                     if (e + up > 0) acc[e] = 0.0;
             }
-            if (!ok) {   // a wait that gave up leaves NaN, never a half-summed tile
-#pragma unroll
-                for (int e = 0; e < 8; ++e) acc[e] = __longlong_as_double(-1LL);
-            }
             if ((flags & kLast) && in) {
                 double *p = x.cd + (size_t)cw * x.ldcd + lrow;
                 // entry e lies e + up columns right of the diagonal; lo .. hi are written
@@ -585,6 +593,11 @@ size_t dense_slice_q_offset(int M, int ncol) {
     return (size_t)dense_blocks(ncol) * ((M + kRowsA - 1) / kRowsA) * kBlockA;
 }
 
+static thread_local long long t_wait_cycles = dg::kTcWaitCycles;
+extern "C" void hcore_gpu_test_wait_cycles(long long cycles) {
+    t_wait_cycles = cycles > 0 ? cycles : dg::kTcWaitCycles;
+}
+
 cudaError_t configure_dense_tc() {
     return cudaFuncSetAttribute(dense_tile_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
 }
@@ -604,13 +617,14 @@ cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, co
 cudaError_t launch_dense_tiles_tc(const DenseWork *d_work,
                                   const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
                                   const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
-                                  int *d_exps, cudaStream_t s) {
+                                  int *d_exps, int *gave_up, cudaStream_t s) {
     const int mb = (b.maxM + kRowsA - 1) / kRowsA, nq = (b.maxN + kRowsA - 1) / kRowsA;
     dense_slice_kernel<<<dim3(mb + nq, b.nchunks), 256, 0, s>>>(d_work, d_cols, d_shift,
                                                                 d_chunks + b.chunk0, d_slices, d_exps);
     const int grid = b.ntiles < 2 * kSms ? b.ntiles : 2 * kSms;   // two CTAs per SM
     dense_tile_tc_kernel<<<grid, kThreadsTc, kSmem, s>>>(d_work, d_cols, d_chunks,
-                                                         d_jobs + b.job0, b.njobs, b.ntiles, d_slices, d_exps);
+                                                         d_jobs + b.job0, b.njobs, b.ntiles, d_slices, d_exps,
+                                                         gave_up, t_wait_cycles);
     return cudaGetLastError();
 }
 

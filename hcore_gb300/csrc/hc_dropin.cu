@@ -65,7 +65,23 @@ ThreadCtx::~ThreadCtx() {
     // the runtime may already be shut down at thread/process exit: ignore errors
     if (dev) cudaFree(dev);
     if (pin) cudaFreeHost(pin);
+    if (word) cudaFreeHost(word);
     if (stream) cudaStreamDestroy(stream);
+}
+
+int *ThreadCtx::wait_word() {
+    if (!word && cudaMallocHost((void **)&word, 256) != cudaSuccess) {
+        cudaGetLastError();
+        word = nullptr;
+    }
+    if (word) *word = 0;
+    return word;
+}
+
+int check_waits(const int *word, const char *fn) {
+    if (*(const volatile int *)word == 0) return HCORE_GPU_OK;
+    set_error("%s: a bounded wait of the products on the tensor cores gave up; the outputs are not valid", fn);
+    return HCORE_GPU_ECUDA;
 }
 
 cudaError_t ThreadCtx::init() {
@@ -693,9 +709,9 @@ struct DensePrep {
     }
 };
 
-// Run a list of dense tasks (device-accessible pointers) on stream s, in the
-// calling thread's arena.
-static int run_dense(int n, const hcore_dense_task *tasks, cudaStream_t s, bool sync) {
+// Run a list of dense tasks (device-accessible pointers) on stream s and wait, in
+// the calling thread's arena.
+static int run_dense(int n, const hcore_dense_task *tasks, cudaStream_t s) {
     if (n <= 0) return HCORE_GPU_OK;
     DensePrep dp;
     int rc = dp.build(n, tasks);
@@ -703,22 +719,24 @@ static int run_dense(int n, const hcore_dense_task *tasks, cudaStream_t s, bool 
     ThreadCtx &tc = thread_ctx();
     char *arena = (char *)tc.dev_ensure(dp.bytes());
     char *pin = (char *)tc.pin_ensure(dp.ws_offset());
-    if (!arena || !pin) {
+    int *word = tc.wait_word();
+    if (!arena || !pin || !word) {
         set_error("hcore_gpu_dense_batched: out of memory");
         return HCORE_GPU_ENOMEM;
     }
     dp.bind(tasks, (double *)(arena + dp.ws_offset()));
+    dp.pr.gave_up = word;
     // the previous call on this stream may still read the pinned buffer
     cudaStreamSynchronize(s);
     dp.pack(pin, tasks);
     cudaMemcpyAsync(arena, pin, dp.ws_offset(), cudaMemcpyHostToDevice, s);
     cudaError_t e = dp.launch(arena, s);
-    if (e == cudaSuccess && sync) e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         set_error("hcore_gpu_dense_batched: %s", cudaGetErrorString(e));
         return HCORE_GPU_ECUDA;
     }
-    return HCORE_GPU_OK;
+    return check_waits(word, "hcore_gpu_dense_batched");
 }
 
 // stage one dense host block (rows x cols, ld) into dst (ld rows)
@@ -928,7 +946,7 @@ void HCORE_dsyrk(HCORE_enum uplo, HCORE_enum trans, int M, int K, double alpha, 
         stage(buf + 2 * nf, CD, M, M, LDCD, tc.stream);
         t.Au = buf; t.Av = buf + nf; t.lda = N; t.CD = buf + 2 * nf; t.ldcd = M;
     }
-    if (run_dense(1, &t, tc.stream, true)) fatal("HCORE_dsyrk: %s\n", last_error());
+    if (run_dense(1, &t, tc.stream)) fatal("HCORE_dsyrk: %s\n", last_error());
     if (!dev) unstage(CD, LDCD, t.CD, M, M, tc.stream, "HCORE_dsyrk");
     if (flops)  // hcore_dsyrk.c:104-188
         flops->syrk += flop_counts('m', K, K, N, 0) + flop_counts('m', M, K, K, 0) +
@@ -960,7 +978,7 @@ void HCORE_dgemmcd(HCORE_enum transA, HCORE_enum transB, int M, double alpha, do
         t.Au = buf; t.Av = buf + na; t.Bu = buf + 2 * na; t.Bv = buf + 2 * na + nb;
         t.lda = M; t.ldb = M; t.CD = buf + 2 * na + 2 * nb; t.ldcd = M;
     }
-    if (run_dense(1, &t, tc.stream, true)) fatal("HCORE_dgemmcd: %s\n", last_error());
+    if (run_dense(1, &t, tc.stream)) fatal("HCORE_dgemmcd: %s\n", last_error());
     if (!dev) unstage(CD, M, t.CD, M, M, tc.stream, "HCORE_dgemmcd");
 }
 
@@ -990,7 +1008,7 @@ void HCORE_duncompress(HCORE_enum transA, HCORE_enum transB, int M, int N, doubl
         stage(buf + na, BV, N, (int)a, LDB, tc.stream);
         t.Au = buf; t.lda = M; t.Bv = buf + na; t.ldb = N; t.CD = buf + na + nb; t.ldcd = M;
     }
-    if (run_dense(1, &t, tc.stream, true)) fatal("HCORE_duncompress: %s\n", last_error());
+    if (run_dense(1, &t, tc.stream)) fatal("HCORE_duncompress: %s\n", last_error());
     if (!dev) unstage(CD, LDC, t.CD, M, N, tc.stream, "HCORE_duncompress");
 }
 
@@ -1035,7 +1053,7 @@ void HCORE_dgemmbdcd(HCORE_enum transA, HCORE_enum transB, int M, int N, double 
         t.Au = buf; t.Av = buf + nf; t.lda = ld; t.Bd = buf + 2 * nf; t.ldb = K;
         t.CD = buf + 2 * nf + nd; t.ldcd = rows;
     }
-    if (run_dense(1, &t, tc.stream, true)) fatal("HCORE_dgemmbdcd: %s\n", last_error());
+    if (run_dense(1, &t, tc.stream)) fatal("HCORE_dgemmbdcd: %s\n", last_error());
     if (!dev) unstage(CD, LDC, t.CD, rows, N, tc.stream, "HCORE_dgemmbdcd");
 }
 
@@ -1127,7 +1145,7 @@ int hcore_gpu_dense_batched(int n, const hcore_dense_task *tasks, void *stream) 
     std::vector<hcore_dense_task> tt;
     int rc = translate_dense(n, tasks, tt);
     if (rc) return rc;
-    return run_dense(n, tt.data(), (cudaStream_t)stream, true);
+    return run_dense(n, tt.data(), (cudaStream_t)stream);
 }
 
 }  // extern "C"
@@ -1135,6 +1153,7 @@ int hcore_gpu_dense_batched(int n, const hcore_dense_task *tasks, void *stream) 
 struct hcore_gpu_dense_plan_s {
     DensePrep prep;
     char *arena = nullptr;
+    int *word = nullptr;   // pinned: a wait that gave up since the last status call
 };
 
 extern "C" {
@@ -1154,18 +1173,23 @@ int hcore_gpu_dense_plan_create(hcore_gpu_dense_plan *plan, int n, const hcore_d
         delete p;
         return rc;
     }
-    if (cudaMalloc(&p->arena, std::max<size_t>(p->prep.bytes(), 256)) != cudaSuccess) {
+    if (cudaMalloc(&p->arena, std::max<size_t>(p->prep.bytes(), 256)) != cudaSuccess ||
+        cudaMallocHost((void **)&p->word, 256) != cudaSuccess) {
         cudaGetLastError();
-        set_error("hcore_gpu_dense_plan_create: cudaMalloc of %zu bytes failed", p->prep.bytes());
+        set_error("hcore_gpu_dense_plan_create: allocation of %zu bytes failed", p->prep.bytes());
+        cudaFree(p->arena);
         delete p;
         return HCORE_GPU_ENOMEM;
     }
+    *p->word = 0;
+    p->prep.pr.gave_up = p->word;
     p->prep.bind(tt.data(), (double *)(p->arena + p->prep.ws_offset()));
     std::vector<char> host(p->prep.ws_offset());
     p->prep.pack(host.data(), tt.data());
     if (cudaMemcpy(p->arena, host.data(), host.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         set_error("hcore_gpu_dense_plan_create: upload failed");
         cudaFree(p->arena);
+        cudaFreeHost(p->word);
         delete p;
         return HCORE_GPU_ECUDA;
     }
@@ -1187,9 +1211,25 @@ int hcore_gpu_dense_plan_execute(hcore_gpu_dense_plan p, void *stream) {
     return HCORE_GPU_OK;
 }
 
+int hcore_gpu_dense_plan_status(hcore_gpu_dense_plan p, void *stream) {
+    if (!p) {
+        set_error("hcore_gpu_dense_plan_status: null plan");
+        return HCORE_GPU_EINVAL;
+    }
+    const cudaError_t e = cudaStreamSynchronize((cudaStream_t)stream);
+    if (e != cudaSuccess) {
+        set_error("hcore_gpu_dense_plan_status: %s", cudaGetErrorString(e));
+        return HCORE_GPU_ECUDA;
+    }
+    const int rc = check_waits(p->word, "hcore_gpu_dense_plan_execute");
+    *p->word = 0;
+    return rc;
+}
+
 int hcore_gpu_dense_plan_destroy(hcore_gpu_dense_plan p) {
     if (p) {
         cudaFree(p->arena);
+        cudaFreeHost(p->word);
         delete p;
     }
     return HCORE_GPU_OK;
@@ -1395,7 +1435,7 @@ extern "C" void HCORE_zuncompress(HCORE_enum transA, HCORE_enum transB, int M, i
         t[q].Bv = dQ + (size_t)q * N * 2 * r; t[q].ldb = N;
         t[q].CD = dOut + (size_t)q * M * N; t[q].ldcd = M;
     }
-    if (run_dense(2, t, tc.stream, true)) fatal("%s: %s\n", fn, last_error());
+    if (run_dense(2, t, tc.stream)) fatal("%s: %s\n", fn, last_error());
     std::vector<double> o(nout);
     if (cudaMemcpyAsync(o.data(), dOut, nout * sizeof(double), cudaMemcpyDeviceToHost,
                         tc.stream) != cudaSuccess ||

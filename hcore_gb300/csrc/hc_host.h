@@ -35,11 +35,18 @@ struct ThreadCtx {
     size_t dev_bytes = 0;
     void *pin = nullptr;
     size_t pin_bytes = 0;
+    int *word = nullptr;
     ~ThreadCtx();
     cudaError_t init();
     void *dev_ensure(size_t bytes);
     void *pin_ensure(size_t bytes);
+    // a word of pinned memory, zeroed, for the kernels of a synchronous call to report
+    // a wait that gave up; null if it cannot be allocated
+    int *wait_word();
 };
+// what a call returns once its stream has been waited for: ECUDA, with the message,
+// if a kernel's wait gave up
+int check_waits(const int *word, const char *fn);
 ThreadCtx &thread_ctx();
 
 // reference flop model of one update (src/misc/descutil/flop_counts.c:3-70

@@ -279,7 +279,7 @@ cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, co
                                  DenseBalance how, int *d_shift, cudaStream_t s);
 cudaError_t launch_dense_tiles_tc(const DenseWork *d_work, const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
                                   const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
-                                  int *d_exps, cudaStream_t s);
+                                  int *d_exps, int *gave_up, cudaStream_t s);
 template <typename T>
 cudaError_t launch_gemm_dense(int ta, int tb, int M, int N, int K, T alpha, const T *A, int lda,
                               const T *B, int ldb, T beta, T *C, int ldc, cudaStream_t s);

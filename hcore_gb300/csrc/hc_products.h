@@ -25,6 +25,9 @@ struct DenseProducts {
     std::vector<DenseChunk> chunks;
     std::vector<DenseJob> jobs;
     std::vector<DenseBatch> batches;
+    // set to 1 by a launch one of whose bounded waits gave up (its tiles are NaN
+    // then): device-accessible, zeroed and read by the caller
+    int *gave_up = nullptr;
 
     // a product; its kk columns are laid out by add_tile
     int add(const DenseWork &w, int M, int N) {
@@ -150,7 +153,7 @@ struct DenseProducts {
         for (int b = stages[q].batches0; b < b1 && e == cudaSuccess; ++b)
             e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
                                       (const DenseJob *)(arena + o_jobs), batches[b],
-                                      (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), s);
+                                      (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), gave_up, s);
         return e;
     }
     cudaError_t launch(char *arena, cudaStream_t s) const {

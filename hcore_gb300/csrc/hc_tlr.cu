@@ -618,7 +618,8 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
     pr.place_device(all);
     char *arena = (char *)tc.dev_ensure(all);
     char *pin = (char *)tc.pin_ensure(up);
-    if (!arena || !pin) {
+    pr.gave_up = tc.wait_word();
+    if (!arena || !pin || !pr.gave_up) {
         set_error("hcore_gpu_trsm_batched: out of memory");
         return HCORE_GPU_ENOMEM;
     }
@@ -644,7 +645,7 @@ static int run_trsm(int n, const hcore_trsm_task *tasks, cudaStream_t s) {
         set_error("hcore_gpu_trsm_batched: %s", cudaGetErrorString(e));
         return HCORE_GPU_ECUDA;
     }
-    return HCORE_GPU_OK;
+    return check_waits(pr.gave_up, "hcore_gpu_trsm_batched");
 }
 
 // LAPACKE_dpotrf_work's argument checks (its info is LAPACK's minus one)
@@ -716,7 +717,8 @@ static int run_potrf(int n, const hcore_potrf_task *tasks, int *info, cudaStream
     pr.place_device(all);
     char *arena = (char *)tc.dev_ensure(all);
     char *pin = (char *)tc.pin_ensure(up);
-    if (!arena || !pin) {
+    pr.gave_up = tc.wait_word();
+    if (!arena || !pin || !pr.gave_up) {
         set_error("hcore_gpu_potrf_batched: out of memory");
         return HCORE_GPU_ENOMEM;
     }
@@ -750,6 +752,7 @@ static int run_potrf(int n, const hcore_potrf_task *tasks, int *info, cudaStream
         set_error("hcore_gpu_potrf_batched: %s", cudaGetErrorString(e));
         return HCORE_GPU_ECUDA;
     }
+    if (const int rc = check_waits(pr.gave_up, "hcore_gpu_potrf_batched")) return rc;   // (NaN fails a pivot's test)
     for (int q = 0; q < nr; ++q) info[slot[q]] = ((const int *)(pin + bt))[q];
     return HCORE_GPU_OK;
 }

@@ -245,7 +245,15 @@ int hcore_gpu_dense_batched(int n, const hcore_dense_task *tasks, void *stream);
 typedef struct hcore_gpu_dense_plan_s *hcore_gpu_dense_plan;
 int hcore_gpu_dense_plan_create(hcore_gpu_dense_plan *plan, int n, const hcore_dense_task *tasks);
 int hcore_gpu_dense_plan_execute(hcore_gpu_dense_plan plan, void *stream);
+/* waits for the stream; HCORE_GPU_ECUDA if since the last status call a bounded
+ * wait inside an execute gave up (its tiles hold NaN; no counterpart in the
+ * reference).  The one-shot calls return that themselves. */
+int hcore_gpu_dense_plan_status(hcore_gpu_dense_plan plan, void *stream);
 int hcore_gpu_dense_plan_destroy(hcore_gpu_dense_plan plan);
+/* For tests of that: the bound, in clock cycles, of the waits inside the products
+ * on the tensor cores that the calling thread launches from here on (0: the
+ * built-in one, about half a second). */
+void hcore_gpu_test_wait_cycles(long long cycles);
 
 /* Triangular solves with many right-hand sides (HCORE_dtrsm semantics,
  * cblas_dtrsm column-major): B = alpha op(A)^-1 B (side HCORE_Left, A M x M)
