@@ -18,6 +18,22 @@
 // a row of P or Q sends the entries it reaches to an FP64 loop, so they come
 // out as in IEEE arithmetic.
 //
+// Entries of graded rows.  Where a row's large entries meet small ones of the other
+// row only, an entry's terms are all far below the product of the two scales, and
+// 2^-55 of that product may be all of the entry.  So each row notes which columns are
+// within 2^-kNear of its top; an entry whose rows share such a column has a term of
+// 2^-(2 kNear + 2) of the scales at least, and its error is below (1.25 K + 1) 2^-45 of the
+// sum of its terms' magnitudes; so it is if the result or CD's entry is that large.
+// The others, 2e-6 of the entries of low-rank updates with singular values over 16
+// decades, go to the FP64 loop (with kNear = 3 1e-4 of them, and the loop's latency,
+// which holds up the CTA's other warps, shows: 32 tiles of 1024 with 24 updates
+// each 30% slower).  What it costs where no entry takes the loop: 12 gemmbdcd tasks of
+// 777 x 650 x 900 484 -> 499 us, the factorization and solves of 8 tiles of 1024 with 12
+// factors each 4342 -> 4451 us.  Stages without balance are left out (kNoBalance): the
+// compressor's products only have to be small in norm, and a Cholesky factorization's
+// backward error is relative to sqrt(a_ii a_jj), the rows' scales, in FP64 too (of a
+// covariance tile two thirds of the entries would take the loop).
+//
 // Measured on one GB300 (tiles and their preparation): 384 products of 1024 x
 // 1024 x 17 21.9 -> 2.56 ms (3.2 GB written: 1.3 TB/s), 32 tiles of 1024 with
 // 24 syrk or gemmcd updates each of ranks 8-32 25.9 -> 2.78 ms, 12 gemmbdcd
@@ -64,6 +80,13 @@ constexpr int kWorkers = 512, kThreadsTc = kWorkers + 64;
 constexpr int kTmem = 256;
 // T = value 2^(110 - E_r - E_c - S), |value| < 128 2^(E_r + E_c): T < 2^62
 constexpr int kShift = 55;
+// Columns "near the top" of a row: scaled entry within kNear binades of the row's
+// largest, among 32 columns of the chunk (those with the largest products, so that
+// one word a row holds them).  An entry of the product whose rows share no such column
+// is formed in FP64 if both the digits' result and CD's entry are below 2^-(2 kNear + 2)
+// of the rows' scales (kFar, in T's units shifted by 32).  See the file comment.
+constexpr int kNear = 4;
+constexpr int kFarBits = kShift - 2 * kNear - 2, kFar = 1 << (kFarBits - 32);
 constexpr int kNonFinite = INT_MAX / 4;   // (more than any sum of two other scales, less than INT_MAX)
 constexpr int kSms = 152;
 // blocks of a chunk's columns; a chunk without columns takes one of zeros
@@ -73,7 +96,8 @@ __host__ __device__ constexpr int dense_blocks(int ncol) { return ncol > 0 ? (nc
 // column), or of P's alone: 2^s brings its largest entry near 1; a zero column
 // or one with a non-finite entry is left as it is
 __global__ void __launch_bounds__(256) dense_balance_kernel(const DenseWork *work, const int2 *cols,
-                                                            const int2 *dims, int n, bool p_only, int *shift) {
+                                                            const int2 *dims, int n, bool p_only, int *shift,
+                                                            int *mag) {
     const int c = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (c >= n) return;
     const int2 tl = cols[c], mn = dims[tl.x];
@@ -89,6 +113,7 @@ __global__ void __launch_bounds__(256) dense_balance_kernel(const DenseWork *wor
     for (int i = lane; i < mn.y && !p_only; i += 32) eq = max(eq, exp_field(q[i * sq]));
     ep = __reduce_max_sync(0xffffffffu, ep);
     eq = __reduce_max_sync(0xffffffffu, eq);
+    if (lane == 0) mag[c] = p_only ? 0 : ep + eq;
     if (lane == 0 && p_only) shift[c] = ep == 0 || ep == 0x7FF ? 0 : ep - 1023;
     else if (lane == 0) shift[c] = ep == 0 || eq == 0 || ep == 0x7FF || eq == 0x7FF ? 0 : (ep - eq) / 2;
 }
@@ -96,7 +121,7 @@ __global__ void __launch_bounds__(256) dense_balance_kernel(const DenseWork *wor
 // the same for operands stored transposed: a thread per column (64 a block,
 // four threads each), so that the loads are coalesced
 __global__ void __launch_bounds__(256) dense_balance_t_kernel(const DenseWork *work, const int2 *cols,
-                                                              const int2 *dims, int n, int *shift) {
+                                                              const int2 *dims, int n, int *shift, int *mag) {
     __shared__ int s_p[64], s_q[64];
     const int tid = threadIdx.x, lc = tid & 63, rg = tid >> 6, c = blockIdx.x * 64 + lc;
     if (tid < 64) s_p[tid] = s_q[tid] = 0;
@@ -116,6 +141,7 @@ __global__ void __launch_bounds__(256) dense_balance_t_kernel(const DenseWork *w
     if (tid < 64 && c < n) {
         const int ep = s_p[tid], eq = s_q[tid];
         shift[c] = ep == 0 || eq == 0 || ep == 0x7FF || eq == 0x7FF ? 0 : (ep - eq) / 2;
+        mag[c] = ep + eq;
     }
 }
 
@@ -127,8 +153,11 @@ __global__ void __launch_bounds__(256) dense_balance_t_kernel(const DenseWork *w
 // a panel of dense tiles 0.53, 0.23.  What is left is the latency of a block's two
 // reads, then the 14 bytes an element that it writes.
 __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work, const int2 *cols,
-                                                          const int *shift, const DenseChunk *chunks,
-                                                          unsigned char *slices, int *exps) {
+                                                          const int *shift, const int *mag,
+                                                          const DenseChunk *chunks, unsigned char *slices, int *exps,
+                                                          unsigned *near_cols) {
+    __shared__ __align__(16) int s_key[128];
+    __shared__ int2 s_near[128];   // a column's shift, and its bit among the 32 of near_cols
     __shared__ const double *s_col[128];
     __shared__ int s_shift[128], s_e[kRowsA], s_ld[128];   // s_ld: distance of two rows
     __shared__ double s_coef[128];
@@ -151,8 +180,22 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
         s_coef[tid] = q ? 1.0 : w.coef;
         s_sign[tid] = q || w.coef == 1.0 ? 0 : (w.coef == -1.0 ? (int)0x80000000 : 1);
     }
+    // order of the columns: by the size of their products, then every second, third or
+    // fourth column first (a solve's triangle is balanced by itself: no sizes)
+    const int stride = (ch.ncol + 31) / 32;
+    if (near_cols && tid < ch.ncol)
+        s_key[tid] = (mag[ch.col0 + tid] << 14) | ((3 - tid % max(stride, 1)) << 7) | (127 - tid);
     if (tid < kRowsA) s_e[tid] = INT_MIN;
     __syncthreads();
+    if (near_cols && tid < 128) {
+        int place = tid < ch.ncol ? tid : 32;
+        if (ch.ncol > 32 && tid < ch.ncol) {
+            place = 0;
+#pragma unroll 8
+            for (int c = 0; c < ch.ncol; ++c) place += s_key[c] > s_key[tid];
+        }
+        s_near[tid] = make_int2(s_shift[tid], place < 32 ? 1 << place : 0);
+    }
     const int row = rb * kRowsA + lrow;
     const bool in = row < n;
     auto entry = [&](int c) -> double { return in && c < ch.ncol ? s_col[c][(size_t)row * s_ld[c]] : 0.0; };
@@ -197,6 +240,9 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
         step = kBlockA;
     }
     const bool zero = E == kNonFinite;
+    // which columns are near the row's top (a row of zeros, or one that goes to FP64
+    // anyway, has all of them)
+    unsigned near = zero || e == INT_MIN ? ~0u : 0u;
     double next[8];   // the next columns, loaded while the digits of these are formed
 #pragma unroll
     for (int t = 0; t < 8; ++t) next[t] = zero ? 0.0 : entry(8 * half + t);
@@ -208,6 +254,12 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
             x[t] = 8 * g + t < ch.ncol ? scaled(8 * g + t, next[t]) : 0.0;
             next[t] = zero ? 0.0 : entry(8 * g + 16 + t);
         }
+        if (near_cols)
+#pragma unroll
+            for (int t = 0; t < 8; ++t) {   // (a zero is not near: its exponent field is 0)
+                const int2 col = s_near[min(8 * g + t, 127)];
+                if (exp_field(x[t]) >= max(1, e - kNear + col.x)) near |= (unsigned)col.y;
+            }
         uint32_t w[7][4];
 #pragma unroll
         for (int h = 0; h < 4; ++h) {
@@ -222,18 +274,24 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
         for (int s = 0; s < 7; ++s)
             *reinterpret_cast<uint4 *>(d + s * slice) = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
     }
+    if (near_cols && in) near_cols[2 * ((size_t)(q ? ch.eq : ch.ep) + row) + half] = near;
 }
 
-// an entry that a NaN or an infinity reaches, in FP64
+// an entry that a NaN or an infinity reaches, or with no large term, in FP64
 __device__ __noinline__ double dense_entry(const DenseWork *work, const int2 *cols, int col0, int ncol,
                                            int row, int col) {
     double v = 0.0;
-    for (int l = 0; l < ncol; ++l) {
+    for (int l = 0; l < ncol;) {   // a task's columns are consecutive
         const int2 tl = cols[col0 + l];
         const DenseWork w = work[tl.x];
-        const double p = w.P[w.tr & 1 ? (size_t)row * w.ldp + tl.y : (size_t)tl.y * w.ldp + row];
-        const double q = w.Q[w.tr & 2 ? (size_t)col * w.ldq + tl.y : (size_t)tl.y * w.ldq + col];
-        v += w.coef * p * q;
+        const bool tp = w.tr & 1, tq = w.tr & 2;
+        const double *p = w.P + (tp ? (size_t)row * w.ldp + tl.y : (size_t)tl.y * w.ldp + row);
+        const double *q = w.Q + (tq ? (size_t)col * w.ldq + tl.y : (size_t)tl.y * w.ldq + col);
+        const size_t sp = tp ? 1 : w.ldp, sq = tq ? 1 : w.ldq;
+        const int run = min(ncol - l, w.kk - tl.y);
+#pragma unroll 1
+        for (int i = 0; i < run; ++i) v += w.coef * p[i * sp] * q[i * sq];
+        l += run;
     }
     return v;
 }
@@ -276,6 +334,7 @@ __device__ __forceinline__ void combine4(long long (&acc)[4], uint32_t taddr) {
 struct Unit {
     double *cd;         // the tile's first entry
     const int *ep, *eq; // row scales of P and Q from the tile's first row and column
+    const uint2 *np, *nq;   // their columns near the top (of each half of the columns)
     double beta;
     int ldcd, rows, cols;
     int row0, col0;     // the tile's place in CD
@@ -353,7 +412,7 @@ __device__ __noinline__ void poison_tiles(const DenseJob *jobs, int njobs, const
 __global__ void __launch_bounds__(kThreadsTc, 2)
     dense_tile_tc_kernel(const DenseWork *work, const int2 *cols, const DenseChunk *chunks,
                          const DenseJob *jobs, int njobs, int ntiles, const unsigned char *slices,
-                         const int *exps, int *gave_up, long long limit) {
+                         const int *exps, const uint2 *near_cols, int *gave_up, long long limit) {
     extern __shared__ __align__(1024) unsigned char sm[];
     unsigned char *misc = sm + kStages * kStage;
     uint64_t *full = reinterpret_cast<uint64_t *>(misc), *empty = full + kStages;
@@ -410,6 +469,8 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                         x.ldcd = ldcd;
                         x.ep = exps + ch.ep + w.row0;
                         x.eq = exps + ch.eq + w.col0;
+                        x.np = near_cols ? near_cols + ch.ep + w.row0 : nullptr;
+                        x.nq = near_cols + ch.eq + w.col0;
                         x.beta = ch.beta;
                         x.rows = w.job.M - w.row0;
                         x.cols = w.job.N - w.col0;
@@ -515,6 +576,11 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             }
             const int Er = in ? x.ep[lrow] + kShift - 110 : 0;
             const int Ecl = (lane & 7) < nc ? x.eq[cw + (lane & 7)] : 0;
+            unsigned nr = ~0u, ncl = ~0u;
+            if (x.np) {
+                if (in) nr = x.np[lrow].x | x.np[lrow].y;
+                if ((lane & 7) < nc) ncl = x.nq[cw + (lane & 7)].x | x.nq[cw + (lane & 7)].y;
+            }
             ok = tc::mbar_wait(done, u & 1, limit);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) {   // (no later unit: its phase of `done` would be taken for this one's)
@@ -522,7 +588,7 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 break;
             }
             tc::fence_after_sync();
-            unsigned slow = 0;   // entries that a NaN, an infinity or a subnormal result needs
+            unsigned slow = 0;   // entries that FP64 forms: NaN, infinity, subnormal, no large term
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
                 long long a4[4];
@@ -534,7 +600,11 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                     const int p = Er + __shfl_sync(0xffffffffu, Ecl, 4 * h + e);
                     bool fits;
                     v[e] = i64_times_pow2(a4[e], p, fits);
-                    if (!fits || p >= kNonFinite / 2) {
+                    // no column near both tops, |T| < kFar 2^32, CD's entry small too
+                    const unsigned common = nr & __shfl_sync(0xffffffffu, ncl, 4 * h + e);
+                    const bool far = common == 0 && (unsigned)((int)(a4[e] >> 32) + kFar) < 2u * kFar &&
+                                     exp_field(acc[4 * h + e]) - 1023 < p + kFarBits;
+                    if (!fits || p >= kNonFinite / 2 || far) {
                         v[e] = 0.0;
                         slow |= 1u << (4 * h + e);
                     }
@@ -603,28 +673,29 @@ cudaError_t configure_dense_tc() {
 }
 
 cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, const int2 *d_dims, int ncols,
-                                 DenseBalance how, int *d_shift, cudaStream_t s) {
+                                 DenseBalance how, int *d_shift, int *d_mag, cudaStream_t s) {
     if (ncols <= 0) return cudaSuccess;
     if (how == kNoBalance) return cudaMemsetAsync(d_shift, 0, (size_t)ncols * sizeof(int), s);
     if (how == kBalanceByThread)
-        dense_balance_t_kernel<<<(ncols + 63) / 64, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, d_shift);
+        dense_balance_t_kernel<<<(ncols + 63) / 64, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, d_shift, d_mag);
     else
         dense_balance_kernel<<<(ncols + 7) / 8, 256, 0, s>>>(d_work, d_cols, d_dims, ncols, how == kBalanceP,
-                                                             d_shift);
+                                                             d_shift, d_mag);
     return cudaGetLastError();
 }
 
 cudaError_t launch_dense_tiles_tc(const DenseWork *d_work,
-                                  const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
+                                  const int2 *d_cols, const int *d_shift, const int *d_mag, const DenseChunk *d_chunks,
                                   const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
-                                  int *d_exps, int *gave_up, cudaStream_t s) {
+                                  int *d_exps, unsigned *d_near, int *gave_up, cudaStream_t s) {
     const int mb = (b.maxM + kRowsA - 1) / kRowsA, nq = (b.maxN + kRowsA - 1) / kRowsA;
-    dense_slice_kernel<<<dim3(mb + nq, b.nchunks), 256, 0, s>>>(d_work, d_cols, d_shift,
-                                                                d_chunks + b.chunk0, d_slices, d_exps);
+    dense_slice_kernel<<<dim3(mb + nq, b.nchunks), 256, 0, s>>>(d_work, d_cols, d_shift, d_mag,
+                                                                d_chunks + b.chunk0, d_slices, d_exps, d_near);
     const int grid = b.ntiles < 2 * kSms ? b.ntiles : 2 * kSms;   // two CTAs per SM
     dense_tile_tc_kernel<<<grid, kThreadsTc, kSmem, s>>>(d_work, d_cols, d_chunks,
                                                          d_jobs + b.job0, b.njobs, b.ntiles, d_slices, d_exps,
-                                                         gave_up, t_wait_cycles);
+                                                         reinterpret_cast<const uint2 *>(d_near), gave_up,
+                                                         t_wait_cycles);
     return cudaGetLastError();
 }
 

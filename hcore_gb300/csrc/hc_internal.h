@@ -271,15 +271,17 @@ size_t dense_slice_bytes(int M, int N, int ncol);
 size_t dense_slice_q_offset(int M, int ncol);
 int dense_tiles(int M, int N);   // tiles of one job
 // how the columns of a stage's products are balanced: not at all (the caller's
-// operands need none), by both operands (a warp per column, or a thread per
+// operands need none, and its results only have to be accurate relative to the
+// rows' scales), by both operands (a warp per column, or a thread per
 // column where both are stored transposed), or by P alone (its slices then do
 // not depend on Q)
 enum DenseBalance { kNoBalance, kBalanceByWarp, kBalanceByThread, kBalanceP };
 cudaError_t launch_dense_balance(const DenseWork *d_work, const int2 *d_cols, const int2 *d_dims, int ncols,
-                                 DenseBalance how, int *d_shift, cudaStream_t s);
-cudaError_t launch_dense_tiles_tc(const DenseWork *d_work, const int2 *d_cols, const int *d_shift, const DenseChunk *d_chunks,
+                                 DenseBalance how, int *d_shift, int *d_mag, cudaStream_t s);
+cudaError_t launch_dense_tiles_tc(const DenseWork *d_work, const int2 *d_cols, const int *d_shift,
+                                  const int *d_mag, const DenseChunk *d_chunks,
                                   const DenseJob *d_jobs, const DenseBatch &b, unsigned char *d_slices,
-                                  int *d_exps, int *gave_up, cudaStream_t s);
+                                  int *d_exps, unsigned *d_near, int *gave_up, cudaStream_t s);
 template <typename T>
 cudaError_t launch_gemm_dense(int ta, int tb, int M, int N, int K, T alpha, const T *A, int lda,
                               const T *B, int ldb, T beta, T *C, int ldc, cudaStream_t s);

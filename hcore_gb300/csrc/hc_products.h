@@ -109,6 +109,8 @@ struct DenseProducts {
     void place_device(size_t &at) {
         place(at, o_shift, cols.size() * sizeof(int));
         place(at, o_exps, max_exps * sizeof(int));
+        place(at, o_near, max_exps * sizeof(uint2));
+        place(at, o_mag, cols.size() * sizeof(int));
         place(at, o_slices, slice_bytes);
     }
     void pack(char *host) const {
@@ -144,16 +146,18 @@ struct DenseProducts {
     cudaError_t launch_stage(char *arena, int q, cudaStream_t s) const {
         const DenseWork *d_work = device_work(arena);
         const int2 *d_cols = (const int2 *)(arena + o_cols), *d_dims = (const int2 *)(arena + o_dims);
-        int *d_shift = (int *)(arena + o_shift);
+        int *d_shift = (int *)(arena + o_shift), *d_mag = (int *)(arena + o_mag);
         const bool last = q + 1 == nstages();
         const int c0 = stages[q].cols0, c1 = last ? (int)cols.size() : stages[q + 1].cols0;
         const int b1 = last ? (int)batches.size() : stages[q + 1].batches0;
         cudaError_t e = launch_dense_balance(d_work, d_cols + c0, d_dims, c1 - c0, stages[q].balance,
-                                             d_shift + c0, s);
+                                             d_shift + c0, d_mag + c0, s);
         for (int b = stages[q].batches0; b < b1 && e == cudaSuccess; ++b)
-            e = launch_dense_tiles_tc(d_work, d_cols, d_shift, (const DenseChunk *)(arena + o_chunks),
+            e = launch_dense_tiles_tc(d_work, d_cols, d_shift, d_mag, (const DenseChunk *)(arena + o_chunks),
                                       (const DenseJob *)(arena + o_jobs), batches[b],
-                                      (unsigned char *)(arena + o_slices), (int *)(arena + o_exps), gave_up, s);
+                                      (unsigned char *)(arena + o_slices), (int *)(arena + o_exps),
+                                      stages[q].balance == kNoBalance ? nullptr : (unsigned *)(arena + o_near),
+                                      gave_up, s);
         return e;
     }
     cudaError_t launch(char *arena, cudaStream_t s) const {
@@ -187,7 +191,7 @@ private:
     };
     std::vector<Stage> stages;
     size_t slice_bytes = 0, max_exps = 0, cur_slices = 0, cur_exps = 0;
-    size_t o_work = 0, o_cols = 0, o_dims = 0, o_chunks = 0, o_jobs = 0, o_shift = 0, o_exps = 0, o_slices = 0;
+    size_t o_work = 0, o_cols = 0, o_dims = 0, o_chunks = 0, o_jobs = 0, o_shift = 0, o_exps = 0, o_near = 0, o_mag = 0, o_slices = 0;
 
     static void place(size_t &at, size_t &o, size_t bytes) {
         o = at;
