@@ -25,14 +25,13 @@
 // 2^-(2 kNear + 2) of the scales at least, and its error is below (1.25 K + 1) 2^-45 of the
 // sum of its terms' magnitudes; so it is if the result or CD's entry is that large.
 // The others, 2e-6 of the entries of low-rank updates with singular values over 16
-// decades, go to the FP64 loop (with kNear = 3 1e-4 of them, and the loop's latency,
-// which holds up the CTA's other warps, shows: 32 tiles of 1024 with 24 updates
-// each 30% slower).  What it costs where no entry takes the loop: 12 gemmbdcd tasks of
-// 777 x 650 x 900 484 -> 499 us, the factorization and solves of 8 tiles of 1024 with 12
-// factors each 4342 -> 4451 us.  Stages without balance are left out (kNoBalance): the
-// compressor's products only have to be small in norm, and a Cholesky factorization's
-// backward error is relative to sqrt(a_ii a_jj), the rows' scales, in FP64 too (of a
-// covariance tile two thirds of the entries would take the loop).
+// decades (1e-4 with kNear = 3), are summed in FP64.  Stages without balance are left
+// out (kNoBalance): the compressor's products only have to be small in norm, and a
+// Cholesky factorization's backward error is relative to sqrt(a_ii a_jj), the rows'
+// scales, in FP64 too (of a covariance tile two thirds of the entries would be slow).
+// Cost: 12 gemmbdcd tasks of 777 x 650 x 900 485 -> 500 us, 32 tiles of 1024 with 24
+// updates each 2554 -> 2685, the factorization and solves of 8 tiles of 1024 with 12
+// factors each 4332 -> 4367.
 //
 // Measured on one GB300 (tiles and their preparation): 384 products of 1024 x
 // 1024 x 17 21.9 -> 2.56 ms (3.2 GB written: 1.3 TB/s), 32 tiles of 1024 with
@@ -277,23 +276,41 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
     if (near_cols && in) near_cols[2 * ((size_t)(q ? ch.eq : ch.ep) + row) + half] = near;
 }
 
-// an entry that a NaN or an infinity reaches, or with no large term, in FP64
-__device__ __noinline__ double dense_entry(const DenseWork *work, const int2 *cols, int col0, int ncol,
-                                           int row, int col) {
-    double v = 0.0;
-    for (int l = 0; l < ncol;) {   // a task's columns are consecutive
-        const int2 tl = cols[col0 + l];
+// Entries that a NaN, an infinity, a subnormal result or graded rows send to FP64: those
+// of the mask `slow`, of this lane's row and 8 columns from `col`, added to acc.  Few of
+// a warp are formed one after the other by all its lanes, a column of the K axis each
+// (one lane's loop over them is a chain of loads, which the CTA's other warps wait
+// for), many by their own lanes.
+__device__ __noinline__ void slow_entries(const DenseWork *work, const int2 *cols, int ncol, int row, int col,
+                                          unsigned slow, double *acc) {
+    const int lane = threadIdx.x & 31;
+    auto term = [&](int l, int i, int j) -> double {
+        const int2 tl = cols[l];
         const DenseWork w = work[tl.x];
-        const bool tp = w.tr & 1, tq = w.tr & 2;
-        const double *p = w.P + (tp ? (size_t)row * w.ldp + tl.y : (size_t)tl.y * w.ldp + row);
-        const double *q = w.Q + (tq ? (size_t)col * w.ldq + tl.y : (size_t)tl.y * w.ldq + col);
-        const size_t sp = tp ? 1 : w.ldp, sq = tq ? 1 : w.ldq;
-        const int run = min(ncol - l, w.kk - tl.y);
+        const double p = w.P[w.tr & 1 ? (size_t)i * w.ldp + tl.y : (size_t)tl.y * w.ldp + i];
+        const double q = w.Q[w.tr & 2 ? (size_t)j * w.ldq + tl.y : (size_t)tl.y * w.ldq + j];
+        return w.coef * p * q;
+    };
 #pragma unroll 1
-        for (int i = 0; i < run; ++i) v += w.coef * p[i * sp] * q[i * sq];
-        l += run;
+    for (int e = 0; e < 8; ++e) {
+        const bool mine = slow >> e & 1;
+        unsigned left = __ballot_sync(0xffffffffu, mine);
+        if (__popc(left) * (ncol / 32 + 3) < ncol) {
+            for (; left; left &= left - 1) {
+                const int s = __ffs(left) - 1;
+                double v = 0.0;
+                for (int l = lane; l < ncol; l += 32) v += term(l, row - lane + s, col + e);
+                __syncwarp();
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+                if (lane == s) acc[e] += v;
+            }
+        } else if (mine) {
+            double v = 0.0;
+            for (int l = 0; l < ncol; ++l) v += term(l, row, col + e);
+            acc[e] += v;
+        }
     }
-    return v;
 }
 
 // The eight planes of 4 columns combined, sum of plane_d 2^(96 - 8 d - 55 - 8)
@@ -620,11 +637,14 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
                 }
             }
             unset = false;
-            if (slow && in) {
+            slow &= in && nc > 0 ? (1u << nc) - 1 : 0u;
+            if (__any_sync(0xffffffffu, slow != 0)) {
+                double v[8];
 #pragma unroll
-                for (int e = 0; e < 8; ++e)
-                    if ((slow >> e & 1) && e < nc)
-                        acc[e] += dense_entry(work, cols, x.kcol0, x.ncol, x.row0 + lrow, x.col0 + cw + e);
+                for (int e = 0; e < 8; ++e) v[e] = acc[e];
+                slow_entries(work, cols + x.kcol0, x.ncol, x.row0 + lrow, x.col0 + cw, slow, v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e) acc[e] = v[e];
             }
             if (flags & kZeroUpper) {
                 const int up = x.col0 + cw - (x.row0 + lrow);   // entry e lies above the diagonal if e + up > 0

@@ -617,7 +617,10 @@ struct DensePrep {
             w.tr = 3;
             pr.add_tile({pr.add(w, t.N ? t.N : t.M, t.a)});
         }
-        pr.stage(kBalanceByWarp);
+        // (AU's or BU's columns are brought to one size: S, whose rows and columns may differ
+        // by 16 decades, keeps its own, and the entries that need FP64 are 4e-3 of all, not
+        // two thirds)
+        pr.stage(kBalanceP);
         for (int i : factor) {
             const hcore_dense_task &t = tasks[i];
             const int q = t.kind == 0 ? t.a : t.b;
