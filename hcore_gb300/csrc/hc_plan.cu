@@ -443,6 +443,10 @@ static void plan_free(hcore_gpu_plan p) {
     delete p;
 }
 
+// the default tuning's lanes: the library's own choice by the list (svd_smem_lanes,
+// svd_spread), of which four lanes are the usual one
+constexpr int kDefaultLanes = 4;
+
 extern "C" int hcore_gpu_tuning_default(hcore_gpu_tuning *t) {
     if (!t) {
         set_error("hcore_gpu_tuning_default: null argument");
@@ -451,9 +455,7 @@ extern "C" int hcore_gpu_tuning_default(hcore_gpu_tuning *t) {
     t->stream_groups = 16;
     if (const char *env = getenv("HCORE_GPU_STREAMS")) t->stream_groups = atoi(env);
     t->stream_groups = std::max(1, std::min(t->stream_groups, 64));
-    t->svd_lanes[0] = 4;   // the fastest on a TLR panel's updates (svd_smem_lanes)
-    t->svd_lanes[1] = 4;
-    t->svd_lanes[2] = 4;
+    for (int &lanes : t->svd_lanes) lanes = kDefaultLanes;
     t->bucket_width = 8;
     t->phase_sync = 0;
     t->qr_warps = 4;
@@ -523,7 +525,8 @@ int hc::plan_create(hcore_gpu_plan *plan, int precision, int n, const hcore_lr_t
     const std::vector<Desc> sorted = descs;
     p->phase_sync = tune.phase_sync != 0;
     auto set_shape_tuning = [&](LaunchShape &sh) {
-        for (int q = 0; q < 3 && tuning; ++q) sh.svd_lanes[q] = tune.svd_lanes[q];
+        for (int q = 0; q < 3; ++q)
+            sh.svd_lanes[q] = tune.svd_lanes[q] == kDefaultLanes ? -1 : tune.svd_lanes[q];
         sh.updates = n;
         sh.bucket_width = tune.bucket_width;
         sh.qr_warps = tune.qr_warps;
@@ -1045,7 +1048,8 @@ extern "C" int hcore_gpu_autotune(int precision, int n, const hcore_lr_task *tas
     int rc = time_cfg(cur, cur_ms);
     // one parameter at a time, keeping a change only if it gains 0.5 %
     const int groups[] = {4, 8, 16, 24, 32};
-    const int lanes0[] = {0, 1, 2}, lanes1[] = {0, 1, 2, 4, 8}, lanes2[] = {0, 1, 2, 4};
+    // (four lanes, the default, are the library's choice and may be a cluster an update)
+    const int lanes0[] = {0, 1, 2, 8}, lanes1[] = {0, 1, 2, 8}, lanes2[] = {0, 1, 2, 8};
     const int widths[] = {8, 16};
     // field(t) is the parameter being searched, as a reference into t
     auto try_values = [&](auto field, const int *vals, int nv) {
@@ -1066,9 +1070,9 @@ extern "C" int hcore_gpu_autotune(int precision, int n, const hcore_lr_task *tas
     try_values([](hcore_gpu_tuning &t) -> int & { return t.stream_groups; }, groups, 5);
     const int qrw[] = {8, 4, 2};
     try_values([](hcore_gpu_tuning &t) -> int & { return t.qr_warps; }, qrw, 3);
-    try_values([](hcore_gpu_tuning &t) -> int & { return t.svd_lanes[1]; }, lanes1, 5);
+    try_values([](hcore_gpu_tuning &t) -> int & { return t.svd_lanes[1]; }, lanes1, 4);
     try_values([](hcore_gpu_tuning &t) -> int & { return t.svd_lanes[2]; }, lanes2, 4);
-    try_values([](hcore_gpu_tuning &t) -> int & { return t.svd_lanes[0]; }, lanes0, 3);
+    try_values([](hcore_gpu_tuning &t) -> int & { return t.svd_lanes[0]; }, lanes0, 4);
     try_values([](hcore_gpu_tuning &t) -> int & { return t.bucket_width; }, widths, 2);
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);

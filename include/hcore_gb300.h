@@ -170,7 +170,10 @@ int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
  *   svd_lanes[3]       lanes per column pair of the shared-memory SVD buckets
  *                      with <= 24, <= 64 and more column pairs (1..32, a
  *                      power of two, above 8 as 8; 0: as many as fit in the
- *                      warps that one lane per pair needs)
+ *                      warps that one lane per pair needs; 4, the default: the
+ *                      library's choice, which gives a short list of small
+ *                      updates eight lanes and the SVDs of few wide ones a
+ *                      cluster of CTAs each)
  *   bucket_width       rank-bucket edges every 8 (fine) or 16 (coarse)
  *   phase_sync         0: each group runs its four phases as soon as it can
  *                      (phases of different groups overlap); 1: every group
@@ -179,9 +182,8 @@ int hcore_gpu_plan_destroy(hcore_gpu_plan plan);
  *                      update), 4 or 2 (two or four times the CTAs per SM)
  * hcore_gpu_tuning_default fills the built-in choice (16 groups, 4 lanes per
  * pair, width 8, no phase sync, 4 QR warps: the autotuner's pick on a TLR
- * panel of 1953 updates; HCORE_GPU_STREAMS overrides the groups; a plan
- * created without a tuning also gives a short list of small updates eight
- * lanes, and the SVDs of few wide ones a cluster of CTAs each).  hcore_gpu_autotune
+ * panel of 1953 updates; HCORE_GPU_STREAMS overrides the groups), with which a
+ * plan is the same as without a tuning.  hcore_gpu_autotune
  * times plans of the given tasks over a search of these parameters
  * (coordinate descent; each candidate's execute captured in a CUDA graph on
  * a private stream and replayed `reps` times) and returns the fastest; the
