@@ -29,9 +29,11 @@
 // out (kNoBalance): the compressor's products only have to be small in norm, and a
 // Cholesky factorization's backward error is relative to sqrt(a_ii a_jj), the rows'
 // scales, in FP64 too (of a covariance tile two thirds of the entries would be slow).
-// Cost: 12 gemmbdcd tasks of 777 x 650 x 900 485 -> 500 us, 32 tiles of 1024 with 24
-// updates each 2554 -> 2685, the factorization and solves of 8 tiles of 1024 with 12
-// factors each 4332 -> 4367.
+// Cost: 12 gemmbdcd tasks of 777 x 650 x 900 482 -> 500 us, 32 tiles of 1024 with 24
+// updates each 2595 -> 2752, the factorization and solves of 8 tiles of 1024 with 12
+// factors each 4279 -> 4370; 4094 updates of covariance tiles, whose singular vectors
+// fall by many decades from point to point, so that most entries of the factors AU S
+// are slow, 10.2 -> 12.0 ms (the factors 2.4 of them, as long as in FP64 alone).
 //
 // Measured on one GB300 (tiles and their preparation): 384 products of 1024 x
 // 1024 x 17 21.9 -> 2.56 ms (3.2 GB written: 1.3 TB/s), 32 tiles of 1024 with
@@ -277,40 +279,58 @@ __global__ void __launch_bounds__(256) dense_slice_kernel(const DenseWork *work,
 }
 
 // Entries that a NaN, an infinity, a subnormal result or graded rows send to FP64: those
-// of the mask `slow`, of this lane's row and 8 columns from `col`, added to acc.  Few of
-// a warp are formed one after the other by all its lanes, a column of the K axis each
-// (one lane's loop over them is a chain of loads, which the CTA's other warps wait
-// for), many by their own lanes.
+// of the mask `slow`, of this lane's row and 8 columns from `col`, added to acc.  A
+// lane's sum over the K axis is a chain of loads, which the CTA's other warps wait for:
+// a few entries are formed one after the other by the whole warp, a column of the K
+// axis a lane, many by their own lanes, the eight columns at the same time.
 __device__ __noinline__ void slow_entries(const DenseWork *work, const int2 *cols, int ncol, int row, int col,
                                           unsigned slow, double *acc) {
     const int lane = threadIdx.x & 31;
-    auto term = [&](int l, int i, int j) -> double {
-        const int2 tl = cols[l];
-        const DenseWork w = work[tl.x];
-        const double p = w.P[w.tr & 1 ? (size_t)i * w.ldp + tl.y : (size_t)tl.y * w.ldp + i];
-        const double q = w.Q[w.tr & 2 ? (size_t)j * w.ldq + tl.y : (size_t)tl.y * w.ldq + j];
-        return w.coef * p * q;
-    };
+    const int all = __reduce_add_sync(0xffffffffu, __popc(slow));
+    if (all * (ncol / 32 + 2) > ncol + 3) {
+        if (slow) {
+            const int last = 31 - __clz(slow);   // (the columns after it may not exist)
+            double v[8] = {};
+            for (int l = 0; l < ncol;) {   // a task's columns are consecutive
+                const int2 tl = cols[l];
+                const DenseWork w = work[tl.x];
+                const bool tp = w.tr & 1, tq = w.tr & 2;
+                const double *p = w.P + (tp ? (size_t)row * w.ldp + tl.y : (size_t)tl.y * w.ldp + row);
+                const double *q = w.Q + (tq ? (size_t)col * w.ldq + tl.y : (size_t)tl.y * w.ldq + col);
+                const size_t sp = tp ? 1 : w.ldp, sq = tq ? 1 : w.ldq, sc = tq ? w.ldq : 1;
+                const int run = min(ncol - l, w.kk - tl.y);
 #pragma unroll 1
-    for (int e = 0; e < 8; ++e) {
-        const bool mine = slow >> e & 1;
-        unsigned left = __ballot_sync(0xffffffffu, mine);
-        if (__popc(left) * (ncol / 32 + 3) < ncol) {
-            for (; left; left &= left - 1) {
-                const int s = __ffs(left) - 1;
-                double v = 0.0;
-                for (int l = lane; l < ncol; l += 32) v += term(l, row - lane + s, col + e);
-                __syncwarp();
+                for (int i = 0; i < run; ++i, p += sp, q += sq) {
+                    const double x = w.coef * *p;
 #pragma unroll
-                for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                if (lane == s) acc[e] += v;
+                    for (int e = 0; e < 8; ++e) v[e] = fma(x, q[min(e, last) * sc], v[e]);
+                }
+                l += run;
             }
-        } else if (mine) {
-            double v = 0.0;
-            for (int l = 0; l < ncol; ++l) v += term(l, row, col + e);
-            acc[e] += v;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+                if (slow >> e & 1) acc[e] += v[e];
         }
+        __syncwarp();
+        return;
     }
+#pragma unroll 1
+    for (int e = 0; e < 8; ++e)
+        for (unsigned left = __ballot_sync(0xffffffffu, slow >> e & 1); left; left &= left - 1) {
+            const int s = __ffs(left) - 1, r = row - lane + s, c = col + e;
+            double v = 0.0;
+            for (int l = lane; l < ncol; l += 32) {
+                const int2 tl = cols[l];
+                const DenseWork w = work[tl.x];
+                const double p = w.P[w.tr & 1 ? (size_t)r * w.ldp + tl.y : (size_t)tl.y * w.ldp + r];
+                const double q = w.Q[w.tr & 2 ? (size_t)c * w.ldq + tl.y : (size_t)tl.y * w.ldq + c];
+                v += w.coef * p * q;
+            }
+            __syncwarp();
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+            if (lane == s) acc[e] += v;
+        }
 }
 
 // The eight planes of 4 columns combined, sum of plane_d 2^(96 - 8 d - 55 - 8)
@@ -638,6 +658,8 @@ __global__ void __launch_bounds__(kThreadsTc, 2)
             }
             unset = false;
             slow &= in && nc > 0 ? (1u << nc) - 1 : 0u;
+            if (flags & kZeroUpper)   // (what becomes zero anyway)
+                slow &= (1u << max(0, min(8, x.row0 + lrow - x.col0 - cw + 1))) - 1;
             if (__any_sync(0xffffffffu, slow != 0)) {
                 double v[8];
 #pragma unroll
