@@ -36,10 +36,10 @@ METRIC = "TLR-GEMM updates/s batched vs plain per-tile on 1 GB300 at rel err <= 
 # DRAM bytes (read + write) per algorithmic byte of each phase's kernels:
 # dram__bytes_read.sum + dram__bytes_write.sum from ncu captures of the
 # 300-update case (a working set beyond L2), divided by the algorithmic bytes.
-# QR: every panel and trailing-update launch of one execute of the blocked QR
-# (406 MB against 353 MB); stack: one 300-update launch.  The full phase's
-# traffic is this ratio times its own algorithmic bytes.
-DRAM_PER_ALG_BYTE = {"stack": 0.46, "qr": 1.15, "svd": None, "rebuild": None}
+# all launches of a phase in one replay of the plan's graph (16 stream groups;
+# QR 446 MB against 353 MB, stack 209 against 503).  The full phase's traffic is
+# this ratio times its own algorithmic bytes.
+DRAM_PER_ALG_BYTE = {"stack": 0.42, "qr": 1.26, "svd": None, "rebuild": None}
 WORKLOAD = dict(workload="TLR Cholesky panel-0 Schur updates (HCORE_dgemm recompression)",
                 points=65536, dim=2, nb=1024, tiles_per_dim=64, kernel="exp(-|x-y|^2/0.01)",
                 acc=1e-8, maxrank=128, tile_compression="relative sigma >= acc*sigma_max",
@@ -423,7 +423,7 @@ def run_gb300(args):
                                          "MEASURED_PEAKS.json has no FP64 figure)",
                           "peak_probe": ceiling,
                           "flops_basis": "reference flop model (flop_counts.c) of that phase",
-                          "note": "FP64-equivalent: for a + c <= 64 the QR is blocked and its "
+                          "note": "FP64-equivalent: the QR is blocked and its "
                                   "trailing updates, and the rebuild, run as exact digit "
                                   "products on the tensor cores; the model counts the "
                                   "unblocked FP64 flops, so frac can exceed what the FP64 "

@@ -37,8 +37,8 @@
 //
 // Measured on one GB300 (tiles and their preparation): 384 products of 1024 x
 // 1024 x 17 21.9 -> 2.56 ms (3.2 GB written: 1.3 TB/s), 32 tiles of 1024 with
-// 24 syrk or gemmcd updates each of ranks 8-32 25.9 -> 2.78 ms, 12 gemmbdcd
-// tasks of 777 x 650 x 900, rank 40, 1.77 -> 0.54 ms; one 32 x 32 x 4 product
+// 24 syrk or gemmcd updates each of ranks 8-32 25.9 -> 2.75 ms, 12 gemmbdcd
+// tasks of 777 x 650 x 900, rank 40, 1.77 -> 0.50 ms; one 32 x 32 x 4 product
 // alone 25 -> 19 us (so no size keeps the FP64 kernel that this replaced).
 //
 // What bounds it.  In FP64 a term costs 1/2 clock of an SM (the FP64 pipe), so

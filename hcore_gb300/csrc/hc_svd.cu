@@ -30,7 +30,9 @@
 // Range safety (as LAPACK's dgesvd scales the matrix first): T is scaled by 2^-e
 // so that its largest entry lies in [1, 2) (exact; the singular values and V S
 // are scaled back by 2^e), and a column whose squared norm is below safmin is
-// negligible (< 2^-485 relative in FP64, 2^-51 in FP32) and not rotated.  A
+// negligible (< 2^-485 relative in FP64, 2^-51 in FP32) and not rotated.  In FP32 a
+// pair whose inner product is below 2^-75 counts as orthogonal too, its square being
+// out of range: columns of norms 2^-38 or so, far below the 2^-24 of T's rounding.  A
 // non-finite T or singular value marks the update NOCONV.
 //
 // svd_smem_kernel is written for latency, because a CTA's serial chain of Jacobi
@@ -154,7 +156,7 @@ __device__ __forceinline__ T group_sum(bool act, int start, int k, int lig, F f)
 // alpha (most columns of a graded T): tau is 2 and y_j becomes -y_j with one
 // rounding.  With an unscaled v = (alpha - beta, x) and 1 / (beta (beta - alpha)) the
 // factor 2 comes out of four rounded operations, and the QR's backward error was four
-// times as large (products of FP32 updates 1.83e-7 from their 64-bit values, 1.41e-7
+// times as large (products of FP32 updates 1.83e-7 from their 64-bit values, 1.42e-7
 // so).
 template <typename T>
 __device__ __forceinline__ T reflector_scal(T alpha, T beta) {

@@ -321,7 +321,8 @@ __global__ void __launch_bounds__(kZqThreads) zgeqrf_kernel(const ZDesc *__restr
 // phase of a column of both cancels in U_r conj(W_r S_r)^T, so none is kept).  With
 // s = x_p^H x_q, m = |a_pq| = sqrt(w_p w_q) |s| and t the real Jacobi tangent of
 // (a_pp, a_qq, m): x_p -= (t / m) w_q conj(s) x_q, x_q += (t / m) w_p s x_p, w_p and
-// w_q divided by 1 + t^2: no square root but 1 / m, no complex scale.
+// w_q divided by 1 + t^2: no square root but 1 / m, no complex scale.  (A pair whose
+// |a_pq|^2 is subnormal, |a_pq| < 2^-511 of T's largest entry, counts as orthogonal.)
 // SVD phase of 48 updates of order 512, ranks 16-32 (k 32-64): 4.87 ms with one CTA
 // an update, four lanes a pair, complex scales, a thread per column in the QR and in
 // U_r; 2.77 now.
